@@ -16,6 +16,7 @@ LIB_PATH = Path(__file__).resolve().parent / "lib" / "libmindpipe_b200.so"
 
 _lock = threading.Lock()
 _lib = None
+_host = None
 
 # name -> (restype, argtypes); mirrors include/mindpipe_b200.h one to one.
 _P, _I, _Z = c_void_p, c_int, c_size_t
@@ -121,6 +122,20 @@ def load() -> ctypes.CDLL:
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+def host():
+    """The native host side of the module forwards (``csrc/host_path.cpp``), loaded on first use."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host as ext
+        except ImportError as e:
+            raise RuntimeError("mindpipe_b200/_host.so is missing or does not load: build it with "
+                               "`python -m mindpipe_b200.build`") from e
+        _host = ext
+    return _host
 
 
 def check(status: int, op: str, **shapes) -> None:

@@ -2,8 +2,10 @@
 
 ``python -m mindpipe_b200.build`` (or :func:`build`) compiles every ``.cu``
 under ``csrc/`` to an object file in parallel and links one shared library
-at ``mindpipe_b200/lib/libmindpipe_b200.so``.  nvcc cross-compiles without a
-GPU, so this also runs on a CPU-only machine.
+at ``mindpipe_b200/lib/libmindpipe_b200.so``, then compiles
+``csrc/host_path.cpp`` (the modules' host side, against the torch headers) to
+the extension module ``mindpipe_b200/_host.so``.  nvcc cross-compiles without
+a GPU, so this also runs on a CPU-only machine.
 """
 from __future__ import annotations
 
@@ -11,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -19,6 +22,7 @@ CSRC = PKG / "csrc"
 LIB_DIR = PKG / "lib"
 LIB_PATH = LIB_DIR / "libmindpipe_b200.so"
 OBJ_DIR = PKG / "build"
+HOST_PATH = PKG / "_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -44,6 +48,26 @@ def _stale(target: Path, deps: list[Path]) -> bool:
         return True
     t = target.stat().st_mtime
     return any(d.stat().st_mtime > t for d in deps)
+
+
+def _build_host(force: bool) -> None:
+    src = CSRC / "host_path.cpp"
+    if not (force or _stale(HOST_PATH, [src, PKG.parent / "include" / "mindpipe_b200.h"])):
+        return
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parents[1]
+    gxx = shutil.which("g++") or "g++"
+    cmd = [gxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wno-deprecated-declarations",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{root / 'include'}", f"-I{root / 'include/torch/csrc/api/include'}", f"-I{cuda / 'include'}",
+           f"-I{sysconfig.get_paths()['include']}", str(src), "-o", str(HOST_PATH),
+           f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10",
+           f"-L{LIB_DIR}", "-lmindpipe_b200", "-Wl,-rpath,$ORIGIN/lib"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError(f"g++ failed for {src.name}")
 
 
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> Path:
@@ -77,6 +101,7 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
         if res.returncode != 0:
             sys.stderr.write(res.stdout + res.stderr)
             raise RuntimeError("link failed")
+    _build_host(force)
     return LIB_PATH
 
 

@@ -16,7 +16,20 @@ from __future__ import annotations
 import torch
 from torch import nn
 
-from . import ops
+from . import _lib, ops
+
+
+def _native_plan(make, module, attributes, *args):
+    """``module``'s native plan (``csrc/host_path.cpp``) if it is still good, else a new one; None where the buffers are
+    not what the kernels take (the checked path reports it).  ``attributes``: the buffers and attributes it depends on."""
+    if module._plan is not None and module._plan.fresh(module):
+        return module._plan
+    buffers = module._buffers
+    guards = [(None, "_buffers")] + [(buffers if name in buffers else None, name) for name in attributes]
+    try:
+        return make(module, guards, *args)
+    except (TypeError, ValueError):
+        return None
 
 
 class VllmPackedInt4Linear(nn.Module):
@@ -32,32 +45,33 @@ class VllmPackedInt4Linear(nn.Module):
     def __init__(self, *, packed_weight: torch.Tensor, scale: torch.Tensor, bias: torch.Tensor | None,
                  in_features: int, out_features: int, zero_point: torch.Tensor | None = None) -> None:
         super().__init__()
-        self.register_buffer("weight_packed", packed_weight.detach().contiguous())
-        self.register_buffer("weight_scale", scale.detach().to(torch.float16).contiguous())
+        packed, scale = packed_weight.detach().contiguous(), scale.detach().to(torch.float16).contiguous()
+        self.register_buffer("weight_packed", packed)
+        self.register_buffer("weight_scale", scale)
         self.register_buffer("weight_shape", torch.tensor([out_features, in_features], dtype=torch.int64))
+        plain = {}                       # attributes that are neither buffers nor modules
         if zero_point is not None:
             self.register_buffer("weight_zero_point", zero_point.detach().contiguous())
         else:
-            self.weight_zero_point = None
+            plain["weight_zero_point"] = None
         if bias is not None:
             self.register_buffer("bias", bias.detach().contiguous())
         else:
-            self.bias = None
-        self.in_features = int(in_features)
-        self.out_features = int(out_features)
-        if self.weight_packed.dtype != torch.int32 or tuple(self.weight_packed.shape) != (
-                self.out_features, (self.in_features + 7) // 8):
-            raise ValueError(
-                f"packed_weight must be int32 [{self.out_features}, {(self.in_features + 7) // 8}], got "
-                f"{self.weight_packed.dtype} {tuple(self.weight_packed.shape)}")
-        if self.weight_scale.dim() != 2 or self.weight_scale.shape[0] != self.out_features or (
-                self.in_features % self.weight_scale.shape[1]):
-            raise ValueError(f"scale shape {tuple(self.weight_scale.shape)} does not divide in_features")
-        self.group_size = self.in_features // int(self.weight_scale.shape[1])
-        self._scale_zero = None   # kernel-side layout, built on first use
-        self._host_stage = {}     # (row count, stream) -> (x, y) device staging buffers of forward_host
-        self._host_plans = {}     # (x_host ptr, y_host ptr, shape, stream, weight-side ptrs) -> raw call of forward_host
-        self._derived_from = None  # (address, version) of every tensor _scale_zero was built from
+            plain["bias"] = None
+        in_features, out_features = int(in_features), int(out_features)
+        if packed.dtype != torch.int32 or tuple(packed.shape) != (out_features, (in_features + 7) // 8):
+            raise ValueError(f"packed_weight must be int32 [{out_features}, {(in_features + 7) // 8}], got "
+                             f"{packed.dtype} {tuple(packed.shape)}")
+        if scale.dim() != 2 or scale.shape[0] != out_features or in_features % scale.shape[1]:
+            raise ValueError(f"scale shape {tuple(scale.shape)} does not divide in_features")
+        plain.update(
+            in_features=in_features, out_features=out_features, group_size=in_features // int(scale.shape[1]),
+            _scale_zero=None,    # kernel-side layout, built on first use
+            _host_stage={},      # (row count, stream) -> (x, y) device staging buffers of forward_host
+            _host_plans={},      # (x_host ptr, y_host ptr, shape, stream, weight-side ptrs) -> raw call of forward_host
+            _derived_from=None,  # (address, version) of every tensor _scale_zero was built from
+            _plan=None)          # native forward, made at the first call
+        self.__dict__.update(plain)      # nn.Module.__setattr__ costs 2-3 us per attribute
         self.register_load_state_dict_post_hook(VllmPackedInt4Linear._state_loaded)
 
     # -- construction -------------------------------------------------------
@@ -87,12 +101,14 @@ class VllmPackedInt4Linear(nn.Module):
         self._scale_zero = ops.w4a16_prepare(self.weight_scale, self.weight_zero_point, self.in_features)
         self._derived_from = self._weight_side_state()
         self._host_plans = {}            # they hold the old buffer's address
+        self._plan = None
 
     @staticmethod
     def _state_loaded(module, incompatible_keys) -> None:
         """``load_state_dict`` copied new scales / zero points into the buffers: the derived layout is stale."""
         module._scale_zero = None
         module._host_plans = {}
+        module._plan = None
 
     def _ensure_prepared(self) -> None:
         """(Re)build the derived buffer when it is missing or when scales / zero points were replaced or
@@ -102,24 +118,38 @@ class VllmPackedInt4Linear(nn.Module):
 
     def dequantize(self) -> torch.Tensor:
         """fp16 ``[N, K]`` weights, bit-identical to the reference's fake-quant weight."""
-        return ops.w4a16_dequant(self.weight_packed, self.weight_scale, self.weight_zero_point,
+        b = self._buffers
+        return ops.w4a16_dequant(b["weight_packed"], b["weight_scale"], b.get("weight_zero_point"),
                                  self.out_features, self.in_features)
 
     def _apply(self, fn, *args, **kwargs):
         self._scale_zero = None          # moved/cast: rebuild lazily on the new device
         self._host_stage = {}
         self._host_plans = {}
+        self._plan = None
         return super()._apply(fn, *args, **kwargs)
 
     # -- forward ------------------------------------------------------------
-    @torch.no_grad()
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        plan = self._plan
+        if plan is not None:
+            y = plan.run(self, x)
+            if y is not None:
+                return y
+        return self._forward_checked(x)
+
+    @torch.no_grad()
+    def _forward_checked(self, x: torch.Tensor) -> torch.Tensor:
         self._ensure_prepared()
         shape = x.shape
         x2 = x.reshape(-1, shape[-1])
         if not x2.is_contiguous():
             x2 = x2.contiguous()
         y = ops.w4a16_linear(x2, self.weight_packed, self._scale_zero, self.bias)
+        self._plan = _native_plan(_lib.host().w4_plan, self,
+                                  ("weight_packed", "weight_scale", "weight_zero_point", "bias", "_scale_zero"),
+                                  self.weight_packed, self._scale_zero, self.bias, self.group_size,
+                                  ops._error_word(x2.device).data_ptr())
         return y.reshape(*shape[:-1], self.out_features)
 
     def forward_host(self, x_host: torch.Tensor, y_host: torch.Tensor | None = None, stream=None,
@@ -144,7 +174,6 @@ class VllmPackedInt4Linear(nn.Module):
             call, args, y_keep, shapes, _keep = plan
             status = call(*args, st)
             if status != 0:
-                from . import _lib
                 _lib.check(status, "w4a16_linear_decode_host", **shapes)
             return y_keep
         m = x_host.shape[0]
@@ -169,7 +198,6 @@ class VllmPackedInt4Linear(nn.Module):
         if y_host is not None and x_host.is_pinned() and y_host.is_pinned():
             # validated once: remember the raw call (the tensors are kept alive by the plan)
             import ctypes
-            from . import _lib
             y_out, y_copy = stage[1].data_ptr(), y_host.data_ptr()
             if zero_copy_output:
                 # pinned memory is mapped into the device's address space: let the kernel store the result there
@@ -205,7 +233,6 @@ def forward_host_many(linears, x_hosts, y_hosts, stream=None):
     tensors, one pair per module (<= 16 rows); returns ``y_hosts``, valid once the stream is synchronised.  The
     first call with a given set of modules, buffers and stream goes through each module's own ``forward_host``
     (argument checks, staging and scratch buffers); repeats reuse the recorded call."""
-    from . import _lib
     st = torch.cuda.current_stream().cuda_stream if stream is None else stream.cuda_stream
     key = (st,) + tuple((id(m), x.data_ptr(), y.data_ptr(), x.shape[0]) for m, x, y in zip(linears, x_hosts, y_hosts))
     plan = _HOST_MANY_PLANS.get(key)
@@ -285,6 +312,7 @@ class SmoothQuantLinear(nn.Module):
         self.quantize_output = bool(quantize_output)
         self.output_quant_name = act_quant if quantize_output else "none"
         self._weight_scale_fp32 = None
+        self._plan = None
 
     @staticmethod
     @torch.no_grad()
@@ -307,9 +335,11 @@ class SmoothQuantLinear(nn.Module):
         (acceleration/runtime_patches/vllm_ascend.patch:4029-4031)."""
         self._weight_scale_fp32 = self.weight_scale.detach().flatten().to(torch.float32).contiguous()
         self._derived_from = (self.weight_scale.data_ptr(), self.weight_scale._version)
+        self._plan = None
 
     def _apply(self, fn, *args, **kwargs):
         self._weight_scale_fp32 = None
+        self._plan = None
         return super()._apply(fn, *args, **kwargs)
 
     def _ensure_prepared(self) -> None:
@@ -323,10 +353,18 @@ class SmoothQuantLinear(nn.Module):
         """The reference's fake-quantised fp16 weight: ``f16(code * scale)``."""
         return (self.weight.to(torch.float16) * self.weight_scale).to(torch.float16)
 
-    @torch.no_grad()
     def forward(self, x):
         """``x`` is an fp16 tensor, or a ``(int8 codes, per-token scale)`` pair produced upstream
         (the tuple input of AscendW8A8DynamicLinearMethod.apply, vllm_ascend.patch:3945-3962)."""
+        plan = self._plan
+        if plan is not None:
+            y = plan.run(self, x)
+            if y is not None:
+                return y
+        return self._forward_checked(x)
+
+    @torch.no_grad()
+    def _forward_checked(self, x):
         self._ensure_prepared()
         if isinstance(x, tuple):
             q, s = x
@@ -342,6 +380,11 @@ class SmoothQuantLinear(nn.Module):
         y = ops.w8a8_gemm(q2.contiguous(), s2.contiguous(), self.weight, self._weight_scale_fp32, self.bias)
         if self.quantize_output:
             _, _, y = ops.act_quant_per_token(y, want_codes=False, want_fake=True)
+        else:
+            self._plan = _native_plan(_lib.host().w8_plan, self,
+                                      ("weight", "weight_scale", "bias", "_weight_scale_fp32", "quantize_output"),
+                                      self.weight, self._weight_scale_fp32, self.bias,
+                                      ops._error_word(q2.device).data_ptr())
         return y.reshape(*lead, self.out_features)
 
     def __repr__(self):
@@ -388,6 +431,11 @@ class QuantLinear(nn.Module):
             self.bias = None
         self.use_weight_quant = True
         self.use_act_quant = True
+        self._plan = None
+
+    def _apply(self, fn, *args, **kwargs):
+        self._plan = None
+        return super()._apply(fn, *args, **kwargs)
 
     def set_quant_state(self, weight_quant: bool = False, act_quant: bool = False) -> None:
         if not (weight_quant and act_quant):
@@ -399,12 +447,23 @@ class QuantLinear(nn.Module):
         return ((self.weight.to(torch.float16) - self.zeros.to(torch.float16)[:, None])
                 * self.scales.to(torch.float16)[:, None]).to(torch.float16)
 
-    @torch.no_grad()
     def forward(self, input: torch.Tensor) -> torch.Tensor:
+        plan = self._plan
+        if plan is not None:
+            y = plan.run(self, input)
+            if y is not None:
+                return y
+        return self._forward_checked(input)
+
+    @torch.no_grad()
+    def _forward_checked(self, input: torch.Tensor) -> torch.Tensor:
         lead = input.shape[:-1]
         x2 = input.reshape(-1, input.shape[-1]).contiguous()
         q, s, z, rs, _ = ops.affine_quant_per_row(x2)
         y = ops.w8a8_affine_gemm(q, s, z, rs, self.weight, self.scales, self.zeros, self.weight_rowsum, self.bias)
+        self._plan = _native_plan(_lib.host().affine_plan, self,
+                                  ("weight", "scales", "zeros", "weight_rowsum", "bias"), self.weight, self.scales,
+                                  self.zeros, self.weight_rowsum, self.bias, ops._error_word(x2.device).data_ptr())
         return y.reshape(*lead, self.out_features)
 
 
@@ -484,6 +543,11 @@ class SmoothQuantPackedMoeExperts(nn.Module):
         self.register_buffer("gate_up_proj_scale", gs)
         self.register_buffer("down_proj", dq)
         self.register_buffer("down_proj_scale", ds)
+        self._plan = None
+
+    def _apply(self, fn, *args, **kwargs):
+        self._plan = None
+        return super()._apply(fn, *args, **kwargs)
 
     @staticmethod
     @torch.no_grad()
@@ -499,8 +563,16 @@ class SmoothQuantPackedMoeExperts(nn.Module):
                                            weight_bits=weight_bits, activation_bits=activation_bits,
                                            expert_range=expert_range, num_experts=num_experts)
 
-    @torch.no_grad()
     def forward(self, hidden_states: torch.Tensor, top_k_index: torch.Tensor, top_k_weights: torch.Tensor):
+        plan = self._plan
+        if plan is not None:
+            out = plan.run(self, hidden_states, top_k_index, top_k_weights)
+            if out is not None:
+                return out
+        return self._forward_checked(hidden_states, top_k_index, top_k_weights)
+
+    @torch.no_grad()
+    def _forward_checked(self, hidden_states, top_k_index, top_k_weights):
         shape = hidden_states.shape
         hs = hidden_states.reshape(-1, shape[-1]).contiguous()
         ids = top_k_index.reshape(hs.shape[0], -1).to(torch.int32).contiguous()
@@ -510,6 +582,10 @@ class SmoothQuantPackedMoeExperts(nn.Module):
         d = ops.moe_expert_stage(routing.routed_q, routing.routed_scale, routing.plan, hi - lo,
                                  self.gate_up_proj, self.gate_up_proj_scale, self.down_proj, self.down_proj_scale)
         out = ops.moe_combine(d, routing.dest_row, ids, w, hs.shape[0])
+        self._plan = _native_plan(_lib.host().moe_plan, self,
+                                  ("gate_up_proj", "gate_up_proj_scale", "down_proj", "down_proj_scale", "expert_range"),
+                                  self.gate_up_proj, self.gate_up_proj_scale, self.down_proj, self.down_proj_scale,
+                                  lo, hi, ops._error_word(hs.device).data_ptr())
         return out.reshape(shape)
 
     def __repr__(self):

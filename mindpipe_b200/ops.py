@@ -9,14 +9,10 @@ the CUDA library.  Nothing here falls back to torch math.
 """
 from __future__ import annotations
 
-import threading
-
 import torch
 
 from . import _lib
 
-_ws_lock = threading.Lock()
-_workspaces: dict[tuple[int, int], torch.Tensor] = {}
 _err_words: dict[int, torch.Tensor] = {}
 
 
@@ -43,22 +39,14 @@ def _ptr(t: torch.Tensor | None) -> int | None:
 
 
 def _workspace(nbytes: int, device: torch.device, kind: str = "decode") -> torch.Tensor:
-    """Zero-initialised scratch, one per (device, stream, kind), grown on demand.
+    """Zero-initialised scratch, one per (device, stream, kind), grown on demand (``csrc/host_path.cpp`` keeps it).
 
     The decode kernels leave their part zeroed where it has to be, so it is
-    cleared only when it is (re)allocated; the prefill split-K partial sums
-    (kind "prefill") overwrite theirs freely, hence the separate buffer.
+    cleared only when it is (re)allocated; the prefill and W8A8 split-K partial
+    sums overwrite theirs freely, hence the separate kinds.
     """
-    key = (device.index if device.index is not None else torch.cuda.current_device(), _stream(), kind)
-    with _ws_lock:
-        ws = _workspaces.get(key)
-        if ws is None or ws.numel() < nbytes:
-            if torch.cuda.is_current_stream_capturing():
-                raise RuntimeError("scratch memory would be allocated during CUDA graph capture; "
-                                   "pass a preallocated workspace= (see new_workspace)")
-            ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-            _workspaces[key] = ws
-    return ws
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    return _lib.host().workspace(nbytes, index, kind)
 
 
 def new_workspace(nbytes: int, device) -> torch.Tensor:
@@ -90,13 +78,10 @@ def w4a16_quantize(weight: torch.Tensor, group_size: int = 128):
     w = _req(weight, "weight", torch.float16, 2)
     n, k = w.shape
     g = group_size if (group_size > 0 and k % group_size == 0) else k
-    groups = k // g
-    packed = torch.empty((n, k // 8), dtype=torch.int32, device=w.device)
-    scale = torch.empty((n, groups), dtype=torch.float16, device=w.device)
-    zero = torch.empty((n, (groups + 7) // 8), dtype=torch.int32, device=w.device)
-    st = _lib.load().mp_w4a16_quantize(w.data_ptr(), n, k, g, packed.data_ptr(), scale.data_ptr(),
-                                       zero.data_ptr(), _stream())
-    _lib.check(st, "w4a16_quantize", N=n, K=k, group=g)
+    made = _lib.host().w4_quantize(w, g)
+    if isinstance(made, int):
+        _lib.check(made, "w4a16_quantize", N=n, K=k, group=g)
+    packed, scale, zero = made
     return packed, scale, zero, g
 
 
@@ -111,10 +96,9 @@ def w4a16_dequant(weight_packed, weight_scale, weight_zero_point, out_features: 
     groups = s.shape[1]
     if s.shape[0] != n or k % groups:
         raise ValueError(f"weight_scale shape {tuple(s.shape)} does not divide K={k}")
-    out = torch.empty((n, k), dtype=torch.float16, device=p.device)
-    st = _lib.load().mp_w4a16_dequant(p.data_ptr(), s.data_ptr(), _ptr(z), n, k, k // groups,
-                                      out.data_ptr(), _stream())
-    _lib.check(st, "w4a16_dequant", N=n, K=k, groups=groups)
+    out = _lib.host().w4_dequant(p, s, z, n, k, k // groups)
+    if isinstance(out, int):
+        _lib.check(out, "w4a16_dequant", N=n, K=k, groups=groups)
     return out
 
 
@@ -371,10 +355,9 @@ def check_device_errors(device=None) -> None:
     import ctypes
 
     def rearm(index=None):
-        with _ws_lock:
-            for (dev_index, _stream_id, _kind), ws in _workspaces.items():
-                if index is None or dev_index == index:
-                    ws.zero_()
+        for dev_index, ws in _lib.host().workspaces():
+            if index is None or dev_index == index:
+                ws.zero_()
         torch.cuda.synchronize(device)
 
     flag = ctypes.c_int(0)
