@@ -30,10 +30,13 @@ inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_
 constexpr int kSmCount = 148;  // B200
 
 // ---- programmatic dependent launch for chains of short kernels -------------
-// With the process-wide switch on (mp_set_programmatic_launch), launch_chained() lets a kernel be scheduled
-// while the previous kernel of the stream is still running; the kernel itself waits for that kernel's results
-// with chain_wait() before it reads or writes anything the stream ordered, and chain_release() lets the next
-// one be scheduled in turn.  Without the attribute both instructions do nothing.
+// launch_chained() lets a kernel be scheduled while the previous kernel of the stream is still running; the kernel
+// itself waits for that kernel's results with chain_wait() before it reads or writes anything the stream ordered, so
+// results are those of a plain launch and only the launch latency (2-3 us) overlaps.  chain_release() lets the next
+// kernel be scheduled in turn; it always comes after chain_wait(), so a kernel that starts early finds everything
+// older than its predecessor complete.
+// launch_chained_opt() does so only with the process-wide switch on (mp_set_programmatic_launch): the kernels that
+// wait for other GPUs.
 bool decode_programmatic_launch();   // w4a16_decode_tma.cu
 
 #ifdef __CUDACC__
@@ -41,7 +44,8 @@ __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
-int launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+int launch_attributed(bool chained, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                      Args... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -51,9 +55,17 @@ int launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
   attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attrs[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attrs;
-  cfg.numAttrs = decode_programmatic_launch() ? 1 : 0;
+  cfg.numAttrs = chained ? 1 : 0;
   MP_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
   return MP_OK;
+}
+template <typename... KArgs, typename... Args>
+int launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  return launch_attributed(true, kernel, grid, block, smem, st, args...);
+}
+template <typename... KArgs, typename... Args>
+int launch_chained_opt(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  return launch_attributed(decode_programmatic_launch(), kernel, grid, block, smem, st, args...);
 }
 #endif
 

@@ -578,7 +578,7 @@ extern "C" int mp_moe_combine_after_peers(const void* arrival_words_u32, int wor
     return MP_ERR_INVALID_ARG;
   if (H % 8 != 0 || k > 8) return MP_ERR_UNSUPPORTED;
   if (!aligned(d_f16, 16) || !aligned(out_f16, 16)) return MP_ERR_ALIGNMENT;
-  return launch_chained(moe_combine_kernel, dim3(T), dim3(256), 0, static_cast<cudaStream_t>(stream),
+  return launch_chained_opt(moe_combine_kernel, dim3(T), dim3(256), 0, static_cast<cudaStream_t>(stream),
                         static_cast<const __half*>(d_f16), static_cast<const int*>(dest_row_i32),
                         static_cast<const int*>(topk_ids_i32), static_cast<const __half*>(topk_weights_f16), T, H, k,
                         static_cast<__half*>(out_f16), static_cast<const unsigned int*>(arrival_words_u32), world,

@@ -302,7 +302,7 @@ extern "C" int mp_peer_barrier_counted(const void* const* peer_flag_ptrs, int wo
   int rc = fill_peers(pf, peer_flag_ptrs, world);
   if (rc != MP_OK) return rc;
   if (rank < 0 || rank >= world || !epoch_counter_u32) return MP_ERR_INVALID_ARG;
-  return launch_chained(peer_barrier_counted_kernel, dim3(1), dim3(32), 0, static_cast<cudaStream_t>(stream), pf, world,
+  return launch_chained_opt(peer_barrier_counted_kernel, dim3(1), dim3(32), 0, static_cast<cudaStream_t>(stream), pf, world,
                         rank, static_cast<unsigned int*>(epoch_counter_u32), error_word);
 }
 
@@ -467,7 +467,7 @@ extern "C" int mp_moe_ep_barrier_plan(const void* const* peer_flag_ptrs, const v
   const int e_loc = num_experts / world;
   const int max_tiles = capacity_rows / kEpTile;
   const int ext = 3 * e_loc + 2 + max_tiles;
-  return launch_chained(ep_barrier_plan_kernel, dim3(1), dim3(64), 0, static_cast<cudaStream_t>(stream), pf, pp, world,
+  return launch_chained_opt(ep_barrier_plan_kernel, dim3(1), dim3(64), 0, static_cast<cudaStream_t>(stream), pf, pp, world,
                         rank, static_cast<unsigned int*>(epoch_counter_u32), num_experts, e_loc, max_tiles, ext,
                         static_cast<int*>(xplan_i32), error_word);
 }
@@ -492,7 +492,7 @@ extern "C" int mp_moe_ep_pull_part(const void* const* peer_q_ptrs, const void* c
   uint4* qd = static_cast<uint4*>(q_sorted_i8);
   float* sd = static_cast<float*>(scale_sorted_f32);
   auto kern = vec == 256 ? ep_pull_kernel<8> : (vec == 128 ? ep_pull_kernel<4> : ep_pull_kernel<0>);
-  return launch_chained(kern, dim3(grid), dim3(256), 0, st, pq, ps, xp, world, num_local_experts, ext, vec, qd, sd, part);
+  return launch_chained_opt(kern, dim3(grid), dim3(256), 0, st, pq, ps, xp, world, num_local_experts, ext, vec, qd, sd, part);
 }
 
 extern "C" int mp_moe_ep_push_part(const void* d_sorted_f16, const void* xplan_i32, int world, int num_local_experts,
@@ -512,7 +512,7 @@ extern "C" int mp_moe_ep_push_part(const void* d_sorted_f16, const void* xplan_i
   const uint4* dd = static_cast<const uint4*>(d_sorted_f16);
   const int* xp = static_cast<const int*>(xplan_i32);
   auto kern = vec == 512 ? ep_push_kernel<16> : (vec == 256 ? ep_push_kernel<8> : ep_push_kernel<0>);
-  return launch_chained(kern, dim3(grid), dim3(256), 0, st, dd, xp, world, num_local_experts, ext, vec, pb, part,
+  return launch_chained_opt(kern, dim3(grid), dim3(256), 0, st, dd, xp, world, num_local_experts, ext, vec, pb, part,
                         EpSignal{});
 }
 
@@ -539,7 +539,7 @@ extern "C" int mp_moe_ep_push_signal(const void* d_sorted_f16, const void* xplan
   int grid = (capacity_rows + 7) / 8;
   if (grid > 4 * kSmCount) grid = 4 * kSmCount;
   auto kern = vec == 512 ? ep_push_kernel<16> : (vec == 256 ? ep_push_kernel<8> : ep_push_kernel<0>);
-  return launch_chained(kern, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream),
+  return launch_chained_opt(kern, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream),
                         static_cast<const uint4*>(d_sorted_f16), static_cast<const int*>(xplan_i32), world,
                         num_local_experts, ext, vec, pb, -1, sig);
 }

@@ -26,9 +26,12 @@
 // cluster barrier, and each owner adds the CK tiles in rank order
 // (deterministic), adds the bias and writes fp16.  No scratch memory.
 //
-// Under programmatic dependent launch the weight and scale boxes of the first
-// stages are requested before griddepcontrol.wait; activations, bias and the
-// output are only touched after it.  Every mbarrier wait is bounded.
+// Launched with programmatic stream serialisation: blocks are scheduled and set
+// up beside the tail of the previous kernel.  With the caller's leave (static
+// weights, mp_set_programmatic_launch) the weight and scale boxes of the first
+// stages are requested before griddepcontrol.wait; everything else, and without
+// that leave the weights too, is only touched after it.  Every mbarrier wait is
+// bounded.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -64,6 +67,7 @@ struct DecodeTmaParams {
   int stages_total;        // ceil(K / 256)
   int stages_per_block;    // per cluster rank
   int groups_per_stage;    // rows of the (scale, zero) box
+  int early_weights;       // 1: fetch weights before the previous kernel of the stream has finished
   int* error_word;
   DecodePush push;         // row-parallel mode (PUSH kernels only)
 };
@@ -211,9 +215,10 @@ w4a16_decode_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         for (int j = 0; j < 4; ++j) tma_load_2d(smem_u32(xb + j * C::kXSub), &tmap_x, full, st * dt::kStageK + j * 64, 0);
       };
       const int prologue = min(n_stages, dt::kStages);
-      for (int i = 0; i < prologue; ++i) issue_weights(i);     // weights never depend on the previous kernel
       asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-      asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (!p.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
+      for (int i = 0; i < prologue; ++i) issue_weights(i);
+      if (p.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
       for (int i = 0; i < prologue; ++i) issue_x(i);
       for (int i = prologue; i < n_stages; ++i) {
         const int s = i % dt::kStages;
@@ -484,7 +489,7 @@ int* decode_error_word_ptr(int* out_rc) {
 
 template <bool HALF, bool FOLD, bool PUSH>
 static int launch_tma(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tsz, const DecodeTmaParams& p,
-                      int row_blocks, int ck, cudaStream_t st, bool pdl) {
+                      int row_blocks, int ck, cudaStream_t st) {
   using C = dt::Cfg<HALF>;
   auto kern = w4a16_decode_tma_kernel<HALF, FOLD, PUSH>;
   static thread_local int configured_device = -1;
@@ -504,17 +509,13 @@ static int launch_tma(const CUtensorMap& tw, const CUtensorMap& tx, const CUtens
   attrs[0].val.clusterDim.x = 1;
   attrs[0].val.clusterDim.y = ck;
   attrs[0].val.clusterDim.z = 1;
-  int n_attrs = 1;
-  // (push launches too: their block counter and call number are touched only after griddepcontrol.wait, i.e. after
-  // the previous push kernel and the finish kernel between them have completed; the early start lets the next
-  // shard's weight fetch run under the exchange)
-  if (pdl) {
-    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attrs[1].val.programmaticStreamSerializationAllowed = 1;
-    n_attrs = 2;
-  }
+  // (push launches: their block counter and call number are touched only after griddepcontrol.wait, i.e. after the
+  // previous push kernel and the finish kernel between them have completed; an early start lets the next shard's
+  // weight fetch run under the exchange, so they take it only with the caller's leave)
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attrs;
-  cfg.numAttrs = n_attrs;
+  cfg.numAttrs = PUSH && !p.early_weights ? 1 : 2;
   MP_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tw, tx, tsz, p));
   return MP_OK;
 }
@@ -577,6 +578,7 @@ int launch_decode_tma(const void* x, const void* packed, const void* sz, const v
   p.M = M; p.N = N; p.K = K; p.group = group;
   p.stages_total = (K + dt::kStageK - 1) / dt::kStageK;
   p.groups_per_stage = gps;
+  p.early_weights = pdl ? 1 : 0;
   {
     int rc_err = MP_OK;
     p.error_word = decode_error_word_ptr(&rc_err);
@@ -602,13 +604,13 @@ int launch_decode_tma(const void* x, const void* packed, const void* sz, const v
   // exact per-weight form.
   if (push) {
     p.push = *push;
-    if (half && group % 128 == 0) return launch_tma<true, true, true>(tw, tx, tsz, p, row_blocks, ck, st, pdl);
-    return half ? launch_tma<true, false, true>(tw, tx, tsz, p, row_blocks, ck, st, pdl)
-                : launch_tma<false, false, true>(tw, tx, tsz, p, row_blocks, ck, st, pdl);
+    if (half && group % 128 == 0) return launch_tma<true, true, true>(tw, tx, tsz, p, row_blocks, ck, st);
+    return half ? launch_tma<true, false, true>(tw, tx, tsz, p, row_blocks, ck, st)
+                : launch_tma<false, false, true>(tw, tx, tsz, p, row_blocks, ck, st);
   }
-  if (half && group % 128 == 0) return launch_tma<true, true, false>(tw, tx, tsz, p, row_blocks, ck, st, pdl);
-  return half ? launch_tma<true, false, false>(tw, tx, tsz, p, row_blocks, ck, st, pdl)
-              : launch_tma<false, false, false>(tw, tx, tsz, p, row_blocks, ck, st, pdl);
+  if (half && group % 128 == 0) return launch_tma<true, true, false>(tw, tx, tsz, p, row_blocks, ck, st);
+  return half ? launch_tma<true, false, false>(tw, tx, tsz, p, row_blocks, ck, st)
+              : launch_tma<false, false, false>(tw, tx, tsz, p, row_blocks, ck, st);
 }
 
 }  // namespace mp

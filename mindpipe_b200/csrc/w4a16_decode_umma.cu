@@ -89,6 +89,7 @@ struct DecodeUmmaParams {
   int stages_per_row;      // ST = ceil(K / 256)
   int total;               // row blocks x ST
   int groups_per_stage;    // rows of the (scale, zero) box
+  int early_weights;       // 1: fetch weights before the previous kernel of the stream has finished
   int gshift;              // log2(group) for groups shorter than 128 columns
   int* counters;           // workspace: [row blocks], zero between calls
   float* tiles;            // workspace: [grid][2][TOK][128] fp32 partial tiles
@@ -244,9 +245,10 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
         for (int j = 0; j < 4; ++j) tma_load_2d(smem_u32(xb + j * kXSub), &tmap_x, full, st * du::kStageK + j * 64, 0);
       };
       const int prologue = min(n_stages, STAGES);
-      for (int i = 0; i < prologue; ++i) issue_weights(i);     // weights never depend on the previous kernel
       asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-      asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (!p.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
+      for (int i = 0; i < prologue; ++i) issue_weights(i);
+      if (p.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
       for (int i = 0; i < prologue; ++i) issue_x(i);
       for (int i = prologue; i < n_stages; ++i) {
         const int s = i % STAGES;
@@ -472,7 +474,7 @@ static bool umma_shape_ok(int M, int N, int K, int group) {
 
 template <int STAGES, int TOK>
 static int launch_umma(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tsz, const DecodeUmmaParams& p,
-                       int grid, size_t smem, cudaStream_t st, bool pdl) {
+                       int grid, size_t smem, cudaStream_t st) {
   auto kern = w4a16_decode_umma_kernel<STAGES, TOK>;
   static thread_local int configured_device = -1;
   int device = 0;
@@ -487,14 +489,10 @@ static int launch_umma(const CUtensorMap& tw, const CUtensorMap& tx, const CUten
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attrs[1];
-  int n_attrs = 0;
-  if (pdl) {
-    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attrs[0].val.programmaticStreamSerializationAllowed = 1;
-    n_attrs = 1;
-  }
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attrs;
-  cfg.numAttrs = n_attrs;
+  cfg.numAttrs = 1;
   MP_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tw, tx, tsz, p));
   return MP_OK;
 }
@@ -529,6 +527,7 @@ int launch_decode_umma(const void* x, const void* packed, const void* sz, const 
   p.stages_per_row = (K + du::kStageK - 1) / du::kStageK;
   p.total = row_blocks * p.stages_per_row;
   p.groups_per_stage = gps;
+  p.early_weights = pdl ? 1 : 0;
   p.gshift = group == 32 ? 5 : group == 64 ? 6 : 7;
   p.counters = static_cast<int*>(workspace);
   p.tiles = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + du::kCounterBytes);
@@ -541,15 +540,15 @@ int launch_decode_umma(const void* x, const void* packed, const void* sz, const 
   // pairs per stage; a 32-token activation tile is 16 KB per stage, a 64-token one 32 KB)
   auto fits = [&](int stages) { return du::smem_bytes(tok, stages, gps) <= du::kSmemBlockMax; };
   if (tok == 16) {
-    if (fits(4)) return launch_umma<4, 16>(tw, tx, tsz, p, grid, du::smem_bytes(16, 4, gps), st, pdl);
-    return launch_umma<3, 16>(tw, tx, tsz, p, grid, du::smem_bytes(16, 3, gps), st, pdl);
+    if (fits(4)) return launch_umma<4, 16>(tw, tx, tsz, p, grid, du::smem_bytes(16, 4, gps), st);
+    return launch_umma<3, 16>(tw, tx, tsz, p, grid, du::smem_bytes(16, 3, gps), st);
   }
   if (tok == 32) {
-    if (fits(3)) return launch_umma<3, 32>(tw, tx, tsz, p, grid, du::smem_bytes(32, 3, gps), st, pdl);
-    if (fits(2)) return launch_umma<2, 32>(tw, tx, tsz, p, grid, du::smem_bytes(32, 2, gps), st, pdl);
+    if (fits(3)) return launch_umma<3, 32>(tw, tx, tsz, p, grid, du::smem_bytes(32, 3, gps), st);
+    if (fits(2)) return launch_umma<2, 32>(tw, tx, tsz, p, grid, du::smem_bytes(32, 2, gps), st);
     return MP_ERR_UNSUPPORTED;
   }
-  if (fits(2)) return launch_umma<2, 64>(tw, tx, tsz, p, grid, du::smem_bytes(64, 2, gps), st, pdl);
+  if (fits(2)) return launch_umma<2, 64>(tw, tx, tsz, p, grid, du::smem_bytes(64, 2, gps), st);
   return MP_ERR_UNSUPPORTED;
 }
 

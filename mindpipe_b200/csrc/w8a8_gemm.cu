@@ -647,7 +647,7 @@ static int launch_gemm(const GemmCall& c, cudaStream_t st) {
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = decode_programmatic_launch() ? 2 : 1;
+    cfg.numAttrs = 2;
     MP_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ta, tb, p));
     return MP_OK;
   }
