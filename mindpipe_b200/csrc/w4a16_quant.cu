@@ -274,9 +274,11 @@ extern "C" int mp_w4a16_quantize(const void* w_f16, int N, int K, int group, voi
   uint32_t* packed = static_cast<uint32_t*>(packed_i32);
   __half* scale = static_cast<__half*>(scale_f16);
   uint32_t* zero = static_cast<uint32_t*>(zero_i32);
-  const int per_warp = quantize_vectors(group / 8) * 256 / group;     // groups a warp takes
+  // groups that a warp of the kernels for these sizes takes
+  const bool own = group == 32 || group == 64 || group == 128 || group == 256;
+  const int per_warp = own ? quantize_vectors(group / 8) * 256 / group : 1;
   const long long units = (long long)N * ((groups + per_warp - 1) / per_warp);
-  if (units > 0x7fffffffLL) return MP_ERR_UNSUPPORTED;
+  if (own && units > 0x7fffffffLL) return MP_ERR_UNSUPPORTED;
   const unsigned blocks = static_cast<unsigned>((units + 7) / 8);
   switch (group) {
     case 32: w4_quantize_groups_kernel<4><<<blocks, 256, 0, st>>>(w, N, K, groups, packed, scale, zero); break;

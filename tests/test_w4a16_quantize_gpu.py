@@ -25,7 +25,7 @@ def _weights(n, k, group, seed):
 
 
 @pytest.mark.filterwarnings("ignore::RuntimeWarning")
-@pytest.mark.parametrize("group", [32, 64, 128, 256, 48, 8])
+@pytest.mark.parametrize("group", [32, 64, 128, 256, 48, 8, 2048])
 @pytest.mark.parametrize("groups_per_row", [1, 7, 8, 9, 24])
 def test_codes_scales_zero_points_and_dequant_bit_exact(group, groups_per_row):
     n, k = 11, group * groups_per_row
