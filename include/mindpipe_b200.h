@@ -147,8 +147,8 @@ int mp_w4a16_rowparallel_finish(void* const* peer_partial0_f32, void* const* pee
 int mp_w4a16_linear_decode_host(const void* x_host_f16, void* x_stage_f16, const void* packed_i32,
                                 const void* sz_f16x2, const void* bias_f16, void* y_stage_f16,
                                 void* y_host_f16, int M, int N, int K, int group, mp_stream_t stream);
-/* The same with a workspace of mp_w4a16_decode_workspace_bytes(M, N, K) bytes (zero-filled once, owned by the caller,
- * not shared between calls that may overlap): the kernel is then chosen as mp_w4a16_linear_decode chooses it. */
+/* The same with a workspace of mp_w4a16_linear_workspace_bytes(M, N, K, group) bytes (zero-filled once, owned by the caller,
+ * not shared between calls that may overlap): the kernel is then chosen as mp_w4a16_linear chooses it. */
 int mp_w4a16_linear_decode_host_ws(const void* x_host_f16, void* x_stage_f16, const void* packed_i32,
                                    const void* sz_f16x2, const void* bias_f16, void* y_stage_f16,
                                    void* y_host_f16, int M, int N, int K, int group, void* workspace,
@@ -182,6 +182,19 @@ int mp_w4a16_linear_decode_host_many(const mp_host_linear* linears, int count, m
  * (the reference's forward runs on host tensors directly).
  */
 int mp_host_buffer_device_alias(const void* host_ptr, size_t bytes, void** device_ptr);
+
+/*
+ * The linear for any number of rows: the decode kernels, the tcgen05 weight-streaming kernel (up to 128 rows) or the
+ * prefill GEMM below, whichever is fastest for the shape (with mp_set_decode_kernel set: as that says).  The forward of
+ * VllmPackedInt4Linear (exporters/vllm.py:85-86) in one call.  The workspace is one for all shapes, under the rules of
+ * mp_w4a16_linear_decode: zero-filled when it is created, left ready for the next call, shared only by calls that cannot
+ * overlap on the device; it may also be shared with the decode entries.  Without one the scratch-free kernels run.  Shapes
+ * that need groups or K the GEMM does not take return MP_ERR_UNSUPPORTED above 16 rows.  error_word as for mp_w8a8_gemm.
+ */
+size_t mp_w4a16_linear_workspace_bytes(int M, int N, int K, int group);
+int mp_w4a16_linear(const void* x_f16, const void* packed_i32, const void* sz_f16x2, const void* bias_f16, void* y_f16,
+                    int M, int N, int K, int group, void* workspace, size_t workspace_bytes, int* error_word,
+                    mp_stream_t stream);
 
 /*
  * Prefill variant (any M; meant for M > 64): the same linear on the fp16 tensor

@@ -29,6 +29,11 @@ inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_
 
 constexpr int kSmCount = 148;  // B200
 
+// Workspace of the W4A16 kernels (zero-filled when it is created): arrival counters and partial tiles, which every call
+// leaves zero, then whatever a call overwrites freely.  The kernels share buffers, so the order is the same for all.
+constexpr size_t kW4CounterBytes = 16384;                       // room for 4096 row blocks
+constexpr size_t kW4TileBytes = (size_t)kSmCount * 128 * 512;   // a tile of 128 tokens x 128 rows fp32 per block
+
 // ---- programmatic dependent launch for chains of short kernels -------------
 // launch_chained() lets a kernel be scheduled while the previous kernel of the stream is still running; the kernel
 // itself waits for that kernel's results with chain_wait() before it reads or writes anything the stream ordered, so

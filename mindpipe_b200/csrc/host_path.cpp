@@ -150,7 +150,6 @@ struct Scratch {
   }
 };
 
-// W4A16: the dispatch of ops.w4a16_linear.
 struct W4Plan : Plan {
   at::Tensor packed, scale_zero, bias;
   int n = 0, k = 0, group = 0;
@@ -163,19 +162,10 @@ struct W4Plan : Plan {
     if (rows > (int64_t(1) << 30)) return none();
     const int m = static_cast<int>(rows);
     const cudaStream_t st = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream();
-    const bool decode = m <= 16 || (m <= 64 && mp_w4a16_decode_kernel_choice(m, n, k, 1) == MP_DECODE_KERNEL_UMMA);
-    if (!decode && (k % 64 != 0 || group % 64 != 0)) return none();
     at::Tensor y = output_like(x, n, at::kHalf);
-    int rc;
-    if (decode) {
-      Scratch ws(mp_w4a16_decode_workspace_bytes(m, n, k), device, st, kDecode);
-      rc = mp_w4a16_linear_decode(x.data_ptr(), packed.data_ptr(), scale_zero.data_ptr(), data_or_null(bias), y.data_ptr(),
-                                  m, n, k, group, ws.ptr, ws.bytes, st);
-    } else {
-      Scratch ws(mp_w4a16_prefill_workspace_bytes(m, n, k), device, st, kPrefill);
-      rc = mp_w4a16_linear_prefill_ex(x.data_ptr(), packed.data_ptr(), scale_zero.data_ptr(), data_or_null(bias),
-                                      y.data_ptr(), m, n, k, group, ws.ptr, ws.bytes, error_word, st);
-    }
+    Scratch ws(mp_w4a16_linear_workspace_bytes(m, n, k, group), device, st, kDecode);
+    const int rc = mp_w4a16_linear(x.data_ptr(), packed.data_ptr(), scale_zero.data_ptr(), data_or_null(bias), y.data_ptr(),
+                                   m, n, k, group, ws.ptr, ws.bytes, error_word, st);
     return rc == MP_OK ? THPVariable_Wrap(std::move(y)) : none();
   }
 };

@@ -35,10 +35,12 @@ int launch_decode_tma(const void* x, const void* packed, const void* sz, const v
 void set_decode_programmatic_launch(bool on);
 bool decode_programmatic_launch();
 int read_and_clear_decode_error(int* value);
-// tcgen05 kernel for M <= 16 with the weights as the tensor-memory operand (w4a16_decode_umma.cu)
+// tcgen05 kernel for M <= 128 with the weights as the tensor-memory operand (w4a16_decode_umma.cu)
 int launch_decode_umma(const void* x, const void* packed, const void* sz, const void* bias, void* y, int M, int N, int K,
                        int group, void* workspace, size_t workspace_bytes, cudaStream_t st, bool pdl);
-size_t decode_umma_workspace_bytes(int M);   // M <= 64: the activation tile is 16, 32 or 64 token rows
+bool decode_umma_shape_ok(int M, int N, int K, int group);
+int decode_tma_cluster(int row_blocks, int stages);   // cluster size the ring kernel splits K over
+size_t decode_umma_workspace_bytes(int M, int K);
 // Which kernel serves M <= 16 when a call does not say: one of the MP_DECODE_KERNEL_* values.  Shapes the
 // chosen one does not take fall through to the next.
 static int g_decode_kernel = MP_DECODE_KERNEL_AUTO;
@@ -498,7 +500,8 @@ static DecodePlan plan_decode(int M, int N, int K, int k_split_req) {
   return pl;
 }
 
-constexpr size_t kCounterBytes = 16384;  // room for 4096 row blocks
+constexpr size_t kCounterBytes = kW4CounterBytes;
+constexpr size_t kPartialOffset = kW4CounterBytes + kW4TileBytes;   // split-K partial sums in a workspace
 
 template <int MB, bool HALF, int WN, int STAGE>
 static int launch_decode(const DecodeParams& p, const DecodePlan& pl, cudaStream_t st) {
@@ -524,12 +527,12 @@ using namespace mp;
 extern "C" size_t mp_w4a16_decode_workspace_bytes_ex(int M, int N, int K, int k_split) {
   if (M <= 0 || M > 64 || N <= 0 || K <= 0 || K % kChunk != 0) return 0;
   if (M <= 16 && k_split <= 0) {             // partial tiles of the persistent tcgen05 kernels; the mma.sync kernels need none
-    return g_decode_kernel == MP_DECODE_KERNEL_MMA_SYNC ? 0 : decode_umma_workspace_bytes(M);
+    return g_decode_kernel == MP_DECODE_KERNEL_MMA_SYNC ? 0 : decode_umma_workspace_bytes(M, K);
   }
   const DecodePlan pl = plan_decode(M, N, K, k_split);
-  const size_t split_k = kCounterBytes + (size_t)pl.k_split * (size_t)M * (size_t)N * sizeof(float);
-  if (k_split <= 0 && g_decode_kernel != MP_DECODE_KERNEL_MMA_SYNC && decode_umma_workspace_bytes(M) > split_k)
-    return decode_umma_workspace_bytes(M);   // 17..64 rows may take the tcgen05 kernel with a wider activation tile
+  const size_t split_k = kPartialOffset + (size_t)pl.k_split * (size_t)M * (size_t)N * sizeof(float);
+  if (k_split <= 0 && g_decode_kernel != MP_DECODE_KERNEL_MMA_SYNC && decode_umma_workspace_bytes(M, K) > split_k)
+    return decode_umma_workspace_bytes(M, K);   // 17..64 rows may take the tcgen05 kernel with a wider activation tile
   return split_k;
 }
 
@@ -616,11 +619,11 @@ static int decode_linear(const void* x_f16, const void* packed_i32, const void* 
   p.chunks_per_split = pl.chunks_per_split;
   p.k_split = pl.k_split;
   if (pl.k_split > 1) {
-    const size_t need = kCounterBytes + (size_t)pl.k_split * M * N * sizeof(float);
+    const size_t need = kPartialOffset + (size_t)pl.k_split * M * N * sizeof(float);
     if (!workspace || workspace_bytes < need) return MP_ERR_WORKSPACE;
     if (!aligned(workspace, 16)) return MP_ERR_ALIGNMENT;
     p.counters = static_cast<int*>(workspace);
-    p.partials = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + kCounterBytes);
+    p.partials = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + kPartialOffset);
   }
   if (pl.mb == 1 && pl.half) return launch_decode<1, true, 1, 8>(p, pl, st);
   if (pl.mb == 1) return launch_decode<1, false, 2, 8>(p, pl, st);
@@ -746,8 +749,8 @@ extern "C" int mp_w4a16_linear_decode_host_ws(const void* x_host_f16, void* x_st
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   MP_CUDA_TRY(cudaMemcpyAsync(x_stage_f16, x_host_f16, (size_t)M * K * sizeof(__half), cudaMemcpyHostToDevice, st));
   // without a workspace: the scratch-free kernels only
-  const int rc = mp_w4a16_linear_decode_ex(x_stage_f16, packed_i32, sz_f16x2, bias_f16, y_stage_f16, M, N, K, group,
-                                           workspace, workspace ? workspace_bytes : 0, 0, stream);
+  const int rc = mp_w4a16_linear(x_stage_f16, packed_i32, sz_f16x2, bias_f16, y_stage_f16, M, N, K, group, workspace,
+                                 workspace ? workspace_bytes : 0, nullptr, stream);
   if (rc != MP_OK) return rc;
   // no y_host: the result stays where the kernel stored it (y_stage may be the device alias of a pinned host
   // buffer, see mp_host_buffer_device_alias: the kernel's stores then are the device-to-host transfer)
@@ -777,8 +780,8 @@ extern "C" int mp_w4a16_linear_decode_host_many(const mp_host_linear* linears, i
   }
   for (int i = 0; i < count; ++i) {
     const mp_host_linear& c = linears[i];
-    const int rc = mp_w4a16_linear_decode_ex(c.x_stage_f16, c.packed_i32, c.sz_f16x2, c.bias_f16, c.y_stage_f16, c.M, c.N,
-                                             c.K, c.group, c.workspace, c.workspace ? c.workspace_bytes : 0, 0, stream);
+    const int rc = mp_w4a16_linear(c.x_stage_f16, c.packed_i32, c.sz_f16x2, c.bias_f16, c.y_stage_f16, c.M, c.N, c.K,
+                                   c.group, c.workspace, c.workspace ? c.workspace_bytes : 0, nullptr, stream);
     if (rc != MP_OK) return rc;
   }
   for (int i = 0; i < count; ++i) {
@@ -811,6 +814,62 @@ extern "C" int mp_w4a16_linear_decode(const void* x_f16, const void* packed_i32,
                                       void* workspace, size_t workspace_bytes, mp_stream_t stream) {
   return mp_w4a16_linear_decode_ex(x_f16, packed_i32, sz_f16x2, bias_f16, y_f16, M, N, K, group, workspace,
                                    workspace_bytes, 0, stream);
+}
+
+// ---- the linear for any number of rows ---------------------------------------------------------------------------
+// Which kernel.  An explicit process-wide choice (mp_set_decode_kernel) goes as far as it did for the decode entry; else,
+// with "stream" the tcgen05 kernel of w4a16_decode_umma.cu (needs a workspace) and "ring" the mma.sync kernel:
+enum LinearKernel { kRing, kStream, kGemm };
+
+static LinearKernel linear_kernel(int M, int N, int K, int group) {
+  const LinearKernel narrow = M <= 16 ? kRing : kGemm;
+  if (!decode_umma_shape_ok(M, N, K, group) || g_decode_kernel == MP_DECODE_KERNEL_MMA_SYNC) return narrow;
+  if (g_decode_kernel == MP_DECODE_KERNEL_UMMA) return M <= 64 ? kStream : kGemm;
+  const size_t packed = (size_t)N * (size_t)K / 2;
+  if (M > 16) return kStream;
+  // 9..16 rows double the ring kernel's MMAs and cost the stream kernel nothing; below 2 MiB or 16 row blocks the stream
+  // kernel's longer pipeline shows (2048x2048: 4.3 vs 4.5 us, 2048x8192: 6.4 vs 8.9, 12288x4096: 10.4 vs 15.7)
+  if (M > 8) return packed >= ((size_t)2 << 20) && N >= 2048 ? kStream : kRing;
+  // Up to 8 rows the ring kernel's folded form is as fast where its grid is one full wave (8192x8192: 11.0 vs 11.2 us).
+  // Elsewhere the stream kernel's even split wins: grids of more than one wave (6144x4096: 6.3 vs 9.4 us, 12288x4096:
+  // 10.0 vs 11.2), grids that leave SMs empty (2048x8192: 5.5 vs 6.3) and long runs per block (8192x28672: 26 vs 29).
+  const int row_blocks = (N + 127) / 128, stages = (K + 255) / 256;
+  const int blocks = row_blocks * decode_tma_cluster(row_blocks, stages);
+  if (packed < ((size_t)4 << 20)) return kRing;
+  return blocks > 2 * kSmCount || blocks <= kSmCount || packed >= ((size_t)64 << 20) ? kStream : kRing;
+}
+
+extern "C" size_t mp_w4a16_linear_workspace_bytes(int M, int N, int K, int group) {
+  if (M <= 0 || N <= 0 || K <= 0 || group <= 0) return 0;
+  switch (linear_kernel(M, N, K, group)) {
+    case kStream: return decode_umma_workspace_bytes(M, K);
+    case kRing: return 0;
+    default: {
+      const size_t split = mp_w4a16_prefill_workspace_bytes(M, N, K);
+      return split ? kPartialOffset + split : 0;
+    }
+  }
+}
+
+extern "C" int mp_w4a16_linear(const void* x_f16, const void* packed_i32, const void* sz_f16x2, const void* bias_f16,
+                               void* y_f16, int M, int N, int K, int group, void* workspace, size_t workspace_bytes,
+                               int* error_word, mp_stream_t stream) {
+  if (!x_f16 || !packed_i32 || !sz_f16x2 || !y_f16 || M <= 0 || N <= 0 || K <= 0 || group <= 0) return MP_ERR_INVALID_ARG;
+  if (K % group != 0) return MP_ERR_UNSUPPORTED;
+  const LinearKernel kernel = linear_kernel(M, N, K, group);
+  if (kernel == kStream && N % 8 == 0 && K % kChunk == 0) {
+    if (!aligned(x_f16, 16) || !aligned(packed_i32, 16) || !aligned(sz_f16x2, 4) || !aligned(y_f16, 2)) return MP_ERR_ALIGNMENT;
+    const int rc = launch_decode_umma(x_f16, packed_i32, sz_f16x2, bias_f16, y_f16, M, N, K, group, workspace,
+                                      workspace_bytes, static_cast<cudaStream_t>(stream), decode_programmatic_launch());
+    if (rc != MP_ERR_UNSUPPORTED) return rc;                     // (no workspace, odd alignment: the others)
+  }
+  if (M <= 16)
+    return decode_linear(x_f16, packed_i32, sz_f16x2, bias_f16, y_f16, M, N, K, group, workspace, workspace_bytes, 0,
+                         MP_DECODE_KERNEL_MMA_SYNC, -1, stream);
+  const bool scratch = workspace && workspace_bytes > kPartialOffset;
+  return mp_w4a16_linear_prefill_ex(x_f16, packed_i32, sz_f16x2, bias_f16, y_f16, M, N, K, group,
+                                    scratch ? static_cast<unsigned char*>(workspace) + kPartialOffset : nullptr,
+                                    scratch ? workspace_bytes - kPartialOffset : 0, error_word, stream);
 }
 
 extern "C" int mp_w4a16_decode_kernel_choice(int M, int N, int K, int have_workspace) {

@@ -1,48 +1,46 @@
-// W4A16 decode linear (M <= 16; 17..64 rows with a wider activation tile) on the tcgen05
-// tensor core with the weights as the TENSOR-MEMORY operand: y = x @ dequant(W)^T.
+// W4A16 linear for up to 64 rows on the tcgen05 tensor core with the weights as the TENSOR-MEMORY operand:
+// y = x @ dequant(W)^T, the packed weights streamed once.
 //
-// A thread owns ONE weight row: it reads 16 bytes (32 codes) of its row from
-// the shared-memory ring, expands them with dequant8 -- exactly
-// f16((u - z) * s) -- and stores the 16 packed registers straight into tensor
-// memory (tcgen05.st, lane = row, column = pair of K).  One elected thread then
-// issues tcgen05.mma kind::f16 with A = those TMEM columns (128 rows x 16 K per
-// instruction), B = the activation tile in shared memory (16 token rows,
-// K-major, 128-byte swizzle) and the fp32 accumulator [128 rows x 16 tokens] in
-// TMEM.  No dequantised weight touches shared or global memory and no dequant
-// warp issues an MMA, shuffles a fragment or touches an activation.
+// A thread owns ONE weight row: it reads 16 bytes (32 codes) of its row from the shared-memory ring, expands them and
+// stores the packed registers straight into tensor memory (tcgen05.st, lane = row, column = pair of K).  One elected
+// thread then issues tcgen05.mma kind::f16 with A = those TMEM columns (128 rows x 16 K per instruction), B = the
+// activation tile in shared memory (token rows, K-major, 128-byte swizzle) and the fp32 accumulator [128 rows x tokens]
+// in TMEM.  No dequantised weight touches shared or global memory, and no dequant warp issues an MMA, shuffles a fragment
+// or touches an activation.
 //
-// Work is cut stream-K style: the (row block, 256-column stage) pairs, row
-// block major, form one sequence that is divided evenly over a PERSISTENT grid
-// of about two blocks per SM, so every SM streams the same number of bytes
-// whatever the shape, the ring never drains between row blocks, and block
-// start-up is paid once per launch.  A block's range crosses at most a few row
-// blocks; for each it owns a "segment".  A segment that covers the whole K of
-// its row block is written to y directly; otherwise its fp32 tile goes to the
-// caller's workspace and the last segment of the row block to arrive (device
-// counter) adds the tiles in block order -- a fixed order, so results are
-// identical from run to run -- adds the bias and writes fp16.
+// What bounds it (clocks per 16 KB stage of weights and SM; HBM delivers one in about 700):
+//   expansion   exact f16((u - z) * s): 660 (thirteen instructions per eight weights, most of them half rate);
+//               FOLD, the exact integers u - z with the group's scale applied to its dot product: 460
+//   MMA         16 instructions of N / 2 clocks (operand A in tensor memory): 154 at 16 tokens, 517 at 64
+//   producer    one thread per stream, about 200 clocks per iteration plus 60 per TMA instruction: weights and
+//               activations have a thread each and no division in their loops (with both streams in one thread, seven
+//               TMA instructions and two divisions per stage, this thread was what held the kernel at 0.45 of HBM)
+// so every role has its own warps and its own barriers, and none waits for another that is not its input.
 //
-//   warps 0-7   dequant: warp w serves TMEM lanes [32 (w & 3), +32) and the
-//               (w >> 2)-th 128-column half of every 256-column stage; warps
-//               0-3 also run the segment epilogues
-//   warp 8      TMA producer (packed weights, (scale, zero) pairs, activations)
-//   warp 9      TMEM allocation and the MMA issuer
-//   warp 10     activation permuter: dequant8 emits the columns of a packed
-//               word in the order (k0,k4,k1,k5,k2,k6,k3,k7); the same
-//               permutation is applied in place to every 16-byte chunk of the
-//               activation tile (a chunk is one token's eight columns of one
-//               packed word, so the swizzle does not matter), off the dequant
-//               warps' critical path
-// TMEM (256 columns per block, two blocks per SM): accumulator at columns
-// [0,TOK); three 64-column A slots (128 K each) after it, used round robin by the
-// "units" (stage, half) in issue order.  TOK = 16, 32 or 64 token rows (the UMMA N):
-// the wider tiles serve 17..64 rows with the weights still streamed once; their
-// activation tile is 16 / 32 KB per stage, so the ring is 3 / 2 stages deep, and an
-// MMA costs about 110 / 135 / 190 clocks at N = 16 / 32 / 64 (measured end to end on
-// 28672x8192), which is why 32 rows cost 1.2x and 64 rows 1.9x the time of 16.  One accumulator is enough: the first MMA of a
-// segment needs weights from warps 0-3, which they store only after they have
-// read the previous segment's accumulator.
-// Every mbarrier wait is bounded.
+// FOLD (up to 16 rows, groups of a multiple of 128 columns): the accumulator of every 128-column unit is read back by
+// the epilogue warps, which add scale * dot to fp32 registers: more accurate than the fp16-rounded f16((u - z) * s) and
+// three instructions per eight weights cheaper.  Otherwise (more rows, shorter groups) the exact form accumulates in TMEM.
+//
+// Work is cut stream-K style: the (row block, 256-column stage) pairs form one sequence divided evenly over a persistent
+// grid of one block per SM.  A block walks its range BACKWARDS.  Of the row blocks in its range only the first it meets
+// can continue in later blocks: that part's fp32 tile goes to the block's slot in the workspace.  Any other row block ends
+// inside the range, and the block that holds a row block's end adds the tiles of the earlier blocks and writes y.  So a
+// block waits only for blocks of lower number, which wrote their tile at the beginning of their range, and adds in block
+// order (results are identical from run to run).  A tile word is stored inverted and zero means "not there yet": the
+// reader polls the words themselves (bounded) and puts the zeros back, with no fence, counter or second round trip.
+//
+//   warps 0-11   expansion: three sets of four; set j takes units j, j + 3, ... and owns TMEM slot j
+//   warps 12-15  epilogue
+//   warp 16      TMA producer of weights and (scale, zero) pairs
+//   warp 17      TMEM allocation and the MMA issuer
+//   warp 18      TMA producer of activations
+// Expansion emits the columns of a packed word in the order (k0,k4,k1,k5,k2,k6,k3,k7).  The threads of a unit apply the
+// same permutation in place to the 16-byte chunks of the unit's activation tile (a chunk is one token's eight columns of
+// one word, so the swizzle does not matter): two chunks each at 16 tokens.  (Warps of their own for this were starved
+// by the expansion warps: 2100 clocks per stage with one.)
+// Up to 16 rows a block takes less than half an SM (shared memory, registers, 256 TMEM columns), so that in a chain of
+// linears the next one's blocks start, and with the caller's leave fetch weights, beside the ones that finish.
+// Every wait is bounded.
 #include "common.cuh"
 #include "tc.cuh"
 
@@ -53,33 +51,57 @@ using namespace tc;
 namespace du {
 constexpr int kRows = 128;
 constexpr int kStageK = 256;
-constexpr int kDequantWarps = 8;
-constexpr int kProducerWarp = 8, kMmaWarp = 9, kPermuteWarp = 10;
-constexpr int kThreads = 11 * 32;
-constexpr int kWBytes = kRows * (kStageK / 2);       // 16384
-// TOK = token rows of the activation tile = UMMA N: 16, 32 or 64
-__host__ __device__ constexpr int x_sub(int tok) { return tok * 128; }        // [TOK tokens x 64 columns] fp16
-__host__ __device__ constexpr int x_bytes(int tok) { return 4 * x_sub(tok); }
-constexpr int kMaxStages = 4;
-constexpr int kBars = 3 * kMaxStages + 7;
-constexpr size_t kSmemBlockMax = 113 * 1024;         // two blocks per SM
-__host__ __device__ constexpr int stage_bytes(int tok, int groups_per_stage) {   // ring stride, a multiple of 1024
-  return kWBytes + x_bytes(tok) + ((groups_per_stage * kRows * 4 + 1023) & ~1023);
+constexpr int kSets = 2;                              // expansion sets of eight warps, a stage each in turn
+constexpr int kSlots = 3;                             // stages between expansion and MMA: stage i is in slot i % 3
+constexpr int kEpiWarp0 = 8 * kSets;
+constexpr int kWeightWarp = kEpiWarp0 + 4, kMmaWarp = kWeightWarp + 1, kXWarp = kMmaWarp + 1;
+constexpr int kThreads = 32 * (kXWarp + 1);
+constexpr int kWBytes = kRows * (kStageK / 2);        // 16384
+constexpr int kMaxRing = 10, kMaxXRing = 8;
+constexpr uint32_t kTmemCols = 512;
+constexpr uint32_t kASlotCols = 128;                  // 256 columns of K, two per 32-bit register
+constexpr size_t kSmemMax = 224 * 1024;
+
+// TOK: token rows of the MMA (its N); XROWS: token rows of the activation tile in shared memory (8 where no more exist:
+// the MMA then reads whatever follows for the other eight, whose results are not used)
+template <int TOK, int XROWS, bool FOLD>
+struct Cfg {
+  // who puts the activations into the order of expanded words: the expansion warps, in shared memory, or (PERM false) a
+  // small kernel before this one
+  static constexpr bool PERM = TOK <= 32;
+  static constexpr int kXSub = XROWS * 128;           // [XROWS x 64 columns] fp16
+  static constexpr int kXBytes = (PERM ? 4 : 2) * kXSub;        // a tile of the ring: a stage, or half of one
+  // activation tiles in flight: enough to hide the latency of their loads behind the stages before (with one per slot the
+  // expansion warps waited half their time); with PERM at most six, see the wait for a slot
+  static constexpr int kXRing = TOK == 16 ? 6 : TOK == 32 ? 4 : TOK == 64 ? 6 : 4;
+  // accumulators: FOLD two per slot (one for each 128 columns), else one per segment in turn
+  static constexpr int kAccs = FOLD ? 2 * kSlots : TOK > 64 ? 1 : 2;
+  static constexpr uint32_t kASlot0 = kAccs * TOK;
+  static_assert(kASlot0 + kSlots * kASlotCols <= kTmemCols, "tensor memory");
+};
+__host__ __device__ constexpr int sz_bytes(int groups_per_stage) { return (groups_per_stage * kRows * 4 + 1023) & ~1023; }
+constexpr int kBars = 2 * kMaxRing + 2 * kMaxXRing + 2 * kSlots + 4;
+constexpr int kScaleWords = kSlots * 2 * 2 * kRows;   // [slot][use parity][half][row]
+constexpr int kTailBytes = kBars * 8 + kScaleWords * 4 + 64;
+constexpr int kMaxGrid = kSmCount;
+// The least stages a block is given.  More blocks per row block shorten the stream but lengthen the closing step, which
+// reads a tile per block: at b stages per block a row block of ST stages takes about b stages + ST / b tiles, so b is the
+// root of ST times the cost of a tile in stages (0.4 at 16 tokens to 1 at 128; 1024x8192 at 16 tokens: 7.0 us with b = 2,
+// 6.3 with 4).
+inline int min_share(int stages_per_row, int tok) {
+  const int tile_cost_x10 = tok == 16 ? 4 : tok == 32 ? 5 : tok == 64 ? 7 : tok == 96 ? 9 : 10;
+  int b = 2;
+  while (b * b * 10 < stages_per_row * tile_cost_x10) ++b;
+  return b;
 }
-__host__ __device__ constexpr size_t smem_bytes(int tok, int stages, int groups_per_stage) {
-  return 1024 + (size_t)stages * stage_bytes(tok, groups_per_stage) + kBars * 8 + 64;
+__host__ __device__ constexpr int tokens_for(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 96 ? 96 : 128; }
+// workspace: the other kernels' arrival counters | one tile per block | activations in expansion order (M > 32)
+constexpr size_t kTileOffset = kW4CounterBytes;
+constexpr size_t kXOffset = kTileOffset + kW4TileBytes;
+static_assert(kW4TileBytes >= (size_t)kMaxGrid * 128 * kRows * sizeof(uint32_t), "tiles");
+inline size_t workspace_bytes(int M, int K) {
+  return M <= 32 ? kTileOffset + (size_t)kMaxGrid * (M <= 16 ? 16 : 32) * kRows * sizeof(uint32_t) : kXOffset + (size_t)M * K * 2;
 }
-constexpr uint32_t kTmemCols = 256;
-constexpr uint32_t kASlotCols = 64;                  // three A slots (128 K each) after the accumulator columns
-__host__ __device__ constexpr uint32_t a_slot0(int tok) { return tok <= 32 ? 32u : 64u; }
-constexpr int kASlots = 3;
-constexpr int kMaxBlocks = 2 * kSmCount;
-constexpr size_t kCounterBytes = 16384;              // one arrival counter per row block (<= 4096 of them)
-__host__ __device__ constexpr size_t tile_floats(int tok) { return (size_t)tok * kRows; }
-__host__ __device__ constexpr size_t workspace_bytes(int tok) {
-  return kCounterBytes + (size_t)kMaxBlocks * 2 * tile_floats(tok) * sizeof(float);
-}
-__host__ __device__ constexpr int tokens_for(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
 }  // namespace du
 
 struct DecodeUmmaParams {
@@ -87,22 +109,21 @@ struct DecodeUmmaParams {
   __half* y;
   int M, N, K, group;
   int stages_per_row;      // ST = ceil(K / 256)
-  int total;               // row blocks x ST
+  int share, extra;        // stages per block: share, one more for the first `extra` blocks
   int groups_per_stage;    // rows of the (scale, zero) box
+  int gshift;              // log2(group) for groups of up to 128 columns
+  int ring;                // weight stages in the ring
   int early_weights;       // 1: fetch weights before the previous kernel of the stream has finished
-  int gshift;              // log2(group) for groups shorter than 128 columns
-  int* counters;           // workspace: [row blocks], zero between calls
-  float* tiles;            // workspace: [grid][2][TOK][128] fp32 partial tiles
+  uint32_t* tiles;         // workspace: [grid][TOK][128] inverted fp32 words, zero between calls
   int* error_word;
 };
 
-// the stage range of block b in a grid of g blocks: [range_start(b), range_start(b + 1))
-__device__ __forceinline__ int range_start(int b, int g, int total) {
-  return static_cast<int>((static_cast<long long>(b) * total) / g);
-}
+// The stage range of block b is [range_start(b), range_start(b + 1)): p.share stages each, one more for the first p.extra.
+__device__ __forceinline__ int range_start(int b, const DecodeUmmaParams& p) { return b * p.share + min(b, p.extra); }
 // the block whose range holds stage t
-__device__ __forceinline__ int block_of(int t, int g, int total) {
-  return static_cast<int>(((static_cast<long long>(t) + 1) * g - 1) / total);
+__device__ __forceinline__ int block_of(int t, const DecodeUmmaParams& p) {
+  const int longer = p.extra * (p.share + 1);
+  return t < longer ? t / (p.share + 1) : p.extra + (t - longer) / p.share;
 }
 
 __device__ __forceinline__ void tmem_st_32x32_x16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -115,7 +136,7 @@ __device__ __forceinline__ void tmem_st_32x32_x16(uint32_t taddr, const uint32_t
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-__device__ __forceinline__ void tmem_ld_32x32_x16(uint32_t taddr, uint32_t (&r)[16]) {
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -123,6 +144,12 @@ __device__ __forceinline__ void tmem_ld_32x32_x16(uint32_t taddr, uint32_t (&r)[
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
+}
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
 }
 
 // D[tmem] (+)= A[tmem] * B[smem]: the A operand is read from tensor memory (lane = row, one 32-bit
@@ -137,30 +164,37 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
       : "memory");
 }
 
-// Ring accesses by 32-bit shared-window address (the 1 KB-aligned ring pointer hides the address space from the
+// Shared-memory accesses by 32-bit shared-window address (the 1 KB-aligned ring pointer hides the address space from the
 // compiler; plain dereferences of it are generic loads and stores).
 __device__ __forceinline__ uint4 du_lds_v4(uint32_t addr) {
-  uint4 v;
-  asm("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-  return v;
-}
-// volatile instead of a memory clobber: keeps its place among the other volatile statements (barrier waits,
-// stores) without being a compiler barrier between neighbouring loads
-__device__ __forceinline__ uint4 du_lds_v4_ordered(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
   return v;
 }
 __device__ __forceinline__ uint32_t du_lds_u32(uint32_t addr) {
   uint32_t v;
-  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
   return v;
 }
 __device__ __forceinline__ void du_sts_v4(uint32_t addr, const uint4& v) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w));
 }
+__device__ __forceinline__ void du_sts_u32(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v));
+}
+__device__ __forceinline__ uint4 ld_relaxed_gpu_v4(const uint32_t* p) {
+  uint4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed_gpu_v4_zero(uint32_t* p) {
+  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1,%1,%1,%1};" ::"l"(p), "r"(0u) : "memory");
+}
+__device__ __forceinline__ void st_relaxed_gpu(uint32_t* p, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 
-// eight fp16 values (k0..k7) -> (k0,k4,k1,k5,k2,k6,k3,k7), the column order dequant8 emits
+// eight fp16 values (k0..k7) -> (k0,k4,k1,k5,k2,k6,k3,k7), the column order of an expanded word
 __device__ __forceinline__ uint4 pair_permute_u4(const uint4 in) {
   uint4 v;
   v.x = prmt(in.x, in.z, 0x5410);
@@ -170,287 +204,397 @@ __device__ __forceinline__ uint4 pair_permute_u4(const uint4 in) {
   return v;
 }
 
-template <int STAGES, int TOK>
-__global__ void __launch_bounds__(du::kThreads, 2)
+// One packed word -> the exact fp16 integers u - z of its eight columns, in dequant8's order.  zl = 1024 + z and
+// zh = 64 + z: the even nibbles are planted in the mantissa of 1024 (step 1), the odd ones, left in place, in that of
+// 64 (step 1/16), so both differences are exact.
+__device__ __forceinline__ void expand8(uint32_t q, __half2 zl, __half2 zh, uint32_t* v) {
+  const uint32_t q8 = q >> 8;
+  const uint32_t a = lop3_and_or(q, 0x000f000fu, 0x64006400u), b = lop3_and_or(q, 0x00f000f0u, 0x54005400u);
+  const uint32_t c = lop3_and_or(q8, 0x000f000fu, 0x64006400u), d = lop3_and_or(q8, 0x00f000f0u, 0x54005400u);
+  v[0] = h2_as_u32(__hsub2(*reinterpret_cast<const __half2*>(&a), zl));
+  v[1] = h2_as_u32(__hsub2(*reinterpret_cast<const __half2*>(&b), zh));
+  v[2] = h2_as_u32(__hsub2(*reinterpret_cast<const __half2*>(&c), zl));
+  v[3] = h2_as_u32(__hsub2(*reinterpret_cast<const __half2*>(&d), zh));
+}
+
+template <int TOK, int XROWS, bool FOLD>
+__global__ void __launch_bounds__(du::kThreads, 1)
 w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                          const __grid_constant__ CUtensorMap tmap_sz, const DecodeUmmaParams p) {
+  using C = du::Cfg<TOK, XROWS, FOLD>;
+  constexpr int kXSub = C::kXSub, kXBytes = C::kXBytes, kXRing = C::kXRing;
+  constexpr bool PERM = C::PERM;
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  constexpr int kXSub = du::x_sub(TOK), kXBytes = du::x_bytes(TOK);
-  constexpr uint32_t kASlot0 = du::a_slot0(TOK);
-  const int stage_bytes = du::stage_bytes(TOK, p.groups_per_stage);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ring + STAGES * stage_bytes);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + du::kBars);
+  // activation ring | weight ring | barriers, scales, flags
+  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int stage_bytes = du::kWBytes + du::sz_bytes(p.groups_per_stage);
+  unsigned char* tail = base + kXRing * kXBytes + p.ring * stage_bytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(tail);
+  uint32_t* s_scale = reinterpret_cast<uint32_t*>(bars + du::kBars);
+  uint32_t* tmem_slot = s_scale + du::kScaleWords;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile int* epi_word = reinterpret_cast<volatile int*>(tmem_slot + 2);   // [last?, first block, last block]
-  const uint32_t full0 = smem_u32(bars);                      // stage landed (TMA bytes)
-  const uint32_t empty0 = full0 + 8 * du::kMaxStages;         // stage may be overwritten
-  const uint32_t xp0 = empty0 + 8 * du::kMaxStages;           // stage's activations are permuted
-  const uint32_t afull0 = xp0 + 8 * du::kMaxStages;           // A slot holds a unit's dequantised weights
-  const uint32_t aempty0 = afull0 + 8 * du::kASlots;          // A slot has been read by its MMAs
-  const uint32_t dfull = aempty0 + 8 * du::kASlots;           // a segment's accumulator is final
+  const uint32_t xring = smem_u32(base), wring = xring + kXRing * kXBytes;
+  const uint32_t full0 = smem_u32(bars);                      // a stage's weights (PERM: and activations) landed
+  const uint32_t empty0 = full0 + 8 * du::kMaxRing;           // its weights have been read
+  const uint32_t xempty0 = empty0 + 8 * du::kMaxRing;         // activation tile has been read
+  const uint32_t xfull0 = xempty0 + 8 * du::kMaxXRing;        // not PERM: activation tile landed
+  const uint32_t ready0 = xfull0 + 8 * du::kMaxXRing;         // slot holds an expanded stage (FOLD: and its accumulators are free)
+  const uint32_t done0 = ready0 + 8 * du::kSlots;             // its MMAs are complete
+  const uint32_t dfull0 = done0 + 8 * du::kSlots;             // not FOLD: a segment's accumulator is complete
+  const uint32_t dempty0 = dfull0 + 16;                       // ... and has been read
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full0 + 8 * s, 1);
-      mbar_init(empty0 + 8 * s, du::kDequantWarps + 1);       // eight dequant warps + the MMAs' commit
-      mbar_init(xp0 + 8 * s, 1);
+  const int blk = static_cast<int>(blockIdx.x);
+  const int ST = p.stages_per_row;
+  const int t_lo = range_start(blk, p), t_hi = range_start(blk + 1, p) - 1;   // walked from t_hi down
+  const int n_stages = t_hi - t_lo + 1;
+
+  // weight producer: the stage it is at (its first loads are issued before the block is set up)
+  int w_row = 0, w_st = 0;
+  auto load_weights = [&](int s) {
+    const uint32_t full = full0 + 8 * s, dst = wring + s * stage_bytes;
+    mbar_arrive_expect_tx(full, du::kWBytes + p.groups_per_stage * du::kRows * 4);
+    tma_load_2d(dst, &tmap_w, full, w_st * (du::kStageK / 2), w_row);
+    const int group = p.group <= du::kStageK ? w_st * p.groups_per_stage : (w_st * du::kStageK) / p.group;
+    tma_load_2d(dst + du::kWBytes, &tmap_sz, full, w_row, group);
+    if (--w_st < 0) { w_st = ST - 1; w_row -= du::kRows; }
+  };
+  if (warp == du::kWeightWarp) {
+    if (elect_one()) {
+      for (int s = 0; s < p.ring; ++s) {
+        mbar_init(full0 + 8 * s, PERM ? 2 : 1);               // the producers
+        mbar_init(empty0 + 8 * s, 8);
+      }
+      fence_mbar_init();
+      w_row = (t_hi / ST) * du::kRows;
+      w_st = t_hi % ST;
+      if (!p.early_weights) chain_wait();
+      for (int s = 0; s < p.ring && s < n_stages; ++s) load_weights(s);
     }
-    for (int q = 0; q < du::kASlots; ++q) {
-      mbar_init(afull0 + 8 * q, 4);                           // the four warps of one half
-      mbar_init(aempty0 + 8 * q, 1);
+  } else if (warp == du::kXWarp) {
+    if (elect_one()) {
+      prefetch_tensormap(&tmap_x);
+      for (int s = 0; s < kXRing; ++s) {
+        mbar_init(xempty0 + 8 * s, 1);
+        mbar_init(xfull0 + 8 * s, 1);
+      }
+      for (int q = 0; q < du::kSlots; ++q) {
+        mbar_init(ready0 + 8 * q, FOLD ? 12 : 8);
+        mbar_init(done0 + 8 * q, 1);
+      }
+      for (int d = 0; d < 2; ++d) {
+        mbar_init(dfull0 + 8 * d, 1);
+        mbar_init(dempty0 + 8 * d, 4);
+      }
+      *abort_flag = 0;
+      fence_mbar_init();
     }
-    mbar_init(dfull, 1);
-    *abort_flag = 0;
-    fence_mbar_init();
-  }
-  if (warp == du::kMmaWarp) {
+  } else if (warp == du::kMmaWarp) {
     tmem_alloc(smem_u32(tmem_slot), du::kTmemCols);
     tmem_relinquish();
   }
+  __syncwarp();
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const int grid = static_cast<int>(gridDim.x), blk = static_cast<int>(blockIdx.x);
-  const int ST = p.stages_per_row;
-  const int t0 = range_start(blk, grid, p.total);
-  const int n_stages = range_start(blk + 1, grid, p.total) - t0;
-
-  if (warp == du::kProducerWarp) {
-    // ------------------------------------------------------------ TMA producer
+  if (warp == du::kWeightWarp) {
+    // ------------------------------------------------------------ TMA producer: weights
     if (elect_one()) {
-      prefetch_tensormap(&tmap_w);
-      prefetch_tensormap(&tmap_x);
-      prefetch_tensormap(&tmap_sz);
-      const uint32_t tx_bytes = du::kWBytes + kXBytes + p.groups_per_stage * du::kRows * 4;
-      auto issue_weights = [&](int i) {
-        const int s = i % STAGES;
-        const int t = t0 + i, rb = t / ST, st = t - rb * ST;
-        const uint32_t full = full0 + 8 * s;
-        unsigned char* base = ring + s * stage_bytes;
-        mbar_arrive_expect_tx(full, tx_bytes);
-        tma_load_2d(smem_u32(base), &tmap_w, full, st * (du::kStageK / 2), rb * du::kRows);
-        tma_load_2d(smem_u32(base + du::kWBytes + kXBytes), &tmap_sz, full, rb * du::kRows,
-                    (st * du::kStageK) / p.group);
-      };
-      auto issue_x = [&](int i) {
-        const int s = i % STAGES;
-        const int t = t0 + i, st = t % ST;
-        const uint32_t full = full0 + 8 * s;
-        unsigned char* xb = ring + s * stage_bytes + du::kWBytes;
+      int s = 0;
+      uint32_t phase = 0;
+      for (int i = p.ring; i < n_stages; ++i) {
+        if (!mbar_wait(empty0 + 8 * s, phase, abort_flag)) break;
+        load_weights(s);
+        if (++s == p.ring) { s = 0; phase ^= 1; }
+      }
+      chain_release();             // all of this block's loads are issued: the next kernel's blocks may start
+    }
+  } else if (warp == du::kXWarp) {
+    // ------------------------------------------------------------ TMA producer: activations
+    if (elect_one()) {
+      chain_wait();
+      int st = t_hi % ST, s = 0, xs = 0;
+      uint32_t phase = 1;
+      bool ok = true;
+      for (int i = 0; ok && i < n_stages; ++i) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) tma_load_2d(smem_u32(xb + j * kXSub), &tmap_x, full, st * du::kStageK + j * 64, 0);
-      };
-      const int prologue = min(n_stages, STAGES);
-      asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-      if (!p.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
-      for (int i = 0; i < prologue; ++i) issue_weights(i);
-      if (p.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
-      for (int i = 0; i < prologue; ++i) issue_x(i);
-      for (int i = prologue; i < n_stages; ++i) {
-        const int s = i % STAGES;
-        const uint32_t phase = ((i / STAGES) & 1) ^ 1;
-        if (!mbar_wait_sleep(empty0 + 8 * s, phase, abort_flag, 400)) break;
-        issue_weights(i);
-        issue_x(i);
+        for (int h = 0; h < (PERM ? 1 : 2); ++h) {
+          if (!mbar_wait(xempty0 + 8 * xs, phase, abort_flag)) { ok = false; break; }
+          const uint32_t bar = PERM ? full0 + 8 * s : xfull0 + 8 * xs;
+          mbar_arrive_expect_tx(bar, kXBytes);
+          tma_load_3d(xring + xs * kXBytes, &tmap_x, bar, 0, 0, st * (du::kStageK / 64) + h * 2);
+          if (++xs == kXRing) { xs = 0; phase ^= 1; }
+        }
+        if (--st < 0) st = ST - 1;
+        if (++s == p.ring) s = 0;
       }
     }
   } else if (warp == du::kMmaWarp) {
-    // ------------------------------------------------------------ MMA issuer
+    // ------------------------------------------------------------ MMA issuer: one wait, 16 MMAs, one commit per stage
     if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc(kIdescDFormatF32 | kIdescABFormatF16, du::kRows, TOK);
+      bool fresh = true;                                       // the next MMA starts a segment
+      int st = t_hi % ST, q = 0, xs = 0, d = 0;
+      uint32_t phase = 0, xphase = 0, dphase = 1;
       bool ok = true;
-      int st = t0 % ST;
-      bool seg_first = true;
-      for (int i = 0; ok && i < n_stages; ++i) {
-        const int s = i % STAGES;
-        const uint32_t phase = (i / STAGES) & 1;
-        const uint32_t xb = smem_u32(ring + s * stage_bytes + du::kWBytes);
-        const bool seg_last = st == ST - 1 || i == n_stages - 1;
+      const uint64_t b_desc0 = umma_desc_k_sw128(xring);
+      for (int i = 0; i < n_stages; ++i) {
+        if (!FOLD && fresh && !mbar_wait(dempty0 + 8 * d, dphase, abort_flag)) break;
+        if (!mbar_wait(ready0 + 8 * q, phase, abort_flag)) break;
+        tcgen05_fence_after();
+        const uint32_t a_tmem = tmem_base + C::kASlot0 + q * du::kASlotCols;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int u = 2 * i + h, q = u % du::kASlots;
-          const uint32_t aphase = (u / du::kASlots) & 1;
-          if (!mbar_wait_sleep(afull0 + 8 * q, aphase, abort_flag, 100)) { ok = false; break; }
-          if (h == 0 && !mbar_wait_sleep(xp0 + 8 * s, phase, abort_flag, 100)) { ok = false; break; }
-          tcgen05_fence_after();
-          const uint32_t a_tmem = tmem_base + kASlot0 + q * du::kASlotCols;
+          if (!PERM && !mbar_wait(xfull0 + 8 * xs, xphase, abort_flag)) { ok = false; break; }
+          const uint64_t b_desc = b_desc0 + ((xs * kXBytes + (PERM ? h * 2 * kXSub : 0)) >> 4);
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {     // 16 K per instruction: 8 TMEM columns of A, 32 bytes of B's rows
-            const uint64_t b_desc = umma_desc_k_sw128(xb + (h * 2 + (kk >> 2)) * kXSub) + 2 * (kk & 3);
-            umma_f16_ts(tmem_base, a_tmem + kk * 8, b_desc, idesc, !(seg_first && h == 0 && kk == 0));
+            const uint32_t d_tmem = tmem_base + (FOLD ? 2 * q + h : d) * TOK;
+            umma_f16_ts(d_tmem, a_tmem + (h * 8 + kk) * 8, b_desc + ((kk >> 2) * kXSub >> 4) + 2 * (kk & 3), idesc,
+                        FOLD ? kk != 0 : !(fresh && h == 0 && kk == 0));
           }
-          umma_commit(aempty0 + 8 * q);
-          if (h == 1) {
-            umma_commit(empty0 + 8 * s);                        // the stage's activations have been read
-            if (seg_last) umma_commit(dfull);
+          if (!PERM || h == 1) {
+            umma_commit(xempty0 + 8 * xs);
+            if (++xs == kXRing) { xs = 0; xphase ^= 1; }
           }
         }
-        seg_first = seg_last;
-        if (++st == ST) st = 0;
+        if (!ok) break;
+        umma_commit(done0 + 8 * q);
+        fresh = st == 0;
+        if (!FOLD && (fresh || i == n_stages - 1)) {
+          umma_commit(dfull0 + 8 * d);
+          if (++d == C::kAccs) { d = 0; dphase ^= 1; }
+        }
+        if (--st < 0) st = ST - 1;
+        if (++q == du::kSlots) { q = 0; phase ^= 1; }
       }
     }
-  } else if (warp == du::kPermuteWarp) {
-    // ------------------------------------------------------------ activation permuter
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int i = 0; i < n_stages; ++i) {
-      const int s = i % STAGES;
-      const uint32_t phase = (i / STAGES) & 1;
-      if (!__all_sync(0xffffffffu, mbar_wait_sleep(full0 + 8 * s, phase, abort_flag, 400))) break;
-      const uint32_t xt = smem_u32(ring + s * stage_bytes + du::kWBytes);
-      // four chunks per lane in flight: the loads are issued together, then permuted and stored
-      for (int c = lane; c < kXBytes / 16; c += 128) {
-        uint4 v[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = du_lds_v4_ordered(xt + (c + 32 * j) * 16);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) du_sts_v4(xt + (c + 32 * j) * 16, pair_permute_u4(v[j]));
-      }
-      fence_proxy_async_smem();                                // generic-proxy stores -> visible to the MMA's reads
-      __syncwarp();
-      if (lane == 0) mbar_arrive(xp0 + 8 * s);
-    }
-  } else {
-    // ------------------------------------------------------------ dequant warps (+ epilogues on warps 0-3)
-    const int quarter = warp & 3, kh = warp >> 2;
-    const int row = quarter * 32 + lane;
-    const uint32_t lane_field = static_cast<uint32_t>(quarter * 32) << 16;
-    const int sw = row & 7;
-    const bool short_groups = p.group < 128;
-    const int grp0 = p.groups_per_stage > 1 ? (kh * 128) / p.group : 0;
-    int w_off[4];                                  // this row's four 16-byte chunks of its half (128-byte swizzle)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) w_off[j] = row * 128 + (((kh * 4 + j) ^ sw) << 4);
-    const int sz_off = du::kWBytes + kXBytes + row * 4;
-    const uint32_t ring_addr = smem_u32(ring);
-    int rb = t0 / ST, st = t0 - rb * ST;
-    int seg_begin_i = 0, seg_begin_st = st, seg_idx = 0;
-    for (int i = 0; i < n_stages; ++i) {
-      const int s = i % STAGES;
-      const uint32_t phase = (i / STAGES) & 1;
+  } else if (warp < du::kEpiWarp0) {
+    // ------------------------------------------------------------ expansion: a warp does 32 rows of half a stage
+    const int quarter = warp & 3, h = (warp >> 2) & 1, set = warp >> 3;
+    const int row = quarter * 32 + lane, sw = row & 7;
+    const uint32_t a_tmem0 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::kASlot0 + h * (du::kASlotCols / 2);
+    int s = set, xs = set, q = set;
+    uint32_t phase = 0, qphase = 1, parity = 0;
+    for (int i = set; i < n_stages; i += du::kSets) {
       if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, phase, abort_flag))) break;
-      const uint32_t base = ring_addr + s * stage_bytes;
+      const uint32_t stage = wring + s * stage_bytes + row * 128, sz = wring + s * stage_bytes + du::kWBytes + row * 4;
       uint4 q4[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) q4[j] = du_lds_v4(base + w_off[j]);
-      ScaleZero sp;
-      {
-        const uint32_t szw = du_lds_u32(base + sz_off + grp0 * (du::kRows * 4));
-        const __half2 h = *reinterpret_cast<const __half2*>(&szw);
-        sp = make_scale_zero(__low2half(h), __high2half(h));
+      for (int j = 0; j < 4; ++j) q4[j] = du_lds_v4(stage + (((h * 4 + j) ^ sw) << 4));
+      uint32_t szw[FOLD ? 1 : 4];
+      if constexpr (FOLD) {
+        szw[0] = du_lds_u32(sz + (p.groups_per_stage > 1 ? h * (du::kRows * 4) : 0));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          szw[j] = du_lds_u32(sz + (p.groups_per_stage > 1 ? ((h * 128 + j * 32) >> p.gshift) * (du::kRows * 4) : 0));
       }
-      const int u = 2 * i + kh, q = u % du::kASlots;
-      const uint32_t aphase = ((u / du::kASlots) & 1) ^ 1;
-      const uint32_t a_tmem = tmem_base + lane_field + kASlot0 + q * du::kASlotCols;
-      // (waiting for the slot here, before the expansion, measured 8 % faster at 16 tokens than waiting
-      // just before the first store)
-      if (!__all_sync(0xffffffffu, mbar_wait(aempty0 + 8 * q, aphase, abort_flag))) break;
+      // (the slot's use before its last one is over: the activations of stage i were requested after the MMAs of stage
+      // i - kXRing >= i - 6, so the parity is not ambiguous)
+      if (!__all_sync(0xffffffffu, mbar_wait(done0 + 8 * q, qphase, abort_flag))) break;
+      mbar_arrive_warp(empty0 + 8 * s, lane);
       tcgen05_fence_after();
+      const uint32_t a_tmem = a_tmem0 + q * du::kASlotCols;
+      if constexpr (FOLD) {
+        du_sts_u32(smem_u32(s_scale + ((q * 2 + parity) * 2 + h) * du::kRows + row), szw[0]);
+        const __half2 z2 = __high2half2(*reinterpret_cast<const __half2*>(&szw[0]));
+        const __half2 zl = __hadd2(z2, __float2half2_rn(1024.0f)), zh = __hadd2(z2, __float2half2_rn(64.0f));
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (j > 0 && short_groups && ((j * 32) & (p.group - 1)) == 0) {   // groups of 32 or 64 columns: next (scale, zero)
-          const int grp = (kh * 128 + j * 32) >> p.gshift;
-          const uint32_t szw = du_lds_u32(base + sz_off + grp * (du::kRows * 4));
-          const __half2 h = *reinterpret_cast<const __half2*>(&szw);
-          sp = make_scale_zero(__low2half(h), __high2half(h));
+        for (int j = 0; j < 4; ++j) {
+          uint32_t r[16];
+          expand8(q4[j].x, zl, zh, r);
+          expand8(q4[j].y, zl, zh, r + 4);
+          expand8(q4[j].z, zl, zh, r + 8);
+          expand8(q4[j].w, zl, zh, r + 12);
+          tmem_st_32x32_x16(a_tmem + j * 16, r);
         }
-        uint32_t r[16];
+      } else {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const uint32_t word = c == 0 ? q4[j].x : c == 1 ? q4[j].y : c == 2 ? q4[j].z : q4[j].w;
-          __half2 v[4];
-          dequant8(word, sp, v);
+        for (int j = 0; j < 4; ++j) {
+          const __half2 szh = *reinterpret_cast<const __half2*>(&szw[j]);
+          const ScaleZero sp = make_scale_zero(__low2half(szh), __high2half(szh));
+          uint32_t r[16];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) r[4 * c + e] = h2_as_u32(v[e]);
+          for (int c = 0; c < 4; ++c) {
+            const uint32_t word = c == 0 ? q4[j].x : c == 1 ? q4[j].y : c == 2 ? q4[j].z : q4[j].w;
+            __half2 v[4];
+            dequant8(word, sp, v);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) r[4 * c + e] = h2_as_u32(v[e]);
+          }
+          tmem_st_32x32_x16(a_tmem + j * 16, r);
         }
-        tmem_st_32x32_x16(a_tmem + j * 16, r);
+      }
+      if constexpr (PERM) {
+        // this half's activations: chunks of XROWS tokens x 128 columns
+        const uint32_t xt = xring + xs * kXBytes + h * (2 * kXSub) + row * 16;
+#pragma unroll
+        for (int c0 = 0; c0 < 2 * kXSub; c0 += 4096) {
+          constexpr int kAtOnce = 2 * kXSub < 4096 ? kXSub / 1024 : 2;
+          uint4 v[kAtOnce];
+#pragma unroll
+          for (int j = 0; j < kAtOnce; ++j) v[j] = du_lds_v4(xt + c0 + j * 2048);
+#pragma unroll
+          for (int j = 0; j < kAtOnce; ++j) du_sts_v4(xt + c0 + j * 2048, pair_permute_u4(v[j]));
+        }
+        fence_proxy_async_smem();                                // generic-proxy stores -> visible to the MMA's reads
       }
       tmem_st_wait();
       tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(afull0 + 8 * q);
-        mbar_arrive(empty0 + 8 * s);
-      }
-      const bool seg_last = st == ST - 1 || i == n_stages - 1;
-      if (seg_last) {
-        if (kh == 0) {
-          // ---- segment epilogue: lane = weight row, column = token
-          if (!__all_sync(0xffffffffu, mbar_wait(dfull, seg_idx & 1, abort_flag))) break;
-          tcgen05_fence_after();
-          // 16 token columns at a time (more would not fit beside the dequant registers)
-          asm volatile("griddepcontrol.wait;" ::: "memory");   // before anything of the previous kernel is overwritten
-          const int n = rb * du::kRows + row;
-          const float bias = (p.bias && n < p.N) ? h2f(p.bias[n]) : 0.0f;
-          const bool whole = seg_begin_st == 0 && st == ST - 1;   // the whole K of this row block: final
-          const int which = seg_begin_i == 0 ? 0 : 1;              // a block has at most two partial segments
-          float* tile = p.tiles + ((size_t)blk * 2 + which) * du::tile_floats(TOK);
-#pragma unroll 1
-          for (int t0c = 0; t0c < TOK; t0c += 16) {
-            uint32_t acc[16];
-            tmem_ld_32x32_x16(tmem_base + lane_field + t0c, acc);
-            tmem_ld_wait();
-            if (whole) {
-              if (n < p.N) {
+      mbar_arrive_warp(ready0 + 8 * q, lane);
+      s += du::kSets;
+      if (s >= p.ring) { s -= p.ring; phase ^= 1; }
+      if (PERM && (xs += du::kSets) >= kXRing) xs -= kXRing;
+      q += du::kSets;
+      if (q >= du::kSlots) { q -= du::kSlots; qphase ^= 1; parity ^= 1; }
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue: lane = weight row, column = token
+    constexpr int CH = FOLD ? XROWS : 16;                      // tokens held at a time
+    const int quarter = warp & 3;
+    const int row = quarter * 32 + lane;
+    const uint32_t d_tmem = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    chain_wait();                                              // before anything of the previous kernel is overwritten
+    // v = a segment's sums for tokens [m0, m0 + CH): to y, to this block's tile, or to shared memory for the closing step
+    auto finish = [&](const float (&v)[CH], int m0, int rb, bool ends_row_block, bool whole) {
+      if (whole) {
+        const int n = rb * du::kRows + row;
+        if (n < p.N) {
+          const float bias = p.bias ? h2f(p.bias[n]) : 0.0f;
 #pragma unroll
-                for (int m = 0; m < 16; ++m)
-                  if (t0c + m < p.M) p.y[(size_t)(t0c + m) * p.N + n] = f2h(__uint_as_float(acc[m]) + bias);
-              }
-            } else {
-#pragma unroll
-              for (int m = 0; m < 16; ++m)
-                if (t0c + m < p.M) tile[(t0c + m) * du::kRows + row] = __uint_as_float(acc[m]);
-            }
-          }
-          if (!whole) {
-            __threadfence();
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (warp == 0 && lane == 0) {
-              const int fb = block_of(rb * ST, grid, p.total), lb = block_of(rb * ST + ST - 1, grid, p.total);
-              const int old = atomicAdd(p.counters + rb, 1);
-              const int last = old == lb - fb ? 1 : 0;
-              if (last) p.counters[rb] = 0;                    // re-armed for the next call
-              __threadfence();
-              epi_word[0] = last; epi_word[1] = fb; epi_word[2] = lb;
-            }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (epi_word[0]) {
-              const int fb = epi_word[1], lb = epi_word[2];
-#pragma unroll 1
-              for (int t0c = 0; t0c < TOK && t0c < p.M; t0c += 16) {
-                float sum[16];
-#pragma unroll
-                for (int m = 0; m < 16; ++m) sum[m] = 0.0f;
-                for (int b2 = fb; b2 <= lb; ++b2) {            // block order: deterministic
-                  const int w2 = range_start(b2, grid, p.total) >= rb * ST ? 0 : 1;
-                  const float* t2 = p.tiles + ((size_t)b2 * 2 + w2) * du::tile_floats(TOK) + row;
-#pragma unroll
-                  for (int m = 0; m < 16; ++m)
-                    if (t0c + m < p.M) sum[m] += __ldcg(t2 + (t0c + m) * du::kRows);
-                }
-                if (n < p.N) {
-#pragma unroll
-                  for (int m = 0; m < 16; ++m)
-                    if (t0c + m < p.M) p.y[(size_t)(t0c + m) * p.N + n] = f2h(sum[m] + bias);
-                }
-              }
-            }
-          }
-          tcgen05_fence_before();
+          for (int m = 0; m < CH; ++m)
+            if (m0 + m < p.M) p.y[(size_t)(m0 + m) * p.N + n] = f2h(v[m] + bias);
         }
-        ++seg_idx;
-        seg_begin_i = i + 1;
-        seg_begin_st = 0;
+      } else if (!ends_row_block) {
+        uint32_t* tile = p.tiles + ((size_t)blk * TOK + m0) * du::kRows + row;
+#pragma unroll
+        for (int m = 0; m < CH; ++m)
+          if (m0 + m < p.M) {
+            const uint32_t b = ~__float_as_uint(v[m]);
+            st_relaxed_gpu(tile + m * du::kRows, b == 0u ? 0x80000000u : b);     // (one NaN pattern becomes another)
+          }
+      } else {
+        // the block's last segment: every weight stage has been read, so the ring is free
+        const uint32_t own = wring + (m0 * du::kRows + row) * 4;
+#pragma unroll
+        for (int m = 0; m < CH; ++m)
+          if (m0 + m < p.M) du_sts_u32(own + m * du::kRows * 4, __float_as_uint(v[m]));
       }
-      if (++st == ST) { st = 0; ++rb; }
+    };
+    bool ok = true;
+    int q = 0;
+    uint32_t phase = 0;
+    if constexpr (FOLD) {
+      for (int i = 0; i < du::kSlots; ++i) mbar_arrive_warp(ready0 + 8 * i, lane);       // all accumulators are free
+    }
+    int rb = t_hi / ST, d = 0;
+    for (int t = t_hi; ok && t >= t_lo; --rb) {
+      const int row_first = rb * ST, lo = max(t_lo, row_first);
+      const bool ends = t == row_first + ST - 1, whole = ends && lo == row_first;
+      if constexpr (FOLD) {
+        float acc[CH];
+#pragma unroll
+        for (int m = 0; m < CH; ++m) acc[m] = 0.0f;
+        for (; t >= lo; --t) {
+          if (!__all_sync(0xffffffffu, mbar_wait(done0 + 8 * q, phase & 1, abort_flag))) { ok = false; break; }
+          tcgen05_fence_after();
+          uint32_t r0[CH], r1[CH];
+          tmem_ld_cols(d_tmem + 2 * q * TOK, r0);
+          tmem_ld_cols(d_tmem + (2 * q + 1) * TOK, r1);
+          const uint32_t sa = smem_u32(s_scale + ((q * 2 + (phase & 1)) * 2) * du::kRows + row);
+          const uint32_t sz0 = du_lds_u32(sa), sz1 = du_lds_u32(sa + du::kRows * 4);
+          tmem_ld_wait();
+          tcgen05_fence_before();
+          mbar_arrive_warp(ready0 + 8 * q, lane);
+          const float s0 = __low2float(*reinterpret_cast<const __half2*>(&sz0));
+          const float s1 = __low2float(*reinterpret_cast<const __half2*>(&sz1));
+#pragma unroll
+          for (int m = 0; m < CH; ++m)
+            acc[m] = fmaf(s1, __uint_as_float(r1[m]), fmaf(s0, __uint_as_float(r0[m]), acc[m]));
+          if (++q == du::kSlots) { q = 0; phase ^= 1; }
+        }
+        if (!ok) break;
+        finish(acc, 0, rb, ends, whole);
+      } else {
+        if (!__all_sync(0xffffffffu, mbar_wait(dfull0 + 8 * d, phase & 1, abort_flag))) break;
+        tcgen05_fence_after();
+#pragma unroll 1
+        for (int m0 = 0; m0 < TOK && m0 < p.M; m0 += 16) {
+          uint32_t r[CH];
+          tmem_ld_cols(d_tmem + d * TOK + m0, r);
+          tmem_ld_wait();
+          float v[CH];
+#pragma unroll
+          for (int m = 0; m < CH; ++m) v[m] = __uint_as_float(r[m]);
+          finish(v, m0, rb, ends, whole);
+          __syncwarp();
+        }
+        tcgen05_fence_before();
+        mbar_arrive_warp(dempty0 + 8 * d, lane);
+        if (++d == C::kAccs) { d = 0; phase ^= 1; }
+      }
+      t = lo - 1;
     }
   }
 
   tcgen05_fence_before();
   __syncthreads();
+  {
+    // The closing step, all threads: when the block's last segment ends a row block that earlier blocks began, add their
+    // tiles to this block's sums.  Four rows of a token per thread; the words of up to four blocks are requested together.
+    const int rb = t_lo / ST, row_first = rb * ST;
+    if (t_lo > row_first && t_hi >= row_first + ST - 1 && !*abort_flag) {
+      const int first_block = block_of(row_first, p);
+      for (int e = tid; e < p.M * (du::kRows / 4); e += du::kThreads) {
+        const int m = e / (du::kRows / 4), r4 = (e % (du::kRows / 4)) * 4;
+        const uint4 own = du_lds_v4(wring + (m * du::kRows + r4) * 4);
+        float v[4] = {__uint_as_float(own.x), __uint_as_float(own.y), __uint_as_float(own.z), __uint_as_float(own.w)};
+        uint32_t* tile = p.tiles + ((size_t)first_block * TOK + m) * du::kRows + r4;
+        for (int b2 = first_block; b2 < blk && !*abort_flag; b2 += 4, tile += (size_t)4 * TOK * du::kRows) {
+          uint4 w[4];
+          uint64_t since = 0;
+          for (uint32_t it = 1;; ++it) {
+            bool there = true;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              w[j] = b2 + j < blk ? ld_relaxed_gpu_v4(tile + (size_t)j * TOK * du::kRows) : make_uint4(1u, 1u, 1u, 1u);
+              there = there && w[j].x != 0u && w[j].y != 0u && w[j].z != 0u && w[j].w != 0u;
+            }
+            if (there) break;
+            if ((it & 0x3F) == 0) {
+              const uint64_t now = globaltimer_ns();
+              if (since == 0) since = now;
+              if (now - since > kWaitLimitNs) *abort_flag = 1;
+              if (*abort_flag) break;
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (b2 + j < blk) {
+              v[0] += __uint_as_float(~w[j].x);
+              v[1] += __uint_as_float(~w[j].y);
+              v[2] += __uint_as_float(~w[j].z);
+              v[3] += __uint_as_float(~w[j].w);
+              st_relaxed_gpu_v4_zero(tile + (size_t)j * TOK * du::kRows);          // ready for the next call
+            }
+        }
+        const int n = rb * du::kRows + r4;                     // N is a multiple of four
+        if (n < p.N && !*abort_flag) {
+          if (p.bias) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] += h2f(p.bias[n + i]);
+          }
+          __half* y = p.y + (size_t)m * p.N + n;
+          *reinterpret_cast<__half2*>(y) = __floats2half2_rn(v[0], v[1]);
+          *reinterpret_cast<__half2*>(y + 2) = __floats2half2_rn(v[2], v[3]);
+        }
+      }
+    }
+    __syncthreads();
+  }
   if (*abort_flag) {
     if (tid == 0 && p.error_word) atomicExch(p.error_word, 4);
     const uint64_t t_start = globaltimer_ns();
@@ -465,56 +609,70 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
 
 int* decode_error_word_ptr(int* out_rc);   // w4a16_decode_tma.cu: device address of the decode error word
 
-size_t decode_umma_workspace_bytes(int M) { return du::workspace_bytes(du::tokens_for(M)); }
+size_t decode_umma_workspace_bytes(int M, int K) { return du::workspace_bytes(M, K); }
 
-static bool umma_shape_ok(int M, int N, int K, int group) {
-  if (M > 64 || K % 64 != 0 || N % 4 != 0) return false;
+// The activations in expansion order, for the wider tiles: permuting them per block and stage in shared memory, as at up
+// to 16 rows, cost the expansion warps a third of their time at 64.
+__global__ void __launch_bounds__(256)
+w4a16_permute_kernel(const uint4* __restrict__ x, int chunks, uint4* __restrict__ out) {
+  chain_wait();
+  chain_release();
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < chunks; i += gridDim.x * 256) out[i] = pair_permute_u4(x[i]);
+}
+
+bool decode_umma_shape_ok(int M, int N, int K, int group) {
+  if (M > 128 || K % 64 != 0 || N % 4 != 0) return false;
   return group == 32 || group == 64 || group == 128 || group == du::kStageK || group % du::kStageK == 0;
 }
 
-template <int STAGES, int TOK>
-static int launch_umma(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tsz, const DecodeUmmaParams& p,
-                       int grid, size_t smem, cudaStream_t st) {
-  auto kern = w4a16_decode_umma_kernel<STAGES, TOK>;
+template <int TOK, int XROWS, bool FOLD>
+static int launch_umma(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tsz, DecodeUmmaParams p, int grid,
+                       cudaStream_t st) {
+  using C = du::Cfg<TOK, XROWS, FOLD>;
+  auto kern = w4a16_decode_umma_kernel<TOK, XROWS, FOLD>;
   static thread_local int configured_device = -1;
   int device = 0;
   MP_CUDA_TRY(cudaGetDevice(&device));
   if (configured_device != device) {
-    MP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)du::kSmemBlockMax));
+    MP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)du::kSmemMax));
     configured_device = device;
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid, 1, 1);
-  cfg.blockDim = dim3(du::kThreads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attrs[1];
-  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attrs[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attrs;
-  cfg.numAttrs = 1;
-  MP_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tw, tx, tsz, p));
-  return MP_OK;
+  // as many weight stages as fit
+  const int stage = du::kWBytes + du::sz_bytes(p.groups_per_stage);
+  const size_t fixed = 1024 + (size_t)C::kXRing * C::kXBytes + du::kTailBytes;
+  p.ring = (int)((du::kSmemMax - fixed) / stage);
+  if (p.ring > du::kMaxRing) p.ring = du::kMaxRing;
+  return launch_chained(kern, dim3(grid), dim3(du::kThreads), fixed + (size_t)p.ring * stage, st, tw, tx, tsz, p);
 }
 
-// Returns MP_ERR_UNSUPPORTED for shapes this kernel does not take (M > 16, K % 64 != 0, N % 4 != 0, groups
+// Returns MP_ERR_UNSUPPORTED for shapes this kernel does not take (M > 128, K % 64 != 0, N % 4 != 0, groups
 // other than 32, 64, 128, 256 or a multiple of 256) and when the workspace is missing or too small; the
-// caller then uses a scratch-free kernel.  The workspace starts zeroed and is left ready for the next call;
+// caller then uses another kernel.  The workspace starts zeroed and is left ready for the next call;
 // calls that share it must not overlap on the GPU.
 int launch_decode_umma(const void* x, const void* packed, const void* sz, const void* bias, void* y, int M, int N, int K,
-                       int group, void* workspace, size_t workspace_bytes, cudaStream_t st, bool pdl) {
-  if (!umma_shape_ok(M, N, K, group)) return MP_ERR_UNSUPPORTED;
+                       int group, void* workspace, size_t workspace_bytes, cudaStream_t st, bool early_weights) {
+  if (!decode_umma_shape_ok(M, N, K, group)) return MP_ERR_UNSUPPORTED;
   const int tok = du::tokens_for(M);
-  if (!workspace || workspace_bytes < du::workspace_bytes(tok) || !aligned(workspace, 16)) return MP_ERR_UNSUPPORTED;
-  if (!aligned(x, 16) || !aligned(packed, 16) || !aligned(sz, 16)) return MP_ERR_UNSUPPORTED;
+  if (!workspace || workspace_bytes < du::workspace_bytes(M, K) || !aligned(workspace, 16)) return MP_ERR_UNSUPPORTED;
+  if (!aligned(x, 16) || !aligned(packed, 16) || !aligned(sz, 16) || !aligned(y, 4)) return MP_ERR_UNSUPPORTED;
   const int row_blocks = (N + du::kRows - 1) / du::kRows;
-  if ((size_t)row_blocks * sizeof(int) > du::kCounterBytes) return MP_ERR_UNSUPPORTED;
   CUtensorMap tw, tx, tsz;
   int rc = encode_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, packed, (uint64_t)K / 2, (uint64_t)N,
                                 (uint64_t)K / 2, 128, du::kRows, true);
   if (rc != MP_OK) return rc;
-  rc = encode_tensor_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, 64,
-                            tok, true);
+  if (tok > 32) {
+    uint4* xp = reinterpret_cast<uint4*>(static_cast<unsigned char*>(workspace) + du::kXOffset);
+    const int chunks = M * (K / 8), blocks = (chunks + 255) / 256;
+    rc = launch_chained(w4a16_permute_kernel, dim3(blocks < 2 * kSmCount ? blocks : 2 * kSmCount), dim3(256), 0, st,
+                        static_cast<const uint4*>(x), chunks, xp);
+    if (rc != MP_OK) return rc;
+    x = xp;
+    early_weights = true;        // of the kernel before only that one is still running, and it writes no weights
+  }
+  // [64 columns][token][chunk of 64 columns]: one copy brings the sub-tiles of a stage or half of one
+  const uint64_t x_dims[3] = {64, (uint64_t)M, (uint64_t)K / 64}, x_strides[2] = {(uint64_t)K * 2, 128};
+  const uint32_t x_box[3] = {64, (uint32_t)(M <= 8 ? 8 : tok), tok <= 32 ? 4u : 2u};
+  rc = encode_tensor_map_3d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, x_dims, x_strides, x_box);
   if (rc != MP_OK) return rc;
   const int gps = group < du::kStageK ? du::kStageK / group : 1;
   rc = encode_tensor_map_2d(&tsz, CU_TENSOR_MAP_DATA_TYPE_UINT32, sz, (uint64_t)N, (uint64_t)(K / group),
@@ -525,31 +683,28 @@ int launch_decode_umma(const void* x, const void* packed, const void* sz, const 
   p.y = static_cast<__half*>(y);
   p.M = M; p.N = N; p.K = K; p.group = group;
   p.stages_per_row = (K + du::kStageK - 1) / du::kStageK;
-  p.total = row_blocks * p.stages_per_row;
+  const long long total = (long long)row_blocks * p.stages_per_row;
+  if (total > (1 << 24)) return MP_ERR_UNSUPPORTED;
+  // as few blocks as finish as early as a block on every SM would
+  int per_block = ((int)total + du::kMaxGrid - 1) / du::kMaxGrid;
+  if (per_block < du::min_share(p.stages_per_row, tok)) per_block = du::min_share(p.stages_per_row, tok);
+  const int grid = ((int)total + per_block - 1) / per_block;
+  p.share = (int)total / grid;
+  p.extra = (int)total % grid;
   p.groups_per_stage = gps;
-  p.early_weights = pdl ? 1 : 0;
   p.gshift = group == 32 ? 5 : group == 64 ? 6 : 7;
-  p.counters = static_cast<int*>(workspace);
-  p.tiles = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + du::kCounterBytes);
+  p.early_weights = early_weights ? 1 : 0;
+  p.tiles = reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(workspace) + du::kTileOffset);
   int rc_err = MP_OK;
   p.error_word = decode_error_word_ptr(&rc_err);
   if (rc_err != MP_OK) return rc_err;
-  // two blocks per SM, each with at least two stages of work
-  const int grid = max(1, min(du::kMaxBlocks, p.total / 2));
-  // the deepest ring that still lets two blocks share an SM (groups of 32 columns carry 4 KB of (scale, zero)
-  // pairs per stage; a 32-token activation tile is 16 KB per stage, a 64-token one 32 KB)
-  auto fits = [&](int stages) { return du::smem_bytes(tok, stages, gps) <= du::kSmemBlockMax; };
-  if (tok == 16) {
-    if (fits(4)) return launch_umma<4, 16>(tw, tx, tsz, p, grid, du::smem_bytes(16, 4, gps), st);
-    return launch_umma<3, 16>(tw, tx, tsz, p, grid, du::smem_bytes(16, 3, gps), st);
-  }
-  if (tok == 32) {
-    if (fits(3)) return launch_umma<3, 32>(tw, tx, tsz, p, grid, du::smem_bytes(32, 3, gps), st);
-    if (fits(2)) return launch_umma<2, 32>(tw, tx, tsz, p, grid, du::smem_bytes(32, 2, gps), st);
-    return MP_ERR_UNSUPPORTED;
-  }
-  if (fits(2)) return launch_umma<2, 64>(tw, tx, tsz, p, grid, du::smem_bytes(64, 2, gps), st);
-  return MP_ERR_UNSUPPORTED;
+  const bool fold = group % 128 == 0;
+  if (M <= 8) return fold ? launch_umma<16, 8, true>(tw, tx, tsz, p, grid, st) : launch_umma<16, 8, false>(tw, tx, tsz, p, grid, st);
+  if (tok == 16) return fold ? launch_umma<16, 16, true>(tw, tx, tsz, p, grid, st) : launch_umma<16, 16, false>(tw, tx, tsz, p, grid, st);
+  if (tok == 32) return launch_umma<32, 32, false>(tw, tx, tsz, p, grid, st);
+  if (tok == 64) return launch_umma<64, 64, false>(tw, tx, tsz, p, grid, st);
+  if (tok == 96) return launch_umma<96, 96, false>(tw, tx, tsz, p, grid, st);
+  return launch_umma<128, 128, false>(tw, tx, tsz, p, grid, st);
 }
 
 }  // namespace mp

@@ -546,6 +546,21 @@ int encode_tensor_map_2d(CUtensorMap* map, CUtensorMapDataType dtype, const void
   return MP_OK;
 }
 
+int encode_tensor_map_3d(CUtensorMap* map, CUtensorMapDataType dtype, const void* base, const uint64_t (&dims)[3],
+                         const uint64_t (&strides)[2], const uint32_t (&box)[3]) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) return MP_ERR_CUDA;
+  const cuuint64_t d[3] = {dims[0], dims[1], dims[2]}, st[2] = {strides[0], strides[1]};
+  const cuuint32_t bx[3] = {box[0], box[1], box[2]}, estr[3] = {1, 1, 1};
+  const CUresult r = fn(map, dtype, 3, const_cast<void*>(base), d, st, bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    g_last_cuda_error = 100000 + static_cast<int>(r);
+    return MP_ERR_CUDA;
+  }
+  return MP_OK;
+}
+
 // Sum of the K slices' int32 partial tiles, then the epilogue of the unsplit kernel with the same
 // operations in the same order (so a split changes no output bit): f16(float(acc) * s_token * s_channel (+ bias)),
 // or the raw int32 sum.

@@ -183,8 +183,10 @@ class VllmPackedInt4Linear(nn.Module):
             # scratch of this (row count, stream) pair, when the library's choice for the shape needs one: calls on
             # one stream run in order, so they may share it
             ws = None
-            if 0 < m <= 16 and ops.w4a16_decode_kernel_choice(m, self.out_features, self.in_features) == "umma":
-                ws = ops.new_workspace(ops.w4a16_decode_workspace_bytes(m, self.out_features, self.in_features), dev)
+            nbytes = _lib.load().mp_w4a16_linear_workspace_bytes(m, self.out_features, self.in_features,
+                                                                 self.group_size) if 0 < m <= 16 else 0
+            if nbytes:
+                ws = ops.new_workspace(nbytes, dev)
             stage = (torch.empty((m, self.in_features), dtype=torch.float16, device=dev),
                      torch.empty((m, self.out_features), dtype=torch.float16, device=dev), ws)
             self._host_stage[(m, st)] = stage

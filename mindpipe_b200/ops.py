@@ -270,27 +270,33 @@ def w4a16_linear_prefill(x, weight_packed, scale_zero, bias=None, *, workspace=N
 
 
 def w4a16_linear(x, weight_packed, scale_zero, bias=None):
-    """W4A16 linear for any number of rows.
-
-    Up to 16 rows go to the weight-streaming decode kernels; 17..64 rows on
-    large weights to the tcgen05 weight-streaming kernel with a 32- or
-    64-token tile (the library's rule, ``w4a16_decode_kernel_choice``); the
-    rest to the tensor-core prefill kernel (which splits K when the batch gives
-    it few tiles); shapes the prefill kernel does not take (K or the group size
-    not a multiple of 64) are processed by the decode kernels in 64-row slabs.
+    """W4A16 linear for any number of rows: the library picks among the decode kernels, the tcgen05 weight-streaming
+    kernel (up to 128 rows) and the tensor-core prefill kernel (``mp_w4a16_linear``).  Shapes the prefill kernel does
+    not take (K or the group size not a multiple of 64) are processed by the decode kernels in 64-row slabs.
     """
-    m, k = x.shape
-    if m <= 16:
-        return w4a16_linear_decode(x, weight_packed, scale_zero, bias)
-    if m <= 64 and w4a16_decode_kernel_choice(m, weight_packed.shape[0], k) == "umma":
-        return w4a16_linear_decode(x, weight_packed, scale_zero, bias)   # weights streamed once, 32/64-token tile
-    group = k // scale_zero.shape[0]
-    if k % 64 == 0 and group % 64 == 0:
-        return w4a16_linear_prefill(x, weight_packed, scale_zero, bias)
-    if m <= 64:
-        return w4a16_linear_decode(x, weight_packed, scale_zero, bias)
-    outs = [w4a16_linear_decode(x[i:i + 64], weight_packed, scale_zero, bias) for i in range(0, m, 64)]
-    return torch.cat(outs, dim=0)
+    x2 = _req(x, "x", torch.float16, 2)
+    p = _req(weight_packed, "weight_packed", torch.int32, 2)
+    sz = _req(scale_zero, "scale_zero", torch.float16, 3)
+    b = None if bias is None else _req(bias, "bias", torch.float16, 1)
+    m, k = x2.shape
+    n = p.shape[0]
+    groups = sz.shape[0]
+    if p.shape[1] * 8 != k or sz.shape[1] != n or k % groups:
+        raise ValueError(f"shape mismatch: x{tuple(x2.shape)} packed{tuple(p.shape)} sz{tuple(sz.shape)}")
+    group = k // groups
+    if m == 0:
+        return torch.empty((m, n), dtype=torch.float16, device=x2.device)
+    if m > 16 and (k % 64 or group % 64):
+        outs = [w4a16_linear_decode(x2[i:i + 64], p, sz, b) for i in range(0, m, 64)]
+        return outs[0] if len(outs) == 1 else torch.cat(outs, dim=0)
+    y = torch.empty((m, n), dtype=torch.float16, device=x2.device)
+    lib = _lib.load()
+    nbytes = lib.mp_w4a16_linear_workspace_bytes(m, n, k, group)
+    ws = _workspace(nbytes, x2.device) if nbytes else None
+    st = lib.mp_w4a16_linear(x2.data_ptr(), p.data_ptr(), sz.data_ptr(), _ptr(b), y.data_ptr(), m, n, k, group, _ptr(ws),
+                             0 if ws is None else ws.numel(), _error_word(x2.device).data_ptr(), _stream())
+    _lib.check(st, "w4a16_linear", M=m, N=n, K=k, group=group)
+    return y
 
 
 # ------------------------------------------------------------------- W8A8

@@ -1,0 +1,47 @@
+"""``w4a16_linear`` at the row counts where its kernels hand over and at ragged shapes, against fp32 of the expanded
+weights; repeated calls give the same bits and leave the scratch buffer's tiles zero."""
+import pytest
+import torch
+
+from mindpipe_b200 import _lib, ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(n, k, m, group):
+    g = torch.Generator(device="cuda").manual_seed(n + k + m)
+    w = (torch.randn(n, k, generator=g, device="cuda") * 0.02).half()
+    packed, scale, zero, _ = ops.w4a16_quantize(w, group)
+    sz = ops.w4a16_prepare(scale, zero, k)
+    x = torch.randn(m, k, generator=g, device="cuda").half()
+    bias = torch.randn(n, generator=g, device="cuda").half()
+    return x, packed, sz, bias, ops.w4a16_dequant(packed, scale, zero, n, k).float()
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 16, 17, 32, 33, 64, 65, 80, 96, 97, 128, 129])
+@pytest.mark.parametrize("n,k,group", [(264, 1280, 128), (4104, 512, 64), (40, 1408, 128), (2048, 2176, 128),
+                                       (20480, 512, 256), (1032, 4096, 4096)])
+def test_linear_at_row_count_edges(m, n, k, group):
+    x, packed, sz, bias, wdq = _case(n, k, m, group)
+    for b in (None, bias):
+        y = ops.w4a16_linear(x, packed, sz, b)
+        ref = x.float() @ wdq.t() + (0 if b is None else b.float())
+        assert ((y.float() - ref).norm() / ref.norm()).item() <= 1e-3
+        for _ in range(2):
+            assert torch.equal(ops.w4a16_linear(x, packed, sz, b), y)
+    ops.check_device_errors()
+    nbytes = _lib.load().mp_w4a16_linear_workspace_bytes(min(m, 16), 28672, 8192, 128)      # counters and 16-token tiles
+    assert not ops._workspace(nbytes, x.device)[:nbytes].any()
+
+
+@pytest.mark.parametrize("m", [5, 16, 50, 100])
+def test_linear_of_extreme_values(m):
+    """Zeros, infinities and NaNs pass through the partial tiles (whose words mean "not there yet" when zero)."""
+    n, k = 512, 8192
+    x, packed, sz, _, wdq = _case(n, k, m, 128)
+    x.zero_()
+    assert not ops.w4a16_linear(x, packed, sz).any()
+    x[0, 3], x[m - 1, k - 1] = float("inf"), float("nan")
+    y = ops.w4a16_linear(x, packed, sz)
+    assert y[m - 1].isnan().all() and not torch.isfinite(y[0]).any() and not y[1:m - 1].any()
+    ops.check_device_errors()
