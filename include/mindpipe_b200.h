@@ -388,6 +388,25 @@ int mp_w8a8_gemm_ex(const void* qx_i8, const void* x_scale_f32, const void* w_i8
                     void* workspace, size_t workspace_bytes, int* error_word, mp_stream_t stream);
 
 /*
+ * The whole W8A8 linear on fp16 rows: mp_act_quant_per_token, then the product -- SmoothQuantLinear.forward
+ * (fake_quant.py:77-88) in one call, so that the product's weights are on their way while the rows are quantised.  Up to
+ * 128 rows a weight-streaming kernel runs, else mp_w8a8_gemm_ex; the results are those of the two calls, bit for bit.
+ * qx_i8 [M,K] and x_scale_f32 [M] receive the codes and scales.  Workspace: as for mp_w4a16_linear (zero-filled when
+ * created, one for all shapes, may be shared with it); the tiled GEMM runs unsplit without one.
+ */
+size_t mp_w8a8_linear_workspace_bytes(int M, int N, int K);
+int mp_w8a8_linear(const void* x_f16, const void* w_i8, const void* w_scale_f32, const void* bias_f16, void* y_f16, int M,
+                   int N, int K, void* qx_i8, void* x_scale_f32, void* workspace, size_t workspace_bytes,
+                   int* error_word, mp_stream_t stream);
+/* The same for the asymmetric linear: mp_affine_quant_per_row and mp_w8a8_affine_gemm (OmniQuant's QuantLinear.forward,
+ * int_linear.py:42-55). */
+size_t mp_w8a8_affine_linear_workspace_bytes(int M, int N, int K);
+int mp_w8a8_affine_linear(const void* x_f16, const void* w_u8, const void* w_scale_f32, const void* w_zero_f32,
+                          const void* w_rowsum_i32, const void* bias_f16, void* y_f16, int M, int N, int K,
+                          void* qx_u8, void* x_scale_f32, void* x_zero_f32, void* x_rowsum_i32, void* workspace,
+                          size_t workspace_bytes, int* error_word, mp_stream_t stream);
+
+/*
  * Raw accumulators acc[M,N] = qx . w^T as int32: npu_quant_matmul with
  * output_dtype=int32 (acceleration/runtime_patches/vllm.patch:756-760), and
  * the bit-exact check of the tensor-core path.
@@ -539,6 +558,19 @@ int mp_moe_gemm2(const void* plan_i32, int padded_rows, int I, int H, int num_lo
  */
 int mp_moe_combine(const void* d_f16, const void* dest_row_i32, const void* topk_ids_i32,
                    const void* topk_weights_f16, int T, int H, int k, void* out_f16, mp_stream_t stream);
+
+/*
+ * The whole expert layer on one GPU: mp_moe_route_gather_quant, mp_moe_expert_stage and mp_moe_combine in one call, i.e.
+ * SmoothQuantPackedMoeExperts.forward (fake_quant.py:165-191) for the experts [expert_lo, expert_hi).  With few tokens the
+ * grouped products run on a weight-streaming kernel; the results are those of the three calls, bit for bit.  scratch: any
+ * memory, 256-byte aligned.  workspace: as for mp_w8a8_linear, may be NULL (then the tiled GEMMs run).
+ */
+size_t mp_moe_experts_scratch_bytes(int T, int H, int k, int num_local_experts, int I);
+size_t mp_moe_experts_workspace_bytes(int T);
+int mp_moe_experts(const void* hidden_f16, const void* topk_ids_i32, const void* topk_weights_f16, int T, int H, int k,
+                   int expert_lo, int expert_hi, const void* w13_q_i8, const void* w13_scale_f32, const void* w2_q_i8,
+                   const void* w2_scale_f32, int I, void* out_f16, void* scratch, size_t scratch_bytes, void* workspace,
+                   size_t workspace_bytes, int* error_word, mp_stream_t stream);
 
 /*
  * Expert-parallel exchange over peer-mapped (symmetric) memory, without a host

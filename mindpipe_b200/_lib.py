@@ -55,6 +55,10 @@ SIGNATURES = {
     "mp_w8a8_gemm": (_I, [_P, _P, _P, _P, _P, _P, _I, _I, _I, _P, _P]),
     "mp_w8a8_gemm_workspace_bytes": (_Z, [_I, _I, _I]),
     "mp_w8a8_gemm_ex": (_I, [_P, _P, _P, _P, _P, _P, _I, _I, _I, _P, _Z, _P, _P]),
+    "mp_w8a8_linear_workspace_bytes": (_Z, [_I, _I, _I]),
+    "mp_w8a8_linear": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _P, _P, _P, _Z, _P, _P]),
+    "mp_w8a8_affine_linear_workspace_bytes": (_Z, [_I, _I, _I]),
+    "mp_w8a8_affine_linear": (_I, [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _P, _P, _P, _P, _P, _Z, _P, _P]),
     "mp_w8a8_gemm_i32": (_I, [_P, _P, _P, _I, _I, _I, _P, _P]),
     "mp_affine_quant_per_row": (_I, [_P, _I, _I, _P, _P, _P, _P, _P, _P]),
     "mp_w8a8_affine_gemm": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _P, _P]),
@@ -65,6 +69,9 @@ SIGNATURES = {
     "mp_moe_expert_stage_workspace_bytes": (_Z, [_I, _I]),
     "mp_moe_expert_stage": (_I, [_P, _P, _P, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _Z, _P, _P]),
     "mp_moe_expert_stage_scatter": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _Z, _P, _P]),
+    "mp_moe_experts_scratch_bytes": (_Z, [_I, _I, _I, _I, _I]),
+    "mp_moe_experts_workspace_bytes": (_Z, [_I]),
+    "mp_moe_experts": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _I, _P, _P, _Z, _P, _Z, _P, _P]),
     "mp_moe_combine": (_I, [_P, _P, _P, _P, _I, _I, _I, _P, _P]),
     "mp_moe_gemm1_swiglu": (_I, [_P, _P, _P, _I, _I, _I, _I, _P, _P, _P, _Z, _I, _P, _P]),
     "mp_moe_requant": (_I, [_P, _I, _I, _I, _P, _Z, _P]),

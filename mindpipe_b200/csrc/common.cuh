@@ -172,6 +172,14 @@ __device__ __forceinline__ uint32_t pack_biased_codes(float2 a, float2 b) {
 
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 
+// (max, -min) of the pairs mx / mn as one register, for reductions that want both.  The sign is flipped on the bits: with
+// __hneg2 in front of the rearranged maximum the compiler lost the negation in some instantiations.
+__device__ __forceinline__ __half2 max_and_neg_min(__half2 mx, __half2 mn) {
+  const uint32_t flipped = h2_bits(mn) ^ 0x80008000u;
+  const __half2 neg = *reinterpret_cast<const __half2*>(&flipped);
+  return __hmax2(__lows2half2(mx, neg), __highs2half2(mx, neg));
+}
+
 // Eight fp16 values (one 128-bit load) -> eight packed int8 codes.
 __device__ __forceinline__ uint2 quant8_pack(const uint4& raw, const RowQuant& rq) {
   const __half2* h2 = reinterpret_cast<const __half2*>(&raw);

@@ -187,11 +187,9 @@ struct W8Plan : Plan {
     const size_t codes = align256(static_cast<size_t>(m) * k);
     at::Tensor q = scratch(codes + static_cast<size_t>(m) * 4, x);
     char* qp = static_cast<char*>(q.data_ptr());
-    Scratch ws(mp_w8a8_gemm_workspace_bytes(m, n, k), device, st, kW8A8);
-    int rc = mp_act_quant_per_token(x.data_ptr(), m, k, qp, qp + codes, nullptr, st);
-    if (rc == MP_OK)
-      rc = mp_w8a8_gemm_ex(qp, qp + codes, weight.data_ptr(), weight_scale.data_ptr(), data_or_null(bias), y.data_ptr(), m,
-                           n, k, ws.ptr, ws.bytes, error_word, st);
+    Scratch ws(mp_w8a8_linear_workspace_bytes(m, n, k), device, st, kDecode);
+    const int rc = mp_w8a8_linear(x.data_ptr(), weight.data_ptr(), weight_scale.data_ptr(), data_or_null(bias), y.data_ptr(),
+                                  m, n, k, qp, qp + codes, ws.ptr, ws.bytes, error_word, st);
     return rc == MP_OK ? THPVariable_Wrap(std::move(y)) : none();
   }
 };
@@ -214,15 +212,15 @@ struct AffinePlan : Plan {
     at::Tensor q = scratch(codes + 3 * per_row, x);
     char* qp = static_cast<char*>(q.data_ptr());
     char *sp = qp + codes, *zp = sp + per_row, *rp = zp + per_row;
-    int rc = mp_affine_quant_per_row(x.data_ptr(), m, k, qp, sp, zp, rp, nullptr, st);
-    if (rc == MP_OK)
-      rc = mp_w8a8_affine_gemm(qp, sp, zp, rp, weight.data_ptr(), scale.data_ptr(), zero.data_ptr(), rowsum.data_ptr(),
-                               data_or_null(bias), y.data_ptr(), m, n, k, error_word, st);
+    Scratch ws(mp_w8a8_affine_linear_workspace_bytes(m, n, k), device, st, kDecode);
+    const int rc = mp_w8a8_affine_linear(x.data_ptr(), weight.data_ptr(), scale.data_ptr(), zero.data_ptr(),
+                                         rowsum.data_ptr(), data_or_null(bias), y.data_ptr(), m, n, k, qp, sp, zp, rp, ws.ptr,
+                                         ws.bytes, error_word, st);
     return rc == MP_OK ? THPVariable_Wrap(std::move(y)) : none();
   }
 };
 
-// W8A8 experts: routing + gather + quantisation, expert stage, weighted combine; one scratch tensor for all of it.
+// W8A8 experts; one scratch tensor for the whole layer.
 struct MoePlan : Plan {
   at::Tensor w13, w13_scale, w2, w2_scale;
   int h = 0, i = 0, lo = 0, hi = 0;
@@ -238,24 +236,13 @@ struct MoePlan : Plan {
     if (entries != wp->numel() || entries % rows != 0 || entries > (int64_t(1) << 24)) return none();
     const int t = static_cast<int>(rows), k = static_cast<int>(entries / rows), e = hi - lo;
     const cudaStream_t st = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream();
-    const int padded = mp_moe_padded_rows(e, t * k);
-    const size_t stage_bytes = mp_moe_expert_stage_workspace_bytes(padded, i);
-    const size_t b_plan = align256(4 * mp_moe_plan_ints(e, t * k)), b_dest = align256(4 * static_cast<size_t>(entries));
-    const size_t b_scale = align256(4 * static_cast<size_t>(padded)), b_q = align256(static_cast<size_t>(padded) * h);
-    const size_t b_d = align256(2 * static_cast<size_t>(padded) * h);
     at::Tensor out = output_like(x, h, at::kHalf);
-    at::Tensor buf = scratch(b_plan + b_dest + b_scale + b_q + b_d + stage_bytes, x);
-    char* plan = static_cast<char*>(buf.data_ptr());
-    char* dest = plan + b_plan;
-    char* rscale = dest + b_dest;
-    char* rq = rscale + b_scale;
-    char* d = rq + b_q;
-    char* stage = d + b_d;
-    int rc = mp_moe_route_gather_quant(x.data_ptr(), idp->data_ptr(), t, h, k, lo, hi, plan, dest, rq, rscale, st);
-    if (rc == MP_OK)
-      rc = mp_moe_expert_stage(rq, rscale, plan, padded, h, i, e, w13.data_ptr(), w13_scale.data_ptr(), w2.data_ptr(),
-                               w2_scale.data_ptr(), d, stage, stage_bytes, error_word, st);
-    if (rc == MP_OK) rc = mp_moe_combine(d, dest, idp->data_ptr(), wp->data_ptr(), t, h, k, out.data_ptr(), st);
+    const size_t bytes = mp_moe_experts_scratch_bytes(t, h, k, e, i);
+    at::Tensor buf = scratch(bytes, x);
+    Scratch ws(mp_moe_experts_workspace_bytes(t), device, st, kDecode);
+    const int rc = mp_moe_experts(x.data_ptr(), idp->data_ptr(), wp->data_ptr(), t, h, k, lo, hi, w13.data_ptr(),
+                                  w13_scale.data_ptr(), w2.data_ptr(), w2_scale.data_ptr(), i, out.data_ptr(), buf.data_ptr(),
+                                  bytes, ws.ptr, ws.bytes, error_word, st);
     return rc == MP_OK ? THPVariable_Wrap(std::move(out)) : none();
   }
 };

@@ -13,6 +13,7 @@
 // a multiple of 128 rows, so a 128-row GEMM tile never straddles experts.
 #include "common.cuh"
 #include "moe_api.cuh"
+#include "w8a8_stream.cuh"
 
 namespace mp {
 
@@ -21,26 +22,57 @@ constexpr int kMaxExperts = 256;
 
 // softmax(fp32) -> top-k -> renormalise -> fp16, one thread per token
 // (algorithm/quantization/qat/flatquant/source/flatquant/model_tools/mixtral_utils.py:330-333,349).
-__global__ void moe_router_topk_kernel(const float* __restrict__ logits, int T, int E, int k,
-                                       int* __restrict__ idx, __half* __restrict__ w) {
+// MAX_E: the probabilities of up to that many experts stay in registers; 0: any number, recomputed for every choice.
+// A few chained latencies long whatever T is (8192 tokens, 8 experts: 6.8 us when every choice called expf per expert).
+template <int MAX_E>
+__global__ void __launch_bounds__(128)
+moe_router_topk_kernel(const float* __restrict__ logits, int T, int E, int k, int* __restrict__ idx,
+                       __half* __restrict__ w) {
+  chain_wait();
+  chain_release();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T) return;
   const float* l = logits + (size_t)t * E;
-  float mx = -INFINITY;
-  for (int e = 0; e < E; ++e) mx = fmaxf(mx, l[e]);
-  float sum = 0.0f;
-  for (int e = 0; e < E; ++e) sum += expf(l[e] - mx);
+  constexpr int NREG = MAX_E > 0 ? MAX_E : 1;
+  float p[NREG];
+  float mx = -INFINITY, sum = 0.0f;
+  if constexpr (MAX_E > 0) {
+#pragma unroll
+    for (int e = 0; e < NREG; ++e) p[e] = e < E ? l[e] : -INFINITY;
+#pragma unroll
+    for (int e = 0; e < NREG; ++e) mx = fmaxf(mx, p[e]);
+#pragma unroll
+    for (int e = 0; e < NREG; ++e)
+      if (e < E) {
+        p[e] = expf(p[e] - mx);
+        sum += p[e];
+      }
+#pragma unroll
+    for (int e = 0; e < NREG; ++e) p[e] = e < E ? p[e] / sum : -2.0f;
+  } else {
+    for (int e = 0; e < E; ++e) mx = fmaxf(mx, l[e]);
+    for (int e = 0; e < E; ++e) sum += expf(l[e] - mx);
+  }
   float chosen_p[8];
   int chosen[8];
   float psum = 0.0f;
   for (int j = 0; j < k; ++j) {
     float best = -1.0f;
     int bi = 0;
-    for (int e = 0; e < E; ++e) {
-      bool taken = false;
-      for (int i = 0; i < j; ++i) taken |= (chosen[i] == e);
-      const float pe = expf(l[e] - mx) / sum;
-      if (!taken && pe > best) { best = pe; bi = e; }     // strict >: ties go to the lower index
+    if constexpr (MAX_E > 0) {
+#pragma unroll
+      for (int e = 0; e < NREG; ++e)
+        if (p[e] > best) { best = p[e]; bi = e; }           // strict >: ties go to the lower index
+#pragma unroll
+      for (int e = 0; e < NREG; ++e)
+        if (e == bi) p[e] = -2.0f;                           // taken
+    } else {
+      for (int e = 0; e < E; ++e) {
+        bool taken = false;
+        for (int i = 0; i < j; ++i) taken |= (chosen[i] == e);
+        const float pe = expf(l[e] - mx) / sum;
+        if (!taken && pe > best) { best = pe; bi = e; }
+      }
     }
     chosen[j] = bi;
     chosen_p[j] = best;
@@ -258,6 +290,28 @@ moe_requant_kernel(const __half* __restrict__ h, const float* __restrict__ absma
   }
 }
 
+// The same for the rows of a few routed entries, a block each (padding rows are neither computed nor read).
+__global__ void __launch_bounds__(256)
+moe_requant_rows_kernel(const __half* __restrict__ h, const float* __restrict__ absmax, int slots, int I,
+                        const int* __restrict__ dest_row, int8_t* __restrict__ q, float* __restrict__ scale) {
+  chain_wait();
+  chain_release();
+  const int row = dest_row[blockIdx.x];
+  if (row < 0) return;
+  const int lane = threadIdx.x & 31;
+  float m = 0.0f;
+  for (int j = lane; j < slots; j += 32) m = fmaxf(m, absmax[(size_t)row * slots + j]);      // every warp for itself
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  const float sf = h2f(f2h(__fdiv_rn(fmaxf(m, h2f(f2h(1e-5f))), 127.0f)));
+  if (threadIdx.x == 0 && blockIdx.y == 0) scale[row] = sf;
+  const RowQuant rq = make_row_quant(sf);
+  const __half* hr = h + (size_t)row * I;
+  int8_t* qr = q + (size_t)row * I;
+  for (int c = blockIdx.y * 256 + threadIdx.x; c < (I >> 3); c += gridDim.y * 256)
+    *reinterpret_cast<uint2*>(qr + c * 8) = quant8_pack(*reinterpret_cast<const uint4*>(hr + c * 8), rq);
+}
+
 static int launch_requant(const __half* h, const float* absmax, int I, const int* num_tiles, int padded_rows,
                           int8_t* q2, float* scale2, cudaStream_t st) {
   const int grid = padded_rows < 8 * kSmCount ? padded_rows : 8 * kSmCount;
@@ -352,10 +406,11 @@ extern "C" int mp_moe_router_topk(const void* logits_f32, int T, int E, int k, v
                                   mp_stream_t stream) {
   if (!logits_f32 || !idx_i32 || !weights_f16 || T <= 0 || E <= 0 || k <= 0) return MP_ERR_INVALID_ARG;
   if (k > 8 || k > E) return MP_ERR_UNSUPPORTED;
-  moe_router_topk_kernel<<<(T + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const float*>(logits_f32), T, E, k, static_cast<int*>(idx_i32), static_cast<__half*>(weights_f16));
-  MP_LAUNCH_CHECK();
-  return MP_OK;
+  auto kern = E <= 8 ? moe_router_topk_kernel<8> : E <= 16 ? moe_router_topk_kernel<16> : E <= 32 ? moe_router_topk_kernel<32>
+                                                                                        : moe_router_topk_kernel<0>;
+  return launch_chained(kern, dim3((T + 127) / 128), dim3(128), 0, static_cast<cudaStream_t>(stream),
+                        static_cast<const float*>(logits_f32), T, E, k, static_cast<int*>(idx_i32),
+                        static_cast<__half*>(weights_f16));
 }
 
 extern "C" size_t mp_moe_plan_ints(int num_local_experts, int max_rows) {
@@ -567,6 +622,110 @@ extern "C" int mp_moe_combine(const void* d_f16, const void* dest_row_i32, const
                         static_cast<const int*>(topk_ids_i32), static_cast<const __half*>(topk_weights_f16), T, H, k,
                         static_cast<__half*>(out_f16), static_cast<const unsigned int*>(nullptr), 0,
                         static_cast<const unsigned int*>(nullptr), static_cast<int*>(nullptr));
+}
+
+// ---- the whole expert layer on one GPU ---------------------------------------------------------------------------
+// Up to 64 tokens the experts' weights are a stream over a handful of rows each: the grouped products run on the
+// weight-streaming kernel, whose first weights are requested while the rows are gathered or re-quantised (32 tokens over
+// eight 4096x14336 experts: 1.41 GB, 344 us with 256-row tiles).  With more, on the tiled grouped GEMMs.
+constexpr int kStreamTokens = 64;
+
+struct LayerBuffers {
+  int padded;
+  size_t plan, dest, scale, q, d, stage, total;
+};
+static LayerBuffers layer_buffers(int T, int H, int k, int E, int I) {
+  LayerBuffers b;
+  b.padded = mp_moe_padded_rows(E, T * k);
+  b.plan = 0;
+  b.dest = b.plan + align256(4 * mp_moe_plan_ints(E, T * k));
+  b.scale = b.dest + align256(4 * (size_t)T * k);
+  b.q = b.scale + align256(4 * (size_t)b.padded);
+  b.d = b.q + align256((size_t)b.padded * H);
+  b.stage = b.d + align256(2 * (size_t)b.padded * H);
+  b.total = b.stage + mp_moe_expert_stage_workspace_bytes(b.padded, I);
+  return b;
+}
+
+extern "C" size_t mp_moe_experts_scratch_bytes(int T, int H, int k, int num_local_experts, int I) {
+  if (T <= 0 || H <= 0 || k <= 0 || num_local_experts <= 0 || I <= 0) return 0;
+  return layer_buffers(T, H, k, num_local_experts, I).total;
+}
+
+extern "C" size_t mp_moe_experts_workspace_bytes(int T) {
+  if (T <= 0 || T > kStreamTokens) return 0;
+  return w8a8_stream_workspace_bytes(STREAM_SWIGLU, T);
+}
+
+extern "C" int mp_moe_experts(const void* hidden_f16, const void* topk_ids_i32, const void* topk_weights_f16, int T, int H,
+                              int k, int expert_lo, int expert_hi, const void* w13_q_i8, const void* w13_scale_f32,
+                              const void* w2_q_i8, const void* w2_scale_f32, int I, void* out_f16, void* scratch,
+                              size_t scratch_bytes, void* workspace, size_t workspace_bytes, int* error_word,
+                              mp_stream_t stream) {
+  const int E = expert_hi - expert_lo;
+  if (!scratch || T <= 0 || H <= 0 || k <= 0 || I <= 0 || E <= 0 || !w13_q_i8 || !w13_scale_f32 || !w2_q_i8 || !w2_scale_f32 ||
+      !topk_weights_f16 || !out_f16)
+    return MP_ERR_INVALID_ARG;
+  const LayerBuffers b = layer_buffers(T, H, k, E, I);
+  if (scratch_bytes < b.total) return MP_ERR_WORKSPACE;
+  if (!aligned(scratch, 256)) return MP_ERR_ALIGNMENT;
+  unsigned char* base = static_cast<unsigned char*>(scratch);
+  int* plan = reinterpret_cast<int*>(base + b.plan);
+  int* dest = reinterpret_cast<int*>(base + b.dest);
+  float* rscale = reinterpret_cast<float*>(base + b.scale);
+  int8_t* rq = reinterpret_cast<int8_t*>(base + b.q);
+  __half* d = reinterpret_cast<__half*>(base + b.d);
+  int rc = mp_moe_route_gather_quant(hidden_f16, topk_ids_i32, T, H, k, expert_lo, expert_hi, plan, dest, rq, rscale, stream);
+  if (rc != MP_OK) return rc;
+  const size_t stage_bytes = b.total - b.stage;
+  const bool stream_path = T <= kStreamTokens && workspace && H % 16 == 0 && I % 16 == 0 && T * k <= 8192 &&
+                           workspace_bytes >= w8a8_stream_workspace_bytes(STREAM_SWIGLU, T) && aligned(workspace, 16);
+  if (stream_path) {
+    StageBuffers sb;
+    rc = stage_buffers(base + b.stage, stage_bytes, b.padded, I, sb);
+    if (rc != MP_OK) return rc;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    StreamParams p{};
+    p.N = I; p.K = H;
+    p.early_weights = 1;                         // the kernel before is the gather, which waited for the plan
+    p.counts = plan;
+    p.segments = plan + 2 * E;
+    p.experts = E;
+    p.rows_per_expert = 2 * I;
+    p.up_row_offset = I;
+    p.a_scale = rscale;
+    p.b_scale = static_cast<const float*>(w13_scale_f32);
+    p.out = sb.h;
+    p.row_absmax = sb.absmax;
+    p.error_word = error_word;
+    rc = launch_w8a8_stream(STREAM_SWIGLU, rq, b.padded, w13_q_i8, E * 2 * I, p, T, workspace, workspace_bytes, st);
+    if (rc == MP_OK) {
+      const int parts = (I / 8 + 1023) / 1024;   // about a thousand eight-value pieces per block
+      rc = launch_chained(moe_requant_rows_kernel, dim3(T * k, parts), dim3(256), 0, st, static_cast<const __half*>(sb.h),
+                          static_cast<const float*>(sb.absmax), moe_absmax_slots(I), I, static_cast<const int*>(dest), sb.q2,
+                          sb.scale2);
+      if (rc != MP_OK) return rc;
+      StreamParams p2{};
+      p2.N = H; p2.K = I;
+      p2.early_weights = 1;
+      p2.counts = plan;
+      p2.segments = plan + 2 * E;
+      p2.experts = E;
+      p2.rows_per_expert = H;
+      p2.a_scale = sb.scale2;
+      p2.b_scale = static_cast<const float*>(w2_scale_f32);
+      p2.out = d;
+      p2.error_word = error_word;
+      rc = launch_w8a8_stream(STREAM_F16, sb.q2, b.padded, w2_q_i8, E * H, p2, T, workspace, workspace_bytes, st);
+      if (rc != MP_OK) return rc;
+      return mp_moe_combine(d, dest, topk_ids_i32, topk_weights_f16, T, H, k, out_f16, stream);
+    }
+    if (rc != MP_ERR_UNSUPPORTED) return rc;
+  }
+  rc = mp_moe_expert_stage(rq, rscale, plan, b.padded, H, I, E, w13_q_i8, w13_scale_f32, w2_q_i8, w2_scale_f32, d,
+                           base + b.stage, stage_bytes, error_word, stream);
+  if (rc != MP_OK) return rc;
+  return mp_moe_combine(d, dest, topk_ids_i32, topk_weights_f16, T, H, k, out_f16, stream);
 }
 
 extern "C" int mp_moe_combine_after_peers(const void* arrival_words_u32, int world, const void* epoch_counter_u32,

@@ -69,8 +69,7 @@ w4_quantize_groups_kernel(const __half* __restrict__ w, int N, int K, int groups
   for (int v = 0; v < V; ++v) {
     const __half2* h = reinterpret_cast<const __half2*>(&raw[v]);
     const __half2 mx = __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3]));
-    const __half2 neg = __hneg2(__hmin2(__hmin2(h[0], h[1]), __hmin2(h[2], h[3])));
-    m[v] = __hmax2(__lows2half2(mx, neg), __highs2half2(mx, neg));
+    m[v] = max_and_neg_min(mx, __hmin2(__hmin2(h[0], h[1]), __hmin2(h[2], h[3])));
   }
 #pragma unroll
   for (int st = 0; st < S; ++st) {

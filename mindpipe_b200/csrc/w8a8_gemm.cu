@@ -25,6 +25,7 @@
 #include "common.cuh"
 #include "tc.cuh"
 #include "moe_api.cuh"
+#include "w8a8_stream.cuh"
 
 namespace mp {
 
@@ -77,12 +78,6 @@ struct GemmCfg {
   static constexpr int kScaleBytes = 3 * 4 * 256 * 4;   // per epilogue warp: 256 channel scales (+ zero points, row sums)
   static constexpr size_t kSmem = 1024 + (size_t)kStages * (kABytes + kBBytes) + kBarBytes + kScaleBytes;
 };
-
-// acc * s_token * s_channel (+ bias) with every fp32 operation rounded on its own (no contraction into
-// an fma), so that the GEMM epilogue and the split-K reduce kernel produce the same bits.
-__device__ __forceinline__ float scaled_output(int acc, float s_token, float s_channel) {
-  return __fmul_rn(__fmul_rn(static_cast<float>(acc), s_token), s_channel);
-}
 
 // Tile order.  Concurrent CTAs work on consecutive tile numbers; a group of `group_m` M tiles is swept
 // over all N tiles before the next group starts (M fastest inside the group).  The activation rows of
@@ -372,14 +367,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll
             for (int jj = 0; jj < 2; ++jj) {
               const float sg = my_scales[c0 + j + jj], su = my_scales[128 + c0 + j + jj];
-              // the reference rounds gate/up (F.linear output), silu(gate) and the product to fp16
-              const __half g16 = f2h(static_cast<float>(static_cast<int>(rg[j + jj])) * sa * sg);
-              const __half u16 = f2h(static_cast<float>(static_cast<int>(ru[j + jj])) * sa * su);
-              const float gf = h2f(g16);
-              // silu in fp32 with the hardware exp2 / reciprocal: the result is rounded to fp16 right
-              // away (as the reference does), which hides their ~2 ulp fp32 error
-              const __half s16 = f2h(__fdividef(gf, 1.0f + __expf(-gf)));
-              const __half h16 = hmul_t(s16, u16);
+              const __half h16 = swiglu_f16(static_cast<int>(rg[j + jj]), static_cast<int>(ru[j + jj]), sa, sg, su);
               h2v[jj] = h16;
               hmax = fmaxf(hmax, fabsf(h2f(h16)));
             }
@@ -427,21 +415,19 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             }
           } else {
             uint32_t hp[16];
-            long long zx = 0, xs = 0;
+            float zx = 0.0f;
+            int xs = 0;
             if (EPI == EPI_AFFINE && row_ok) {
-              zx = static_cast<long long>(p.a_zero[row]);
+              zx = p.a_zero[row];
               xs = p.a_rowsum[row];
             }
 #pragma unroll
             for (int j = 0; j < 32; j += 2) {
               float v0, v1;
               if (EPI == EPI_AFFINE) {
-                // sum (qx - zx)(qw - zw) = acc - zw * sum(qx) - zx * sum(qw) + K * zx * zw, exactly, in int64
-                const long long zw0 = static_cast<long long>(my_zero[c0 + j]), zw1 = static_cast<long long>(my_zero[c0 + j + 1]);
-                const long long t0 = static_cast<long long>(r[j]) - zw0 * xs - zx * my_wsum[c0 + j] + (long long)p.K * zx * zw0;
-                const long long t1 = static_cast<long long>(r[j + 1]) - zw1 * xs - zx * my_wsum[c0 + j + 1] + (long long)p.K * zx * zw1;
-                v0 = static_cast<float>(t0) * sa * my_scales[c0 + j];
-                v1 = static_cast<float>(t1) * sa * my_scales[c0 + j + 1];
+                v0 = affine_output(static_cast<int>(r[j]), p.K, zx, xs, my_zero[c0 + j], my_wsum[c0 + j], sa, my_scales[c0 + j]);
+                v1 = affine_output(static_cast<int>(r[j + 1]), p.K, zx, xs, my_zero[c0 + j + 1], my_wsum[c0 + j + 1], sa,
+                                   my_scales[c0 + j + 1]);
               } else {
                 v0 = scaled_output(static_cast<int>(r[j]), sa, my_scales[c0 + j]);
                 v1 = scaled_output(static_cast<int>(r[j + 1]), sa, my_scales[c0 + j + 1]);
@@ -562,12 +548,14 @@ int encode_tensor_map_3d(CUtensorMap* map, CUtensorMapDataType dtype, const void
 }
 
 // Sum of the K slices' int32 partial tiles, then the epilogue of the unsplit kernel with the same
-// operations in the same order (so a split changes no output bit): f16(float(acc) * s_token * s_channel (+ bias)),
-// or the raw int32 sum.
-template <bool F16OUT>
+// operations in the same order (so a split changes no output bit).
+template <bool AFFINE>
 __global__ void __launch_bounds__(256)
-w8a8_splitk_reduce_kernel(const int* __restrict__ partial, int k_split, int M, int N, const float* __restrict__ a_scale,
-                          const float* __restrict__ b_scale, const __half* __restrict__ bias, void* __restrict__ out) {
+w8a8_splitk_reduce_kernel(const int* __restrict__ partial, int k_split, int M, int N, int K,
+                          const float* __restrict__ a_scale, const float* __restrict__ b_scale,
+                          const __half* __restrict__ bias, const float* __restrict__ a_zero,
+                          const int* __restrict__ a_rowsum, const float* __restrict__ b_zero,
+                          const int* __restrict__ b_rowsum, void* __restrict__ out) {
   chain_wait();
   chain_release();
   const int quads = N >> 2;
@@ -579,19 +567,17 @@ w8a8_splitk_reduce_kernel(const int* __restrict__ partial, int k_split, int M, i
       const int4 v = *reinterpret_cast<const int4*>(partial + s * slice + (size_t)m * N + n);
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
-    if (F16OUT) {
-      const float sa = a_scale[m];
-      float v0 = scaled_output(acc.x, sa, b_scale[n]), v1 = scaled_output(acc.y, sa, b_scale[n + 1]);
-      float v2 = scaled_output(acc.z, sa, b_scale[n + 2]), v3 = scaled_output(acc.w, sa, b_scale[n + 3]);
-      if (bias) {
-        v0 = __fadd_rn(v0, h2f(bias[n])); v1 = __fadd_rn(v1, h2f(bias[n + 1]));
-        v2 = __fadd_rn(v2, h2f(bias[n + 2])); v3 = __fadd_rn(v3, h2f(bias[n + 3]));
-      }
-      const __half2 lo = __floats2half2_rn(v0, v1), hi = __floats2half2_rn(v2, v3);
-      *reinterpret_cast<uint2*>(static_cast<__half*>(out) + (size_t)m * N + n) = make_uint2(h2_as_u32(lo), h2_as_u32(hi));
-    } else {
-      *reinterpret_cast<int4*>(static_cast<int*>(out) + (size_t)m * N + n) = acc;
+    const float sa = a_scale[m];
+    const int a[4] = {acc.x, acc.y, acc.z, acc.w};
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[i] = AFFINE ? affine_output(a[i], K, a_zero[m], a_rowsum[m], b_zero[n + i], b_rowsum[n + i], sa, b_scale[n + i])
+                    : scaled_output(a[i], sa, b_scale[n + i]);
+      if (bias) v[i] = __fadd_rn(v[i], h2f(bias[n + i]));
     }
+    const __half2 lo = __floats2half2_rn(v[0], v[1]), hi = __floats2half2_rn(v[2], v[3]);
+    *reinterpret_cast<uint2*>(static_cast<__half*>(out) + (size_t)m * N + n) = make_uint2(h2_as_u32(lo), h2_as_u32(hi));
   }
 }
 
@@ -687,12 +673,12 @@ static int w8a8_k_split(int M, int N, int K) {
   return (k_blocks + per - 1) / per;                        // no empty slice
 }
 
-template <bool F16OUT>
+template <bool AFFINE>
 static int launch_splitk_reduce(const GemmCall& c, cudaStream_t st) {
   int blocks = (c.M * (c.N / 4) + 255) / 256;
   if (blocks > 2 * kSmCount) blocks = 2 * kSmCount;
-  return launch_chained(w8a8_splitk_reduce_kernel<F16OUT>, dim3(blocks), dim3(256), 0, st, c.partial, c.k_split, c.M, c.N,
-                        c.a_scale, c.b_scale, c.bias, c.out);
+  return launch_chained(w8a8_splitk_reduce_kernel<AFFINE>, dim3(blocks), dim3(256), 0, st, c.partial, c.k_split, c.M, c.N,
+                        c.K, c.a_scale, c.b_scale, c.bias, c.a_zero, c.a_rowsum, c.b_zero, c.b_rowsum, c.out);
 }
 
 // The CTA-pair form pays once there are enough 256-row tiles to occupy the 74 pairs.
@@ -771,7 +757,7 @@ extern "C" int mp_w8a8_gemm_ex(const void* qx_i8, const void* x_scale_f32, const
     c.partial = static_cast<int*>(workspace);
     rc = launch_gemm<128, EPI_F16>(c, st);
     if (rc != MP_OK) return rc;
-    return launch_splitk_reduce<true>(c, st);
+    return launch_splitk_reduce<false>(c, st);
   }
   const long long tiles256 = (long long)((M + 127) / 128) * ((N + 255) / 256);
   if (N <= 128 || tiles256 < kSmCount) return launch_gemm<128, EPI_F16>(c, st);
@@ -796,6 +782,15 @@ extern "C" int mp_w8a8_affine_gemm(const void* qx_u8, const void* x_scale_f32, c
                                    const void* x_rowsum_i32, const void* w_u8, const void* w_scale_f32,
                                    const void* w_zero_f32, const void* w_rowsum_i32, const void* bias_f16,
                                    void* y_f16, int M, int N, int K, int* error_word, mp_stream_t stream) {
+  return w8a8_affine_gemm(qx_u8, x_scale_f32, x_zero_f32, x_rowsum_i32, w_u8, w_scale_f32, w_zero_f32, w_rowsum_i32, bias_f16,
+                          y_f16, M, N, K, nullptr, 0, error_word, static_cast<cudaStream_t>(stream));
+}
+
+namespace mp {
+int w8a8_affine_gemm(const void* qx_u8, const void* x_scale_f32, const void* x_zero_f32, const void* x_rowsum_i32,
+                     const void* w_u8, const void* w_scale_f32, const void* w_zero_f32, const void* w_rowsum_i32,
+                     const void* bias_f16, void* y_f16, int M, int N, int K, void* workspace, size_t workspace_bytes,
+                     int* error_word, cudaStream_t st) {
   int rc = check_gemm_args(qx_u8, w_u8, y_f16, M, N, K);
   if (rc != MP_OK) return rc;
   if (!x_scale_f32 || !x_zero_f32 || !x_rowsum_i32 || !w_scale_f32 || !w_zero_f32 || !w_rowsum_i32) return MP_ERR_INVALID_ARG;
@@ -806,9 +801,18 @@ extern "C" int mp_w8a8_affine_gemm(const void* qx_u8, const void* x_scale_f32, c
   c.a_zero = static_cast<const float*>(x_zero_f32); c.a_rowsum = static_cast<const int*>(x_rowsum_i32);
   c.b_zero = static_cast<const float*>(w_zero_f32); c.b_rowsum = static_cast<const int*>(w_rowsum_i32);
   c.bias = static_cast<const __half*>(bias_f16); c.out = y_f16; c.error_word = error_word;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (use_pair(M, N)) return launch_gemm<256, EPI_AFFINE, true>(c, st);
+  const int ks = workspace ? w8a8_k_split(M, N, K) : 1;        // without scratch: one K slice per tile
+  if (ks > 1) {
+    if (workspace_bytes < (size_t)ks * M * N * sizeof(int)) return MP_ERR_WORKSPACE;
+    if (!aligned(workspace, 16)) return MP_ERR_ALIGNMENT;
+    c.k_split = ks;
+    c.partial = static_cast<int*>(workspace);
+    rc = launch_gemm<128, EPI_AFFINE>(c, st);
+    return rc != MP_OK ? rc : launch_splitk_reduce<true>(c, st);
+  }
   const long long tiles256 = (long long)((M + 127) / 128) * ((N + 255) / 256);
   if (N <= 128 || tiles256 < kSmCount) return launch_gemm<128, EPI_AFFINE>(c, st);
   return launch_gemm<256, EPI_AFFINE>(c, st);
 }
+}  // namespace mp

@@ -131,12 +131,22 @@ class VllmPackedInt4Linear(nn.Module):
 
     # -- forward ------------------------------------------------------------
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        plan = self._plan
+        plan = self._plan or self._make_plan()
         if plan is not None:
             y = plan.run(self, x)
             if y is not None:
                 return y
         return self._forward_checked(x)
+
+    def _make_plan(self):
+        if not self.weight_packed.is_cuda:
+            return None
+        self._ensure_prepared()
+        self._plan = _native_plan(_lib.host().w4_plan, self,
+                                  ("weight_packed", "weight_scale", "weight_zero_point", "bias", "_scale_zero"),
+                                  self.weight_packed, self._scale_zero, self.bias, self.group_size,
+                                  ops._error_word(self.weight_packed.device).data_ptr())
+        return self._plan
 
     @torch.no_grad()
     def _forward_checked(self, x: torch.Tensor) -> torch.Tensor:
@@ -146,10 +156,7 @@ class VllmPackedInt4Linear(nn.Module):
         if not x2.is_contiguous():
             x2 = x2.contiguous()
         y = ops.w4a16_linear(x2, self.weight_packed, self._scale_zero, self.bias)
-        self._plan = _native_plan(_lib.host().w4_plan, self,
-                                  ("weight_packed", "weight_scale", "weight_zero_point", "bias", "_scale_zero"),
-                                  self.weight_packed, self._scale_zero, self.bias, self.group_size,
-                                  ops._error_word(x2.device).data_ptr())
+        self._make_plan()
         return y.reshape(*shape[:-1], self.out_features)
 
     def forward_host(self, x_host: torch.Tensor, y_host: torch.Tensor | None = None, stream=None,
@@ -358,12 +365,22 @@ class SmoothQuantLinear(nn.Module):
     def forward(self, x):
         """``x`` is an fp16 tensor, or a ``(int8 codes, per-token scale)`` pair produced upstream
         (the tuple input of AscendW8A8DynamicLinearMethod.apply, vllm_ascend.patch:3945-3962)."""
-        plan = self._plan
+        plan = self._plan or self._make_plan()
         if plan is not None:
             y = plan.run(self, x)
             if y is not None:
                 return y
         return self._forward_checked(x)
+
+    def _make_plan(self):
+        if self.quantize_output or not self.weight.is_cuda:
+            return None
+        self._ensure_prepared()
+        self._plan = _native_plan(_lib.host().w8_plan, self,
+                                  ("weight", "weight_scale", "bias", "_weight_scale_fp32", "quantize_output"),
+                                  self.weight, self._weight_scale_fp32, self.bias,
+                                  ops._error_word(self.weight.device).data_ptr())
+        return self._plan
 
     @torch.no_grad()
     def _forward_checked(self, x):
@@ -382,11 +399,7 @@ class SmoothQuantLinear(nn.Module):
         y = ops.w8a8_gemm(q2.contiguous(), s2.contiguous(), self.weight, self._weight_scale_fp32, self.bias)
         if self.quantize_output:
             _, _, y = ops.act_quant_per_token(y, want_codes=False, want_fake=True)
-        else:
-            self._plan = _native_plan(_lib.host().w8_plan, self,
-                                      ("weight", "weight_scale", "bias", "_weight_scale_fp32", "quantize_output"),
-                                      self.weight, self._weight_scale_fp32, self.bias,
-                                      ops._error_word(q2.device).data_ptr())
+        self._make_plan()
         return y.reshape(*lead, self.out_features)
 
     def __repr__(self):
@@ -450,12 +463,21 @@ class QuantLinear(nn.Module):
                 * self.scales.to(torch.float16)[:, None]).to(torch.float16)
 
     def forward(self, input: torch.Tensor) -> torch.Tensor:
-        plan = self._plan
+        plan = self._plan or self._make_plan()
         if plan is not None:
             y = plan.run(self, input)
             if y is not None:
                 return y
         return self._forward_checked(input)
+
+    def _make_plan(self):
+        if not self.weight.is_cuda:
+            return None
+        self._plan = _native_plan(_lib.host().affine_plan, self,
+                                  ("weight", "scales", "zeros", "weight_rowsum", "bias"), self.weight, self.scales,
+                                  self.zeros, self.weight_rowsum, self.bias,
+                                  ops._error_word(self.weight.device).data_ptr())
+        return self._plan
 
     @torch.no_grad()
     def _forward_checked(self, input: torch.Tensor) -> torch.Tensor:
@@ -463,9 +485,7 @@ class QuantLinear(nn.Module):
         x2 = input.reshape(-1, input.shape[-1]).contiguous()
         q, s, z, rs, _ = ops.affine_quant_per_row(x2)
         y = ops.w8a8_affine_gemm(q, s, z, rs, self.weight, self.scales, self.zeros, self.weight_rowsum, self.bias)
-        self._plan = _native_plan(_lib.host().affine_plan, self,
-                                  ("weight", "scales", "zeros", "weight_rowsum", "bias"), self.weight, self.scales,
-                                  self.zeros, self.weight_rowsum, self.bias, ops._error_word(x2.device).data_ptr())
+        self._make_plan()
         return y.reshape(*lead, self.out_features)
 
 
@@ -566,12 +586,22 @@ class SmoothQuantPackedMoeExperts(nn.Module):
                                            expert_range=expert_range, num_experts=num_experts)
 
     def forward(self, hidden_states: torch.Tensor, top_k_index: torch.Tensor, top_k_weights: torch.Tensor):
-        plan = self._plan
+        plan = self._plan or self._make_plan()
         if plan is not None:
             out = plan.run(self, hidden_states, top_k_index, top_k_weights)
             if out is not None:
                 return out
         return self._forward_checked(hidden_states, top_k_index, top_k_weights)
+
+    def _make_plan(self):
+        if not self.gate_up_proj.is_cuda:
+            return None
+        lo, hi = self.expert_range
+        self._plan = _native_plan(_lib.host().moe_plan, self,
+                                  ("gate_up_proj", "gate_up_proj_scale", "down_proj", "down_proj_scale", "expert_range"),
+                                  self.gate_up_proj, self.gate_up_proj_scale, self.down_proj, self.down_proj_scale,
+                                  lo, hi, ops._error_word(self.gate_up_proj.device).data_ptr())
+        return self._plan
 
     @torch.no_grad()
     def _forward_checked(self, hidden_states, top_k_index, top_k_weights):
@@ -584,10 +614,7 @@ class SmoothQuantPackedMoeExperts(nn.Module):
         d = ops.moe_expert_stage(routing.routed_q, routing.routed_scale, routing.plan, hi - lo,
                                  self.gate_up_proj, self.gate_up_proj_scale, self.down_proj, self.down_proj_scale)
         out = ops.moe_combine(d, routing.dest_row, ids, w, hs.shape[0])
-        self._plan = _native_plan(_lib.host().moe_plan, self,
-                                  ("gate_up_proj", "gate_up_proj_scale", "down_proj", "down_proj_scale", "expert_range"),
-                                  self.gate_up_proj, self.gate_up_proj_scale, self.down_proj, self.down_proj_scale,
-                                  lo, hi, ops._error_word(hs.device).data_ptr())
+        self._make_plan()
         return out.reshape(shape)
 
     def __repr__(self):

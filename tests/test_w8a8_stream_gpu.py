@@ -1,0 +1,89 @@
+"""The weight-streaming W8A8 product against the tiled GEMM: integer sums and the same output arithmetic, so the same
+bits, at the row counts where its tiles change, ragged shapes and cuts of K over many blocks."""
+import numpy as np
+import pytest
+import torch
+
+from mindpipe_b200 import ops
+from mindpipe_b200.modules import QuantLinear, SmoothQuantLinear, SmoothQuantPackedMoeExperts
+from oracle import pseudo_quant as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _linear(n, k, bias):
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    lin = torch.nn.Linear(k, n, bias=bias, device="cuda", dtype=torch.float16)
+    with torch.no_grad():
+        lin.weight.normal_(0, 0.02, generator=g)
+        lin.weight[0] = lin.weight[0].abs() + 0.01             # one-sided rows: zero points outside the codes
+        lin.weight[n // 2] = -lin.weight[n // 2].abs() - 0.01
+    return lin
+
+
+@pytest.mark.parametrize("kind", [SmoothQuantLinear.from_float, QuantLinear], ids=["symmetric", "affine"])
+@pytest.mark.parametrize("m", [1, 16, 17, 32, 33, 64, 65, 128, 129])
+@pytest.mark.parametrize("n,k", [(40, 512), (384, 4112), (1026, 1024), (20480, 256), (256, 16384), (4096, 4096)])
+def test_streamed_product_gives_the_tiled_gemm_s_bits(kind, m, n, k):
+    mod = kind(_linear(n, k, bias=m % 2 == 0))
+    x = torch.randn(m, k, device="cuda").half()
+    x[:, ::97] *= 20
+    x[m // 2] = x[m // 2].abs() + 1
+    want = mod._forward_checked(x)
+    assert mod._plan is not None
+    for _ in range(3):
+        assert torch.equal(mod(x), want)
+    ops.check_device_errors()
+
+
+@pytest.mark.filterwarnings("ignore::RuntimeWarning")
+@pytest.mark.parametrize("k", [8, 1024, 2056, 4096, 8192, 11008, 16392])
+def test_affine_quantiser_bit_exact_at_every_row_length(k):
+    rng = np.random.default_rng(k)
+    x = rng.normal(0, 1, (12, k))
+    x[0], x[1], x[2] = 0.0, 3.25, -np.abs(x[2]) - 5.0          # constant and one-sided rows
+    x[3], x[4] = np.abs(x[3]) * 1e-3 + 50.0, x[4] * 1e-5       # far from zero; scale below 2^-14
+    x[5], x[6, 0] = x[5] * 9000.0, 60000.0
+    x[7] = np.arange(k) % 511 * 0.25
+    x = x.astype(np.float16)
+    q, s, z, rs, f = ops.affine_quant_per_row(torch.from_numpy(x).cuda(), want_fake=True)
+    fake, codes, sc, zp = O.affine_quant_last_dim(x)
+    assert np.array_equal(q.cpu().numpy(), codes)
+    assert np.array_equal(s.cpu().numpy(), sc.astype(np.float32).reshape(-1))
+    assert np.array_equal(z.cpu().numpy(), zp.astype(np.float32).reshape(-1))
+    assert np.array_equal(rs.cpu().numpy(), codes.astype(np.int64).sum(axis=1).astype(np.int32))
+    assert np.array_equal(f.cpu().numpy(), fake)
+
+
+@pytest.mark.parametrize("t", [1, 16, 17, 33, 64, 65])
+@pytest.mark.parametrize("e,h,i,k", [(4, 256, 384, 2), (8, 1024, 144, 2), (40, 512, 272, 4)])
+@pytest.mark.parametrize("routing", ["random", "one expert", "twice the same"])
+def test_expert_layer_of_few_tokens_gives_the_staged_layer_s_bits(t, e, h, i, k, routing):
+    g = torch.Generator(device="cuda").manual_seed(t + e)
+    mod = SmoothQuantPackedMoeExperts(torch.randn(e, 2 * i, h, generator=g, device="cuda").half() * 0.05,
+                                      torch.randn(e, h, i, generator=g, device="cuda").half() * 0.05)
+    x = torch.randn(t, h, generator=g, device="cuda").half()
+    ids = torch.rand(t, e, generator=g, device="cuda").topk(k, dim=1).indices.int()
+    if routing == "one expert":
+        ids = torch.arange(k, device="cuda", dtype=torch.int32).expand(t, k).contiguous()
+    elif routing == "twice the same":
+        ids[:, 1] = ids[:, 0]
+    w = torch.rand(t, k, generator=g, device="cuda").half()
+    want = mod._forward_checked(x, ids, w)
+    assert mod._plan is not None
+    for _ in range(3):
+        assert torch.equal(mod(x, ids, w), want)
+    ops.check_device_errors()
+
+
+@pytest.mark.parametrize("e", [4, 8, 12, 32, 40])
+def test_router_matches_softmax_topk_at_every_width(e):
+    logits = torch.randn(300, e, device="cuda") * 2
+    logits[0] = 0.5                                            # all equal: lower indices first
+    logits[1, 1], logits[1, 3] = 9.0, 9.0
+    idx, w = ops.moe_router_topk(logits, 2)
+    p = logits.softmax(dim=-1)
+    top, ref = p.sort(dim=-1, descending=True, stable=True)
+    assert torch.equal(idx.long(), ref[:, :2])
+    want = top[:, :2] / top[:, :2].sum(dim=-1, keepdim=True)
+    assert (w.float() - want).abs().max().item() <= 1e-3
