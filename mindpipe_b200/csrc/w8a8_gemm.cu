@@ -2,10 +2,10 @@
 // then a scale epilogue.  One persistent CTA per SM, warp specialised:
 //
 //   warp 0     TMA producer: 128-byte-swizzled [128 x 128 B] activation tile and
-//              [BN x 128 B] weight tile per stage, multi-stage mbarrier ring
-//   warp 1     MMA issuer: tcgen05.mma kind::i8 (M=128, N=BN, K=32), four per
+//              [bn x 128 B] weight tile per stage, multi-stage mbarrier ring
+//   warp 1     MMA issuer: tcgen05.mma kind::i8 (M=128, N=bn, K=32), four per
 //              stage; tcgen05.commit releases the stage / publishes the tile
-//   warps 2-5  epilogue: tcgen05.ld the int32 accumulators (TMEM is double
+//   warps 2-9  epilogue (two warps to a quarter of the rows, 32 columns in turn): tcgen05.ld the int32 accumulators (TMEM is double
 //              buffered, so this overlaps the next tile's main loop), apply
 //              acc * s_token[m] * s_channel[n] (+bias) and store
 //
@@ -20,8 +20,15 @@
 // expert * rows_per_expert (segments are 256-row aligned, so a CTA pair's 256-row
 // tile belongs to one expert as well).
 //
+// The epilogue's columns come from one table entry each (a broadcast 8- or 16-byte load); with zero points the table holds
+// the integers of the exact sum, so an element costs two 32-bit multiply-adds more than a symmetric one.  Four epilogue
+// warps, three loads and four float <-> integer conversions an element took 51.8 us where the symmetric product took 27.8
+// (333 x 12288 x 4096); now 21.9 and 21.1.
+//
 // Every mbarrier wait is bounded; on a timeout the block records an error
 // word, lets its copies land, frees its TMEM and returns.
+#include <algorithm>
+
 #include "common.cuh"
 #include "tc.cuh"
 #include "moe_api.cuh"
@@ -34,12 +41,15 @@ using namespace tc;
 constexpr int kBM = 128;
 constexpr int kBK = 128;      // int8 elements (= bytes) of K per stage
 constexpr int kUmmaK = 32;    // K of one kind::i8 instruction
+constexpr int kEpilogueWarps = 8;               // two per quarter of the tile's rows, half of its columns each
+constexpr int kThreads = 64 + 32 * kEpilogueWarps;
 
 enum : int { EPI_F16 = 0, EPI_I32 = 1, EPI_SWIGLU = 2, EPI_AFFINE = 3 };   // AFFINE: unsigned codes with zero points
 
 struct GemmParams {
   int M, N, K;
   int m_tiles, n_tiles, k_blocks;
+  int bn;                      // columns of a tile, a multiple of 32
   int k_split;                 // > 1: a tile's K range is cut into this many work items of kb_per_split k-blocks,
   int kb_per_split;            //      whose raw int32 partial tiles go to `partial` ([k_split][M][N])
   int* partial;
@@ -63,21 +73,27 @@ struct GemmParams {
   int* error_word;
 };
 
-// PAIR: two CTAs (a cluster of 2) share each MMA -- a 256 x BN tile, 128 rows of A and of the
-// accumulator per CTA, and each CTA stages only its half of the BN weight rows.  Per CTA and k-block
-// the shared memory then carries 16 KB (A) + BN/2 x 128 B (B) in and the same out, instead of
-// 16 KB + BN x 128 B: at BN = 256 that is 64 KB rather than 96 KB per 512 tensor cycles, which takes
+// PAIR: two CTAs (a cluster of 2) share each MMA -- a 256 x bn tile, 128 rows of A and of the
+// accumulator per CTA, and each CTA stages only its half of the bn weight rows.  Per CTA and k-block
+// the shared memory then carries 16 KB (A) + bn/2 x 128 B (B) in and the same out, instead of
+// 16 KB + bn x 128 B: at bn = 256 that is 64 KB rather than 96 KB per 512 tensor cycles, which takes
 // the kernel off the 128 B/clk shared-memory limit that held the single-CTA form at ~70 % tensor use.
-template <int BN, bool PAIR = false>
-struct GemmCfg {
-  static constexpr int kABytes = kBM * kBK;
-  static constexpr int kBBytes = (PAIR ? BN / 2 : BN) * kBK;
-  static constexpr int kStages = PAIR ? (BN == 256 ? 6 : 8) : (BN == 256 ? 4 : 6);
-  static constexpr int kTmemCols = 2 * BN;
-  static constexpr int kBarBytes = 256;
-  static constexpr int kScaleBytes = 3 * 4 * 256 * 4;   // per epilogue warp: 256 channel scales (+ zero points, row sums)
-  static constexpr size_t kSmem = 1024 + (size_t)kStages * (kABytes + kBBytes) + kBarBytes + kScaleBytes;
-};
+constexpr int kABytes = kBM * kBK;
+constexpr int kMaxStages = 8;
+constexpr int kBarBytes = 256;
+constexpr int kColumnBytes = kEpilogueWarps * 128 * 16;   // per epilogue warp: what its <= 128 columns need
+constexpr int kTmemCols = 512;                            // two accumulators of up to 256 columns
+constexpr int kMaxBN = 256;
+
+__host__ __device__ constexpr int b_stage_bytes(int bn, bool pair) { return (pair ? bn / 2 : bn) * kBK; }
+// as many stages as 192 KB hold, eight at most
+__host__ __device__ constexpr int gemm_stages(int bn, bool pair) {
+  const int n = 196608 / (kABytes + b_stage_bytes(bn, pair));
+  return n < kMaxStages ? n : kMaxStages;
+}
+constexpr size_t gemm_smem(int bn, bool pair) {
+  return 1024 + (size_t)gemm_stages(bn, pair) * (kABytes + b_stage_bytes(bn, pair)) + kBarBytes + kColumnBytes;
+}
 
 // Tile order.  Concurrent CTAs work on consecutive tile numbers; a group of `group_m` M tiles is swept
 // over all N tiles before the next group starts (M fastest inside the group).  The activation rows of
@@ -112,20 +128,20 @@ __device__ __forceinline__ void tile_coords_grouped(int tile, int n_tiles, const
   n_tile = in_group / gsize;
 }
 
-template <int BN, int EPI, bool PAIR>
-__global__ void __launch_bounds__(192, 1)
+template <int EPI, bool PAIR>
+__global__ void __launch_bounds__(kThreads, 1)
 w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const GemmParams p) {
-  using Cfg = GemmCfg<BN, PAIR>;
-  constexpr int STAGES = Cfg::kStages;
+  const int bn = EPI == EPI_SWIGLU ? kMaxBN : p.bn;
+  const int b_bytes = b_stage_bytes(bn, PAIR), STAGES = gemm_stages(bn, PAIR);
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sA = smem;
-  unsigned char* sB = smem + STAGES * Cfg::kABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sB + STAGES * Cfg::kBBytes);
+  unsigned char* sB = smem + STAGES * kABytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sB + STAGES * b_bytes);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* s_scales = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(bars) + Cfg::kBarBytes);
+  int4* s_columns = reinterpret_cast<int4*>(reinterpret_cast<unsigned char*>(bars) + kBarBytes);
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
   const uint32_t tfull0 = smem_u32(bars + 2 * STAGES), tempty0 = smem_u32(bars + 2 * STAGES + 2);
 
@@ -135,24 +151,28 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   // commits arrive on.  Every WAIT in the kernel is on a barrier of the waiting CTA.
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
   const bool leader = rank == 0;
+  __shared__ float s_hmax[2][kBM];                 // SWIGLU: the row maxima of the second half of a tile's columns ...
+  __shared__ uint64_t s_hmax_bar[2][4];            // ... per accumulator buffer and quarter of the rows
   if (threadIdx.x == 0) {
+    if (EPI == EPI_SWIGLU)
+      for (int i = 0; i < 8; ++i) mbar_init(smem_u32(&s_hmax_bar[i >> 2][i & 3]), 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull0 + 8 * b, 1);
-      mbar_init(tempty0 + 8 * b, PAIR ? 8 : 4);     // one arrival per epilogue warp (of both CTAs)
+      mbar_init(tempty0 + 8 * b, PAIR ? 2 * kEpilogueWarps : kEpilogueWarps);     // one arrival per epilogue warp (of both CTAs)
     }
     *abort_flag = 0;
     fence_mbar_init();
   }
   if (warp == 1) {
     if (PAIR) {
-      tmem_alloc_pair(smem_u32(tmem_slot), Cfg::kTmemCols);
+      tmem_alloc_pair(smem_u32(tmem_slot), kTmemCols);
       tmem_relinquish_pair();
     } else {
-      tmem_alloc(smem_u32(tmem_slot), Cfg::kTmemCols);
+      tmem_alloc(smem_u32(tmem_slot), kTmemCols);
       tmem_relinquish();
     }
   }
@@ -228,25 +248,25 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           if (PAIR) {
             // both CTAs' bytes are counted on the leader's barrier
             const uint32_t full = map_to_cta(full0 + 8 * stage, 0);
-            if (leader) mbar_arrive_expect_tx(full0 + 8 * stage, 2 * (Cfg::kABytes + Cfg::kBBytes));
-            tma_load_2d_pair(smem_u32(sA + stage * Cfg::kABytes), &tmap_a, full, kb * kBK, m0);
+            if (leader) mbar_arrive_expect_tx(full0 + 8 * stage, 2 * (kABytes + b_bytes));
+            tma_load_2d_pair(smem_u32(sA + stage * kABytes), &tmap_a, full, kb * kBK, m0);
             // this CTA's half of the tile's weight rows; with SwiGLU the halves are the gate rows
             // (accumulator columns [0,128)) and the matching up rows (columns [128,256))
             const int b_row = EPI == EPI_SWIGLU
                                   ? e_row0 + (rank ? p.up_row_offset : 0) + n_tile * 128
-                                  : e_row0 + n_tile * BN + static_cast<int>(rank) * (BN / 2);
-            tma_load_2d_pair(smem_u32(sB + stage * Cfg::kBBytes), &tmap_b, full, kb * kBK, b_row);
+                                  : e_row0 + n_tile * bn + static_cast<int>(rank) * (bn / 2);
+            tma_load_2d_pair(smem_u32(sB + stage * b_bytes), &tmap_b, full, kb * kBK, b_row);
           } else {
             const uint32_t full = full0 + 8 * stage;
-            mbar_arrive_expect_tx(full, Cfg::kABytes + Cfg::kBBytes);
-            tma_load_2d(smem_u32(sA + stage * Cfg::kABytes), &tmap_a, full, kb * kBK, m0);
+            mbar_arrive_expect_tx(full, kABytes + b_bytes);
+            tma_load_2d(smem_u32(sA + stage * kABytes), &tmap_a, full, kb * kBK, m0);
             if (EPI == EPI_SWIGLU) {
               // gate rows then the matching up rows: the tile's columns [0,128) and [128,256)
-              const uint32_t dst = smem_u32(sB + stage * Cfg::kBBytes);
+              const uint32_t dst = smem_u32(sB + stage * b_bytes);
               tma_load_2d(dst, &tmap_b, full, kb * kBK, e_row0 + n_tile * 128);
               tma_load_2d(dst + 128 * kBK, &tmap_b, full, kb * kBK, e_row0 + p.up_row_offset + n_tile * 128);
             } else {
-              tma_load_2d(smem_u32(sB + stage * Cfg::kBBytes), &tmap_b, full, kb * kBK, e_row0 + n_tile * BN);
+              tma_load_2d(smem_u32(sB + stage * b_bytes), &tmap_b, full, kb * kBK, e_row0 + n_tile * bn);
             }
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -255,8 +275,8 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp == 1) {
     if (leader && elect_one()) {
-      constexpr uint32_t idesc =
-          umma_idesc(kIdescDFormatS32 | (EPI == EPI_AFFINE ? kIdescABFormatU8 : kIdescABFormatS8), kRowsPerTile, BN);
+      const uint32_t idesc =
+          umma_idesc(kIdescDFormatS32 | (EPI == EPI_AFFINE ? kIdescABFormatU8 : kIdescABFormatS8), kRowsPerTile, bn);
       int stage = 0;
       uint32_t phase = 0;
       int buf = 0;
@@ -266,12 +286,12 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const int kb0 = (work % p.k_split) * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
         if (!mbar_wait(tempty0 + 8 * buf, buf_phase ^ 1, abort_flag)) break;
         tcgen05_fence_after();
-        const uint32_t d_tmem = tmem_base + buf * BN;
+        const uint32_t d_tmem = tmem_base + buf * kMaxBN;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(full0 + 8 * stage, phase, abort_flag)) { ok = false; break; }
           tcgen05_fence_after();
-          const uint64_t a_desc = umma_desc_k_sw128(smem_u32(sA + stage * Cfg::kABytes));
-          const uint64_t b_desc = umma_desc_k_sw128(smem_u32(sB + stage * Cfg::kBBytes));
+          const uint64_t a_desc = umma_desc_k_sw128(smem_u32(sA + stage * kABytes));
+          const uint64_t b_desc = umma_desc_k_sw128(smem_u32(sB + stage * b_bytes));
 #pragma unroll
           for (int kk = 0; kk < kBK / kUmmaK; ++kk) {
             // advancing K by 32 bytes inside the 128-byte swizzle row: +2 in 16-byte address units
@@ -300,10 +320,13 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       }
     }
   } else {
-    const int quarter = warp & 3;               // TMEM lanes [32*quarter, +32) belong to this warp
-    float* my_scales = s_scales + quarter * 768; // this warp's copy of the tile's channel scales
-    float* my_zero = my_scales + 256;             // AFFINE: channel zero points ...
-    int* my_wsum = reinterpret_cast<int*>(my_scales + 512);   // ... and channel code sums
+    const int quarter = warp & 3;               // TMEM lanes [32*quarter, +32) belong to this warp ...
+    const int half = (warp - 2) >> 2;           // ... and every other 32 of the tile's output columns
+    const int cols = EPI == EPI_SWIGLU ? 128 : bn;
+    // this warp's table of its columns: {scale, bias}, AFFINE {zero, sum - K * zero, scale, bias}, SWIGLU {gate scale,
+    // up scale}; one broadcast load per column or two.  A bias that is not there is -0, which added changes no value.
+    int4* column4 = s_columns + (warp - 2) * 128;
+    float2* column2 = reinterpret_cast<float2*>(column4);
     int buf = 0;
     uint32_t buf_phase = 0;
     const uint32_t tempty_leader0 = PAIR ? map_to_cta(tempty0, 0) : tempty0;
@@ -312,24 +335,29 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       int m_tile, n_tile;
       coords(tile, m_tile, n_tile);
       const int e_row0 = p.tile_expert ? p.tile_expert[PAIR ? 2 * m_tile : m_tile] * p.b_rows_per_expert : 0;
-      // channel scales of this tile -> shared memory (each warp keeps its own copy: no cross-warp barrier)
-      if (EPI != EPI_I32) {
+      const int n0 = n_tile * cols;
+      bool wide = false;                        // AFFINE: a zero point beyond the codes
+      if (EPI != EPI_I32 && p.k_split == 1) {
         __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int c = lane + 32 * i;             // column of the accumulator tile
-          int n, src;
+        for (int c0 = 32 * half; c0 < cols; c0 += 64) {
+          const int c = (c0 >> 1 & ~31) + lane, n = n0 + c0 + lane;      // place in the table, output column
+          const bool in = n < p.N;
+          const float scale = in ? __ldg(p.b_scale + e_row0 + n) : 0.0f;
           if (EPI == EPI_SWIGLU) {
-            n = n_tile * 128 + (c & 127);
-            src = e_row0 + (c >= 128 ? p.up_row_offset : 0) + n;
+            column2[c] = make_float2(scale, in ? __ldg(p.b_scale + e_row0 + p.up_row_offset + n) : 0.0f);
           } else {
-            n = n_tile * BN + c;
-            src = e_row0 + n;
-          }
-          my_scales[c] = (c < BN && n < p.N) ? __ldg(p.b_scale + src) : 0.0f;
-          if (EPI == EPI_AFFINE) {
-            my_zero[c] = (c < BN && n < p.N) ? __ldg(p.b_zero + src) : 0.0f;
-            my_wsum[c] = (c < BN && n < p.N) ? __ldg(p.b_rowsum + src) : 0;
+            const float bias = in && p.bias ? h2f(p.bias[n]) : -0.0f;
+            if (EPI == EPI_AFFINE) {
+              const float zw = in ? __ldg(p.b_zero + n) : 0.0f;
+              wide |= !(zw >= 0.0f && zw <= 255.0f);
+              const unsigned int w = wide ? 0u : static_cast<unsigned int>(zw);
+              column4[c] = make_int4(static_cast<int>(w),
+                                     static_cast<int>((in ? static_cast<unsigned int>(__ldg(p.b_rowsum + n)) : 0u) -
+                                                      static_cast<unsigned int>(p.K) * w),
+                                     __float_as_int(scale), __float_as_int(bias));
+            } else {
+              column2[c] = make_float2(scale, bias);
+            }
           }
         }
         __syncwarp();
@@ -349,13 +377,13 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         out_row = static_cast<__half*>(p.scatter.back[home_rank]) + (size_t)home_row * p.N;
       }
       const float sa = (EPI != EPI_I32 && row_ok) ? p.a_scale[row] : 0.0f;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * kMaxBN;
       if (EPI == EPI_SWIGLU) {
-        const int n0 = n_tile * 128;
         float hmax = 0.0f;
         __half* out = static_cast<__half*>(p.out);
 #pragma unroll 1
-        for (int c0 = 0; c0 < 128; c0 += 32) {
+        for (int c0 = 32 * half; c0 < 128; c0 += 64) {
+          const float2* col2 = column2 + (c0 >> 1 & ~31);
           uint32_t rg[32], ru[32];
           tmem_ld_32x32(taddr + c0, rg);
           tmem_ld_32x32(taddr + 128 + c0, ru);
@@ -366,8 +394,8 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             __half h2v[2];
 #pragma unroll
             for (int jj = 0; jj < 2; ++jj) {
-              const float sg = my_scales[c0 + j + jj], su = my_scales[128 + c0 + j + jj];
-              const __half h16 = swiglu_f16(static_cast<int>(rg[j + jj]), static_cast<int>(ru[j + jj]), sa, sg, su);
+              const float2 col = col2[j + jj];
+              const __half h16 = swiglu_f16(static_cast<int>(rg[j + jj]), static_cast<int>(ru[j + jj]), sa, col.x, col.y);
               h2v[jj] = h16;
               hmax = fmaxf(hmax, fabsf(h2f(h16)));
             }
@@ -389,11 +417,32 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             }
           }
         }
-        if (row_ok) p.row_absmax[(size_t)row * p.n_tiles + n_tile] = hmax;   // one slot per (row, column tile): no atomics, nothing to zero
+        // one slot per (row, column tile): no atomics, nothing to zero.  The two halves of the columns meet in shared
+        // memory, in one place per accumulator buffer, which the second half writes again only after the first half has
+        // released that buffer.
+        if (half) {
+          s_hmax[buf][quarter * 32 + lane] = hmax;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&s_hmax_bar[buf][quarter]));
+        } else {
+          if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_hmax_bar[buf][quarter]), buf_phase, abort_flag))) break;
+          if (row_ok)
+            p.row_absmax[(size_t)row * p.n_tiles + n_tile] = fmaxf(hmax, s_hmax[buf][quarter * 32 + lane]);
+        }
       } else {
-        const int n0 = n_tile * BN;
+        float zx = 0.0f;
+        int xs = 0;
+        unsigned int x = 0;
+        if (EPI == EPI_AFFINE && p.k_split == 1) {
+          zx = row_ok ? p.a_zero[row] : 0.0f;
+          xs = row_ok ? p.a_rowsum[row] : 0;
+          wide = __any_sync(0xffffffffu, wide || !(zx >= 0.0f && zx <= 255.0f));
+          x = wide ? 0u : static_cast<unsigned int>(zx);
+        }
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
+        for (int c0 = 32 * half; c0 < bn; c0 += 64) {
+          const int4* col4 = column4 + (c0 >> 1 & ~31);
+          const float2* col2 = column2 + (c0 >> 1 & ~31);
           uint32_t r[32];
           tmem_ld_32x32(taddr + c0, r);
           tmem_ld_wait();
@@ -415,29 +464,34 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             }
           } else {
             uint32_t hp[16];
-            float zx = 0.0f;
-            int xs = 0;
-            if (EPI == EPI_AFFINE && row_ok) {
-              zx = p.a_zero[row];
-              xs = p.a_rowsum[row];
+            if (EPI == EPI_AFFINE && wide) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                const int n = n0 + c0 + j;
+                const float v = n < p.N ? __fadd_rn(affine_output(static_cast<int>(r[j]), p.K, zx, xs, p.b_zero[n], p.b_rowsum[n],
+                                                                  sa, p.b_scale[n]),
+                                                    __int_as_float(col4[j].w))
+                                        : 0.0f;
+                r[j] = __float_as_uint(v);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                if (EPI == EPI_AFFINE) {
+                  // both zero points lie in [0, 255], so the true value fits 32 bits and wrapping products are exact
+                  const int4 col = col4[j];
+                  const int t = static_cast<int>(r[j] - static_cast<unsigned int>(col.x) * static_cast<unsigned int>(xs) -
+                                                 x * static_cast<unsigned int>(col.y));
+                  r[j] = __float_as_uint(__fadd_rn(scaled_output(t, sa, __int_as_float(col.z)), __int_as_float(col.w)));
+                } else {
+                  const float2 col = col2[j];
+                  r[j] = __float_as_uint(__fadd_rn(scaled_output(static_cast<int>(r[j]), sa, col.x), col.y));
+                }
+              }
             }
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              float v0, v1;
-              if (EPI == EPI_AFFINE) {
-                v0 = affine_output(static_cast<int>(r[j]), p.K, zx, xs, my_zero[c0 + j], my_wsum[c0 + j], sa, my_scales[c0 + j]);
-                v1 = affine_output(static_cast<int>(r[j + 1]), p.K, zx, xs, my_zero[c0 + j + 1], my_wsum[c0 + j + 1], sa,
-                                   my_scales[c0 + j + 1]);
-              } else {
-                v0 = scaled_output(static_cast<int>(r[j]), sa, my_scales[c0 + j]);
-                v1 = scaled_output(static_cast<int>(r[j + 1]), sa, my_scales[c0 + j + 1]);
-              }
-              if (p.bias) {
-                if (n0 + c0 + j < p.N) v0 = __fadd_rn(v0, h2f(p.bias[n0 + c0 + j]));
-                if (n0 + c0 + j + 1 < p.N) v1 = __fadd_rn(v1, h2f(p.bias[n0 + c0 + j + 1]));
-              }
-              hp[j >> 1] = h2_as_u32(__floats2half2_rn(v0, v1));
-            }
+            for (int j = 0; j < 32; j += 2)
+              hp[j >> 1] = h2_as_u32(__floats2half2_rn(__uint_as_float(r[j]), __uint_as_float(r[j + 1])));
             if (row_ok) {
               __half* dst = out_row + n0 + c0;
               if (n0 + c0 + 32 <= p.N && (p.N % 8) == 0) {
@@ -487,9 +541,9 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   if (warp == 1) {
     tcgen05_fence_after();
     if (PAIR) {
-      tmem_dealloc_pair(tmem_base, Cfg::kTmemCols);
+      tmem_dealloc_pair(tmem_base, kTmemCols);
     } else {
-      tmem_dealloc(tmem_base, Cfg::kTmemCols);
+      tmem_dealloc(tmem_base, kTmemCols);
     }
   }
 }
@@ -581,8 +635,15 @@ w8a8_splitk_reduce_kernel(const int* __restrict__ partial, int k_split, int M, i
   }
 }
 
+// How a product is cut: 256-row tiles on CTA pairs or 128-row tiles on single CTAs, the tile's columns, K slices.
+struct GemmShape {
+  bool pair;
+  int bn;
+  int k_split;
+};
+
 struct GemmCall {
-  int k_split = 1; int* partial = nullptr;
+  int* partial = nullptr;
   const RowScatter* scatter = nullptr;
   const float* a_zero = nullptr; const int* a_rowsum = nullptr; const float* b_zero = nullptr; const int* b_rowsum = nullptr;
   const void* a; const void* b;
@@ -597,20 +658,21 @@ struct GemmCall {
   int tile_part = -1;
 };
 
-template <int BN, int EPI, bool PAIR = false>
-static int launch_gemm(const GemmCall& c, cudaStream_t st) {
-  using Cfg = GemmCfg<BN, PAIR>;
+template <int EPI, bool PAIR>
+static int launch_gemm(const GemmCall& c, const GemmShape& shape, cudaStream_t st) {
+  const int bn = shape.bn;
   CUtensorMap ta, tb;
   int rc = encode_tensor_map_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, c.a, (uint64_t)c.K, (uint64_t)c.a_rows,
                                 (uint64_t)c.K, kBK, kBM);
   if (rc != MP_OK) return rc;
   rc = encode_tensor_map_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, c.b, (uint64_t)c.K, (uint64_t)c.b_rows_total,
-                            (uint64_t)c.K, kBK, PAIR ? BN / 2 : (EPI == EPI_SWIGLU ? 128 : BN));
+                            (uint64_t)c.K, kBK, PAIR ? bn / 2 : (EPI == EPI_SWIGLU ? 128 : bn));
   if (rc != MP_OK) return rc;
   GemmParams p{};
   p.M = c.M; p.N = c.N; p.K = c.K;
   p.m_tiles = (c.a_rows + kBM - 1) / kBM;
-  p.n_tiles = (c.N + (EPI == EPI_SWIGLU ? 128 : BN) - 1) / (EPI == EPI_SWIGLU ? 128 : BN);
+  p.bn = bn;
+  p.n_tiles = (c.N + (EPI == EPI_SWIGLU ? 128 : bn) - 1) / (EPI == EPI_SWIGLU ? 128 : bn);
   p.k_blocks = (c.K + kBK - 1) / kBK;
   p.m_tiles_dev = c.m_tiles_dev; p.tile_expert = c.tile_expert;
   p.b_rows_per_expert = c.b_rows_per_expert; p.up_row_offset = c.up_row_offset;
@@ -618,27 +680,27 @@ static int launch_gemm(const GemmCall& c, cudaStream_t st) {
   p.row_absmax = c.row_absmax; p.error_word = c.error_word;
   p.group_m = PAIR ? 8 : 16;            // 2048 activation rows per group
   p.tile_part = c.m_tiles_dev ? c.tile_part : -1;
-  p.k_split = c.k_split > 1 ? c.k_split : 1;
+  p.k_split = shape.k_split;
   p.kb_per_split = (p.k_blocks + p.k_split - 1) / p.k_split;
   p.partial = c.partial;
   if (c.scatter) p.scatter = *c.scatter;
   p.a_zero = c.a_zero; p.a_rowsum = c.a_rowsum; p.b_zero = c.b_zero; p.b_rowsum = c.b_rowsum;
-  auto kern = w8a8_gemm_kernel<BN, EPI, PAIR>;
+  auto kern = w8a8_gemm_kernel<EPI, PAIR>;
   static thread_local int configured_device = -1;
   int device = 0;
   MP_CUDA_TRY(cudaGetDevice(&device));
   if (configured_device != device) {
-    MP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem));
+    MP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem(kMaxBN, PAIR)));
     configured_device = device;
   }
   if (PAIR) {
     // one cluster of two CTAs per 256-row tile in flight: 74 pairs fill the 148 SMs
-    const long long total = (long long)((p.m_tiles + 1) / 2) * p.n_tiles;
+    const long long total = (long long)((p.m_tiles + 1) / 2) * p.n_tiles * p.k_split;
     const int pairs = (int)(total < kSmCount / 2 ? total : kSmCount / 2);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(2 * pairs, 1, 1);
-    cfg.blockDim = dim3(192, 1, 1);
-    cfg.dynamicSmemBytes = Cfg::kSmem;
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = gemm_smem(bn, PAIR);
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -654,36 +716,84 @@ static int launch_gemm(const GemmCall& c, cudaStream_t st) {
   }
   const long long total = (long long)p.m_tiles * p.n_tiles * p.k_split;
   const int grid = (int)(total < kSmCount ? total : kSmCount);
-  return launch_chained(kern, dim3(grid), dim3(192), Cfg::kSmem, st, ta, tb, p);
+  return launch_chained(kern, dim3(grid), dim3(kThreads), gemm_smem(bn, PAIR), st, ta, tb, p);
 }
 
-// Few output tiles (decode and small batches: the GEMM is a weight stream, and a CTA sustains only
-// ~130 GB/s on its own): cut K until about one work item per SM exists.  Needs N % 4 == 0.
-static int w8a8_k_split(int M, int N, int K) {
-  if (N % 4 != 0 || N <= 128) return 1;
-  const long long tiles256 = (long long)((M + 127) / 128) * ((N + 255) / 256);
-  if (tiles256 >= kSmCount) return 1;                       // the 128 x 256 form fills the machine
-  const int tiles = ((M + 127) / 128) * ((N + 127) / 128);  // 128 x 128 tiles are used below that
+// The most K slices the caller's scratch has room for (1: no scratch): as many as bring 128 x 128 tiles to one work item
+// per SM, of four k-blocks at least.  Needs N % 4 == 0.
+static int max_k_split(int M, int N, int K) {
+  if (N % 4 != 0 || N <= 128 || (long long)((M + 255) / 256) * ((N + 255) / 256) >= kSmCount / 2) return 1;
+  const int tiles = ((M + 127) / 128) * ((N + 127) / 128);
   const int k_blocks = (K + kBK - 1) / kBK;
-  int ks = kSmCount / tiles;
-  if (ks > k_blocks / 4) ks = k_blocks / 4;
-  if (ks > 16) ks = 16;
-  if (ks < 2) return 1;
-  const int per = (k_blocks + ks - 1) / ks;
-  return (k_blocks + per - 1) / per;                        // no empty slice
+  const int ks = std::min(std::min(kSmCount / tiles, k_blocks / 4), 16);
+  return ks < 2 ? 1 : ks;
+}
+
+// The cut with the shortest estimated time, in SM clocks.  A k-block (128 bytes of K) costs a CTA
+//   * 2 * bn in the tensor core (four instructions of bn / 2), and
+//   * the bytes of its two operand tiles in and out of shared memory at 128 B/clk, which is also their way from L2 at
+//     64 B/clk: 2 * (128 + bn) alone, 2 * (128 + bn / 2) in a pair -- always the larger number.
+// Work items go over the CTAs (pairs) in whole waves, so narrower tiles win where they fill the last one: 333 rows x 12288
+// columns are 96 items of 256 x 256 on 74 pairs (two waves of 512 a k-block), 128 of 256 x 192 (two of 448) or 144 of
+// 128 x 256 (one of 768).  A tile's last epilogue, pipeline fill and launch are in kTileClocks and 8 clocks a column; a K
+// split adds kReduceClocks and its partial sums' way through L2 and back.  Ties go to the wider tile.
+// Measured over 129..4096 rows of six layer shapes, every cut timed: the choice is the fastest or within 4 % of it, but for
+// 129..256 rows of 4096 columns (10.2 us, 9.2 with 128 x 64).  Before, with 128 or 256 columns only (us): 12288 x 4096 at
+// 129 / 333 / 1024 rows 19.8 / 27.8 / 39.7 -> 17.1 / 21.1 / 38.0, 22016 x 4096 30.0 / 38.4 / 68.1 -> 23.7 / 36.5 / 66.8.
+static GemmShape gemm_shape(int M, int N, int K, int max_split) {
+  constexpr long long kTileClocks = 1500, kReduceClocks = 8000, kReduceBytesPerClock = 2000;
+  const int k_blocks = (K + kBK - 1) / kBK;
+  const int bn_max = N >= kMaxBN ? kMaxBN : (N + 31) / 32 * 32;
+  GemmShape best{false, bn_max, 1};
+  long long best_cost = -1;
+  for (int pair = 1; pair >= 0; --pair) {
+    const int slots = pair ? kSmCount / 2 : kSmCount;
+    const long long m_tiles = pair ? (M + 255) / 256 : (M + 127) / 128;
+    for (int bn = bn_max; bn >= 32; bn -= 32) {
+      const long long tiles = m_tiles * ((N + bn - 1) / bn);
+      const int per_block = 256 + (pair ? bn : 2 * bn);
+      for (int want = 1; want <= (tiles < slots ? max_split : 1); ++want) {
+        const int per = (k_blocks + want - 1) / want, ks = (k_blocks + per - 1) / per;     // no empty slice
+        if (ks != want) continue;
+        const long long waves = (tiles * ks + slots - 1) / slots;
+        long long cost = waves * per * per_block + kTileClocks + 8 * bn;
+        if (ks > 1) cost += kReduceClocks + 8LL * ks * M * N / kReduceBytesPerClock;
+        if (best_cost < 0 || cost < best_cost) {
+          best_cost = cost;
+          best = GemmShape{pair != 0, bn, ks};
+        }
+      }
+    }
+  }
+  return best;
 }
 
 template <bool AFFINE>
-static int launch_splitk_reduce(const GemmCall& c, cudaStream_t st) {
+static int launch_splitk_reduce(const GemmCall& c, int k_split, cudaStream_t st) {
   int blocks = (c.M * (c.N / 4) + 255) / 256;
   if (blocks > 2 * kSmCount) blocks = 2 * kSmCount;
-  return launch_chained(w8a8_splitk_reduce_kernel<AFFINE>, dim3(blocks), dim3(256), 0, st, c.partial, c.k_split, c.M, c.N,
+  return launch_chained(w8a8_splitk_reduce_kernel<AFFINE>, dim3(blocks), dim3(256), 0, st, c.partial, k_split, c.M, c.N,
                         c.K, c.a_scale, c.b_scale, c.bias, c.a_zero, c.a_rowsum, c.b_zero, c.b_rowsum, c.out);
 }
 
-// The CTA-pair form pays once there are enough 256-row tiles to occupy the 74 pairs.
-static bool use_pair(int M, int N) {
-  return (long long)((M + 255) / 256) * ((N + 255) / 256) >= kSmCount / 2 && N > 128;
+template <int EPI>
+static int launch_shape(const GemmCall& c, const GemmShape& shape, cudaStream_t st) {
+  return shape.pair ? launch_gemm<EPI, true>(c, shape, st) : launch_gemm<EPI, false>(c, shape, st);
+}
+
+// With scratch the product may be split over K; a second kernel then adds the slices and scales.
+template <int EPI>
+static int run_gemm(GemmCall& c, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+  const int max_split = workspace ? max_k_split(c.M, c.N, c.K) : 1;
+  if (max_split > 1 && workspace_bytes < (size_t)max_split * c.M * c.N * sizeof(int)) return MP_ERR_WORKSPACE;
+  const GemmShape shape = gemm_shape(c.M, c.N, c.K, max_split);
+  if (shape.k_split > 1) {
+    if (!aligned(workspace, 16)) return MP_ERR_ALIGNMENT;
+    c.partial = static_cast<int*>(workspace);
+  }
+  const int rc = launch_shape<EPI>(c, shape, st);
+  if (rc != MP_OK || shape.k_split == 1) return rc;
+  return launch_splitk_reduce<EPI == EPI_AFFINE>(c, shape.k_split, st);
 }
 
 static int check_gemm_args(const void* a, const void* b, void* out, int M, int N, int K) {
@@ -704,7 +814,7 @@ int launch_moe_gemm1_swiglu(const void* routed_q, const float* routed_scale, con
   c.m_tiles_dev = num_tiles_dev; c.tile_expert = tile_expert; c.b_rows_per_expert = 2 * I; c.up_row_offset = I;
   c.row_absmax = row_absmax; c.error_word = error_word;
   c.tile_part = tile_part;
-  return launch_gemm<256, EPI_SWIGLU, true>(c, st);   // expert segments are 256-row aligned: pair tiles fit
+  return launch_gemm<EPI_SWIGLU, true>(c, GemmShape{true, kMaxBN, 1}, st);   // expert segments are 256-row aligned: pair tiles fit
 }
 
 int launch_moe_gemm2(const void* q2, const float* scale2, const void* w2_q, const float* w2_scale, int padded_rows,
@@ -717,7 +827,7 @@ int launch_moe_gemm2(const void* q2, const float* scale2, const void* w2_q, cons
   c.error_word = error_word;
   c.scatter = scatter;
   c.tile_part = tile_part;
-  return launch_gemm<256, EPI_F16, true>(c, st);
+  return launch_gemm<EPI_F16, true>(c, GemmShape{true, kMaxBN, 1}, st);
 }
 
 }  // namespace mp
@@ -725,8 +835,8 @@ int launch_moe_gemm2(const void* q2, const float* scale2, const void* w2_q, cons
 using namespace mp;
 
 extern "C" size_t mp_w8a8_gemm_workspace_bytes(int M, int N, int K) {
-  if (M <= 0 || N <= 0 || K <= 0 || use_pair(M, N)) return 0;
-  const int ks = w8a8_k_split(M, N, K);
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const int ks = max_k_split(M, N, K);
   return ks > 1 ? (size_t)ks * M * N * sizeof(int) : 0;
 }
 
@@ -747,21 +857,7 @@ extern "C" int mp_w8a8_gemm_ex(const void* qx_i8, const void* x_scale_f32, const
   c.a = qx_i8; c.b = w_i8; c.M = M; c.N = N; c.K = K; c.a_rows = M; c.b_rows_total = N;
   c.a_scale = static_cast<const float*>(x_scale_f32); c.b_scale = static_cast<const float*>(w_scale_f32);
   c.bias = static_cast<const __half*>(bias_f16); c.out = y_f16; c.error_word = error_word;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (use_pair(M, N)) return launch_gemm<256, EPI_F16, true>(c, st);
-  const int ks = workspace ? w8a8_k_split(M, N, K) : 1;        // without scratch: one K slice per tile
-  if (ks > 1) {
-    if (workspace_bytes < (size_t)ks * M * N * sizeof(int)) return MP_ERR_WORKSPACE;
-    if (!aligned(workspace, 16)) return MP_ERR_ALIGNMENT;
-    c.k_split = ks;
-    c.partial = static_cast<int*>(workspace);
-    rc = launch_gemm<128, EPI_F16>(c, st);
-    if (rc != MP_OK) return rc;
-    return launch_splitk_reduce<false>(c, st);
-  }
-  const long long tiles256 = (long long)((M + 127) / 128) * ((N + 255) / 256);
-  if (N <= 128 || tiles256 < kSmCount) return launch_gemm<128, EPI_F16>(c, st);
-  return launch_gemm<256, EPI_F16>(c, st);
+  return run_gemm<EPI_F16>(c, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int mp_w8a8_gemm_i32(const void* qx_i8, const void* w_i8, void* acc_i32, int M, int N, int K,
@@ -771,11 +867,7 @@ extern "C" int mp_w8a8_gemm_i32(const void* qx_i8, const void* w_i8, void* acc_i
   GemmCall c{};
   c.a = qx_i8; c.b = w_i8; c.M = M; c.N = N; c.K = K; c.a_rows = M; c.b_rows_total = N;
   c.out = acc_i32; c.error_word = error_word;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (use_pair(M, N)) return launch_gemm<256, EPI_I32, true>(c, st);
-  const long long tiles256 = (long long)((M + 127) / 128) * ((N + 255) / 256);
-  if (N <= 128 || tiles256 < kSmCount) return launch_gemm<128, EPI_I32>(c, st);
-  return launch_gemm<256, EPI_I32>(c, st);
+  return launch_shape<EPI_I32>(c, gemm_shape(M, N, K, 1), static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int mp_w8a8_affine_gemm(const void* qx_u8, const void* x_scale_f32, const void* x_zero_f32,
@@ -801,18 +893,6 @@ int w8a8_affine_gemm(const void* qx_u8, const void* x_scale_f32, const void* x_z
   c.a_zero = static_cast<const float*>(x_zero_f32); c.a_rowsum = static_cast<const int*>(x_rowsum_i32);
   c.b_zero = static_cast<const float*>(w_zero_f32); c.b_rowsum = static_cast<const int*>(w_rowsum_i32);
   c.bias = static_cast<const __half*>(bias_f16); c.out = y_f16; c.error_word = error_word;
-  if (use_pair(M, N)) return launch_gemm<256, EPI_AFFINE, true>(c, st);
-  const int ks = workspace ? w8a8_k_split(M, N, K) : 1;        // without scratch: one K slice per tile
-  if (ks > 1) {
-    if (workspace_bytes < (size_t)ks * M * N * sizeof(int)) return MP_ERR_WORKSPACE;
-    if (!aligned(workspace, 16)) return MP_ERR_ALIGNMENT;
-    c.k_split = ks;
-    c.partial = static_cast<int*>(workspace);
-    rc = launch_gemm<128, EPI_AFFINE>(c, st);
-    return rc != MP_OK ? rc : launch_splitk_reduce<true>(c, st);
-  }
-  const long long tiles256 = (long long)((M + 127) / 128) * ((N + 255) / 256);
-  if (N <= 128 || tiles256 < kSmCount) return launch_gemm<128, EPI_AFFINE>(c, st);
-  return launch_gemm<256, EPI_AFFINE>(c, st);
+  return run_gemm<EPI_AFFINE>(c, workspace, workspace_bytes, st);
 }
 }  // namespace mp
