@@ -200,17 +200,17 @@ int mp_w4a16_linear(const void* x_f16, const void* packed_i32, const void* sz_f1
  * Prefill variant (any M; meant for M > 64): the same linear on the fp16 tensor
  * cores (tcgen05 kind::f16, fp32 accumulators in TMEM), activations fed by TMA,
  * int4 unpack + group dequant fused in as a producer stage that writes the
- * dequantised tile straight into shared memory.  K % 64 == 0, group % 64 == 0.
+ * dequantised tile straight into tensor memory.  K % 64 == 0, group % 64 == 0.
  * error_word as for mp_w8a8_gemm.
  */
 int mp_w4a16_linear_prefill(const void* x_f16, const void* packed_i32, const void* sz_f16x2,
                             const void* bias_f16, void* y_f16, int M, int N, int K, int group,
                             int* error_word, mp_stream_t stream);
 /*
- * Same, with scratch for split-K: with few output tiles (M <= 256 and a narrow
- * N) the K range of every tile is cut into slices so that all SMs stream
- * weights; the slices' fp32 partial tiles go to `workspace` and a second kernel
- * adds them in slice order (deterministic).  mp_w4a16_prefill_workspace_bytes
+ * Same, with scratch for split tiles: where whole tiles would leave CTA pairs
+ * idle, every pair gets an equal run of the tiles' K steps; the fp32 partial
+ * tiles of those cut in between go to `workspace` and a second kernel
+ * adds them in K order (deterministic).  mp_w4a16_prefill_workspace_bytes
  * returns the size needed (0 = no split for this shape); a null workspace
  * means no split.
  */

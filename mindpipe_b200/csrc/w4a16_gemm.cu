@@ -1,20 +1,34 @@
-// W4A16 prefill GEMM: y[M,N] = x[M,K] @ dequant(W)[N,K]^T on the fp16 tensor
-// cores, with the int4 unpack + group dequant fused in as a producer stage.
+// W4A16 product for many tokens: y[M,N] = x[M,K] @ dequant(W)[N,K]^T on the fp16 tensor cores, the int4 unpack and
+// group dequantisation fused in as a producer stage.
 //
-// One persistent CTA per SM, 14 warps (128-row tile, MT = 1) or 18 warps (256-row tile, MT = 2):
-//   warp 0      TMA producer for the activation tile x[128 MT x 64] (128-byte swizzle)
-//   warp 1      MMA issuer: tcgen05.mma kind::f16, M=128, N=256, K=16, fp32 in TMEM
-//   next 4 MT   epilogue warps: tcgen05.ld -> (+bias) -> fp16 -> global
-//               (for M > 256 two CTAs of a cluster share each MMA, see Cfg)
-//   last 8      dequant producers: stream the packed int4 words of the weight tile
-//               [256 rows x 64 columns] from global memory with 128-bit loads, expand
-//               them with dequant8 (exactly f16((u - z) * s), the reference's Wdq) and
-//               store them into shared memory in the canonical K-major 128-byte-swizzle
-//               layout the MMA reads -- the dequantised weights never exist in HBM.
+// The weights are the A operand, in tensor memory: a pair of CTAs (a cluster of 2, cta_group::2) multiplies 256 weight
+// rows -- 128 in each CTA -- with up to 256 tokens, whose activations are the B operand, half of them in each CTA's shared
+// memory.  Why this way round:
+//   * expanded weights never pass through shared memory.  Per 256 columns of K a CTA takes 16 KB of packed words and at
+//     256 tokens 64 KB of activations into shared memory and reads them once, 1250 clocks at 128 B/clk, beside 2048 clocks
+//     of MMA.  With the expanded tile as B in shared memory (512 tokens x 256 rows to a pair) it was 1800 of 2048, and a
+//     batch of 129 rows was multiplied as 256, one of 300 as 512.
+//   * the tokens are the MMA's N, any multiple of 32, so little is multiplied for padding.
+//   * expanding 32768 weights takes the SM's ALUs 660 clocks of those 2048.
+// A persistent pair per two SMs, roles by warp:
+//   warps 0-11   expansion, three sets of four warps taking 128-column steps in turn: a lane holds a weight row, makes
+//                exactly f16((u - z) * s) of its words and stores them to a tensor memory slot
+//   warps 12-19  epilogue: accumulators -> fp16 (+ bias), transposed through shared memory -> y; or fp32 partial tiles
+//   warp 20      TMA producer of the packed words (256 columns a stage)
+//   warp 21      MMA issuer (the even CTA's)
+//   warp 22      TMA producer of the activations (128 columns a step)
+// Work is cut into (tile, step) units, and with scratch every pair gets an equal run of them: a tile whose run ends in
+// between is left as fp32 partial tiles, which a second kernel adds in K order.  Without scratch pairs take whole tiles.
 //
-// A stage is full when the TMA bytes have landed and all dequant warps have
-// arrived (after a fence that makes their generic-proxy stores visible to the
-// tensor core).  Every wait is bounded (see tc.cuh).
+// Measured (us, groups of 128; in brackets the form it replaces, expanded weights as the B operand in shared memory):
+// 12288 x 4096 at 129 / 333 / 512 / 2048 rows 22.0 / 35.8 / 42.1 / 155.8 [40.8 / 59.7 / 59.6 / 171.6], 4096 x 11008 at
+// 129 / 2048 rows 23.5 / 142.4 [38.1 / 149.5].  With many rows the MMAs bound it (1050 clocks a step of 1024 at 256 tokens,
+// 5000 of 38000 a tile in the epilogue); below 160 rows the expansion warps (about 800 a step).
+//
+// Every mbarrier wait is bounded (tc.cuh); on a timeout the pair records an error word, lets its copies land, frees its
+// tensor memory and returns.
+#include <algorithm>
+
 #include "common.cuh"
 #include "tc.cuh"
 
@@ -23,467 +37,537 @@ namespace mp {
 using namespace tc;
 
 namespace w4 {
-constexpr int kBN = 256;
-constexpr int kBK = 64;            // fp16 elements of K per stage = one 128-byte swizzle row
-constexpr int kUmmaK = 16;
-constexpr int kSubBytes = 128 * kBK * 2;   // one 128-row activation sub-tile: 16 KB
-constexpr int kTmemCols = 2 * kBN;         // all 512 columns
-constexpr int kDequantWarps = 8;
-// MT = 128-row activation sub-tiles per block tile.  MT = 1: 128 x 256 tile, two accumulator
-// buffers (the epilogue of a tile overlaps the next main loop).  MT = 2: 256 x 256 tile whose two
-// accumulators share one dequantised weight tile -- half the dequant work per flop, one buffer.
-// PAIR (with MT = 2): two CTAs of a cluster share every MMA (cta_group::2, M = 256 per instruction:
-// 128 rows from each CTA), so a pair computes a 512 x 256 tile and each CTA dequantises and stages
-// only 128 of the 256 weight rows -- half the dequant work and a third less shared-memory traffic
-// per flop than the single-CTA 256 x 256 tile.
-template <int MT, bool PAIR = false>
-struct Cfg {
-  static constexpr int kBM = 128 * MT;                       // activation rows per CTA
-  static constexpr int kStages = PAIR ? 4 : (MT == 1 ? 4 : 3);
-  static constexpr int kABytes = MT * kSubBytes;
-  static constexpr int kBRows = PAIR ? kBN / 2 : kBN;        // weight rows this CTA dequantises
-  static constexpr int kBStage = kBRows * kBK * 2;
-  static constexpr int kBufs = MT == 1 ? 2 : 1;
-  static constexpr int kEpiWarps = 4 * MT;
-  static constexpr int kFirstDequantWarp = 2 + kEpiWarps;
-  static constexpr int kThreads = 32 * (2 + kEpiWarps + kDequantWarps);
-  static constexpr size_t kSmem = 1024 + (size_t)kStages * (kABytes + kBStage) + 256;
-};
+constexpr int kRows = 128;                 // weight rows of a CTA
+constexpr int kStepK = 128, kStageK = 256;
+constexpr int kSets = 3;
+constexpr int kEpiWarp0 = 4 * kSets, kEpiWarps = 8, kWeightWarp = kEpiWarp0 + kEpiWarps, kMmaWarp = kWeightWarp + 1,
+              kXWarp = kWeightWarp + 2;
+constexpr int kThreads = 32 * (kXWarp + 1);
+constexpr int kStageBytes = kRows * kStageK / 2;
+constexpr int kMaxT = 256;
+constexpr int kSlotCols = kStepK / 2;      // tensor memory columns of a step's expanded weights
+constexpr int kMaxSlots = 6, kMaxXRing = 6, kMaxRing = 8;
+constexpr int kRingBytes = 208 * 1024;     // both rings
+constexpr int kStagingBytes = kEpiWarps * 2048;
+constexpr int kTailBytes = 512;
+constexpr size_t kSmem = 1024 + kRingBytes + kStagingBytes + kTailBytes;
+constexpr int kTmemCols = 512;
+constexpr int kPairs = kSmCount / 2;
+
+__host__ __device__ constexpr int accumulators(int T) { return T <= 128 ? 2 : 1; }
+// slots and weight stages: four or more, see the waits of the expansion
+__host__ __device__ constexpr int slots(int T) {
+  const int n = (kTmemCols - accumulators(T) * T) / kSlotCols;
+  return n < kMaxSlots ? n : kMaxSlots;
+}
+__host__ __device__ constexpr int x_step_bytes(int T) { return T / 2 * kStepK * 2; }
+__host__ __device__ constexpr int x_ring(int T) { return T > 128 ? 4 : kMaxXRing; }
+__host__ __device__ constexpr int ring(int T) {
+  const int n = (kRingBytes - x_ring(T) * x_step_bytes(T)) / kStageBytes;
+  return n < kMaxRing ? n : kMaxRing;
+}
+static_assert(slots(256) == 4 && slots(128) == 4 && slots(160) == 5 && ring(256) == 5 && ring(128) >= 4, "rings");
 }  // namespace w4
 
 struct W4GemmParams {
-  const uint32_t* packed;   // [N, K/8]
   const uint32_t* sz;       // [K/group, N] (scale, zero) f16 pairs
   const __half* bias;
   __half* y;
   int M, N, K, group;
-  int m_tiles, n_tiles, k_blocks;
-  int k_split;              // > 1: each tile's K range is cut into this many work items ...
-  int kb_per_split;         // ... of this many k-blocks, whose fp32 partial tiles go to `partial`
-  float* partial;           // [k_split][M][N] fp32 (split-K only)
+  int T;                    // tokens of a tile, a multiple of 32
+  int m_tiles, steps;       // tiles along the tokens; 128-column steps of a tile
+  int unit_steps;           // 1, or `steps` when pairs take whole tiles
+  int share, extra;         // units of a pair: share, one more for the first `extra` pairs
+  float* partial;           // [pair][2][rank][T][128]: the first segment of a pair that begins inside a tile, and the last
+                            // one that ends inside a tile whose beginning it holds
   int* error_word;
 };
 
-template <int MT, bool PAIR>
-__global__ void __launch_bounds__(w4::Cfg<MT, PAIR>::kThreads, 1)
-w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4GemmParams p) {
+__host__ __device__ inline int w4_range_start(int pair, int share, int extra) {
+  return pair * share + (pair < extra ? pair : extra);
+}
+__device__ __forceinline__ int w4_pair_of(int unit, int share, int extra) {
+  const int longer = extra * (share + 1);
+  return unit < longer ? unit / (share + 1) : extra + (unit - longer) / share;
+}
+
+// A pair's walk over its units: one segment per tile.
+struct W4Segment {
+  int tile, s0, s1;         // steps [s0, s1) of the tile
+};
+
+// D[tmem] (+)= A[tmem] * B[smem] over a CTA pair: M = 256, 128 lanes of A and D in each CTA's tensor memory, B's rows
+// split in halves between the two shared memories.
+__device__ __forceinline__ void umma_f16_ts_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                                 uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+__device__ __forceinline__ uint4 w4_lds_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+
+// One packed word -> f16((u - z) * s) of its eight columns in order.
+__device__ __forceinline__ void expand_word(uint32_t word, const ScaleZero& sp, uint32_t* out) {
+  __half2 v[4];
+  dequant8(word, sp, v);
+  const uint32_t a = h2_as_u32(v[0]), b = h2_as_u32(v[1]), c = h2_as_u32(v[2]), d = h2_as_u32(v[3]);
+  out[0] = prmt(a, b, 0x5410);
+  out[1] = prmt(c, d, 0x5410);
+  out[2] = prmt(a, b, 0x7632);
+  out[3] = prmt(c, d, 0x7632);
+}
+
+__global__ void __launch_bounds__(w4::kThreads, 1)
+w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
+                  const W4GemmParams p) {
   using namespace w4;
-  using C = Cfg<MT, PAIR>;
-  constexpr int kBStage = C::kBStage;
-  constexpr int kStages = C::kStages;
-  constexpr int kABytes = C::kABytes;
-  constexpr int kBM = C::kBM;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* sA = smem;
-  unsigned char* sB = smem + kStages * kABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sB + kStages * kBStage);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4);
+  const int T = p.T, n_slots = slots(T), n_x = x_ring(T), n_w = ring(T), n_acc = accumulators(T);
+  const int x_bytes = x_step_bytes(T), x_half = x_bytes / 2;
+  unsigned char* tail = smem + kRingBytes + kStagingBytes;
+  const uint32_t xring = smem_u32(smem), wring = xring + n_x * x_bytes, staging = xring + kRingBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(tail);
+  const uint32_t wfull0 = smem_u32(bars);                  // packed words landed
+  const uint32_t wempty0 = wfull0 + 8 * kMaxRing;          // ... and were read
+  const uint32_t xfull0 = wempty0 + 8 * kMaxRing;          // leader: both CTAs' activations landed
+  const uint32_t xempty0 = xfull0 + 8 * kMaxXRing;         // ... and were multiplied
+  const uint32_t ready0 = xempty0 + 8 * kMaxXRing;         // leader: both CTAs' slots hold an expanded step
+  const uint32_t done0 = ready0 + 8 * kMaxSlots;           // ... and it was multiplied
+  const uint32_t tfull0 = done0 + 8 * kMaxSlots;           // a segment's accumulator is complete
+  const uint32_t tempty0 = tfull0 + 16;                    // leader: both CTAs have read it
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 8 * (2 * kMaxRing + 2 * kMaxXRing + 2 * kMaxSlots + 4));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + kStages);
-  const uint32_t tfull0 = smem_u32(bars + 2 * kStages), tempty0 = smem_u32(bars + 2 * kStages + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // PAIR: rank 0 of the cluster leads: it issues the MMAs and owns the "stage full" and "accumulator
-  // free" barriers, on which the peer's TMA bytes, dequant warps and epilogue warps arrive remotely;
-  // both CTAs own "stage empty" and "accumulator full" barriers that the leader's commits arrive on.
-  // Every wait is on a barrier of the waiting CTA.
-  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+  const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
-  constexpr int kCtas = PAIR ? 2 : 1;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      // leader: the TMA producer's expect_tx arrival + its dequant warps (+ one relayed arrival for the
-      // peer's dequant warps); peer: its dequant warps only (its relay thread waits on this one)
-      mbar_init(full0 + 8 * s, leader ? 1 + kDequantWarps + (PAIR ? 1 : 0) : kDequantWarps);
-      mbar_init(empty0 + 8 * s, 1);
+    for (int s = 0; s < n_w; ++s) {
+      mbar_init(wfull0 + 8 * s, 1);
+      mbar_init(wempty0 + 8 * s, 8);                       // four warps for each of the stage's two steps
+    }
+    for (int s = 0; s < n_x; ++s) {
+      mbar_init(xfull0 + 8 * s, 1);
+      mbar_init(xempty0 + 8 * s, 1);
+    }
+    for (int q = 0; q < n_slots; ++q) {
+      mbar_init(ready0 + 8 * q, 8);                        // four warps of each CTA
+      mbar_init(done0 + 8 * q, 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull0 + 8 * b, 1);
-      mbar_init(tempty0 + 8 * b, kCtas * C::kEpiWarps);
+      mbar_init(tempty0 + 8 * b, 2 * kEpiWarps);
     }
     *abort_flag = 0;
     fence_mbar_init();
   }
-  if (warp == 1) {
-    if (PAIR) {
-      tmem_alloc_pair(smem_u32(tmem_slot), kTmemCols);
-      tmem_relinquish_pair();
-    } else {
-      tmem_alloc(smem_u32(tmem_slot), kTmemCols);
-      tmem_relinquish();
-    }
+  if (warp == kMmaWarp) {
+    tmem_alloc_pair(smem_u32(tmem_slot), kTmemCols);
+    tmem_relinquish_pair();
   }
   tcgen05_fence_before();
   __syncthreads();
-  if (PAIR) {            // the peer's barriers exist before anything signals them
-    cluster_arrive();
-    cluster_wait();
-  }
+  cluster_arrive();              // the peer's barriers exist before anything signals them
+  cluster_wait();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // work item = (tile, K slice); m_tiles counts tiles of kCtas * kBM rows
-  const int total = p.m_tiles * p.n_tiles * p.k_split;
-  const int first_tile = PAIR ? blockIdx.x >> 1 : blockIdx.x;
-  const int tile_step = PAIR ? gridDim.x >> 1 : gridDim.x;
-  const uint32_t full_leader0 = PAIR ? map_to_cta(full0, 0) : full0;
 
-  if (warp == 0) {
+  chain_wait();
+  chain_release();
+
+  const int pair = static_cast<int>(blockIdx.x) >> 1, steps = p.steps;
+  const int u0 = w4_range_start(pair, p.share, p.extra) * p.unit_steps,
+            u1 = w4_range_start(pair + 1, p.share, p.extra) * p.unit_steps;          // this pair's steps
+  // the segment that begins at unit u
+  auto segment_at = [&](int u, W4Segment& g) {
+    g.tile = u / steps;
+    g.s0 = u - g.tile * steps;
+    g.s1 = min(steps, g.s0 + u1 - u);
+  };
+  auto first_row = [&](int tile) { return (tile / p.m_tiles) * (2 * kRows) + static_cast<int>(rank) * kRows; };
+  const uint32_t peer_or_own = rank ^ 1u;
+
+  if (warp == kWeightWarp) {
+    if (elect_one()) {
+      prefetch_tensormap(&tmap_w);
+      int s = 0;
+      uint32_t phase = 1;
+      bool ok = true;
+      W4Segment g;
+      for (int u = u0; ok && u < u1; u += g.s1 - g.s0) {
+        segment_at(u, g);
+        const int row = first_row(g.tile);
+        for (int st = g.s0 >> 1; st <= (g.s1 - 1) >> 1; ++st) {
+          if (!mbar_wait(wempty0 + 8 * s, phase, abort_flag)) { ok = false; break; }
+          mbar_arrive_expect_tx(wfull0 + 8 * s, kStageBytes);
+          tma_load_2d(wring + s * kStageBytes, &tmap_w, wfull0 + 8 * s, st * (kStageK / 2), row);
+          if (++s == n_w) { s = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == kXWarp) {
     if (elect_one()) {
       prefetch_tensormap(&tmap_x);
-      int stage = 0;
-      uint32_t phase = 0;
+      const uint32_t xfull_leader0 = map_to_cta(xfull0, 0);
+      int s = 0;
+      uint32_t phase = 1;
       bool ok = true;
-      for (int work = first_tile; ok && work < total; work += tile_step) {
-        const int tile = work / p.k_split;
-        const int kb0 = (work - tile * p.k_split) * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
-        const int m0 = (tile % p.m_tiles) * (kCtas * kBM) + static_cast<int>(rank) * kBM;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(empty0 + 8 * stage, phase ^ 1, abort_flag)) { ok = false; break; }
-          if (PAIR) {
-            const uint32_t full = full_leader0 + 8 * stage;      // both CTAs' bytes are counted by the leader
-            if (leader) mbar_arrive_expect_tx(full0 + 8 * stage, 2 * kABytes);
-#pragma unroll
-            for (int sub = 0; sub < MT; ++sub)
-              tma_load_2d_pair(smem_u32(sA + stage * kABytes + sub * kSubBytes), &tmap_x, full, kb * kBK,
-                               m0 + sub * 128);
-          } else {
-            const uint32_t full = full0 + 8 * stage;
-            mbar_arrive_expect_tx(full, kABytes);
-#pragma unroll
-            for (int sub = 0; sub < MT; ++sub)
-              tma_load_2d(smem_u32(sA + stage * kABytes + sub * kSubBytes), &tmap_x, full, kb * kBK, m0 + sub * 128);
+      W4Segment g;
+      for (int u = u0; ok && u < u1; u += g.s1 - g.s0) {
+        segment_at(u, g);
+        const int m0 = (g.tile % p.m_tiles) * T + static_cast<int>(rank) * (T / 2);
+        for (int st = g.s0; st < g.s1; ++st) {
+          if (!mbar_wait(xempty0 + 8 * s, phase, abort_flag)) { ok = false; break; }
+          const int k0 = st * kStepK;
+          const bool both = k0 + 64 < p.K;
+          if (leader) mbar_arrive_expect_tx(xfull0 + 8 * s, both ? 2 * x_bytes : x_bytes);     // of both CTAs
+          tma_load_2d_pair(xring + s * x_bytes, &tmap_x, xfull_leader0 + 8 * s, k0, m0);
+          if (both) tma_load_2d_pair(xring + s * x_bytes + x_half, &tmap_x, xfull_leader0 + 8 * s, k0 + 64, m0);
+          if (++s == n_x) { s = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == kMmaWarp) {
+    if (leader && elect_one()) {
+      const uint32_t idesc = umma_idesc(kIdescDFormatF32 | kIdescABFormatF16, 2 * kRows, T);
+      const uint32_t xempty_peer0 = map_to_cta(xempty0, peer_or_own), done_peer0 = map_to_cta(done0, peer_or_own),
+                     tfull_peer0 = map_to_cta(tfull0, peer_or_own);
+      const uint64_t b_desc0 = umma_desc_k_sw128(xring);
+      int q = 0, xs = 0, d = 0;
+      uint32_t phase = 0, xphase = 0, dphase = 1;
+      bool ok = true;
+      W4Segment g;
+      for (int u = u0; ok && u < u1; u += g.s1 - g.s0) {
+        segment_at(u, g);
+        if (!mbar_wait(tempty0 + 8 * d, dphase, abort_flag)) break;
+        const uint32_t d_tmem = tmem_base + d * T;
+        for (int st = g.s0; st < g.s1; ++st) {
+          if (!mbar_wait(xfull0 + 8 * xs, xphase, abort_flag) || !mbar_wait(ready0 + 8 * q, phase, abort_flag)) {
+            ok = false;
+            break;
           }
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
-        }
-      }
-    }
-  } else if (warp == 1 && !leader) {
-    // peer CTA: relay "my half of the weight tile is in place" to the leader with ONE cluster-scope
-    // arrival per stage (the eight dequant warps arrive on the local barrier, which is cheap)
-    if (elect_one()) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int work = first_tile; ok && work < total; work += tile_step) {
-        const int kb0 = (work % p.k_split) * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(full0 + 8 * stage, phase, abort_flag)) { ok = false; break; }
-          mbar_arrive_cluster(full_leader0 + 8 * stage);
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
-        }
-      }
-    }
-  } else if (warp == 1) {
-    if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc(kIdescDFormatF32 | kIdescABFormatF16, kCtas * 128, kBN);
-      int stage = 0;
-      uint32_t phase = 0;
-      int buf = 0;
-      uint32_t buf_phase = 0;
-      bool ok = true;
-      for (int work = first_tile; ok && work < total; work += tile_step) {
-        const int kb0 = (work % p.k_split) * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
-        if (!mbar_wait(tempty0 + 8 * buf, buf_phase ^ 1, abort_flag)) break;
-        tcgen05_fence_after();
-        const uint32_t d_tmem = tmem_base + buf * kBN;        // MT == 2: the accumulators sit at columns 0 and 256
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(full0 + 8 * stage, phase, abort_flag)) { ok = false; break; }
           tcgen05_fence_after();
-          const uint64_t b_desc = umma_desc_k_sw128(smem_u32(sB + stage * kBStage));
+          const uint32_t a_tmem = tmem_base + n_acc * T + q * kSlotCols;
+          const int halves = st * kStepK + 64 < p.K ? 2 : 1;
+          for (int h = 0; h < halves; ++h) {
+            const uint64_t b_desc = b_desc0 + ((xs * x_bytes + h * x_half) >> 4);
 #pragma unroll
-          for (int sub = 0; sub < MT; ++sub) {
-            const uint64_t a_desc = umma_desc_k_sw128(smem_u32(sA + stage * kABytes + sub * kSubBytes));
-#pragma unroll
-            for (int kk = 0; kk < kBK / kUmmaK; ++kk) {  // +32 bytes of K per step
-              if (PAIR) {
-                umma_f16_pair(d_tmem + sub * kBN, a_desc + 2 * kk, b_desc + 2 * kk, idesc, (kb != kb0 || kk != 0));
-              } else {
-                umma_f16(d_tmem + sub * kBN, a_desc + 2 * kk, b_desc + 2 * kk, idesc, (kb != kb0 || kk != 0));
-              }
-            }
+            for (int kk = 0; kk < 4; ++kk)       // 16 K per instruction: 8 columns of A, 32 bytes of B's rows
+              umma_f16_ts_pair(d_tmem, a_tmem + (h * 4 + kk) * 8, b_desc + 2 * kk, idesc, st != g.s0 || h != 0 || kk != 0);
           }
-          if (PAIR) {                      // release the stage in both CTAs
-            umma_commit_pair(empty0 + 8 * stage);
-            umma_commit_pair(map_to_cta(empty0 + 8 * stage, 1));
-          } else {
-            umma_commit(empty0 + 8 * stage);
-          }
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
+          umma_commit_pair(xempty0 + 8 * xs);
+          umma_commit_pair(xempty_peer0 + 8 * xs);
+          umma_commit_pair(done0 + 8 * q);
+          umma_commit_pair(done_peer0 + 8 * q);
+          if (++xs == n_x) { xs = 0; xphase ^= 1; }
+          if (++q == n_slots) { q = 0; phase ^= 1; }
         }
         if (!ok) break;
-        if (PAIR) {                        // publish the accumulators to both CTAs' epilogues
-          umma_commit_pair(tfull0 + 8 * buf);
-          umma_commit_pair(map_to_cta(tfull0 + 8 * buf, 1));
-        } else {
-          umma_commit(tfull0 + 8 * buf);
-        }
-        if (++buf == C::kBufs) { buf = 0; buf_phase ^= 1; }
+        umma_commit_pair(tfull0 + 8 * d);
+        umma_commit_pair(tfull_peer0 + 8 * d);
+        if (++d == n_acc) { d = 0; dphase ^= 1; }
       }
     }
-  } else if (warp < C::kFirstDequantWarp) {
-    const int quarter = warp & 3;                 // TMEM lanes [32*quarter, +32) belong to this warp
-    const int sub = (warp - 2) >> 2;              // which 128-row accumulator (MT == 2)
-    int buf = 0;
-    uint32_t buf_phase = 0;
-    const uint32_t tempty_leader0 = PAIR ? map_to_cta(tempty0, 0) : tempty0;
-    for (int work = first_tile; work < total; work += tile_step) {
-      const int tile = work / p.k_split, split = work - tile * p.k_split;
-      const int m_tile = tile % p.m_tiles, n_tile = tile / p.m_tiles;
-      if (!__all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * buf, buf_phase, abort_flag))) break;
-      tcgen05_fence_after();
-      const int row = m_tile * (kCtas * kBM) + static_cast<int>(rank) * kBM + sub * 128 + quarter * 32 + lane;
-      const bool row_ok = row < p.M;
-      const int n0 = n_tile * kBN;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + (buf + sub) * kBN;
-#pragma unroll 1
-      for (int c0 = 0; c0 < kBN; c0 += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32(taddr + c0, r);
-        tmem_ld_wait();
-        if (p.k_split > 1) {
-          // split-K: this K slice's fp32 partial tile; a second kernel adds the slices in order
-          if (row_ok) {
-            float* dst = p.partial + ((size_t)split * p.M + row) * p.N + n0 + c0;
-            if (n0 + c0 + 32 <= p.N && (p.N % 4) == 0) {
-#pragma unroll
-              for (int v = 0; v < 8; ++v)
-                reinterpret_cast<uint4*>(dst)[v] = make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (n0 + c0 + j < p.N) dst[j] = __uint_as_float(r[j]);
-            }
-          }
-          continue;
-        }
-        uint32_t packed_out[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int n = n0 + c0 + 2 * j;
-          float v0 = __uint_as_float(r[2 * j]), v1 = __uint_as_float(r[2 * j + 1]);
-          if (p.bias) {
-            if (n < p.N) v0 += h2f(p.bias[n]);
-            if (n + 1 < p.N) v1 += h2f(p.bias[n + 1]);
-          }
-          packed_out[j] = h2_as_u32(__floats2half2_rn(v0, v1));
-        }
-        if (row_ok) {
-          __half* dst = p.y + (size_t)row * p.N + n0 + c0;
-          if (n0 + c0 + 32 <= p.N && (p.N % 8) == 0) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v)
-              reinterpret_cast<uint4*>(dst)[v] =
-                  make_uint4(packed_out[4 * v], packed_out[4 * v + 1], packed_out[4 * v + 2], packed_out[4 * v + 3]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {                     // static indices keep the values in registers
-              const uint32_t w = packed_out[j >> 1];
-              if (n0 + c0 + j < p.N)
-                dst[j] = __ushort_as_half(static_cast<unsigned short>((j & 1) ? (w >> 16) : (w & 0xFFFFu)));
-            }
-          }
-        }
+  } else if (warp < kEpiWarp0) {
+    // ---- expansion: this warp's 32 rows of every third step
+    const int quarter = warp & 3, set = warp >> 2;
+    const int row = quarter * 32 + lane, sw = row & 7;
+    const uint32_t a_tmem0 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + n_acc * T;
+    const uint32_t ready_leader0 = map_to_cta(ready0, 0);
+    const int sub_blocks = p.K / 64;
+    // the group of a step's first 64 columns and how many such blocks of it come before, kept by addition from step to step
+    const int g64 = p.group / 64, g_step = 2 * kSets / g64, r_step = 2 * kSets % g64;
+    int grp = 0, rem = 0;
+    int q = set % n_slots, s = 0, ord = 0;                // slot; weight stage and its running number
+    uint32_t qphase = 1, phase = 0;
+    W4Segment g{0, 0, 0};
+    int n = 0, base = 0, end = u0, next_base = 0;          // of the segment [.., end): row, first stage's running number
+    // (scale, zero) of this row for a step's two halves
+    auto load_sz = [&](int st, uint32_t (&z)[2]) {
+      const uint32_t* src = p.sz + (size_t)grp * p.N + n;
+      const bool live = n < p.N;
+      z[0] = live ? __ldg(src) : 0u;
+      z[1] = live && 2 * st + 1 < sub_blocks ? __ldg(rem + 1 >= g64 ? src + p.N : src) : 0u;
+    };
+    auto seek = [&](int u) {                               // the segment that holds unit u
+      while (u >= end) {
+        segment_at(end, g);
+        base = next_base;
+        next_base = base + ((g.s1 - 1) >> 1) - (g.s0 >> 1) + 1;
+        end += g.s1 - g.s0;
+        n = first_row(g.tile) + row;
       }
-      tcgen05_fence_before();
+      const int st = g.s1 - (end - u);
+      grp = 2 * st / g64;
+      rem = 2 * st - grp * g64;
+      return st;
+    };
+    int u = u0 + set, st = 0;
+    uint32_t sz_next[2];
+    if (u < u1) {
+      st = seek(u);
+      load_sz(st, sz_next);
+    }
+    while (u < u1) {
+      const int now = base + (st >> 1) - (g.s0 >> 1);
+      for (; ord < now; ++ord)
+        if (++s == n_w) { s = 0; phase ^= 1; }
+      const uint32_t sz_now[2] = {sz_next[0], sz_next[1]};
+      const bool alone = (st ^ 1) < g.s0 || (st ^ 1) >= g.s1;        // the stage's other step is not this pair's
+      // The slot first: when the MMAs of the step n_slots >= 4 before this one are done, the stages before the last four
+      // have been filled and read, so that the parity of the stage's barrier is not ambiguous.
+      if (!__all_sync(0xffffffffu, mbar_wait(done0 + 8 * q, qphase, abort_flag) &&
+                                       mbar_wait(wfull0 + 8 * s, phase, abort_flag))) break;
+      tcgen05_fence_after();
+      const uint32_t src = wring + s * kStageBytes + row * 128;
+      uint4 w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = w4_lds_v4(src + ((((st & 1) * 4 + j) ^ sw) << 4));
+      u += kSets;
+      const int this_st = st;
+      if (u < u1) {                                        // the next step's scales, while this one is expanded
+        if (u < end) {
+          st += kSets;
+          grp += g_step;
+          rem += r_step;
+          if (rem >= g64) { rem -= g64; ++grp; }
+        } else {
+          st = seek(u);
+        }
+        load_sz(st, sz_next);
+      }
+      const uint32_t a_tmem = a_tmem0 + q * kSlotCols;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (j == 2 && 2 * this_st + 1 >= sub_blocks) break;             // K ends in the middle of the step
+        const __half2 szh = *reinterpret_cast<const __half2*>(&sz_now[j >> 1]);
+        uint32_t r[16];
+        const ScaleZero sp = make_scale_zero(__low2half(szh), __high2half(szh));
+        expand_word(w[j].x, sp, r);
+        expand_word(w[j].y, sp, r + 4);
+        expand_word(w[j].z, sp, r + 8);
+        expand_word(w[j].w, sp, r + 12);
+        tmem_st_32x32_x16(a_tmem + j * 16, r);
+      }
       __syncwarp();
       if (lane == 0) {
-        if (PAIR) {
-          mbar_arrive_cluster(tempty_leader0 + 8 * buf);
-        } else {
-          mbar_arrive(tempty0 + 8 * buf);
-        }
+        mbar_arrive(wempty0 + 8 * s);
+        if (alone) mbar_arrive(wempty0 + 8 * s);
       }
-      if (++buf == C::kBufs) { buf = 0; buf_phase ^= 1; }
+      tmem_st_wait();
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_tmem(ready_leader0 + 8 * q);
+      q += kSets;
+      if (q >= n_slots) { q -= n_slots; qphase ^= 1; }
     }
   } else {
-    // ---- dequant producers: 256 threads expand this CTA's rows of the weight tile; a thread owns one
-    // row (all 64 columns of the k-block) or, with 128 rows per CTA (PAIR), one 32-column half of a row ----
-    constexpr int kTPR = 256 / C::kBRows;                              // threads per row: 1 or 2
-    constexpr int kVec = 2 / kTPR;                                     // 128-bit loads per thread and k-block
-    const int dt = threadIdx.x - C::kFirstDequantWarp * 32;            // 0..255
-    const int r = dt / kTPR;                                           // row of this CTA's weight tile
-    const int part = dt % kTPR;                                        // which half of the row's k-block
-    const int words_per_row = p.K >> 3;
-    int stage = 0;
-    uint32_t phase = 0;
-    bool ok = true;
-    const int row_off = (r >> 3) * 1024 + (r & 7) * 128;     // row r of a K-major tile with 128-byte rows
-    const int sw = r & 7;
-    for (int work = first_tile; ok && work < total; work += tile_step) {
-      const int tile = work / p.k_split;
-      const int kb0 = (work - tile * p.k_split) * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
-      const int n = (tile / p.m_tiles) * kBN + static_cast<int>(rank) * C::kBRows + r;
-      const bool n_ok = n < p.N;
-      const uint32_t* row = p.packed + (size_t)(n_ok ? n : 0) * words_per_row + part * 4;
-      const uint32_t* szp = p.sz + (n_ok ? n : 0);
-      // software pipeline: the words of the next kPrefetch k-blocks are in flight while one is
-      // expanded (a k-block lasts about 1000 tensor cycles, a global load under load about as long)
-      constexpr int kPrefetch = 3;
-      uint4 q[kPrefetch][kVec];
-      uint32_t szq[kPrefetch];
-      auto fetch = [&](int kb, uint4 (&dst)[kVec], uint32_t& z) {
-        const bool live = n_ok && kb < kb1;
-        const uint32_t* src = row + kb * (kBK / 8);
+    // ---- epilogue: lane = weight row, column = token; two warps to a quarter of the rows take 32 tokens in turn
+    const int quarter = warp & 3, half = (warp - kEpiWarp0) >> 2;
+    const int row = quarter * 32 + lane;
+    const uint32_t tempty_leader0 = map_to_cta(tempty0, 0);
+    const uint32_t stage = staging + (warp - kEpiWarp0) * 2048;
+    const bool vec = p.N % 8 == 0;
+    int d = 0;
+    uint32_t dphase = 0;
+    W4Segment g;
+    for (int u = u0; u < u1; u += g.s1 - g.s0) {
+      segment_at(u, g);
+      const int n0 = first_row(g.tile) + quarter * 32, n = n0 + lane, m0 = (g.tile % p.m_tiles) * T;
+      const bool whole = g.s0 == 0 && g.s1 == steps;
+      const float bias = p.bias && n < p.N ? h2f(p.bias[n]) : 0.0f;
+      if (!__all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * d, dphase, abort_flag))) break;
+      tcgen05_fence_after();
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + d * T;
+      const int last = min(T, p.M - m0);                     // tokens that exist
+      const int chunks = (last - 32 * half + 63) >> 6;       // of 32 tokens; this warp's are c, c + 2, ...: four at most
+      uint32_t r[32], h0[16];                        // h: two tokens each
+      auto load = [&](int i) { tmem_ld_32x32(taddr + 32 * half + 64 * i, r); };
+      auto pack = [&](uint32_t (&h)[16]) {
 #pragma unroll
-        for (int v = 0; v < kVec; ++v) dst[v] = live ? ldg_stream_v4(src + 4 * v) : make_uint4(0, 0, 0, 0);
-        z = live ? __ldg(szp + (size_t)((kb * kBK) / p.group) * p.N) : 0u;
+        for (int j = 0; j < 16; ++j) {
+          float v0 = __uint_as_float(r[2 * j]), v1 = __uint_as_float(r[2 * j + 1]);
+          if (p.bias) { v0 += bias; v1 += bias; }
+          h[j] = h2_as_u32(__floats2half2_rn(v0, v1));
+        }
       };
+      auto store = [&](const uint32_t (&h)[16], int i) {
+        const int c0 = 32 * half + 64 * i, left = last - c0;
+        __half* y = p.y + (size_t)(m0 + c0) * p.N;
+        if (vec && n0 + 32 <= p.N) {
+          // 16 token pairs x 32 rows of words; the 16-byte pieces of odd pairs trade places, against bank conflicts
+          __syncwarp();
 #pragma unroll
-      for (int d = 0; d < kPrefetch; ++d) fetch(kb0 + d, q[d], szq[d]);
-      for (int kb = kb0; kb < kb1; ++kb) {
-        uint4 cur[kVec];
+          for (int j = 0; j < 16; ++j)
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(stage + j * 128 + (((lane >> 2) ^ (j & 1)) << 4) + (lane & 3) * 4), "r"(h[j]) : "memory");
+          __syncwarp();
 #pragma unroll
-        for (int v = 0; v < kVec; ++v) cur[v] = q[0][v];
-        const uint32_t szc = szq[0];
+          for (int k = 0; k < 2; ++k) {
+            const int j = k * 8 + (lane >> 2), piece = (lane & 3) * 2;      // pair of tokens, eight rows
+            const uint4 a = w4_lds_v4(stage + j * 128 + ((piece ^ (j & 1)) << 4));
+            const uint4 b = w4_lds_v4(stage + j * 128 + (((piece + 1) ^ (j & 1)) << 4));
+            __half* dst = y + (size_t)(2 * j) * p.N + n0 + (lane & 3) * 8;
+            if (2 * j < left)
+              *reinterpret_cast<uint4*>(dst) = make_uint4(prmt(a.x, a.y, 0x5410), prmt(a.z, a.w, 0x5410), prmt(b.x, b.y, 0x5410), prmt(b.z, b.w, 0x5410));
+            if (2 * j + 1 < left)
+              *reinterpret_cast<uint4*>(dst + p.N) = make_uint4(prmt(a.x, a.y, 0x7632), prmt(a.z, a.w, 0x7632), prmt(b.x, b.y, 0x7632), prmt(b.z, b.w, 0x7632));
+          }
+        } else if (n < p.N) {
 #pragma unroll
-        for (int d = 0; d + 1 < kPrefetch; ++d) {
-#pragma unroll
-          for (int v = 0; v < kVec; ++v) q[d][v] = q[d + 1][v];
-          szq[d] = szq[d + 1];
+          for (int j = 0; j < 32; ++j)
+            if (j < left)
+              y[(size_t)j * p.N + n] = __ushort_as_half(static_cast<unsigned short>((j & 1) ? h[j >> 1] >> 16 : h[j >> 1]));
         }
-        fetch(kb + kPrefetch, q[kPrefetch - 1], szq[kPrefetch - 1]);
-        const __half2 hz = *reinterpret_cast<const __half2*>(&szc);
-        const ScaleZero sp = make_scale_zero(__low2half(hz), __high2half(hz));
-        if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * stage, phase ^ 1, abort_flag))) { ok = false; break; }
-        const uint32_t row_base = smem_u32(sB + stage * kBStage + row_off);   // st.shared below, not generic stores
-#pragma unroll
-        for (int jj = 0; jj < 4 * kVec; ++jj) {                   // 16-byte chunk j = columns 8j..8j+7
-          const int j = part * 4 + jj;
-          const uint4& src = cur[jj >> 2];
-          const uint32_t word = (jj & 3) == 0 ? src.x : (jj & 3) == 1 ? src.y : (jj & 3) == 2 ? src.z : src.w;
-          __half2 v[4];
-          dequant8(word, sp, v);
-          const uint32_t a = h2_as_u32(v[0]), b = h2_as_u32(v[1]), c = h2_as_u32(v[2]), d = h2_as_u32(v[3]);
-          uint4 o;                                                // natural column order for the MMA
-          o.x = prmt(a, b, 0x5410);
-          o.y = prmt(c, d, 0x5410);
-          o.z = prmt(a, b, 0x7632);
-          o.w = prmt(c, d, 0x7632);
-          asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(row_base + ((j ^ sw) << 4)), "r"(o.x), "r"(o.y),
-                       "r"(o.z), "r"(o.w) : "memory");                // 128-byte swizzle
-        }
-        fence_proxy_async_smem();      // generic-proxy stores -> visible to the tensor core's async proxy
+      };
+      auto release = [&]() {
+        tcgen05_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(full0 + 8 * stage);      // this CTA's barrier (the peer's is relayed)
-        if (++stage == kStages) { stage = 0; phase ^= 1; }
+        if (lane == 0) mbar_arrive_tmem(tempty_leader0 + 8 * d);
+      };
+      if (!whole) {
+        float* dst = p.partial + (((size_t)pair * 2 + (g.s0 == 0)) * 2 + rank) * ((size_t)T * kRows) + row;
+#pragma unroll 1
+        for (int i = 0; i < chunks; ++i) {
+          load(i);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) dst[(32 * half + 64 * i + j) * kRows] = __uint_as_float(r[j]);
+        }
+        release();
+      } else {
+        // the accumulator is given back as soon as its last 32 columns are in registers
+        if (chunks <= 0) release();
+        if (chunks > 0) load(0);
+#pragma unroll 1
+        for (int i = 0; i < chunks; ++i) {
+          tmem_ld_wait();
+          if (i == chunks - 1) release();
+          pack(h0);
+          if (i < chunks - 1) load(i + 1);
+          store(h0, i);
+        }
       }
+      if (++d == n_acc) { d = 0; dphase ^= 1; }
     }
   }
 
   __syncthreads();
-  if (PAIR) {
-    // a CTA that gave up tells its peer (whose waits poll the flag) before both meet at the cluster
-    // barrier; the peer cannot have left yet, so its shared memory is still there
-    if (*abort_flag && threadIdx.x == 0) st_cluster_u32(map_to_cta(smem_u32(const_cast<int*>(abort_flag)), rank ^ 1u), 1u);
-    cluster_arrive();       // the leader's MMAs read the peer's shared memory: nobody leaves early
-    cluster_wait();
-  }
+  // a CTA that gave up tells its peer (whose waits poll the flag) before both meet at the cluster barrier; the peer
+  // cannot have left yet, so its shared memory is still there
+  if (*abort_flag && threadIdx.x == 0) st_cluster_u32(map_to_cta(smem_u32(const_cast<int*>(abort_flag)), rank ^ 1u), 1u);
+  cluster_arrive();       // the leader's MMAs read the peer's shared memory: nobody leaves early
+  cluster_wait();
   if (*abort_flag) {
     if (threadIdx.x == 0 && p.error_word) atomicExch(p.error_word, 2);
     const uint64_t t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
     __syncthreads();
   }
-  if (warp == 1) {
+  if (warp == kMmaWarp) {
     tcgen05_fence_after();
-    if (PAIR) {
-      tmem_dealloc_pair(tmem_base, w4::kTmemCols);
-    } else {
-      tmem_dealloc(tmem_base, w4::kTmemCols);
-    }
+    tmem_dealloc_pair(tmem_base, kTmemCols);
   }
 }
 
-// y = f16(sum of the K slices' partial tiles, in slice order (+ bias))
+// The tiles that more than one pair worked on: y = f16(sum of their partial tiles in K order (+ bias)).  Block (b, z): the
+// tile in which pair b + 1 begins, slice z of its tokens.
 __global__ void __launch_bounds__(256)
-w4a16_splitk_reduce_kernel(const float* __restrict__ partial, int k_split, int M, int N,
-                           const __half* __restrict__ bias, __half* __restrict__ y) {
-  const int quads = N >> 2;
-  const size_t slice = (size_t)M * N;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M * quads; i += gridDim.x * blockDim.x) {
-    const int m = i / quads, n = (i - m * quads) << 2;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < k_split; ++s) {
-      const float4 v = *reinterpret_cast<const float4*>(partial + s * slice + (size_t)m * N + n);
-      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+w4a16_gemm_reduce_kernel(const W4GemmParams p) {
+  chain_wait();
+  chain_release();
+  const int start = w4_range_start(static_cast<int>(blockIdx.x) + 1, p.share, p.extra);
+  const int tile = start / p.steps;
+  if (start == tile * p.steps) return;                       // the pair begins with the tile
+  const int first = w4_pair_of(tile * p.steps, p.share, p.extra);
+  if (first != static_cast<int>(blockIdx.x)) return;         // an earlier boundary in the same tile does it
+  const int last = w4_pair_of((tile + 1) * p.steps - 1, p.share, p.extra);
+  const int m0 = (tile % p.m_tiles) * p.T, n0 = (tile / p.m_tiles) * (2 * w4::kRows);
+  const int tokens = min(p.T, p.M - m0);
+  const size_t tile_words = (size_t)p.T * w4::kRows;
+  const int i = blockIdx.y * 256 + threadIdx.x;              // four rows of a token to a thread
+  if (i < tokens * (2 * w4::kRows / 4)) {
+    const int t = i / (2 * w4::kRows / 4), r = (i % (2 * w4::kRows / 4)) * 4;
+    const int rank = r / w4::kRows;
+    const float* src = p.partial + rank * tile_words + (size_t)t * w4::kRows + (r - rank * w4::kRows);
+    float4 acc = *reinterpret_cast<const float4*>(src + ((size_t)first * 2 + 1) * 2 * tile_words);
+    for (int q = first + 1; q <= last; q += 4) {             // four requests at a time
+      float4 v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (q + j <= last) v[j] = *reinterpret_cast<const float4*>(src + (size_t)(q + j) * 4 * tile_words);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (q + j <= last) { acc.x += v[j].x; acc.y += v[j].y; acc.z += v[j].z; acc.w += v[j].w; }
     }
-    if (bias) {
-      acc.x += h2f(bias[n]); acc.y += h2f(bias[n + 1]); acc.z += h2f(bias[n + 2]); acc.w += h2f(bias[n + 3]);
+    const float v[4] = {acc.x, acc.y, acc.z, acc.w};
+    const int n = n0 + r;
+    __half h[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) h[j] = f2h(p.bias && n + j < p.N ? v[j] + h2f(p.bias[n + j]) : v[j]);
+    __half* y = p.y + (size_t)(m0 + t) * p.N + n;
+    if (n + 4 <= p.N && p.N % 4 == 0) {
+      *reinterpret_cast<uint2*>(y) = make_uint2(h2_as_u32(__halves2half2(h[0], h[1])), h2_as_u32(__halves2half2(h[2], h[3])));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (n + j < p.N) y[j] = h[j];
     }
-    const __half2 lo = __floats2half2_rn(acc.x, acc.y), hi = __floats2half2_rn(acc.z, acc.w);
-    *reinterpret_cast<uint2*>(y + (size_t)m * N + n) = make_uint2(h2_as_u32(lo), h2_as_u32(hi));
   }
 }
 
-// With few output tiles (batch sizes just above the decode kernels' range, or a narrow N) most SMs
-// would idle while a handful stream all the weights: cut K so that about one work item per SM (per
-// CTA pair for M > 256) exists.  Returns 1 when the tiles alone fill the machine or N % 4 != 0.
-static int prefill_k_split(int M, int N, int K) {
-  if (N % 4 != 0) return 1;
-  const int n_tiles = (N + w4::kBN - 1) / w4::kBN;
-  int tiles, units;
-  if (M > 256) {
-    tiles = ((M + 511) / 512) * n_tiles;
-    units = kSmCount / 2;
-  } else {
-    tiles = (M > 128 ? (M + 255) / 256 : (M + 127) / 128) * n_tiles;
-    units = kSmCount;
+// Tokens of a tile, and whether pairs get equal runs of units (scratch needed) or whole tiles: the shortest estimate in
+// SM clocks.  A step is 4 T clocks of MMA but no less than 360 (8 KB of packed words at HBM rate, and about their
+// expansion), and 60 for its barriers; the last tile's epilogue 10 T; splitting adds 16 T for writing and reading partial
+// tiles and 5500 for the second launch.
+struct W4Shape {
+  int T;
+  bool split;
+  int pairs;
+};
+static W4Shape w4_gemm_shape(int M, int N, int K, bool may_split) {
+  const long long n_tiles = (N + 2 * w4::kRows - 1) / (2 * w4::kRows), steps = (K + w4::kStepK - 1) / w4::kStepK;
+  W4Shape best{};
+  long long best_cost = -1;
+  for (int T = w4::kMaxT; T >= 32; T -= 32) {
+    const long long tiles = n_tiles * ((M + T - 1) / T), units = tiles * steps;
+    const long long step = std::max(4 * T, 360) + 60;
+    const long long waves = (tiles + w4::kPairs - 1) / w4::kPairs;
+    const long long whole = waves * steps * step + 10 * T;
+    if (best_cost < 0 || whole < best_cost) {
+      best_cost = whole;
+      best = W4Shape{T, false, (int)std::min<long long>(tiles, w4::kPairs)};
+    }
+    const long long pairs = std::min<long long>(w4::kPairs, units / 4);
+    if (!may_split || pairs < 2 || units % pairs == 0 && units / pairs % steps == 0) continue;
+    const long long split = (units + pairs - 1) / pairs * step + 26 * T + 5500;
+    if (split < best_cost) {
+      best_cost = split;
+      best = W4Shape{T, true, (int)pairs};
+    }
   }
-  const int k_blocks = K / w4::kBK;
-  int ks = units / tiles;
-  if (ks > k_blocks / 4) ks = k_blocks / 4;          // at least four k-blocks per slice
-  if (ks > 16) ks = 16;
-  if (ks < 2) return 1;
-  const int per = (k_blocks + ks - 1) / ks;
-  return (k_blocks + per - 1) / per;                  // no empty slice
+  return best;
 }
 
-template <int MT, bool PAIR = false>
-static int launch_w4_gemm(const CUtensorMap& tx, W4GemmParams p, cudaStream_t st) {
-  using C = w4::Cfg<MT, PAIR>;
-  constexpr int kTileRows = (PAIR ? 2 : 1) * C::kBM;
-  p.m_tiles = (p.M + kTileRows - 1) / kTileRows;
-  auto kern = w4a16_gemm_kernel<MT, PAIR>;
-  static thread_local int configured_device = -1;
-  int device = 0;
-  MP_CUDA_TRY(cudaGetDevice(&device));
-  if (configured_device != device) {
-    MP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem));
-    configured_device = device;
-  }
-  const long long total = (long long)p.m_tiles * p.n_tiles * p.k_split;
-  if (PAIR) {
-    const int pairs = (int)(total < kSmCount / 2 ? total : kSmCount / 2);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(2 * pairs, 1, 1);
-    cfg.blockDim = dim3(C::kThreads, 1, 1);
-    cfg.dynamicSmemBytes = C::kSmem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    MP_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tx, p));
-    return MP_OK;
-  }
-  const int grid = (int)(total < kSmCount ? total : kSmCount);
-  kern<<<grid, C::kThreads, C::kSmem, st>>>(tx, p);
-  MP_LAUNCH_CHECK();
-  return MP_OK;
-}
+static size_t w4_partial_bytes(int pairs, int T) { return (size_t)pairs * 4 * T * w4::kRows * sizeof(float); }
 
 }  // namespace mp
 
 using namespace mp;
 
+// Room for the partial tiles wherever they may be wanted: when the split is chosen, and for fewer tiles than pairs.
 extern "C" size_t mp_w4a16_prefill_workspace_bytes(int M, int N, int K) {
-  if (M <= 0 || N <= 0 || K <= 0 || K % w4::kBK != 0) return 0;
-  const int ks = prefill_k_split(M, N, K);
-  return ks > 1 ? (size_t)ks * M * N * sizeof(float) : 0;
+  if (M <= 0 || N <= 0 || K <= 0 || K % 64 != 0) return 0;
+  const W4Shape s = w4_gemm_shape(M, N, K, true);
+  return s.split || s.pairs < w4::kPairs ? w4_partial_bytes(s.pairs, s.T) : 0;
 }
 
 extern "C" int mp_w4a16_linear_prefill(const void* x_f16, const void* packed_i32, const void* sz_f16x2,
@@ -498,38 +582,63 @@ extern "C" int mp_w4a16_linear_prefill_ex(const void* x_f16, const void* packed_
                                           void* workspace, size_t workspace_bytes, int* error_word,
                                           mp_stream_t stream) {
   if (!x_f16 || !packed_i32 || !sz_f16x2 || !y_f16 || M <= 0 || N <= 0 || K <= 0 || group <= 0) return MP_ERR_INVALID_ARG;
-  if (K % w4::kBK != 0 || group % w4::kBK != 0 || K % group != 0) return MP_ERR_UNSUPPORTED;
+  if (K % 64 != 0 || group % 64 != 0 || K % group != 0) return MP_ERR_UNSUPPORTED;
   if (!aligned(x_f16, 16) || !aligned(packed_i32, 16) || !aligned(sz_f16x2, 4) || !aligned(y_f16, 16)) return MP_ERR_ALIGNMENT;
-  CUtensorMap tx;
-  int rc = encode_tensor_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x_f16, (uint64_t)K, (uint64_t)M,
-                                (uint64_t)K * 2, w4::kBK, 128);
+  const W4Shape shape = w4_gemm_shape(M, N, K, workspace != nullptr);
+  if (workspace) {
+    if (workspace_bytes < mp_w4a16_prefill_workspace_bytes(M, N, K)) return MP_ERR_WORKSPACE;
+    if (!aligned(workspace, 16)) return MP_ERR_ALIGNMENT;
+  }
+  CUtensorMap tx, tw;
+  int rc = encode_tensor_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x_f16, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, 64,
+                                shape.T / 2);
+  if (rc != MP_OK) return rc;
+  rc = encode_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, packed_i32, (uint64_t)K / 2, (uint64_t)N, (uint64_t)K / 2,
+                            w4::kStageK / 2, w4::kRows);
   if (rc != MP_OK) return rc;
   W4GemmParams p{};
-  p.packed = static_cast<const uint32_t*>(packed_i32);
   p.sz = static_cast<const uint32_t*>(sz_f16x2);
   p.bias = static_cast<const __half*>(bias_f16);
   p.y = static_cast<__half*>(y_f16);
   p.M = M; p.N = N; p.K = K; p.group = group;
-  p.n_tiles = (N + w4::kBN - 1) / w4::kBN;
-  p.k_blocks = K / w4::kBK;
+  p.T = shape.T;
+  p.m_tiles = (M + shape.T - 1) / shape.T;
+  p.steps = (K + w4::kStepK - 1) / w4::kStepK;
   p.error_word = error_word;
-  p.k_split = 1;
-  p.kb_per_split = p.k_blocks;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int ks = workspace ? prefill_k_split(M, N, K) : 1;    // without scratch: one K slice per tile
-  if (ks > 1) {
-    if (workspace_bytes < (size_t)ks * M * N * sizeof(float)) return MP_ERR_WORKSPACE;
-    if (!aligned(workspace, 16)) return MP_ERR_ALIGNMENT;
-    p.k_split = ks;
-    p.kb_per_split = (p.k_blocks + ks - 1) / ks;
+  const long long tiles = (long long)p.m_tiles * ((N + 2 * w4::kRows - 1) / (2 * w4::kRows)), units = tiles * p.steps;
+  if (units > 2000000000LL) return MP_ERR_UNSUPPORTED;
+  if (shape.split) {
     p.partial = static_cast<float*>(workspace);
+    p.share = (int)(units / shape.pairs);
+    p.extra = (int)(units % shape.pairs);
+  } else {
+    p.share = (int)(tiles / shape.pairs);
+    p.extra = (int)(tiles % shape.pairs);
   }
-  rc = M > 256 ? launch_w4_gemm<2, true>(tx, p, st)          // 512 x 256 tiles on CTA pairs
-       : M > 128 ? launch_w4_gemm<2>(tx, p, st) : launch_w4_gemm<1>(tx, p, st);
-  if (rc != MP_OK || ks == 1) return rc;
-  int blocks = (M * (N / 4) + 255) / 256;
-  if (blocks > 2 * kSmCount) blocks = 2 * kSmCount;
-  w4a16_splitk_reduce_kernel<<<blocks, 256, 0, st>>>(p.partial, ks, M, N, p.bias, p.y);
-  MP_LAUNCH_CHECK();
-  return MP_OK;
+  p.unit_steps = shape.split ? 1 : p.steps;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  static thread_local int configured_device = -1;
+  int device = 0;
+  MP_CUDA_TRY(cudaGetDevice(&device));
+  if (configured_device != device) {
+    MP_CUDA_TRY(cudaFuncSetAttribute(w4a16_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w4::kSmem));
+    configured_device = device;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(2 * shape.pairs, 1, 1);
+  cfg.blockDim = dim3(w4::kThreads, 1, 1);
+  cfg.dynamicSmemBytes = w4::kSmem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  MP_CUDA_TRY(cudaLaunchKernelEx(&cfg, w4a16_gemm_kernel, tx, tw, p));
+  if (!shape.split) return MP_OK;
+  return launch_chained(w4a16_gemm_reduce_kernel, dim3(shape.pairs - 1, shape.T / 4), dim3(256), 0, st, p);
 }

@@ -514,7 +514,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       __syncwarp();
       if (lane == 0) {
         if (PAIR) {
-          mbar_arrive_cluster(tempty_leader0 + 8 * buf);
+          mbar_arrive_tmem(tempty_leader0 + 8 * buf);
         } else {
           mbar_arrive(tempty0 + 8 * buf);
         }
