@@ -265,11 +265,11 @@ __device__ __forceinline__ void umma_i8_pair(uint32_t tmem_d, uint64_t desc_a, u
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrive (once the pair's MMAs issued so far have completed) on an mbarrier given by its
-// shared::cluster address: this CTA's own (its shared::cta address is valid here) or the peer's.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster)
-               : "memory");
+// Arrive, once the pair's MMAs issued so far have completed, on the mbarrier at this shared-memory offset in both CTAs of
+// the pair.
+__device__ __forceinline__ void umma_commit_both(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"(static_cast<unsigned short>(3)) : "memory");
 }
 
 // Arrive on an mbarrier of this CTA once all MMAs issued so far by this

@@ -11,7 +11,7 @@
 //   * the tokens are the MMA's N, any multiple of 32, so little is multiplied for padding.
 //   * expanding 32768 weights takes the SM's ALUs 660 clocks of those 2048.
 // A persistent pair per two SMs, roles by warp:
-//   warps 0-11   expansion, three sets of four warps taking 128-column steps in turn: a lane holds a weight row, makes
+//   warps 0-11   expansion, three sets of four warps taking 256-column stages in turn: a lane holds a weight row, makes
 //                exactly f16((u - z) * s) of its words and stores them to a tensor memory slot
 //   warps 12-19  epilogue: accumulators -> fp16 (+ bias), transposed through shared memory -> y; or fp32 partial tiles
 //   warp 20      TMA producer of the packed words (256 columns a stage)
@@ -28,6 +28,7 @@
 // Every mbarrier wait is bounded (tc.cuh); on a timeout the pair records an error word, lets its copies land, frees its
 // tensor memory and returns.
 #include <algorithm>
+#include <climits>
 
 #include "common.cuh"
 #include "tc.cuh"
@@ -46,7 +47,7 @@ constexpr int kThreads = 32 * (kXWarp + 1);
 constexpr int kStageBytes = kRows * kStageK / 2;
 constexpr int kMaxT = 256;
 constexpr int kSlotCols = kStepK / 2;      // tensor memory columns of a step's expanded weights
-constexpr int kMaxSlots = 6, kMaxXRing = 6, kMaxRing = 8;
+constexpr int kMaxSlots = 6, kMaxRing = 8;
 constexpr int kRingBytes = 208 * 1024;     // both rings
 constexpr int kStagingBytes = kEpiWarps * 2048;
 constexpr int kTailBytes = 512;
@@ -55,18 +56,18 @@ constexpr int kTmemCols = 512;
 constexpr int kPairs = kSmCount / 2;
 
 __host__ __device__ constexpr int accumulators(int T) { return T <= 128 ? 2 : 1; }
-// slots and weight stages: four or more, see the waits of the expansion
+// Slots of a step's operands: tensor memory for the expanded weights, shared memory for the activations.  There are four
+// or more, and at least as many weight stages, see the waits of the expansion.
 __host__ __device__ constexpr int slots(int T) {
   const int n = (kTmemCols - accumulators(T) * T) / kSlotCols;
   return n < kMaxSlots ? n : kMaxSlots;
 }
 __host__ __device__ constexpr int x_step_bytes(int T) { return T / 2 * kStepK * 2; }
-__host__ __device__ constexpr int x_ring(int T) { return T > 128 ? 4 : kMaxXRing; }
 __host__ __device__ constexpr int ring(int T) {
-  const int n = (kRingBytes - x_ring(T) * x_step_bytes(T)) / kStageBytes;
+  const int n = (kRingBytes - slots(T) * x_step_bytes(T)) / kStageBytes;
   return n < kMaxRing ? n : kMaxRing;
 }
-static_assert(slots(256) == 4 && slots(128) == 4 && slots(160) == 5 && ring(256) == 5 && ring(128) >= 4, "rings");
+static_assert(slots(256) == 4 && slots(128) == 4 && slots(160) == 5 && ring(256) == 5 && ring(192) == 5 && ring(128) >= 6, "rings");
 }  // namespace w4
 
 struct W4GemmParams {
@@ -131,20 +132,18 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   using namespace w4;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int T = p.T, n_slots = slots(T), n_x = x_ring(T), n_w = ring(T), n_acc = accumulators(T);
+  const int T = p.T, n_slots = slots(T), n_w = ring(T), n_acc = accumulators(T);
   const int x_bytes = x_step_bytes(T), x_half = x_bytes / 2;
   unsigned char* tail = smem + kRingBytes + kStagingBytes;
-  const uint32_t xring = smem_u32(smem), wring = xring + n_x * x_bytes, staging = xring + kRingBytes;
+  const uint32_t xring = smem_u32(smem), wring = xring + n_slots * x_bytes, staging = xring + kRingBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(tail);
   const uint32_t wfull0 = smem_u32(bars);                  // packed words landed
   const uint32_t wempty0 = wfull0 + 8 * kMaxRing;          // ... and were read
-  const uint32_t xfull0 = wempty0 + 8 * kMaxRing;          // leader: both CTAs' activations landed
-  const uint32_t xempty0 = xfull0 + 8 * kMaxXRing;         // ... and were multiplied
-  const uint32_t ready0 = xempty0 + 8 * kMaxXRing;         // leader: both CTAs' slots hold an expanded step
-  const uint32_t done0 = ready0 + 8 * kMaxSlots;           // ... and it was multiplied
+  const uint32_t ready0 = wempty0 + 8 * kMaxRing;          // leader: both CTAs' halves of a slot's operands are in place
+  const uint32_t done0 = ready0 + 8 * kMaxSlots;           // ... and were multiplied
   const uint32_t tfull0 = done0 + 8 * kMaxSlots;           // a segment's accumulator is complete
   const uint32_t tempty0 = tfull0 + 16;                    // leader: both CTAs have read it
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 8 * (2 * kMaxRing + 2 * kMaxXRing + 2 * kMaxSlots + 4));
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 8 * (2 * kMaxRing + 2 * kMaxSlots + 4));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -153,14 +152,10 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   if (threadIdx.x == 0) {
     for (int s = 0; s < n_w; ++s) {
       mbar_init(wfull0 + 8 * s, 1);
-      mbar_init(wempty0 + 8 * s, 8);                       // four warps for each of the stage's two steps
-    }
-    for (int s = 0; s < n_x; ++s) {
-      mbar_init(xfull0 + 8 * s, 1);
-      mbar_init(xempty0 + 8 * s, 1);
+      mbar_init(wempty0 + 8 * s, 4);                       // a set's warps
     }
     for (int q = 0; q < n_slots; ++q) {
-      mbar_init(ready0 + 8 * q, 8);                        // four warps of each CTA
+      mbar_init(ready0 + 8 * q, 9);                        // four warps of each CTA, the leader's TMA producer
       mbar_init(done0 + 8 * q, 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -194,7 +189,6 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     g.s1 = min(steps, g.s0 + u1 - u);
   };
   auto first_row = [&](int tile) { return (tile / p.m_tiles) * (2 * kRows) + static_cast<int>(rank) * kRows; };
-  const uint32_t peer_or_own = rank ^ 1u;
 
   if (warp == kWeightWarp) {
     if (elect_one()) {
@@ -217,7 +211,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   } else if (warp == kXWarp) {
     if (elect_one()) {
       prefetch_tensormap(&tmap_x);
-      const uint32_t xfull_leader0 = map_to_cta(xfull0, 0);
+      const uint32_t ready_leader0 = map_to_cta(ready0, 0);
       int s = 0;
       uint32_t phase = 1;
       bool ok = true;
@@ -226,24 +220,22 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         segment_at(u, g);
         const int m0 = (g.tile % p.m_tiles) * T + static_cast<int>(rank) * (T / 2);
         for (int st = g.s0; st < g.s1; ++st) {
-          if (!mbar_wait(xempty0 + 8 * s, phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait(done0 + 8 * s, phase, abort_flag)) { ok = false; break; }
           const int k0 = st * kStepK;
           const bool both = k0 + 64 < p.K;
-          if (leader) mbar_arrive_expect_tx(xfull0 + 8 * s, both ? 2 * x_bytes : x_bytes);     // of both CTAs
-          tma_load_2d_pair(xring + s * x_bytes, &tmap_x, xfull_leader0 + 8 * s, k0, m0);
-          if (both) tma_load_2d_pair(xring + s * x_bytes + x_half, &tmap_x, xfull_leader0 + 8 * s, k0 + 64, m0);
-          if (++s == n_x) { s = 0; phase ^= 1; }
+          if (leader) mbar_arrive_expect_tx(ready0 + 8 * s, both ? 2 * x_bytes : x_bytes);     // of both CTAs
+          tma_load_2d_pair(xring + s * x_bytes, &tmap_x, ready_leader0 + 8 * s, k0, m0);
+          if (both) tma_load_2d_pair(xring + s * x_bytes + x_half, &tmap_x, ready_leader0 + 8 * s, k0 + 64, m0);
+          if (++s == n_slots) { s = 0; phase ^= 1; }
         }
       }
     }
   } else if (warp == kMmaWarp) {
     if (leader && elect_one()) {
       const uint32_t idesc = umma_idesc(kIdescDFormatF32 | kIdescABFormatF16, 2 * kRows, T);
-      const uint32_t xempty_peer0 = map_to_cta(xempty0, peer_or_own), done_peer0 = map_to_cta(done0, peer_or_own),
-                     tfull_peer0 = map_to_cta(tfull0, peer_or_own);
       const uint64_t b_desc0 = umma_desc_k_sw128(xring);
-      int q = 0, xs = 0, d = 0;
-      uint32_t phase = 0, xphase = 0, dphase = 1;
+      int q = 0, d = 0;
+      uint32_t phase = 0, dphase = 1;
       bool ok = true;
       W4Segment g;
       for (int u = u0; ok && u < u1; u += g.s1 - g.s0) {
@@ -251,124 +243,112 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         if (!mbar_wait(tempty0 + 8 * d, dphase, abort_flag)) break;
         const uint32_t d_tmem = tmem_base + d * T;
         for (int st = g.s0; st < g.s1; ++st) {
-          if (!mbar_wait(xfull0 + 8 * xs, xphase, abort_flag) || !mbar_wait(ready0 + 8 * q, phase, abort_flag)) {
-            ok = false;
-            break;
-          }
+          if (!mbar_wait(ready0 + 8 * q, phase, abort_flag)) { ok = false; break; }
           tcgen05_fence_after();
           const uint32_t a_tmem = tmem_base + n_acc * T + q * kSlotCols;
           const int halves = st * kStepK + 64 < p.K ? 2 : 1;
           for (int h = 0; h < halves; ++h) {
-            const uint64_t b_desc = b_desc0 + ((xs * x_bytes + h * x_half) >> 4);
+            const uint64_t b_desc = b_desc0 + ((q * x_bytes + h * x_half) >> 4);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)       // 16 K per instruction: 8 columns of A, 32 bytes of B's rows
               umma_f16_ts_pair(d_tmem, a_tmem + (h * 4 + kk) * 8, b_desc + 2 * kk, idesc, st != g.s0 || h != 0 || kk != 0);
           }
-          umma_commit_pair(xempty0 + 8 * xs);
-          umma_commit_pair(xempty_peer0 + 8 * xs);
-          umma_commit_pair(done0 + 8 * q);
-          umma_commit_pair(done_peer0 + 8 * q);
-          if (++xs == n_x) { xs = 0; xphase ^= 1; }
+          umma_commit_both(done0 + 8 * q);
           if (++q == n_slots) { q = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma_commit_pair(tfull0 + 8 * d);
-        umma_commit_pair(tfull_peer0 + 8 * d);
+        umma_commit_both(tfull0 + 8 * d);
         if (++d == n_acc) { d = 0; dphase ^= 1; }
       }
     }
   } else if (warp < kEpiWarp0) {
-    // ---- expansion: this warp's 32 rows of every third step
+    // ---- expansion: this warp's 32 rows of every third stage (two steps, one where the pair's run begins or ends in it)
     const int quarter = warp & 3, set = warp >> 2;
     const int row = quarter * 32 + lane, sw = row & 7;
     const uint32_t a_tmem0 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + n_acc * T;
     const uint32_t ready_leader0 = map_to_cta(ready0, 0);
-    const int sub_blocks = p.K / 64;
-    // the group of a step's first 64 columns and how many such blocks of it come before, kept by addition from step to step
-    const int g64 = p.group / 64, g_step = 2 * kSets / g64, r_step = 2 * kSets % g64;
-    int grp = 0, rem = 0;
-    int q = set % n_slots, s = 0, ord = 0;                // slot; weight stage and its running number
-    uint32_t qphase = 1, phase = 0;
+    const int sub_blocks = p.K / 64, g64 = p.group / 64;
+    // x / d for the small quotients here is the high word of x * ceil(2^32 / d), d > 1
+    const uint32_t by_slots = 0xffffffffu / n_slots + 1, by_ring = 0xffffffffu / n_w + 1, by_group = 0xffffffffu / g64 + 1;
     W4Segment g{0, 0, 0};
-    int n = 0, base = 0, end = u0, next_base = 0;          // of the segment [.., end): row, first stage's running number
-    // (scale, zero) of this row for a step's two halves
-    auto load_sz = [&](int st, uint32_t (&z)[2]) {
-      const uint32_t* src = p.sz + (size_t)grp * p.N + n;
-      const bool live = n < p.N;
-      z[0] = live ? __ldg(src) : 0u;
-      z[1] = live && 2 * st + 1 < sub_blocks ? __ldg(rem + 1 >= g64 ? src + p.N : src) : 0u;
-    };
-    auto seek = [&](int u) {                               // the segment that holds unit u
-      while (u >= end) {
+    int n = 0, end = u0, g_unit = 0, g_stage = 0, g_stages = 0;   // the segment's row, end, first unit and first stage of this pair
+    const int sets = n_slots < 5 ? 2 : kSets;                     // four slots are for many tokens, and two sets enough
+    int o = set < sets ? set : INT_MAX / 2;                       // running number of this set's stage
+    auto seek = [&]() {
+      while (o >= g_stage + g_stages) {
+        if (end >= u1) return false;
+        g_unit = end - u0;
+        g_stage += g_stages;
         segment_at(end, g);
-        base = next_base;
-        next_base = base + ((g.s1 - 1) >> 1) - (g.s0 >> 1) + 1;
+        g_stages = ((g.s1 - 1) >> 1) - (g.s0 >> 1) + 1;
         end += g.s1 - g.s0;
         n = first_row(g.tile) + row;
       }
-      const int st = g.s1 - (end - u);
-      grp = 2 * st / g64;
-      rem = 2 * st - grp * g64;
-      return st;
+      return true;
     };
-    int u = u0 + set, st = 0;
-    uint32_t sz_next[2];
-    if (u < u1) {
-      st = seek(u);
-      load_sz(st, sz_next);
-    }
-    while (u < u1) {
-      const int now = base + (st >> 1) - (g.s0 >> 1);
-      for (; ord < now; ++ord)
-        if (++s == n_w) { s = 0; phase ^= 1; }
-      const uint32_t sz_now[2] = {sz_next[0], sz_next[1]};
-      const bool alone = (st ^ 1) < g.s0 || (st ^ 1) >= g.s1;        // the stage's other step is not this pair's
-      // The slot first: when the MMAs of the step n_slots >= 4 before this one are done, the stages before the last four
-      // have been filled and read, so that the parity of the stage's barrier is not ambiguous.
-      if (!__all_sync(0xffffffffu, mbar_wait(done0 + 8 * q, qphase, abort_flag) &&
-                                       mbar_wait(wfull0 + 8 * s, phase, abort_flag))) break;
-      tcgen05_fence_after();
-      const uint32_t src = wring + s * kStageBytes + row * 128;
-      uint4 w[4];
+    // (scale, zero) of this row for the stage's four blocks of 64 columns
+    auto load_sz = [&](int stage, uint32_t (&z)[4]) {
+      const bool live = n < p.N;
+      int before = -1;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = w4_lds_v4(src + ((((st & 1) * 4 + j) ^ sw) << 4));
-      u += kSets;
-      const int this_st = st;
-      if (u < u1) {                                        // the next step's scales, while this one is expanded
-        if (u < end) {
-          st += kSets;
-          grp += g_step;
-          rem += r_step;
-          if (rem >= g64) { rem -= g64; ++grp; }
-        } else {
-          st = seek(u);
+      for (int i = 0; i < 4; ++i) {
+        const int b = 4 * stage + i;
+        const int grp = g64 == 1 ? b : static_cast<int>(__umulhi(static_cast<uint32_t>(b), by_group));
+        if (b >= sub_blocks) z[i] = 0u;
+        else if (i > 0 && grp == before) z[i] = z[i > 0 ? i - 1 : 0];
+        else z[i] = live ? __ldg(p.sz + (size_t)grp * p.N + n) : 0u;
+        before = grp;
+      }
+    };
+    uint32_t sz_next[4];
+    bool more = seek();
+    if (more) load_sz((g.s0 >> 1) + o - g_stage, sz_next);
+    bool ok = true;
+    while (ok && more) {
+      const int stage = (g.s0 >> 1) + o - g_stage;
+      const int first = max(2 * stage, g.s0), last = min(2 * stage + 2, g.s1);
+      int unit = g_unit + first - g.s0;
+      const int lap = static_cast<int>(__umulhi(static_cast<uint32_t>(o), by_ring)), s = o - lap * n_w;
+      const uint32_t sz_now[4] = {sz_next[0], sz_next[1], sz_next[2], sz_next[3]};
+      o += sets;
+      more = seek();
+      if (more) load_sz((g.s0 >> 1) + o - g_stage, sz_next);     // arrives while this stage is expanded
+#pragma unroll 1
+      for (int st = first; st < last; ++st, ++unit) {
+        const int use = static_cast<int>(__umulhi(static_cast<uint32_t>(unit), by_slots)), q = unit - use * n_slots;
+        // The parity of the slot's barrier is not ambiguous: of three sets this one's stage before held no unit older than
+        // five before this one, which waited for the unit n_slots before it, and two turns of five slots or more ago is no
+        // later than that; of two sets it is three, and four slots will do.  Nor is that of the stage's barrier: when the
+        // unit n_slots before this one is done, every stage n_w >= n_slots before this one has been filled and read.
+        if (!__all_sync(0xffffffffu, mbar_wait(done0 + 8 * q, (use & 1) ^ 1, abort_flag))) { ok = false; break; }
+        if (st == first && !__all_sync(0xffffffffu, mbar_wait(wfull0 + 8 * s, lap & 1, abort_flag))) { ok = false; break; }
+        tcgen05_fence_after();
+        const uint32_t src = wring + s * kStageBytes + row * 128;
+        const int h = st & 1;
+        uint4 w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = w4_lds_v4(src + (((h * 4 + j) ^ sw) << 4));
+        const uint32_t sz_h[2] = {h ? sz_now[2] : sz_now[0], h ? sz_now[3] : sz_now[1]};
+        const uint32_t a_tmem = a_tmem0 + q * kSlotCols;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (j == 2 && 2 * st + 1 >= sub_blocks) break;                // K ends in the middle of the step
+          const __half2 szh = *reinterpret_cast<const __half2*>(&sz_h[j >> 1]);
+          const ScaleZero sp = make_scale_zero(__low2half(szh), __high2half(szh));
+          uint32_t r[16];
+          expand_word(w[j].x, sp, r);
+          expand_word(w[j].y, sp, r + 4);
+          expand_word(w[j].z, sp, r + 8);
+          expand_word(w[j].w, sp, r + 12);
+          tmem_st_32x32_x16(a_tmem + j * 16, r);
         }
-        load_sz(st, sz_next);
+        __syncwarp();
+        if (st == last - 1 && lane == 0) mbar_arrive(wempty0 + 8 * s);
+        tmem_st_wait();
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_tmem(ready_leader0 + 8 * q);
       }
-      const uint32_t a_tmem = a_tmem0 + q * kSlotCols;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (j == 2 && 2 * this_st + 1 >= sub_blocks) break;             // K ends in the middle of the step
-        const __half2 szh = *reinterpret_cast<const __half2*>(&sz_now[j >> 1]);
-        uint32_t r[16];
-        const ScaleZero sp = make_scale_zero(__low2half(szh), __high2half(szh));
-        expand_word(w[j].x, sp, r);
-        expand_word(w[j].y, sp, r + 4);
-        expand_word(w[j].z, sp, r + 8);
-        expand_word(w[j].w, sp, r + 12);
-        tmem_st_32x32_x16(a_tmem + j * 16, r);
-      }
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(wempty0 + 8 * s);
-        if (alone) mbar_arrive(wempty0 + 8 * s);
-      }
-      tmem_st_wait();
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_tmem(ready_leader0 + 8 * q);
-      q += kSets;
-      if (q >= n_slots) { q -= n_slots; qphase ^= 1; }
     }
   } else {
     // ---- epilogue: lane = weight row, column = token; two warps to a quarter of the rows take 32 tokens in turn
@@ -525,8 +505,7 @@ w4a16_gemm_reduce_kernel(const W4GemmParams p) {
 }
 
 // Tokens of a tile, and whether pairs get equal runs of units (scratch needed) or whole tiles: the shortest estimate in
-// SM clocks.  A step is 4 T clocks of MMA but no less than 360 (8 KB of packed words at HBM rate, and about their
-// expansion), and 60 for its barriers; the last tile's epilogue 10 T; splitting adds 16 T for writing and reading partial
+// SM clocks.  A step is 4 T clocks of MMA but no less than the 600 of its expansion, and 60 for its barriers; the last tile's epilogue 10 T; splitting adds 16 T for writing and reading partial
 // tiles and 5500 for the second launch.
 struct W4Shape {
   int T;
@@ -539,7 +518,7 @@ static W4Shape w4_gemm_shape(int M, int N, int K, bool may_split) {
   long long best_cost = -1;
   for (int T = w4::kMaxT; T >= 32; T -= 32) {
     const long long tiles = n_tiles * ((M + T - 1) / T), units = tiles * steps;
-    const long long step = std::max(4 * T, 360) + 60;
+    const long long step = std::max(4 * T, 600) + 60;
     const long long waves = (tiles + w4::kPairs - 1) / w4::kPairs;
     const long long whole = waves * steps * step + 10 * T;
     if (best_cost < 0 || whole < best_cost) {

@@ -302,8 +302,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             }
           }
           if (PAIR) {                      // release the stage in both CTAs
-            umma_commit_pair(empty0 + 8 * stage);
-            umma_commit_pair(map_to_cta(empty0 + 8 * stage, 1));
+            umma_commit_both(empty0 + 8 * stage);
           } else {
             umma_commit(empty0 + 8 * stage);
           }
@@ -311,8 +310,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
         if (!ok) break;
         if (PAIR) {                        // publish the accumulator halves to both CTAs' epilogues
-          umma_commit_pair(tfull0 + 8 * buf);
-          umma_commit_pair(map_to_cta(tfull0 + 8 * buf, 1));
+          umma_commit_both(tfull0 + 8 * buf);
         } else {
           umma_commit(tfull0 + 8 * buf);
         }
