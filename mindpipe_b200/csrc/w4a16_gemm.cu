@@ -11,7 +11,7 @@
 //   * the tokens are the MMA's N, any multiple of 32, so little is multiplied for padding.
 //   * expanding 32768 weights takes the SM's ALUs 660 clocks of those 2048.
 // A persistent pair per two SMs, roles by warp:
-//   warps 0-11   expansion, three sets of four warps taking 256-column stages in turn: a lane holds a weight row, makes
+//   warps 0-11   expansion, three sets of four warps taking 128-column steps in turn: a lane holds a weight row, makes
 //                exactly f16((u - z) * s) of its words and stores them to a tensor memory slot
 //   warps 12-19  epilogue: accumulators -> fp16 (+ bias), transposed through shared memory -> y; or fp32 partial tiles
 //   warp 20      TMA producer of the packed words (256 columns a stage)
@@ -28,7 +28,6 @@
 // Every mbarrier wait is bounded (tc.cuh); on a timeout the pair records an error word, lets its copies land, frees its
 // tensor memory and returns.
 #include <algorithm>
-#include <climits>
 
 #include "common.cuh"
 #include "tc.cuh"
@@ -48,26 +47,28 @@ constexpr int kStageBytes = kRows * kStageK / 2;
 constexpr int kMaxT = 256;
 constexpr int kSlotCols = kStepK / 2;      // tensor memory columns of a step's expanded weights
 constexpr int kMaxSlots = 6, kMaxRing = 8;
-constexpr int kRingBytes = 208 * 1024;     // both rings
-constexpr int kStagingBytes = kEpiWarps * 2048;
+constexpr int kRingBytes = 192 * 1024;     // both rings
+constexpr int kStagingBytes = kEpiWarps * 4096;           // two chunks of 32 tokens x 32 rows for each epilogue warp
 constexpr int kTailBytes = 512;
 constexpr size_t kSmem = 1024 + kRingBytes + kStagingBytes + kTailBytes;
 constexpr int kTmemCols = 512;
 constexpr int kPairs = kSmCount / 2;
 
 __host__ __device__ constexpr int accumulators(int T) { return T <= 128 ? 2 : 1; }
+__host__ __device__ constexpr int x_step_bytes(int T) { return T / 2 * kStepK * 2; }
 // Slots of a step's operands: tensor memory for the expanded weights, shared memory for the activations.  There are four
 // or more, and at least as many weight stages, see the waits of the expansion.
 __host__ __device__ constexpr int slots(int T) {
-  const int n = (kTmemCols - accumulators(T) * T) / kSlotCols;
-  return n < kMaxSlots ? n : kMaxSlots;
+  int n = (kTmemCols - accumulators(T) * T) / kSlotCols;
+  if (n > kMaxSlots) n = kMaxSlots;
+  while ((kRingBytes - n * x_step_bytes(T)) / kStageBytes < n) --n;
+  return n;
 }
-__host__ __device__ constexpr int x_step_bytes(int T) { return T / 2 * kStepK * 2; }
 __host__ __device__ constexpr int ring(int T) {
   const int n = (kRingBytes - slots(T) * x_step_bytes(T)) / kStageBytes;
   return n < kMaxRing ? n : kMaxRing;
 }
-static_assert(slots(256) == 4 && slots(128) == 4 && slots(160) == 5 && ring(256) == 5 && ring(192) == 5 && ring(128) >= 6, "rings");
+static_assert(slots(256) == 4 && slots(128) == 4 && slots(160) == 5 && slots(192) == 4 && slots(224) == 4 && ring(256) == 4 && ring(160) == 5, "rings");
 }  // namespace w4
 
 struct W4GemmParams {
@@ -99,14 +100,21 @@ struct W4Segment {
 
 // D[tmem] (+)= A[tmem] * B[smem] over a CTA pair: M = 256, 128 lanes of A and D in each CTA's tensor memory, B's rows
 // split in halves between the two shared memories.
-__device__ __forceinline__ void umma_f16_ts_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
-                                                 uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
+template <bool ACCUMULATE = true>
+__device__ __forceinline__ void umma_f16_ts_pair(uint32_t tmem_d, uint32_t tmem_a, uint32_t desc_lo, uint32_t desc_hi,
+                                                 uint32_t idesc, bool accumulate = true) {
+  if (ACCUMULATE) {
+    asm volatile(
+        "{\n\t.reg .b64 b;\n\tmov.b64 b, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], b, %4, 1;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(desc_lo), "r"(desc_hi), "r"(idesc) : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .b64 b;\n\t.reg .pred p;\n\tmov.b64 b, {%2, %3};\n\tsetp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(desc_lo), "r"(desc_hi), "r"(idesc), "r"(static_cast<uint32_t>(accumulate))
+        : "memory");
+  }
 }
 
 __device__ __forceinline__ uint4 w4_lds_v4(uint32_t addr) {
@@ -152,7 +160,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   if (threadIdx.x == 0) {
     for (int s = 0; s < n_w; ++s) {
       mbar_init(wfull0 + 8 * s, 1);
-      mbar_init(wempty0 + 8 * s, 4);                       // a set's warps
+      mbar_init(wempty0 + 8 * s, 8);                       // four warps for each of the stage's two steps
     }
     for (int q = 0; q < n_slots; ++q) {
       mbar_init(ready0 + 8 * q, 9);                        // four warps of each CTA, the leader's TMA producer
@@ -233,7 +241,12 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   } else if (warp == kMmaWarp) {
     if (leader && elect_one()) {
       const uint32_t idesc = umma_idesc(kIdescDFormatF32 | kIdescABFormatF16, 2 * kRows, T);
+      // This thread's instructions wait their turn among those of the expansion: at 160 tokens and fewer they set the pace, so
+      // a step has as few as possible.
       const uint64_t b_desc0 = umma_desc_k_sw128(xring);
+      const uint32_t desc_hi = static_cast<uint32_t>(b_desc0 >> 32), desc_lo0 = static_cast<uint32_t>(b_desc0);
+      const uint32_t a0 = tmem_base + n_acc * T, slot_step = x_bytes >> 4, half_step = x_half >> 4;
+      uint32_t desc = desc_lo0, a_tmem = a0;
       int q = 0, d = 0;
       uint32_t phase = 0, dphase = 1;
       bool ok = true;
@@ -245,16 +258,19 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         for (int st = g.s0; st < g.s1; ++st) {
           if (!mbar_wait(ready0 + 8 * q, phase, abort_flag)) { ok = false; break; }
           tcgen05_fence_after();
-          const uint32_t a_tmem = tmem_base + n_acc * T + q * kSlotCols;
-          const int halves = st * kStepK + 64 < p.K ? 2 : 1;
-          for (int h = 0; h < halves; ++h) {
-            const uint64_t b_desc = b_desc0 + ((q * x_bytes + h * x_half) >> 4);
+          // 16 K per instruction: 8 columns of A, 32 bytes of B's rows
+          umma_f16_ts_pair<false>(d_tmem, a_tmem, desc, desc_hi, idesc, st != g.s0);
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)       // 16 K per instruction: 8 columns of A, 32 bytes of B's rows
-              umma_f16_ts_pair(d_tmem, a_tmem + (h * 4 + kk) * 8, b_desc + 2 * kk, idesc, st != g.s0 || h != 0 || kk != 0);
+          for (int kk = 1; kk < 4; ++kk) umma_f16_ts_pair(d_tmem, a_tmem + kk * 8, desc + 2 * kk, desc_hi, idesc);
+          if (st * kStepK + 64 < p.K) {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              umma_f16_ts_pair(d_tmem, a_tmem + 32 + kk * 8, desc + half_step + 2 * kk, desc_hi, idesc);
           }
           umma_commit_both(done0 + 8 * q);
-          if (++q == n_slots) { q = 0; phase ^= 1; }
+          desc += slot_step;
+          a_tmem += kSlotCols;
+          if (++q == n_slots) { q = 0; phase ^= 1; desc = desc_lo0; a_tmem = a0; }
         }
         if (!ok) break;
         umma_commit_both(tfull0 + 8 * d);
@@ -262,7 +278,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       }
     }
   } else if (warp < kEpiWarp0) {
-    // ---- expansion: this warp's 32 rows of every third stage (two steps, one where the pair's run begins or ends in it)
+    // ---- expansion: this warp's 32 rows of every third step
     const int quarter = warp & 3, set = warp >> 2;
     const int row = quarter * 32 + lane, sw = row & 7;
     const uint32_t a_tmem0 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + n_acc * T;
@@ -271,91 +287,86 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     // x / d for the small quotients here is the high word of x * ceil(2^32 / d), d > 1
     const uint32_t by_slots = 0xffffffffu / n_slots + 1, by_ring = 0xffffffffu / n_w + 1, by_group = 0xffffffffu / g64 + 1;
     W4Segment g{0, 0, 0};
-    int n = 0, end = u0, g_unit = 0, g_stage = 0, g_stages = 0;   // the segment's row, end, first unit and first stage of this pair
-    const int sets = n_slots < 5 ? 2 : kSets;                     // four slots are for many tokens, and two sets enough
-    int o = set < sets ? set : INT_MAX / 2;                       // running number of this set's stage
-    auto seek = [&]() {
-      while (o >= g_stage + g_stages) {
-        if (end >= u1) return false;
-        g_unit = end - u0;
-        g_stage += g_stages;
+    int n = 0, end = u0;                       // the segment's row, and the unit after it
+    int stage0 = 0, stages = 0;                // its first weight stage's number in this pair's run, and how many it has
+    auto seek = [&](int u) {
+      while (u >= end) {
+        stage0 += stages;
         segment_at(end, g);
-        g_stages = ((g.s1 - 1) >> 1) - (g.s0 >> 1) + 1;
+        stages = ((g.s1 - 1) >> 1) - (g.s0 >> 1) + 1;
         end += g.s1 - g.s0;
-        n = first_row(g.tile) + row;
+        n = min(first_row(g.tile) + row, p.N - 1);
       }
-      return true;
+      return g.s1 - (end - u);
     };
-    // (scale, zero) of this row for the stage's four blocks of 64 columns
-    auto load_sz = [&](int stage, uint32_t (&z)[4]) {
-      const bool live = n < p.N;
-      int before = -1;
+    // (scale, zero) of this row for the step's two blocks of 64 columns.  Two loads, the same word twice or not: a copy of
+    // one would wait for it here.  Rows and columns that do not exist take another's; nothing of theirs is kept.
+    auto load_sz = [&](int st, uint32_t (&z)[2]) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int b = 4 * stage + i;
+      for (int i = 0; i < 2; ++i) {
+        const int b = min(2 * st + i, sub_blocks - 1);
         const int grp = g64 == 1 ? b : static_cast<int>(__umulhi(static_cast<uint32_t>(b), by_group));
-        if (b >= sub_blocks) z[i] = 0u;
-        else if (i > 0 && grp == before) z[i] = z[i > 0 ? i - 1 : 0];
-        else z[i] = live ? __ldg(p.sz + (size_t)grp * p.N + n) : 0u;
-        before = grp;
+        z[i] = __ldg(p.sz + (size_t)grp * p.N + n);
       }
     };
-    uint32_t sz_next[4];
-    bool more = seek();
-    if (more) load_sz((g.s0 >> 1) + o - g_stage, sz_next);
-    bool ok = true;
-    while (ok && more) {
-      const int stage = (g.s0 >> 1) + o - g_stage;
-      const int first = max(2 * stage, g.s0), last = min(2 * stage + 2, g.s1);
-      int unit = g_unit + first - g.s0;
-      const int lap = static_cast<int>(__umulhi(static_cast<uint32_t>(o), by_ring)), s = o - lap * n_w;
-      const uint32_t sz_now[4] = {sz_next[0], sz_next[1], sz_next[2], sz_next[3]};
-      o += sets;
-      more = seek();
-      if (more) load_sz((g.s0 >> 1) + o - g_stage, sz_next);     // arrives while this stage is expanded
-#pragma unroll 1
-      for (int st = first; st < last; ++st, ++unit) {
-        const int use = static_cast<int>(__umulhi(static_cast<uint32_t>(unit), by_slots)), q = unit - use * n_slots;
-        // The parity of the slot's barrier is not ambiguous: of three sets this one's stage before held no unit older than
-        // five before this one, which waited for the unit n_slots before it, and two turns of five slots or more ago is no
-        // later than that; of two sets it is three, and four slots will do.  Nor is that of the stage's barrier: when the
-        // unit n_slots before this one is done, every stage n_w >= n_slots before this one has been filled and read.
-        if (!__all_sync(0xffffffffu, mbar_wait(done0 + 8 * q, (use & 1) ^ 1, abort_flag))) { ok = false; break; }
-        if (st == first && !__all_sync(0xffffffffu, mbar_wait(wfull0 + 8 * s, lap & 1, abort_flag))) { ok = false; break; }
-        tcgen05_fence_after();
-        const uint32_t src = wring + s * kStageBytes + row * 128;
-        const int h = st & 1;
-        uint4 w[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) w[j] = w4_lds_v4(src + (((h * 4 + j) ^ sw) << 4));
-        const uint32_t sz_h[2] = {h ? sz_now[2] : sz_now[0], h ? sz_now[3] : sz_now[1]};
-        const uint32_t a_tmem = a_tmem0 + q * kSlotCols;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (j == 2 && 2 * st + 1 >= sub_blocks) break;                // K ends in the middle of the step
-          const __half2 szh = *reinterpret_cast<const __half2*>(&sz_h[j >> 1]);
-          const ScaleZero sp = make_scale_zero(__low2half(szh), __high2half(szh));
-          uint32_t r[16];
-          expand_word(w[j].x, sp, r);
-          expand_word(w[j].y, sp, r + 4);
-          expand_word(w[j].z, sp, r + 8);
-          expand_word(w[j].w, sp, r + 12);
-          tmem_st_32x32_x16(a_tmem + j * 16, r);
-        }
-        __syncwarp();
-        if (st == last - 1 && lane == 0) mbar_arrive(wempty0 + 8 * s);
-        tmem_st_wait();
-        tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_tmem(ready_leader0 + 8 * q);
+    int u = u0 + set, st = 0;
+    uint32_t sz_next[2];
+    if (u < u1) {
+      st = seek(u);
+      load_sz(st, sz_next);
+    }
+    while (u < u1) {
+      const int use = static_cast<int>(__umulhi(static_cast<uint32_t>(u - u0), by_slots)), q = u - u0 - use * n_slots;
+      const int stage = stage0 + (st >> 1) - (g.s0 >> 1);
+      const int lap = static_cast<int>(__umulhi(static_cast<uint32_t>(stage), by_ring)), s = stage - lap * n_w;
+      const int reads = (st ^ 1) < g.s0 || (st ^ 1) >= g.s1 ? 2 : 1;    // the stage's other step may not be this pair's
+      const int h = st & 1;
+      const bool both = 2 * st + 1 < sub_blocks;                         // K may end in the middle of the step
+      const uint32_t sz_now[2] = {sz_next[0], sz_next[1]};
+      u += kSets;
+      if (u < u1) {                            // the next step's scales arrive while this one is expanded
+        st = seek(u);
+        load_sz(st, sz_next);
       }
+      // The slot first: the unit three before this one waited for the unit n_slots before it, which is no earlier than the
+      // slot's use before its last one, so the barrier's parity is not ambiguous; and when the unit n_slots before this one
+      // is done, every stage n_w >= n_slots before this one has been filled and read, so the stage's is not either.
+      if (!__all_sync(0xffffffffu, mbar_wait(done0 + 8 * q, (use & 1) ^ 1, abort_flag) &&
+                                       mbar_wait(wfull0 + 8 * s, lap & 1, abort_flag))) break;
+      tcgen05_fence_after();
+      const uint32_t src = wring + s * kStageBytes + row * 128;
+      uint4 w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = w4_lds_v4(src + (((h * 4 + j) ^ sw) << 4));
+      const uint32_t a_tmem = a_tmem0 + q * kSlotCols;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (j == 2 && !both) break;
+        const __half2 szh = *reinterpret_cast<const __half2*>(&sz_now[j >> 1]);
+        const ScaleZero sp = make_scale_zero(__low2half(szh), __high2half(szh));
+        uint32_t r[16];
+        expand_word(w[j].x, sp, r);
+        expand_word(w[j].y, sp, r + 4);
+        expand_word(w[j].z, sp, r + 8);
+        expand_word(w[j].w, sp, r + 12);
+        tmem_st_32x32_x16(a_tmem + j * 16, r);
+      }
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(wempty0 + 8 * s);
+        if (reads == 2) mbar_arrive(wempty0 + 8 * s);
+      }
+      tmem_st_wait();
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_tmem(ready_leader0 + 8 * q);
     }
   } else {
     // ---- epilogue: lane = weight row, column = token; two warps to a quarter of the rows take 32 tokens in turn
     const int quarter = warp & 3, half = (warp - kEpiWarp0) >> 2;
     const int row = quarter * 32 + lane;
     const uint32_t tempty_leader0 = map_to_cta(tempty0, 0);
-    const uint32_t stage = staging + (warp - kEpiWarp0) * 2048;
+    const uint32_t stage = staging + (warp - kEpiWarp0) * 4096;
     const bool vec = p.N % 8 == 0;
     int d = 0;
     uint32_t dphase = 0;
@@ -370,7 +381,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + d * T;
       const int last = min(T, p.M - m0);                     // tokens that exist
       const int chunks = (last - 32 * half + 63) >> 6;       // of 32 tokens; this warp's are c, c + 2, ...: four at most
-      uint32_t r[32], h0[16];                        // h: two tokens each
+      uint32_t r[32], h[16];
       auto load = [&](int i) { tmem_ld_32x32(taddr + 32 * half + 64 * i, r); };
       auto pack = [&](uint32_t (&h)[16]) {
 #pragma unroll
@@ -380,32 +391,27 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           h[j] = h2_as_u32(__floats2half2_rn(v0, v1));
         }
       };
-      auto store = [&](const uint32_t (&h)[16], int i) {
-        const int c0 = 32 * half + 64 * i, left = last - c0;
-        __half* y = p.y + (size_t)(m0 + c0) * p.N;
-        if (vec && n0 + 32 <= p.N) {
-          // 16 token pairs x 32 rows of words; the 16-byte pieces of odd pairs trade places, against bank conflicts
-          __syncwarp();
+      // a chunk through shared memory: 16 token pairs x 32 rows of words; the 16-byte pieces of odd pairs trade places,
+      // against bank conflicts
+      auto stage_chunk = [&](const uint32_t (&h)[16], int buf) {
+        __syncwarp();
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
-            asm volatile("st.shared.u32 [%0], %1;" ::"r"(stage + j * 128 + (((lane >> 2) ^ (j & 1)) << 4) + (lane & 3) * 4), "r"(h[j]) : "memory");
-          __syncwarp();
+        for (int j = 0; j < 16; ++j)
+          asm volatile("st.shared.u32 [%0], %1;" ::"r"(stage + buf * 2048 + j * 128 + (((lane >> 2) ^ (j & 1)) << 4) + (lane & 3) * 4), "r"(h[j]) : "memory");
+        __syncwarp();
+      };
+      auto flush = [&](int buf, int i) {
+        const int c0 = 32 * half + 64 * i;
 #pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const int j = k * 8 + (lane >> 2), piece = (lane & 3) * 2;      // pair of tokens, eight rows
-            const uint4 a = w4_lds_v4(stage + j * 128 + ((piece ^ (j & 1)) << 4));
-            const uint4 b = w4_lds_v4(stage + j * 128 + (((piece + 1) ^ (j & 1)) << 4));
-            __half* dst = y + (size_t)(2 * j) * p.N + n0 + (lane & 3) * 8;
-            if (2 * j < left)
-              *reinterpret_cast<uint4*>(dst) = make_uint4(prmt(a.x, a.y, 0x5410), prmt(a.z, a.w, 0x5410), prmt(b.x, b.y, 0x5410), prmt(b.z, b.w, 0x5410));
-            if (2 * j + 1 < left)
-              *reinterpret_cast<uint4*>(dst + p.N) = make_uint4(prmt(a.x, a.y, 0x7632), prmt(a.z, a.w, 0x7632), prmt(b.x, b.y, 0x7632), prmt(b.z, b.w, 0x7632));
-          }
-        } else if (n < p.N) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (j < left)
-              y[(size_t)j * p.N + n] = __ushort_as_half(static_cast<unsigned short>((j & 1) ? h[j >> 1] >> 16 : h[j >> 1]));
+        for (int k = 0; k < 2; ++k) {
+          const int j = k * 8 + (lane >> 2), piece = (lane & 3) * 2, t = c0 + 2 * j;      // pair of tokens, eight rows
+          const uint32_t src = stage + buf * 2048 + j * 128;
+          const uint4 a = w4_lds_v4(src + ((piece ^ (j & 1)) << 4)), b = w4_lds_v4(src + (((piece + 1) ^ (j & 1)) << 4));
+          __half* dst = p.y + (size_t)(m0 + t) * p.N + n0 + (lane & 3) * 8;
+          if (t < last)
+            *reinterpret_cast<uint4*>(dst) = make_uint4(prmt(a.x, a.y, 0x5410), prmt(a.z, a.w, 0x5410), prmt(b.x, b.y, 0x5410), prmt(b.z, b.w, 0x5410));
+          if (t + 1 < last)
+            *reinterpret_cast<uint4*>(dst + p.N) = make_uint4(prmt(a.x, a.y, 0x7632), prmt(a.z, a.w, 0x7632), prmt(b.x, b.y, 0x7632), prmt(b.z, b.w, 0x7632));
         }
       };
       auto release = [&]() {
@@ -423,18 +429,57 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           for (int j = 0; j < 32; ++j) dst[(32 * half + 64 * i + j) * kRows] = __uint_as_float(r[j]);
         }
         release();
-      } else {
-        // the accumulator is given back as soon as its last 32 columns are in registers
-        if (chunks <= 0) release();
+      } else if (vec && n0 + 32 <= p.N) {
+        // The accumulator is given back as soon as its last columns are in registers: nothing is stored to memory before
+        // (with the chunks stored one after another the MMAs waited 5800 clocks a tile for 256 tokens).
         if (chunks > 0) load(0);
+        tmem_ld_wait();
+        if (chunks <= 1) release();
+        if (chunks > 0) pack(h);
+        if (chunks > 1) load(1);
+        if (chunks > 0) stage_chunk(h, 0);
+        if (chunks > 1) {
+          tmem_ld_wait();
+          if (chunks == 2) release();
+          pack(h);
+          if (chunks > 2) load(2);
+          stage_chunk(h, 1);
+        }
+        if (chunks > 2) {
+          tmem_ld_wait();
+          if (chunks == 3) release();
+          pack(h);
+        }
+        if (chunks > 3) {
+          load(3);
+          tmem_ld_wait();
+          release();
+        }
+        if (chunks > 0) flush(0, 0);
+        if (chunks > 2) stage_chunk(h, 0);
+        if (chunks > 1) flush(1, 1);
+        if (chunks > 3) {
+          pack(h);
+          stage_chunk(h, 1);
+        }
+        if (chunks > 2) flush(0, 2);
+        if (chunks > 3) flush(1, 3);
+      } else {
 #pragma unroll 1
         for (int i = 0; i < chunks; ++i) {
+          load(i);
           tmem_ld_wait();
-          if (i == chunks - 1) release();
-          pack(h0);
-          if (i < chunks - 1) load(i + 1);
-          store(h0, i);
+          pack(h);
+          const int c0 = 32 * half + 64 * i;
+          __half* y = p.y + (size_t)(m0 + c0) * p.N + n;
+          if (n < p.N) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (c0 + j < last)
+                y[(size_t)j * p.N] = __ushort_as_half(static_cast<unsigned short>((j & 1) ? h[j >> 1] >> 16 : h[j >> 1]));
+          }
         }
+        release();
       }
       if (++d == n_acc) { d = 0; dphase ^= 1; }
     }
