@@ -266,10 +266,10 @@ __device__ __forceinline__ void umma_i8_pair(uint32_t tmem_d, uint64_t desc_a, u
       : "memory");
 }
 // Arrive, once the pair's MMAs issued so far have completed, on the mbarrier at this shared-memory offset in both CTAs of
-// the pair.
-__device__ __forceinline__ void umma_commit_both(uint32_t bar) {
+// the pair (cta_mask: their ranks in the cluster).
+__device__ __forceinline__ void umma_commit_both(uint32_t bar, unsigned short cta_mask = 3) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"(static_cast<unsigned short>(3)) : "memory");
+               ::"r"(bar), "h"(cta_mask) : "memory");
 }
 
 // Arrive on an mbarrier of this CTA once all MMAs issued so far by this

@@ -79,8 +79,9 @@ struct W4GemmParams {
   int T;                    // tokens of a tile, a multiple of 32
   int m_tiles, steps;       // tiles along the tokens; 128-column steps of a tile
   int unit_steps;           // 1, or `steps` when pairs take whole tiles
+  int split;                // > 1: a cluster of this many pairs shares a tile, a pair takes steps / split of it
   int share, extra;         // units of a pair: share, one more for the first `extra` pairs
-  float* partial;           // [pair][2][rank][T][128]: the first segment of a pair that begins inside a tile, and the last
+  float* partial;           // [pair][2][rank][T / 4][128][4 tokens]: the first segment of a pair that begins inside a tile, and the last
                             // one that ends inside a tile whose beginning it holds
   int* error_word;
 };
@@ -134,6 +135,24 @@ __device__ __forceinline__ void expand_word(uint32_t word, const ScaleZero& sp, 
   out[3] = prmt(c, d, 0x7632);
 }
 
+// Rows n and n + 1 of up to four tokens from `m` on.
+__device__ __forceinline__ void store_quad(const W4GemmParams& p, int m, int tokens, int n, const float (&a)[4],
+                                           const float (&b)[4]) {
+  const float bias0 = p.bias ? h2f(p.bias[n]) : -0.0f, bias1 = p.bias && n + 1 < p.N ? h2f(p.bias[n + 1]) : -0.0f;
+  __half* y = p.y + (size_t)m * p.N + n;
+#pragma unroll
+  for (int j = 0; j < 4; ++j, y += p.N) {
+    if (j >= tokens) break;
+    const __half2 h = __floats2half2_rn(a[j] + bias0, b[j] + bias1);
+    if (p.N % 2 == 0) {
+      *reinterpret_cast<__half2*>(y) = h;
+    } else {
+      y[0] = __low2half(h);
+      if (n + 1 < p.N) y[1] = __high2half(h);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(w4::kThreads, 1)
 w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                   const W4GemmParams p) {
@@ -155,41 +174,19 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();
+  const uint32_t cta = cluster_ctarank(), rank = cta & 1u, leader_cta = cta & ~1u;
   const bool leader = rank == 0;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < n_w; ++s) {
-      mbar_init(wfull0 + 8 * s, 1);
-      mbar_init(wempty0 + 8 * s, 8);                       // four warps for each of the stage's two steps
-    }
-    for (int q = 0; q < n_slots; ++q) {
-      mbar_init(ready0 + 8 * q, 9);                        // four warps of each CTA, the leader's TMA producer
-      mbar_init(done0 + 8 * q, 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(tfull0 + 8 * b, 1);
-      mbar_init(tempty0 + 8 * b, 2 * kEpiWarps);
-    }
-    *abort_flag = 0;
-    fence_mbar_init();
+  const int pair = static_cast<int>(blockIdx.x) >> 1, steps = p.steps, split = p.split;
+  // this pair's steps
+  int u0, u1;
+  if (split > 1) {
+    const int tile = pair / split, i = pair - tile * split;
+    u0 = tile * steps + steps * i / split;
+    u1 = tile * steps + steps * (i + 1) / split;
+  } else {
+    u0 = w4_range_start(pair, p.share, p.extra) * p.unit_steps;
+    u1 = w4_range_start(pair + 1, p.share, p.extra) * p.unit_steps;
   }
-  if (warp == kMmaWarp) {
-    tmem_alloc_pair(smem_u32(tmem_slot), kTmemCols);
-    tmem_relinquish_pair();
-  }
-  tcgen05_fence_before();
-  __syncthreads();
-  cluster_arrive();              // the peer's barriers exist before anything signals them
-  cluster_wait();
-  tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-
-  chain_wait();
-  chain_release();
-
-  const int pair = static_cast<int>(blockIdx.x) >> 1, steps = p.steps;
-  const int u0 = w4_range_start(pair, p.share, p.extra) * p.unit_steps,
-            u1 = w4_range_start(pair + 1, p.share, p.extra) * p.unit_steps;          // this pair's steps
   // the segment that begins at unit u
   auto segment_at = [&](int u, W4Segment& g) {
     g.tile = u / steps;
@@ -198,28 +195,82 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   };
   auto first_row = [&](int tile) { return (tile / p.m_tiles) * (2 * kRows) + static_cast<int>(rank) * kRows; };
 
+  // weight producer: where its walk stands, and a stage's load
+  W4Segment wg{0, 0, 0};
+  int w_end = u0, w_st = 0, w_row = 0;
+  auto next_stage = [&]() {                    // false: none left
+    if (w_st > (wg.s1 - 1) >> 1 || w_end == u0) {
+      if (w_end >= u1) return false;
+      segment_at(w_end, wg);
+      w_end += wg.s1 - wg.s0;
+      w_st = wg.s0 >> 1;
+      w_row = first_row(wg.tile);
+    }
+    return true;
+  };
+  auto load_stage = [&](int s) {
+    mbar_arrive_expect_tx(wfull0 + 8 * s, kStageBytes);
+    tma_load_2d(wring + s * kStageBytes, &tmap_w, wfull0 + 8 * s, w_st++ * (kStageK / 2), w_row);
+  };
+  bool w_more = false;
+
+  // the barriers of the first weights, which come while the rest is set up, are this CTA's own
   if (warp == kWeightWarp) {
     if (elect_one()) {
-      prefetch_tensormap(&tmap_w);
-      int s = 0;
-      uint32_t phase = 1;
-      bool ok = true;
-      W4Segment g;
-      for (int u = u0; ok && u < u1; u += g.s1 - g.s0) {
-        segment_at(u, g);
-        const int row = first_row(g.tile);
-        for (int st = g.s0 >> 1; st <= (g.s1 - 1) >> 1; ++st) {
-          if (!mbar_wait(wempty0 + 8 * s, phase, abort_flag)) { ok = false; break; }
-          mbar_arrive_expect_tx(wfull0 + 8 * s, kStageBytes);
-          tma_load_2d(wring + s * kStageBytes, &tmap_w, wfull0 + 8 * s, st * (kStageK / 2), row);
-          if (++s == n_w) { s = 0; phase ^= 1; }
-        }
+      for (int s = 0; s < n_w; ++s) {
+        mbar_init(wfull0 + 8 * s, 1);
+        mbar_init(wempty0 + 8 * s, 8);                     // four warps for each of the stage's two steps
       }
+      fence_mbar_init();
     }
   } else if (warp == kXWarp) {
     if (elect_one()) {
       prefetch_tensormap(&tmap_x);
-      const uint32_t ready_leader0 = map_to_cta(ready0, 0);
+      for (int q = 0; q < n_slots; ++q) {
+        mbar_init(ready0 + 8 * q, 9);                      // four warps of each CTA, the leader's TMA producer
+        mbar_init(done0 + 8 * q, 1);
+      }
+      for (int b = 0; b < 2; ++b) {
+        mbar_init(tfull0 + 8 * b, 1);
+        mbar_init(tempty0 + 8 * b, 2 * kEpiWarps);
+      }
+      *abort_flag = 0;
+      fence_mbar_init();
+    }
+  } else if (warp == kMmaWarp) {
+    tmem_alloc_pair(smem_u32(tmem_slot), kTmemCols);
+    tmem_relinquish_pair();
+  }
+  __syncwarp();
+  tcgen05_fence_before();
+  cluster_arrive();              // the peer's barriers exist before anything signals them
+  chain_wait();
+  chain_release();
+  if (warp == kWeightWarp && elect_one()) {      // (tensor memory and the cluster's barrier take about 1.1 us)
+    for (int s = 0; s < n_w; ++s) {
+      w_more = next_stage();
+      if (!w_more) break;
+      load_stage(s);
+    }
+  }
+  __syncwarp();
+  cluster_wait();                // (and this CTA's: every thread of the cluster takes part)
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == kWeightWarp) {
+    if (w_more) {                              // the thread that issued the first loads
+      int s = 0;
+      uint32_t phase = 0;
+      while (next_stage()) {
+        if (!mbar_wait(wempty0 + 8 * s, phase, abort_flag)) break;
+        load_stage(s);
+        if (++s == n_w) { s = 0; phase ^= 1; }
+      }
+    }
+  } else if (warp == kXWarp) {
+    if (elect_one()) {
+      const uint32_t ready_leader0 = map_to_cta(ready0, leader_cta);
       int s = 0;
       uint32_t phase = 1;
       bool ok = true;
@@ -241,6 +292,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   } else if (warp == kMmaWarp) {
     if (leader && elect_one()) {
       const uint32_t idesc = umma_idesc(kIdescDFormatF32 | kIdescABFormatF16, 2 * kRows, T);
+      const unsigned short pair_mask = static_cast<unsigned short>(3u << leader_cta);
       // This thread's instructions wait their turn among those of the expansion: at 160 tokens and fewer they set the pace, so
       // a step has as few as possible.
       const uint64_t b_desc0 = umma_desc_k_sw128(xring);
@@ -267,13 +319,13 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             for (int kk = 0; kk < 4; ++kk)
               umma_f16_ts_pair(d_tmem, a_tmem + 32 + kk * 8, desc + half_step + 2 * kk, desc_hi, idesc);
           }
-          umma_commit_both(done0 + 8 * q);
+          umma_commit_both(done0 + 8 * q, pair_mask);
           desc += slot_step;
           a_tmem += kSlotCols;
           if (++q == n_slots) { q = 0; phase ^= 1; desc = desc_lo0; a_tmem = a0; }
         }
         if (!ok) break;
-        umma_commit_both(tfull0 + 8 * d);
+        umma_commit_both(tfull0 + 8 * d, pair_mask);
         if (++d == n_acc) { d = 0; dphase ^= 1; }
       }
     }
@@ -282,7 +334,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     const int quarter = warp & 3, set = warp >> 2;
     const int row = quarter * 32 + lane, sw = row & 7;
     const uint32_t a_tmem0 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + n_acc * T;
-    const uint32_t ready_leader0 = map_to_cta(ready0, 0);
+    const uint32_t ready_leader0 = map_to_cta(ready0, leader_cta);
     const int sub_blocks = p.K / 64, g64 = p.group / 64;
     // x / d for the small quotients here is the high word of x * ceil(2^32 / d), d > 1
     const uint32_t by_slots = 0xffffffffu / n_slots + 1, by_ring = 0xffffffffu / n_w + 1, by_group = 0xffffffffu / g64 + 1;
@@ -365,7 +417,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     // ---- epilogue: lane = weight row, column = token; two warps to a quarter of the rows take 32 tokens in turn
     const int quarter = warp & 3, half = (warp - kEpiWarp0) >> 2;
     const int row = quarter * 32 + lane;
-    const uint32_t tempty_leader0 = map_to_cta(tempty0, 0);
+    const uint32_t tempty_leader0 = map_to_cta(tempty0, leader_cta);
     const uint32_t stage = staging + (warp - kEpiWarp0) * 4096;
     const bool vec = p.N % 8 == 0;
     int d = 0;
@@ -377,6 +429,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       const bool whole = g.s0 == 0 && g.s1 == steps;
       const float bias = p.bias && n < p.N ? h2f(p.bias[n]) : 0.0f;
       if (!__all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * d, dphase, abort_flag))) break;
+      if (split > 1) break;                    // its one segment; exchanged below
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + d * T;
       const int last = min(T, p.M - m0);                     // tokens that exist
@@ -420,13 +473,14 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         if (lane == 0) mbar_arrive_tmem(tempty_leader0 + 8 * d);
       };
       if (!whole) {
-        float* dst = p.partial + (((size_t)pair * 2 + (g.s0 == 0)) * 2 + rank) * ((size_t)T * kRows) + row;
+        float* dst = p.partial + (((size_t)pair * 2 + (g.s0 == 0)) * 2 + rank) * ((size_t)T * kRows) + row * 4;
 #pragma unroll 1
         for (int i = 0; i < chunks; ++i) {
           load(i);
           tmem_ld_wait();
+          uint4* to = reinterpret_cast<uint4*>(dst + (32 * half + 64 * i) * kRows);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) dst[(32 * half + 64 * i + j) * kRows] = __uint_as_float(r[j]);
+          for (int j = 0; j < 8; ++j) to[j * kRows] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
         }
         release();
       } else if (vec && n0 + 32 <= p.N) {
@@ -485,12 +539,58 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
   }
 
-  __syncthreads();
   // a CTA that gave up tells its peer (whose waits poll the flag) before both meet at the cluster barrier; the peer
   // cannot have left yet, so its shared memory is still there
-  if (*abort_flag && threadIdx.x == 0) st_cluster_u32(map_to_cta(smem_u32(const_cast<int*>(abort_flag)), rank ^ 1u), 1u);
+  __syncwarp();
+  if (*abort_flag && lane == 0) st_cluster_u32(map_to_cta(smem_u32(const_cast<int*>(abort_flag)), cta ^ 1u), 1u);
+  __syncwarp();
   cluster_arrive();       // the leader's MMAs read the peer's shared memory: nobody leaves early
   cluster_wait();
+  if (split > 1) {
+    // Every CTA of the cluster has finished its products and its rings are free.  CTA (i, rank) gets, from the CTAs of its
+    // rank, their sums of the i-th part of the tile's tokens, adds them in K order and stores that part.  Through global
+    // memory the partial tiles took 2.1 us to write and about 4 to read again (12 MB each way at 160 tokens).
+    const int tile = pair / split, i = pair - tile * split;
+    const int m0 = (tile % p.m_tiles) * T, last = min(T, p.M - m0);
+    const int quads = T / (4 * split);                       // of tokens, a CTA's part
+    if (warp >= kEpiWarp0 && warp < kEpiWarp0 + kEpiWarps) {
+      const int quarter = warp & 3, half = (warp - kEpiWarp0) >> 2;
+      const uint32_t own = xring + static_cast<uint32_t>(i * quads * kRows + quarter * 32 + lane) * 16;
+      tcgen05_fence_after();
+      for (int c0 = 32 * half; c0 < last; c0 += 64) {
+        uint32_t r[32];
+        tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + c0, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int quad = c0 / 4 + j, to = quad / quads;
+          const uint32_t dst = map_to_cta(own + static_cast<uint32_t>(quad - to * quads) * kRows * 16, 2 * to + rank);
+          asm volatile("st.shared::cluster.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(r[4 * j]), "r"(r[4 * j + 1]),
+                       "r"(r[4 * j + 2]), "r"(r[4 * j + 3]) : "memory");
+        }
+      }
+      tcgen05_fence_before();
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    const int n0 = first_row(tile);
+    for (int e = threadIdx.x; e < quads * (kRows / 2); e += kThreads) {
+      const int quad = e / (kRows / 2), row = (e % (kRows / 2)) * 2, t = (i * quads + quad) * 4, n = n0 + row;
+      if (t >= last || n >= p.N) continue;
+      float v[2][4] = {};
+      for (int from = 0; from < split; ++from) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const uint4 w = w4_lds_v4(xring + static_cast<uint32_t>((from * quads + quad) * kRows + row + k) * 16);
+          v[k][0] += __uint_as_float(w.x); v[k][1] += __uint_as_float(w.y);
+          v[k][2] += __uint_as_float(w.z); v[k][3] += __uint_as_float(w.w);
+        }
+      }
+      store_quad(p, m0 + t, min(4, last - t), n, v[0], v[1]);
+    }
+    __syncthreads();
+  }
   if (*abort_flag) {
     if (threadIdx.x == 0 && p.error_word) atomicExch(p.error_word, 2);
     const uint64_t t0 = globaltimer_ns();
@@ -518,65 +618,101 @@ w4a16_gemm_reduce_kernel(const W4GemmParams p) {
   const int m0 = (tile % p.m_tiles) * p.T, n0 = (tile / p.m_tiles) * (2 * w4::kRows);
   const int tokens = min(p.T, p.M - m0);
   const size_t tile_words = (size_t)p.T * w4::kRows;
-  const int i = blockIdx.y * 256 + threadIdx.x;              // four rows of a token to a thread
-  if (i < tokens * (2 * w4::kRows / 4)) {
-    const int t = i / (2 * w4::kRows / 4), r = (i % (2 * w4::kRows / 4)) * 4;
-    const int rank = r / w4::kRows;
-    const float* src = p.partial + rank * tile_words + (size_t)t * w4::kRows + (r - rank * w4::kRows);
-    float4 acc = *reinterpret_cast<const float4*>(src + ((size_t)first * 2 + 1) * 2 * tile_words);
-    for (int q = first + 1; q <= last; q += 4) {             // four requests at a time
-      float4 v[4];
+  // two rows of four tokens to a thread
+  const int i = blockIdx.y * 256 + threadIdx.x, t = (i / w4::kRows) * 4, r = (i % w4::kRows) * 2;
+  if (t >= tokens) return;
+  const int rank = r / w4::kRows;
+  const float4* src = reinterpret_cast<const float4*>(p.partial + rank * tile_words + (size_t)t * w4::kRows) + (r - rank * w4::kRows);
+  const size_t pair_step = tile_words;                         // four tiles of four words
+  float4 a = src[first * pair_step + tile_words / 2], b = src[first * pair_step + tile_words / 2 + 1];
+  for (int q = first + 1; q <= last; q += 4) {                 // four requests at a time
+    float4 va[4], vb[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (q + j <= last) v[j] = *reinterpret_cast<const float4*>(src + (size_t)(q + j) * 4 * tile_words);
+    for (int j = 0; j < 4; ++j)
+      if (q + j <= last) {
+        va[j] = src[(q + j) * pair_step];
+        vb[j] = src[(q + j) * pair_step + 1];
+      }
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (q + j <= last) { acc.x += v[j].x; acc.y += v[j].y; acc.z += v[j].z; acc.w += v[j].w; }
-    }
-    const float v[4] = {acc.x, acc.y, acc.z, acc.w};
-    const int n = n0 + r;
-    __half h[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) h[j] = f2h(p.bias && n + j < p.N ? v[j] + h2f(p.bias[n + j]) : v[j]);
-    __half* y = p.y + (size_t)(m0 + t) * p.N + n;
-    if (n + 4 <= p.N && p.N % 4 == 0) {
-      *reinterpret_cast<uint2*>(y) = make_uint2(h2_as_u32(__halves2half2(h[0], h[1])), h2_as_u32(__halves2half2(h[2], h[3])));
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (n + j < p.N) y[j] = h[j];
-    }
+    for (int j = 0; j < 4; ++j)
+      if (q + j <= last) {
+        a.x += va[j].x; a.y += va[j].y; a.z += va[j].z; a.w += va[j].w;
+        b.x += vb[j].x; b.y += vb[j].y; b.z += vb[j].z; b.w += vb[j].w;
+      }
   }
+  const int n = n0 + r;
+  if (n >= p.N) return;
+  const float va[4] = {a.x, a.y, a.z, a.w}, vb[4] = {b.x, b.y, b.z, b.w};
+  store_quad(p, m0 + t, min(4, tokens - t), n, va, vb);
 }
 
-// Tokens of a tile, and whether pairs get equal runs of units (scratch needed) or whole tiles: the shortest estimate in
-// SM clocks.  A step is 4 T clocks of MMA but no less than the 600 of its expansion, and 60 for its barriers; the last tile's epilogue 10 T; splitting adds 16 T for writing and reading partial
-// tiles and 5500 for the second launch.
+static void w4_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* cluster, int pairs, int split) {
+  cfg.gridDim = dim3(2 * pairs, 1, 1);
+  cfg.blockDim = dim3(w4::kThreads, 1, 1);
+  cfg.dynamicSmemBytes = w4::kSmem;
+  cluster->id = cudaLaunchAttributeClusterDimension;
+  cluster->val.clusterDim.x = 2 * split;
+  cluster->val.clusterDim.y = 1;
+  cluster->val.clusterDim.z = 1;
+  cfg.attrs = cluster;
+  cfg.numAttrs = 1;
+}
+
+// How a product is cut, by the shortest estimate in SM clocks: the tokens of a tile, and then
+//   * whole tiles to a pair, in as many waves as it takes;
+//   * a tile to a cluster of two or four pairs, which exchange their sums through their shared memories;
+//   * with scratch, an equal run of all tiles' steps to every pair, the cut tiles added by a second kernel.
+// A step is 4 T clocks of MMA but no less than the 600 of its expansion, and 110 for its barriers; the last tile's
+// epilogue 16 T.  The exchange in a cluster takes about 2500 and 6 T, the second kernel 6000 and, for partial tiles written
+// to and read from L2, 40 T.
 struct W4Shape {
   int T;
-  bool split;
+  int split;                // pairs to a tile
+  bool runs;                // equal runs
   int pairs;
 };
-static W4Shape w4_gemm_shape(int M, int N, int K, bool may_split) {
+struct W4Device {
+  int id = -1;
+  int clusters[3];          // clusters of 1, 2, 4 pairs that fit the device at once
+};
+static int w4_device(const W4Device** out) {
+  static thread_local W4Device d;
+  *out = &d;
+  int device = 0;
+  MP_CUDA_TRY(cudaGetDevice(&device));
+  if (d.id == device) return MP_OK;
+  MP_CUDA_TRY(cudaFuncSetAttribute(w4a16_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w4::kSmem));
+  for (int i = 0; i < 3; ++i) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr;
+    w4_launch_config(cfg, &attr, w4::kPairs / 4 * 4, 1 << i);
+    MP_CUDA_TRY(cudaOccupancyMaxActiveClusters(&d.clusters[i], w4a16_gemm_kernel, &cfg));
+  }
+  d.id = device;
+  return MP_OK;
+}
+
+static W4Shape w4_gemm_shape(int M, int N, int K, bool scratch, const int (&clusters)[3]) {
   const long long n_tiles = (N + 2 * w4::kRows - 1) / (2 * w4::kRows), steps = (K + w4::kStepK - 1) / w4::kStepK;
   W4Shape best{};
   long long best_cost = -1;
+  auto offer = [&](long long cost, const W4Shape& shape) {
+    if (best_cost >= 0 && cost >= best_cost) return;
+    best_cost = cost;
+    best = shape;
+  };
   for (int T = w4::kMaxT; T >= 32; T -= 32) {
     const long long tiles = n_tiles * ((M + T - 1) / T), units = tiles * steps;
-    const long long step = std::max(4 * T, 600) + 60;
-    const long long waves = (tiles + w4::kPairs - 1) / w4::kPairs;
-    const long long whole = waves * steps * step + 10 * T;
-    if (best_cost < 0 || whole < best_cost) {
-      best_cost = whole;
-      best = W4Shape{T, false, (int)std::min<long long>(tiles, w4::kPairs)};
+    const long long step = std::max(4 * T, 600) + 110, waves = (tiles + w4::kPairs - 1) / w4::kPairs;
+    offer(waves * steps * step + 16 * T, W4Shape{T, 1, false, (int)std::min<long long>(tiles, w4::kPairs)});
+    for (int i = 1; i <= 2; ++i) {
+      const int split = 1 << i;
+      if (tiles > clusters[i] || steps < 2 * split) continue;
+      offer((steps + split - 1) / split * step + 2500 + (6 + 16 / split) * T, W4Shape{T, split, false, (int)tiles * split});
     }
     const long long pairs = std::min<long long>(w4::kPairs, units / 4);
-    if (!may_split || pairs < 2 || units % pairs == 0 && units / pairs % steps == 0) continue;
-    const long long split = (units + pairs - 1) / pairs * step + 26 * T + 5500;
-    if (split < best_cost) {
-      best_cost = split;
-      best = W4Shape{T, true, (int)pairs};
-    }
+    if (!scratch || pairs < 2 || (units % pairs == 0 && units / pairs % steps == 0)) continue;
+    offer((units + pairs - 1) / pairs * step + 6000 + 56 * T, W4Shape{T, 1, true, (int)pairs});
   }
   return best;
 }
@@ -590,8 +726,10 @@ using namespace mp;
 // Room for the partial tiles wherever they may be wanted: when the split is chosen, and for fewer tiles than pairs.
 extern "C" size_t mp_w4a16_prefill_workspace_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0 || K % 64 != 0) return 0;
-  const W4Shape s = w4_gemm_shape(M, N, K, true);
-  return s.split || s.pairs < w4::kPairs ? w4_partial_bytes(s.pairs, s.T) : 0;
+  const W4Device* d;
+  const int none[3] = {0, 0, 0};
+  const W4Shape s = w4_gemm_shape(M, N, K, true, w4_device(&d) == MP_OK ? d->clusters : none);
+  return s.runs || s.pairs < w4::kPairs ? w4_partial_bytes(s.pairs, s.T) : 0;
 }
 
 extern "C" int mp_w4a16_linear_prefill(const void* x_f16, const void* packed_i32, const void* sz_f16x2,
@@ -608,13 +746,16 @@ extern "C" int mp_w4a16_linear_prefill_ex(const void* x_f16, const void* packed_
   if (!x_f16 || !packed_i32 || !sz_f16x2 || !y_f16 || M <= 0 || N <= 0 || K <= 0 || group <= 0) return MP_ERR_INVALID_ARG;
   if (K % 64 != 0 || group % 64 != 0 || K % group != 0) return MP_ERR_UNSUPPORTED;
   if (!aligned(x_f16, 16) || !aligned(packed_i32, 16) || !aligned(sz_f16x2, 4) || !aligned(y_f16, 16)) return MP_ERR_ALIGNMENT;
-  const W4Shape shape = w4_gemm_shape(M, N, K, workspace != nullptr);
+  const W4Device* d;
+  int rc = w4_device(&d);
+  if (rc != MP_OK) return rc;
+  const W4Shape shape = w4_gemm_shape(M, N, K, workspace != nullptr, d->clusters);
   if (workspace) {
     if (workspace_bytes < mp_w4a16_prefill_workspace_bytes(M, N, K)) return MP_ERR_WORKSPACE;
     if (!aligned(workspace, 16)) return MP_ERR_ALIGNMENT;
   }
   CUtensorMap tx, tw;
-  int rc = encode_tensor_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x_f16, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, 64,
+  rc = encode_tensor_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x_f16, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, 64,
                                 shape.T / 2);
   if (rc != MP_OK) return rc;
   rc = encode_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, packed_i32, (uint64_t)K / 2, (uint64_t)N, (uint64_t)K / 2,
@@ -631,38 +772,21 @@ extern "C" int mp_w4a16_linear_prefill_ex(const void* x_f16, const void* packed_
   p.error_word = error_word;
   const long long tiles = (long long)p.m_tiles * ((N + 2 * w4::kRows - 1) / (2 * w4::kRows)), units = tiles * p.steps;
   if (units > 2000000000LL) return MP_ERR_UNSUPPORTED;
-  if (shape.split) {
-    p.partial = static_cast<float*>(workspace);
-    p.share = (int)(units / shape.pairs);
-    p.extra = (int)(units % shape.pairs);
-  } else {
-    p.share = (int)(tiles / shape.pairs);
-    p.extra = (int)(tiles % shape.pairs);
-  }
-  p.unit_steps = shape.split ? 1 : p.steps;
+  p.split = shape.split;
+  const long long parts = shape.runs ? units : tiles;       // shared out evenly (split > 1: by the cluster's place)
+  p.share = (int)(parts / shape.pairs);
+  p.extra = (int)(parts % shape.pairs);
+  p.unit_steps = shape.runs ? 1 : p.steps;
+  p.partial = static_cast<float*>(workspace);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  static thread_local int configured_device = -1;
-  int device = 0;
-  MP_CUDA_TRY(cudaGetDevice(&device));
-  if (configured_device != device) {
-    MP_CUDA_TRY(cudaFuncSetAttribute(w4a16_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w4::kSmem));
-    configured_device = device;
-  }
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(2 * shape.pairs, 1, 1);
-  cfg.blockDim = dim3(w4::kThreads, 1, 1);
-  cfg.dynamicSmemBytes = w4::kSmem;
-  cfg.stream = st;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  w4_launch_config(cfg, attr, shape.pairs, shape.split);
+  cfg.stream = st;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
   cfg.numAttrs = 2;
   MP_CUDA_TRY(cudaLaunchKernelEx(&cfg, w4a16_gemm_kernel, tx, tw, p));
-  if (!shape.split) return MP_OK;
-  return launch_chained(w4a16_gemm_reduce_kernel, dim3(shape.pairs - 1, shape.T / 4), dim3(256), 0, st, p);
+  if (!shape.runs) return MP_OK;
+  return launch_chained(w4a16_gemm_reduce_kernel, dim3(shape.pairs - 1, (shape.T / 4 * w4::kRows + 255) / 256), dim3(256), 0, st, p);
 }
