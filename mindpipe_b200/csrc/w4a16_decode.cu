@@ -826,7 +826,9 @@ static LinearKernel linear_kernel(int M, int N, int K, int group) {
   if (!decode_umma_shape_ok(M, N, K, group) || g_decode_kernel == MP_DECODE_KERNEL_MMA_SYNC) return narrow;
   if (g_decode_kernel == MP_DECODE_KERNEL_UMMA) return M <= 64 ? kStream : kGemm;
   const size_t packed = (size_t)N * (size_t)K / 2;
-  if (M > 16) return kStream;
+  // Above 96 rows the pair kernel expands less often for its tokens (4096x11008 at 97 / 128 rows: 23.7 / 26.0 vs 21.7 / 22.3
+  // us; the other 7B shapes are level at 97 and a few per cent better at 128); it takes no groups of 32.
+  if (M > 16) return M > 96 && group % 64 == 0 ? kGemm : kStream;
   // 9..16 rows double the ring kernel's MMAs and cost the stream kernel nothing; below 2 MiB or 16 row blocks the stream
   // kernel's longer pipeline shows (2048x2048: 4.3 vs 4.5 us, 2048x8192: 6.4 vs 8.9, 12288x4096: 10.4 vs 15.7)
   if (M > 8) return packed >= ((size_t)2 << 20) && N >= 2048 ? kStream : kRing;

@@ -663,8 +663,9 @@ static void w4_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* clust
 //   * a tile to a cluster of two or four pairs, which exchange their sums through their shared memories;
 //   * with scratch, an equal run of all tiles' steps to every pair, the cut tiles added by a second kernel.
 // A step is 4 T clocks of MMA but no less than the 600 of its expansion, and 110 for its barriers; the last tile's
-// epilogue 16 T.  The exchange in a cluster takes about 2500 and 6 T, the second kernel 6000 and, for partial tiles written
-// to and read from L2, 40 T.
+// epilogue 16 T.  The exchange in a cluster takes about 4000 and 16 T, the second kernel 4000 and, with the partial tiles'
+// way to L2 and back, 100 T.  With these the choice was the fastest of all cuts, or within 4 % of it, over 65..1024 rows of
+// seven shapes from 2688 x 2944 to 22016 x 4096.
 struct W4Shape {
   int T;
   int split;                // pairs to a tile
@@ -708,11 +709,11 @@ static W4Shape w4_gemm_shape(int M, int N, int K, bool scratch, const int (&clus
     for (int i = 1; i <= 2; ++i) {
       const int split = 1 << i;
       if (tiles > clusters[i] || steps < 2 * split) continue;
-      offer((steps + split - 1) / split * step + 2500 + (6 + 16 / split) * T, W4Shape{T, split, false, (int)tiles * split});
+      offer((steps + split - 1) / split * step + 4000 + (16 + 16 / split) * T, W4Shape{T, split, false, (int)tiles * split});
     }
     const long long pairs = std::min<long long>(w4::kPairs, units / 4);
     if (!scratch || pairs < 2 || (units % pairs == 0 && units / pairs % steps == 0)) continue;
-    offer((units + pairs - 1) / pairs * step + 6000 + 56 * T, W4Shape{T, 1, true, (int)pairs});
+    offer((units + pairs - 1) / pairs * step + 4000 + 116 * T, W4Shape{T, 1, true, (int)pairs});
   }
   return best;
 }
