@@ -50,6 +50,9 @@ struct GemmParams {
   int M, N, K;
   int m_tiles, n_tiles, k_blocks;
   int bn;                      // columns of a tile, a multiple of 32
+  int a_box;                   // activation rows a load brings: 128, or as many as there are (a copy that reaches beyond a
+                               // small tensor is slow: 14 us instead of 8 for 24 rows of 4096).  The shared memory behind
+                               // them holds anything: a row of the accumulator depends on its own row alone
   int k_split;                 // > 1: a tile's K range is cut into this many work items of kb_per_split k-blocks,
   int kb_per_split;            //      whose raw int32 partial tiles go to `partial` ([k_split][M][N])
   int* partial;
@@ -248,7 +251,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           if (PAIR) {
             // both CTAs' bytes are counted on the leader's barrier
             const uint32_t full = map_to_cta(full0 + 8 * stage, 0);
-            if (leader) mbar_arrive_expect_tx(full0 + 8 * stage, 2 * (kABytes + b_bytes));
+            if (leader) mbar_arrive_expect_tx(full0 + 8 * stage, 2 * (p.a_box * kBK + b_bytes));
             tma_load_2d_pair(smem_u32(sA + stage * kABytes), &tmap_a, full, kb * kBK, m0);
             // this CTA's half of the tile's weight rows; with SwiGLU the halves are the gate rows
             // (accumulator columns [0,128)) and the matching up rows (columns [128,256))
@@ -258,7 +261,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             tma_load_2d_pair(smem_u32(sB + stage * b_bytes), &tmap_b, full, kb * kBK, b_row);
           } else {
             const uint32_t full = full0 + 8 * stage;
-            mbar_arrive_expect_tx(full, kABytes + b_bytes);
+            mbar_arrive_expect_tx(full, p.a_box * kBK + b_bytes);
             tma_load_2d(smem_u32(sA + stage * kABytes), &tmap_a, full, kb * kBK, m0);
             if (EPI == EPI_SWIGLU) {
               // gate rows then the matching up rows: the tile's columns [0,128) and [128,256)
@@ -659,9 +662,10 @@ struct GemmCall {
 template <int EPI, bool PAIR>
 static int launch_gemm(const GemmCall& c, const GemmShape& shape, cudaStream_t st) {
   const int bn = shape.bn;
+  const int a_box = std::min(c.a_rows, kBM);
   CUtensorMap ta, tb;
   int rc = encode_tensor_map_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, c.a, (uint64_t)c.K, (uint64_t)c.a_rows,
-                                (uint64_t)c.K, kBK, kBM);
+                                (uint64_t)c.K, kBK, (uint32_t)a_box);
   if (rc != MP_OK) return rc;
   rc = encode_tensor_map_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, c.b, (uint64_t)c.K, (uint64_t)c.b_rows_total,
                             (uint64_t)c.K, kBK, PAIR ? bn / 2 : (EPI == EPI_SWIGLU ? 128 : bn));
@@ -670,6 +674,7 @@ static int launch_gemm(const GemmCall& c, const GemmShape& shape, cudaStream_t s
   p.M = c.M; p.N = c.N; p.K = c.K;
   p.m_tiles = (c.a_rows + kBM - 1) / kBM;
   p.bn = bn;
+  p.a_box = a_box;
   p.n_tiles = (c.N + (EPI == EPI_SWIGLU ? 128 : bn) - 1) / (EPI == EPI_SWIGLU ? 128 : bn);
   p.k_blocks = (c.K + kBK - 1) / kBK;
   p.m_tiles_dev = c.m_tiles_dev; p.tile_expert = c.tile_expert;
@@ -730,7 +735,8 @@ static int max_k_split(int M, int N, int K) {
 // The cut with the shortest estimated time, in SM clocks.  A k-block (128 bytes of K) costs a CTA
 //   * 2 * bn in the tensor core (four instructions of bn / 2), and
 //   * the bytes of its two operand tiles in and out of shared memory at 128 B/clk, which is also their way from L2 at
-//     64 B/clk: 2 * (128 + bn) alone, 2 * (128 + bn / 2) in a pair -- always the larger number.
+//     64 B/clk: 2 * (128 + bn) alone (fewer with less than 128 rows), 2 * (128 + bn / 2) in a pair -- the larger number,
+//   * no less than 350: the waits and issues of its two producing threads.
 // Work items go over the CTAs (pairs) in whole waves, so narrower tiles win where they fill the last one: 333 rows x 12288
 // columns are 96 items of 256 x 256 on 74 pairs (two waves of 512 a k-block), 128 of 256 x 192 (two of 448) or 144 of
 // 128 x 256 (one of 768).  A tile's last epilogue, pipeline fill and launch are in kTileClocks and 8 clocks a column; a K
@@ -739,7 +745,7 @@ static int max_k_split(int M, int N, int K) {
 // 129..256 rows of 4096 columns (10.2 us, 9.2 with 128 x 64).  Before, with 128 or 256 columns only (us): 12288 x 4096 at
 // 129 / 333 / 1024 rows 19.8 / 27.8 / 39.7 -> 17.1 / 21.1 / 38.0, 22016 x 4096 30.0 / 38.4 / 68.1 -> 23.7 / 36.5 / 66.8.
 static GemmShape gemm_shape(int M, int N, int K, int max_split) {
-  constexpr long long kTileClocks = 1500, kReduceClocks = 8000, kReduceBytesPerClock = 2000;
+  constexpr long long kTileClocks = 1500, kReduceClocks = 14000, kReduceBytesPerClock = 2000;
   const int k_blocks = (K + kBK - 1) / kBK;
   const int bn_max = N >= kMaxBN ? kMaxBN : (N + 31) / 32 * 32;
   GemmShape best{false, bn_max, 1};
@@ -749,7 +755,7 @@ static GemmShape gemm_shape(int M, int N, int K, int max_split) {
     const long long m_tiles = pair ? (M + 255) / 256 : (M + 127) / 128;
     for (int bn = bn_max; bn >= 32; bn -= 32) {
       const long long tiles = m_tiles * ((N + bn - 1) / bn);
-      const int per_block = 256 + (pair ? bn : 2 * bn);
+      const int per_block = std::max(350, 2 * (pair ? 128 + bn / 2 : std::min(128, M) + bn));
       for (int want = 1; want <= (tiles < slots ? max_split : 1); ++want) {
         const int per = (k_blocks + want - 1) / want, ks = (k_blocks + per - 1) / per;     // no empty slice
         if (ks != want) continue;

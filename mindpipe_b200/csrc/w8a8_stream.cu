@@ -1,4 +1,4 @@
-// W8A8 products with few activation rows (up to 128, or that many per expert): the weights are streamed once as the MMA's
+// W8A8 products with few activation rows (up to 8, or 64 to an expert): the weights are streamed once as the MMA's
 // 128-row operand, the activation rows are its N.
 //
 //   D[128 weight rows][tokens] (int32, TMEM) += W[128 rows x 128 bytes] (shared memory) x X[tokens x 128 bytes]^T
@@ -18,7 +18,7 @@
 //               scales, bias or SwiGLU, stores of 256 contiguous bytes
 //   warp 8      TMA producer: one copy of weights and one of activations per stage
 //   warp 9      TMEM allocation and the MMA issuer
-// Up to 64 rows a block takes less than half an SM, so the next product of a chain starts beside the end of this one; its
+// A block takes less than half an SM, so the next product of a chain starts beside the end of this one; its
 // first weights are then already on the way (see early_weights).
 #include "common.cuh"
 #include "tc.cuh"
@@ -45,7 +45,7 @@ template <int TOK, int EPI>
 struct Cfg {
   static constexpr int kParts = EPI == STREAM_SWIGLU ? 2 : 1;       // gate rows and up rows
   static constexpr int kStageBytes = kWBytes + TOK * kStepK;
-  static constexpr int kSmemMax = TOK <= 64 ? 112 * 1024 : 220 * 1024;
+  static constexpr int kSmemMax = 112 * 1024;
   static constexpr int kFixed = 1024 + 2 * kChunk * kPitch * 4 + (2 * kMaxRing + 4) * 8 + 64;
   static constexpr int kFit = (kSmemMax - kFixed) / kStageBytes;
   static constexpr int kRing = kFit < kMaxRing ? kFit : kMaxRing;
@@ -93,7 +93,7 @@ struct StreamAt {
 };
 
 template <int TOK, int EPI>
-__global__ void __launch_bounds__(ws::kThreads, TOK <= 64 ? 2 : 1)
+__global__ void __launch_bounds__(ws::kThreads, 2)
 w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                    const StreamParams p) {
   using C = ws::Cfg<TOK, EPI>;
@@ -177,7 +177,7 @@ w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       at.set(n_steps > 0 ? t_hi : 0, row_blocks, steps);
       auto load_w = [&](int s, const StreamAt& a, int part) {
         const int e = grouped ? s_group[a.group] & 0xFF : 0;
-        mbar_arrive_expect_tx(full0 + 8 * s, C::kStageBytes);
+        mbar_arrive_expect_tx(full0 + 8 * s, ws::kWBytes + p.x_box * ws::kStepK);
         tma_load_2d(ring + s * C::kStageBytes, &tmap_w, full0 + 8 * s, a.kb * ws::kStepK,
                     e * p.rows_per_expert + part * p.up_row_offset + a.rb * ws::kRows);
       };
@@ -424,7 +424,7 @@ static int launch_stream(const CUtensorMap& tw, const CUtensorMap& tx, const Str
   return launch_chained(kern, dim3(grid), dim3(ws::kThreads), C::kSmem, st, tw, tx, p);
 }
 
-static int stream_tokens(int rows) { return rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : 128; }
+static int stream_tokens(int rows) { return rows <= 16 ? 16 : rows <= 32 ? 32 : 64; }
 
 size_t w8a8_stream_workspace_bytes(int epi, int max_rows) {
   const int parts = epi == STREAM_SWIGLU ? 2 : 1;
@@ -433,9 +433,7 @@ size_t w8a8_stream_workspace_bytes(int epi, int max_rows) {
 
 int launch_w8a8_stream(int epi, const void* x_i8, int x_rows, const void* w_i8, int w_rows, StreamParams p, int max_rows,
                        void* workspace, size_t workspace_bytes, cudaStream_t st) {
-  const int parts = epi == STREAM_SWIGLU ? 2 : 1;
-  if (max_rows > (parts == 2 ? kStreamMaxRowsSwiglu : kStreamMaxRows) || p.K % 16 != 0 || p.K >= (1 << 17) ||
-      p.experts > ws::kMaxExperts)
+  if (max_rows > kStreamMaxExpertRows || p.K % 16 != 0 || p.K >= (1 << 17) || p.experts > ws::kMaxExperts)
     return MP_ERR_UNSUPPORTED;
   if (!workspace || workspace_bytes < w8a8_stream_workspace_bytes(epi, max_rows) || !aligned(workspace, 16))
     return MP_ERR_UNSUPPORTED;
@@ -445,8 +443,9 @@ int launch_w8a8_stream(int epi, const void* x_i8, int x_rows, const void* w_i8, 
   int rc = encode_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, w_i8, (uint64_t)p.K, (uint64_t)w_rows, (uint64_t)p.K,
                                 ws::kStepK, ws::kRows);
   if (rc != MP_OK) return rc;
+  p.x_box = x_rows < tok ? x_rows : tok;
   rc = encode_tensor_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_UINT8, x_i8, (uint64_t)p.K, (uint64_t)x_rows, (uint64_t)p.K,
-                            ws::kStepK, tok);
+                            ws::kStepK, p.x_box);
   if (rc != MP_OK) return rc;
   p.steps = (p.K + ws::kStepK - 1) / ws::kStepK;
   p.row_blocks = (p.N + ws::kRows - 1) / ws::kRows;
@@ -455,8 +454,8 @@ int launch_w8a8_stream(int epi, const void* x_i8, int x_rows, const void* w_i8, 
   const long long most = (long long)groups * p.row_blocks * p.steps;
   if (most > (1 << 24)) return MP_ERR_UNSUPPORTED;
   // as in w4a16_decode_umma.cu: at b steps per block a row block costs b steps and steps / b tiles; a tile costs about 0.4
-  // (16 tokens) to 1 (128) steps
-  const int tile_cost_x10 = (tok == 16 ? 4 : tok == 32 ? 5 : tok == 64 ? 7 : 10);
+  // (16 tokens) to 0.7 (64) steps
+  const int tile_cost_x10 = tok == 16 ? 4 : tok == 32 ? 5 : 7;
   p.min_share = 2;
   while (p.min_share * p.min_share * 10 < p.steps * tile_cost_x10) ++p.min_share;
   p.tiles = reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(workspace) + kW4CounterBytes);
@@ -466,13 +465,12 @@ int launch_w8a8_stream(int epi, const void* x_i8, int x_rows, const void* w_i8, 
   switch (epi) {                                                                     \
     case STREAM_F16: return launch_stream<TOK, STREAM_F16>(tw, tx, p, grid, st);     \
     case STREAM_AFFINE: return launch_stream<TOK, STREAM_AFFINE>(tw, tx, p, grid, st); \
-    default: return launch_stream<(TOK < 128 ? TOK : 64), STREAM_SWIGLU>(tw, tx, p, grid, st); \
+    default: return launch_stream<TOK, STREAM_SWIGLU>(tw, tx, p, grid, st); \
   }
   switch (tok) {
     case 16: MP_STREAM(16)
     case 32: MP_STREAM(32)
-    case 64: MP_STREAM(64)
-    default: MP_STREAM(128)
+    default: MP_STREAM(64)
   }
 #undef MP_STREAM
 }

@@ -30,9 +30,13 @@ struct StreamParams {
   const int* b_rowsum;
   uint32_t* tiles;             // workspace: [grid][parts][tokens][128], zero between calls
   int* error_word;
+  int x_box;                   // activation rows a load brings: no more than there are (a copy that reaches beyond a small
+                               // tensor is slow: 14 us instead of 8 for 24 rows of 4096 in a box of 128)
 };
 
-constexpr int kStreamMaxRows = 128, kStreamMaxRowsSwiglu = 64;
+// Rows of a linear, rows per expert.  From 9 rows on the tiled kernel is as fast or faster (16 rows, us: 4096x4096 10.6 vs
+// 10.0, 28672x4096 26.5 vs 25.4; at 64: 19.5 vs 10.2, 37.3 vs 26.5); at 8 this one is (9.3 vs 9.9, 4096x14336 15.7 vs 17).
+constexpr int kStreamMaxRows = 8, kStreamMaxExpertRows = 64;
 
 // Most rows a call (grouped: an expert of it) has; MP_ERR_UNSUPPORTED where the kernel does not apply.
 int launch_w8a8_stream(int epi, const void* x_i8, int x_rows, const void* w_i8, int w_rows, StreamParams p, int max_rows,
