@@ -175,6 +175,16 @@ typedef struct mp_host_linear {
 } mp_host_linear;
 int mp_w4a16_linear_decode_host_many(const mp_host_linear* linears, int count, mp_stream_t stream);
 /*
+ * The same set recorded once for a stream and run many times: rows and results cross PCIe beside the products, on two
+ * more streams (joined to `stream` again at the end of each run).  All of x_host_f16 / y_host_f16 must be page-locked,
+ * at most 16 entries (MP_ERR_UNSUPPORTED otherwise: use the call above).  The entries' buffers and the host memory outlive
+ * the pipeline.  Destroying it while a run is still
+ * on the device is allowed.
+ */
+int mp_host_pipeline_create(const mp_host_linear* linears, int count, mp_stream_t stream, void** pipeline);
+int mp_host_pipeline_run(void* pipeline);
+void mp_host_pipeline_destroy(void* pipeline);
+/*
  * The address under which the current device can read and write a page-locked
  * host range (cudaHostAlloc / cudaHostRegister memory, e.g. torch's pinned
  * tensors).  MP_ERR_UNSUPPORTED for pageable memory, a range that is not mapped
@@ -184,7 +194,7 @@ int mp_w4a16_linear_decode_host_many(const mp_host_linear* linears, int count, m
 int mp_host_buffer_device_alias(const void* host_ptr, size_t bytes, void** device_ptr);
 
 /*
- * The linear for any number of rows: the decode kernels, the tcgen05 weight-streaming kernel (up to 128 rows) or the
+ * The linear for any number of rows: the decode kernels, the tcgen05 weight-streaming kernel (up to 96 rows) or the
  * prefill GEMM below, whichever is fastest for the shape (with mp_set_decode_kernel set: as that says).  The forward of
  * VllmPackedInt4Linear (exporters/vllm.py:85-86) in one call.  The workspace is one for all shapes, under the rules of
  * mp_w4a16_linear_decode: zero-filled when it is created, left ready for the next call, shared only by calls that cannot

@@ -39,6 +39,9 @@ SIGNATURES = {
     "mp_host_buffer_device_alias": (_I, [_P, _Z, _P]),
     "mp_w4a16_linear_decode_host_ws": (_I, [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P, _Z, _P]),
     "mp_w4a16_linear_decode_host_many": (_I, [_P, _I, _P]),
+    "mp_host_pipeline_create": (_I, [_P, _I, _P, _P]),
+    "mp_host_pipeline_run": (_I, [_P]),
+    "mp_host_pipeline_destroy": (None, [_P]),
     "mp_w4a16_linear_workspace_bytes": (_Z, [_I, _I, _I, _I]),
     "mp_w4a16_linear": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _P, _Z, _P, _P]),
     "mp_w4a16_linear_prefill": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P]),

@@ -853,25 +853,35 @@ extern "C" size_t mp_w4a16_linear_workspace_bytes(int M, int N, int K, int group
   }
 }
 
-extern "C" int mp_w4a16_linear(const void* x_f16, const void* packed_i32, const void* sz_f16x2, const void* bias_f16,
-                               void* y_f16, int M, int N, int K, int group, void* workspace, size_t workspace_bytes,
-                               int* error_word, mp_stream_t stream) {
+namespace mp {
+int w4a16_linear(const void* x_f16, const void* packed_i32, const void* sz_f16x2, const void* bias_f16, void* y_f16, int M,
+                 int N, int K, int group, void* workspace, size_t workspace_bytes, int* error_word, int early,
+                 mp_stream_t stream) {
   if (!x_f16 || !packed_i32 || !sz_f16x2 || !y_f16 || M <= 0 || N <= 0 || K <= 0 || group <= 0) return MP_ERR_INVALID_ARG;
   if (K % group != 0) return MP_ERR_UNSUPPORTED;
   const LinearKernel kernel = linear_kernel(M, N, K, group);
   if (kernel == kStream && N % 8 == 0 && K % kChunk == 0) {
     if (!aligned(x_f16, 16) || !aligned(packed_i32, 16) || !aligned(sz_f16x2, 4) || !aligned(y_f16, 2)) return MP_ERR_ALIGNMENT;
     const int rc = launch_decode_umma(x_f16, packed_i32, sz_f16x2, bias_f16, y_f16, M, N, K, group, workspace,
-                                      workspace_bytes, static_cast<cudaStream_t>(stream), decode_programmatic_launch());
+                                      workspace_bytes, static_cast<cudaStream_t>(stream),
+                                      early < 0 ? decode_programmatic_launch() : early > 0);
     if (rc != MP_ERR_UNSUPPORTED) return rc;                     // (no workspace, odd alignment: the others)
   }
   if (M <= 16)
     return decode_linear(x_f16, packed_i32, sz_f16x2, bias_f16, y_f16, M, N, K, group, workspace, workspace_bytes, 0,
-                         MP_DECODE_KERNEL_MMA_SYNC, -1, stream);
+                         MP_DECODE_KERNEL_MMA_SYNC, early, stream);
   const bool scratch = workspace && workspace_bytes > kPartialOffset;
   return mp_w4a16_linear_prefill_ex(x_f16, packed_i32, sz_f16x2, bias_f16, y_f16, M, N, K, group,
                                     scratch ? static_cast<unsigned char*>(workspace) + kPartialOffset : nullptr,
                                     scratch ? workspace_bytes - kPartialOffset : 0, error_word, stream);
+}
+}  // namespace mp
+
+extern "C" int mp_w4a16_linear(const void* x_f16, const void* packed_i32, const void* sz_f16x2, const void* bias_f16,
+                               void* y_f16, int M, int N, int K, int group, void* workspace, size_t workspace_bytes,
+                               int* error_word, mp_stream_t stream) {
+  return w4a16_linear(x_f16, packed_i32, sz_f16x2, bias_f16, y_f16, M, N, K, group, workspace, workspace_bytes, error_word, -1,
+                      stream);
 }
 
 extern "C" int mp_w4a16_decode_kernel_choice(int M, int N, int K, int have_workspace) {

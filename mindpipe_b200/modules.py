@@ -234,10 +234,28 @@ class VllmPackedInt4Linear(nn.Module):
 _HOST_MANY_PLANS: dict = {}
 
 
+class _HostPipeline:
+    """Owner of an ``mp_host_pipeline``."""
+
+    def __init__(self, calls, count, stream):
+        import ctypes
+        lib = _lib.load()
+        handle = ctypes.c_void_p()
+        self.status = lib.mp_host_pipeline_create(calls, count, stream, ctypes.byref(handle))
+        self.handle, self._run, self._destroy = handle, lib.mp_host_pipeline_run, lib.mp_host_pipeline_destroy
+
+    def run(self):
+        return self._run(self.handle)
+
+    def __del__(self):
+        if self.handle:
+            self._destroy(self.handle)
+
+
 def forward_host_many(linears, x_hosts, y_hosts, stream=None):
     """``forward_host`` of several independent ``VllmPackedInt4Linear`` modules on ONE stream in one library
-    call: all H2D copies first, then the kernels back to back (so that under ``mp_set_programmatic_launch(1)`` each
-    fetches its weights while the one before drains), then the D2H copies.  For linears that do not depend on one
+    call: the first module's rows, then the kernels back to back, each fetching its weights while the one before
+    drains; the other modules' rows and the results cross PCIe meanwhile.  For linears that do not depend on one
     another -- the q/k/v or gate/up projections of a decoder layer.  ``x_hosts`` / ``y_hosts`` are pinned CPU fp16
     tensors, one pair per module (<= 16 rows); returns ``y_hosts``, valid once the stream is synchronised.  The
     first call with a given set of modules, buffers and stream goes through each module's own ``forward_host``
@@ -248,10 +266,10 @@ def forward_host_many(linears, x_hosts, y_hosts, stream=None):
     if plan is not None:
         for m in linears:
             m._ensure_prepared()
-        calls, derived, _keep = plan
+        run, derived, _keep = plan
         if all(m._scale_zero is z and m.weight_packed.data_ptr() == p and (None if m.bias is None else m.bias.data_ptr()) == b
                for m, (z, p, b) in zip(linears, derived)):
-            status = _lib.load().mp_w4a16_linear_decode_host_many(calls, len(derived), st)
+            status = run()
             if status != 0:
                 _lib.check(status, "w4a16_linear_decode_host_many", count=len(derived))
             return y_hosts
@@ -277,7 +295,14 @@ def forward_host_many(linears, x_hosts, y_hosts, stream=None):
         c.workspace_bytes = 0 if ws is None else ws.numel()
     if len(_HOST_MANY_PLANS) >= 256:
         _HOST_MANY_PLANS.clear()
-    _HOST_MANY_PLANS[key] = (calls, [(m._scale_zero, m.weight_packed.data_ptr(), None if m.bias is None else m.bias.data_ptr())
+    pipeline = _HostPipeline(calls, len(linears), st)
+    if pipeline.status == 0:
+        run = pipeline.run
+    else:                                # more than 16 modules, or buffers the device cannot address as the host does
+
+        def run():
+            return _lib.load().mp_w4a16_linear_decode_host_many(calls, len(linears), st)
+    _HOST_MANY_PLANS[key] = (run, [(m._scale_zero, m.weight_packed.data_ptr(), None if m.bias is None else m.bias.data_ptr())
                                      for m in linears], (list(linears), list(x_hosts), list(y_hosts)))
     return y_hosts
 
