@@ -160,6 +160,13 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t smem_dst, const CUtens
       : "memory");
 }
 
+// Bring a tile to L2.  L2 is where all SMs and copies meet, so this is safe before chain_wait() too: whatever the kernel
+// before still writes there is seen by the load that follows the wait.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int crd0, int crd1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(crd0), "r"(crd1) : "memory");
+}
+
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }

@@ -216,7 +216,11 @@ w4a16_decode_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       };
       const int prologue = min(n_stages, dt::kStages);
       asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-      if (!p.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (!p.early_weights) {
+        // the first stages on their way to L2 while the kernel before ends
+        for (int i = 0; i < prologue; ++i) tma_prefetch_2d(&tmap_w, (s_begin + i) * (dt::kStageK / 2), row_block0);
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+      }
       for (int i = 0; i < prologue; ++i) issue_weights(i);
       if (p.early_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
       for (int i = 0; i < prologue; ++i) issue_x(i);

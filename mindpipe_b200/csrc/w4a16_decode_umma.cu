@@ -259,7 +259,13 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
       fence_mbar_init();
       w_row = (t_hi / ST) * du::kRows;
       w_st = t_hi % ST;
-      if (!p.early_weights) chain_wait();
+      if (!p.early_weights) {
+        for (int s = 0, row = w_row, st = w_st; s < p.ring && s < n_stages; ++s) {     // to L2 while the kernel before ends
+          tma_prefetch_2d(&tmap_w, st * (du::kStageK / 2), row);
+          if (--st < 0) { st = ST - 1; row -= du::kRows; }
+        }
+        chain_wait();
+      }
       for (int s = 0; s < p.ring && s < n_stages; ++s) load_weights(s);
     }
   } else if (warp == du::kXWarp) {

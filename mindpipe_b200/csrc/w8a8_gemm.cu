@@ -188,6 +188,16 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  // the first weight tiles on their way to L2 while the kernel before ends (grouped: it decides which)
+  if (warp == 0 && !p.tile_expert && elect_one()) {
+    const int work = PAIR ? blockIdx.x >> 1 : blockIdx.x, tile = work / p.k_split;
+    const int kb0 = (work - tile * p.k_split) * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + min(p.kb_per_split, STAGES));
+    int m_tile, n_tile;
+    tile_coords(tile, PAIR ? (p.m_tiles + 1) / 2 : p.m_tiles, p.n_tiles, p.group_m, m_tile, n_tile);
+    const int row = n_tile * bn + (PAIR ? static_cast<int>(rank) * (bn / 2) : 0);
+    for (int kb = kb0; kb < kb1; ++kb) tma_prefetch_2d(&tmap_b, kb * kBK, row);
+  }
+  __syncwarp();
   // everything above touched only this block's shared and tensor memory: under programmatic dependent launch it
   // ran beside the previous kernel's tail; from here on that kernel's results are read
   chain_wait();
