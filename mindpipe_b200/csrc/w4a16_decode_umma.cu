@@ -66,8 +66,9 @@ constexpr size_t kSmemMax = 224 * 1024;
 // the MMA then reads whatever follows for the other eight, whose results are not used)
 template <int TOK, int XROWS, bool FOLD>
 struct Cfg {
-  // who puts the activations into the order of expanded words: the expansion warps, in shared memory, or (PERM false) a
-  // small kernel before this one
+  // the columns of an expanded word come out as (k0,k4) (k1,k5) ..: the activations are put into that order, in shared
+  // memory, or (PERM false) the words back into theirs.  Permuting the activations of 64 tokens per block and stage cost the
+  // expansion warps a third of their time, permuting them in a kernel of its own 2 us a call.
   static constexpr bool PERM = TOK <= 32;
   static constexpr int kXSub = XROWS * 128;           // [XROWS x 64 columns] fp16
   static constexpr int kXBytes = (PERM ? 4 : 2) * kXSub;        // a tile of the ring: a stage, or half of one
@@ -95,13 +96,10 @@ inline int min_share(int stages_per_row, int tok) {
   return b;
 }
 __host__ __device__ constexpr int tokens_for(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 96 ? 96 : 128; }
-// workspace: the other kernels' arrival counters | one tile per block | activations in expansion order (M > 32)
+// workspace: the other kernels' arrival counters | one tile per block
 constexpr size_t kTileOffset = kW4CounterBytes;
-constexpr size_t kXOffset = kTileOffset + kW4TileBytes;
 static_assert(kW4TileBytes >= (size_t)kMaxGrid * 128 * kRows * sizeof(uint32_t), "tiles");
-inline size_t workspace_bytes(int M, int K) {
-  return M <= 32 ? kTileOffset + (size_t)kMaxGrid * (M <= 16 ? 16 : 32) * kRows * sizeof(uint32_t) : kXOffset + (size_t)M * K * 2;
-}
+inline size_t workspace_bytes(int M) { return kTileOffset + (size_t)kMaxGrid * tokens_for(M) * kRows * sizeof(uint32_t); }
 }  // namespace du
 
 struct DecodeUmmaParams {
@@ -193,6 +191,13 @@ __device__ __forceinline__ uint4 pair_permute_u4(const uint4 in) {
   v.z = prmt(in.y, in.w, 0x5410);
   v.w = prmt(in.y, in.w, 0x7632);
   return v;
+}
+
+// (k0,k4) (k1,k5) (k2,k6) (k3,k7) -> (k0,k1) .. (k6,k7)
+__device__ __forceinline__ void in_order(uint32_t* v) {
+  const uint32_t a = prmt(v[0], v[1], 0x5410), b = prmt(v[2], v[3], 0x5410);
+  const uint32_t c = prmt(v[0], v[1], 0x7632), d = prmt(v[2], v[3], 0x7632);
+  v[0] = a; v[1] = b; v[2] = c; v[3] = d;
 }
 
 // One packed word -> the exact fp16 integers u - z of its eight columns, in dequant8's order.  zl = 1024 + z and
@@ -421,6 +426,7 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
             dequant8(word, sp, v);
 #pragma unroll
             for (int e = 0; e < 4; ++e) r[4 * c + e] = h2_as_u32(v[e]);
+            if constexpr (!PERM) in_order(&r[4 * c]);
           }
           tmem_st_32x32_x16(a_tmem + j * 16, r);
         }
@@ -606,16 +612,7 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
 
 int* decode_error_word_ptr(int* out_rc);   // w4a16_decode_tma.cu: device address of the decode error word
 
-size_t decode_umma_workspace_bytes(int M, int K) { return du::workspace_bytes(M, K); }
-
-// The activations in expansion order, for the wider tiles: permuting them per block and stage in shared memory, as at up
-// to 16 rows, cost the expansion warps a third of their time at 64.
-__global__ void __launch_bounds__(256)
-w4a16_permute_kernel(const uint4* __restrict__ x, int chunks, uint4* __restrict__ out) {
-  chain_wait();
-  chain_release();
-  for (int i = blockIdx.x * 256 + threadIdx.x; i < chunks; i += gridDim.x * 256) out[i] = pair_permute_u4(x[i]);
-}
+size_t decode_umma_workspace_bytes(int M, int K) { return du::workspace_bytes(M); }
 
 bool decode_umma_shape_ok(int M, int N, int K, int group) {
   if (M > 128 || K % 64 != 0 || N % 4 != 0) return false;
@@ -650,22 +647,13 @@ int launch_decode_umma(const void* x, const void* packed, const void* sz, const 
                        int group, void* workspace, size_t workspace_bytes, cudaStream_t st, bool early_weights) {
   if (!decode_umma_shape_ok(M, N, K, group)) return MP_ERR_UNSUPPORTED;
   const int tok = du::tokens_for(M);
-  if (!workspace || workspace_bytes < du::workspace_bytes(M, K) || !aligned(workspace, 16)) return MP_ERR_UNSUPPORTED;
+  if (!workspace || workspace_bytes < du::workspace_bytes(M) || !aligned(workspace, 16)) return MP_ERR_UNSUPPORTED;
   if (!aligned(x, 16) || !aligned(packed, 16) || !aligned(sz, 16) || !aligned(y, 4)) return MP_ERR_UNSUPPORTED;
   const int row_blocks = (N + du::kRows - 1) / du::kRows;
   CUtensorMap tw, tx, tsz;
   int rc = encode_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, packed, (uint64_t)K / 2, (uint64_t)N,
                                 (uint64_t)K / 2, 128, du::kRows, true);
   if (rc != MP_OK) return rc;
-  if (tok > 32) {
-    uint4* xp = reinterpret_cast<uint4*>(static_cast<unsigned char*>(workspace) + du::kXOffset);
-    const int chunks = M * (K / 8), blocks = (chunks + 255) / 256;
-    rc = launch_chained(w4a16_permute_kernel, dim3(blocks < 2 * kSmCount ? blocks : 2 * kSmCount), dim3(256), 0, st,
-                        static_cast<const uint4*>(x), chunks, xp);
-    if (rc != MP_OK) return rc;
-    x = xp;
-    early_weights = true;        // of the kernel before only that one is still running, and it writes no weights
-  }
   // [64 columns][token][chunk of 64 columns]: one copy brings the sub-tiles of a stage or half of one
   const uint64_t x_dims[3] = {64, (uint64_t)M, (uint64_t)K / 64}, x_strides[2] = {(uint64_t)K * 2, 128};
   const uint32_t x_box[3] = {64, (uint32_t)(M <= 8 ? 8 : tok), tok <= 32 ? 4u : 2u};
