@@ -69,12 +69,12 @@ struct Cfg {
   // the columns of an expanded word come out as (k0,k4) (k1,k5) ..: the activations are put into that order, in shared
   // memory, or (PERM false) the words back into theirs.  Permuting the activations of 64 tokens per block and stage cost the
   // expansion warps a third of their time, permuting them in a kernel of its own 2 us a call.
-  static constexpr bool PERM = TOK <= 32;
+  static constexpr bool PERM = TOK <= 16;
   static constexpr int kXSub = XROWS * 128;           // [XROWS x 64 columns] fp16
   static constexpr int kXBytes = (PERM ? 4 : 2) * kXSub;        // a tile of the ring: a stage, or half of one
   // activation tiles in flight: enough to hide the latency of their loads behind the stages before (with one per slot the
   // expansion warps waited half their time); with PERM at most six, see the wait for a slot
-  static constexpr int kXRing = TOK == 16 ? 6 : TOK == 32 ? 4 : TOK == 64 ? 6 : 4;
+  static constexpr int kXRing = TOK == 16 ? 6 : TOK <= 64 ? 6 : 4;
   // accumulators: FOLD two per slot (one for each 128 columns), else one per segment in turn
   static constexpr int kAccs = FOLD ? 2 * kSlots : TOK > 64 ? 1 : 2;
   static constexpr uint32_t kASlot0 = kAccs * TOK;
@@ -656,7 +656,7 @@ int launch_decode_umma(const void* x, const void* packed, const void* sz, const 
   if (rc != MP_OK) return rc;
   // [64 columns][token][chunk of 64 columns]: one copy brings the sub-tiles of a stage or half of one
   const uint64_t x_dims[3] = {64, (uint64_t)M, (uint64_t)K / 64}, x_strides[2] = {(uint64_t)K * 2, 128};
-  const uint32_t x_box[3] = {64, (uint32_t)(M <= 8 ? 8 : tok), tok <= 32 ? 4u : 2u};
+  const uint32_t x_box[3] = {64, (uint32_t)(M <= 8 ? 8 : tok), tok <= 16 ? 4u : 2u};
   rc = encode_tensor_map_3d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, x_dims, x_strides, x_box);
   if (rc != MP_OK) return rc;
   const int gps = group < du::kStageK ? du::kStageK / group : 1;
