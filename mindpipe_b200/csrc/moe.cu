@@ -19,6 +19,7 @@ namespace mp {
 
 constexpr int kTileRows = kMoeTileRows;
 constexpr int kMaxExperts = 256;
+constexpr int kPlanInGather = 256;      // most routed entries for which the gather makes the plan: one to a thread
 
 // softmax(fp32) -> top-k -> renormalise -> fp16, one thread per token
 // (algorithm/quantization/qat/flatquant/source/flatquant/model_tools/mixtral_utils.py:330-333,349).
@@ -119,6 +120,35 @@ __global__ void moe_plan_kernel(int* __restrict__ plan, int E, int max_tiles) {
   *num_tiles = tiles;
 }
 
+// One block: the plan for these counts, laid out by thread 0 exactly as moe_plan_kernel does it, and zero scales for every
+// segment's padding rows, so that whatever codes they hold turn into zeros downstream.  placed: the entries have their rows
+// already, as the cursors will say once they all took one.
+__device__ __forceinline__ void write_plan(const int* s_counts, int* __restrict__ plan, int E, int max_tiles,
+                                           float* __restrict__ routed_scale, bool placed) {
+  int* counts = plan;
+  int* cursors = plan + E;
+  int* seg = plan + 2 * E;
+  if (threadIdx.x == 0) {
+    int* num_tiles = plan + 3 * E + 1;
+    int* tile_expert = plan + 3 * E + 2;
+    int off = 0, tiles = 0;
+    for (int e = 0; e < E; ++e) {
+      counts[e] = s_counts[e];
+      seg[e] = off;
+      cursors[e] = placed ? s_counts[e] : 0;
+      const int nt = moe_segment_tiles(s_counts[e]);
+      for (int i = 0; i < nt && tiles < max_tiles; ++i) tile_expert[tiles++] = e;
+      off += nt * kTileRows;
+    }
+    seg[E] = off;
+    *num_tiles = tiles;
+  }
+  __syncthreads();
+  for (int e = 0; e < E; ++e)
+    for (int r = seg[e] + s_counts[e] + threadIdx.x; r < seg[e + 1]; r += blockDim.x) routed_scale[r] = 0.0f;
+  for (int r = seg[E] + threadIdx.x; r < max_tiles * kTileRows; r += blockDim.x) routed_scale[r] = 0.0f;   // unused tail
+}
+
 // Count and plan in one launch (one block): the per-expert counts are taken in shared memory, thread 0 lays out the
 // padded segments exactly as moe_plan_kernel does, and the scales of every segment's padding rows are zeroed -- so
 // the routing needs no memset of the counters or of the scale buffer and two launches instead of five nodes.
@@ -138,29 +168,7 @@ moe_count_plan_kernel(const int* __restrict__ ids, int n_entries, int lo, int hi
     if (key >= 0 && (threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&s_counts[key], __popc(same));
   }
   __syncthreads();
-  int* counts = plan;
-  int* cursors = plan + E;
-  int* seg = plan + 2 * E;
-  if (threadIdx.x == 0) {
-    int* num_tiles = plan + 3 * E + 1;
-    int* tile_expert = plan + 3 * E + 2;
-    int off = 0, tiles = 0;
-    for (int e = 0; e < E; ++e) {
-      counts[e] = s_counts[e];
-      seg[e] = off;
-      cursors[e] = 0;
-      const int nt = moe_segment_tiles(s_counts[e]);
-      for (int i = 0; i < nt && tiles < max_tiles; ++i) tile_expert[tiles++] = e;
-      off += nt * kTileRows;
-    }
-    seg[E] = off;
-    *num_tiles = tiles;
-  }
-  __syncthreads();
-  // padding rows get scale 0, so whatever codes they hold turn into zeros downstream
-  for (int e = 0; e < E; ++e)
-    for (int r = seg[e] + s_counts[e] + threadIdx.x; r < seg[e + 1]; r += blockDim.x) routed_scale[r] = 0.0f;
-  for (int r = seg[E] + threadIdx.x; r < max_tiles * kTileRows; r += blockDim.x) routed_scale[r] = 0.0f;   // unused tail
+  write_plan(s_counts, plan, E, max_tiles, routed_scale, false);
 }
 
 // One block per routed entry (t, j): claim a row in the expert's segment, record it, and
@@ -169,10 +177,13 @@ moe_count_plan_kernel(const int* __restrict__ ids, int n_entries, int lo, int hi
 // in one pass.  Arithmetic as in act_quant.cu.
 // KEEP: rows of up to 4096 values (two 16-byte pieces per thread) stay in registers between the abs-max pass
 // and the quantising pass instead of being read a second time.
-template <bool KEEP>
+// PLAN: up to 256 entries, whose ids every block reads for itself: it counts them, finds its row (entries of an expert in
+// their order) and needs no launch before it; one block more writes the plan (a launch less: 3 us of the 27 that two tokens
+// took).
+template <bool KEEP, bool PLAN>
 __global__ void __launch_bounds__(256)
 moe_gather_quant_kernel(const __half* __restrict__ hidden, const int* __restrict__ ids, int H, int k, int lo, int hi,
-                        int* __restrict__ plan, int E, int* __restrict__ dest_row,
+                        int* __restrict__ plan, int E, int max_tiles, int* __restrict__ dest_row,
                         int8_t* __restrict__ routed_q, float* __restrict__ routed_scale) {
   chain_wait();
   chain_release();
@@ -180,6 +191,30 @@ moe_gather_quant_kernel(const __half* __restrict__ hidden, const int* __restrict
   __shared__ float s_scale;
   __shared__ int s_dest;
   const int entry = blockIdx.x;
+  int planned = 0;
+  if constexpr (PLAN) {
+    __shared__ int s_counts[kMaxExperts];
+    __shared__ int s_base;
+    const int n = gridDim.x - 1, tid = threadIdx.x;
+    const int id = tid < n ? ids[tid] : -1;
+    if (tid < kMaxExperts) s_counts[tid] = 0;
+    if (tid == 0) s_base = 0;
+    __syncthreads();
+    if (id >= lo && id < hi) atomicAdd(&s_counts[id - lo], 1);
+    __syncthreads();
+    if (entry == n) {
+      write_plan(s_counts, plan, E, max_tiles, routed_scale, true);
+      return;
+    }
+    const int own = ids[entry];
+    planned = __syncthreads_count(tid < entry && id == own);
+    if (own >= lo && tid < own - lo && tid < E) {
+      const int rows = moe_segment_tiles(s_counts[tid]) * kTileRows;
+      if (rows) atomicAdd(&s_base, rows);
+    }
+    __syncthreads();
+    planned += s_base;
+  }
   const int e = ids[entry];
   if (e < lo || e >= hi) {
     if (threadIdx.x == 0) dest_row[entry] = -1;
@@ -223,8 +258,7 @@ moe_gather_quant_kernel(const __half* __restrict__ hidden, const int* __restrict
     for (int i = 1; i < 8; ++i) v = fmaxf(v, s_red[i]);
     const float eps = h2f(f2h(1e-5f));
     s_scale = h2f(f2h(__fdiv_rn(fmaxf(v, eps), 127.0f)));
-    const int pos = atomicAdd(plan + E + (e - lo), 1);
-    s_dest = plan[2 * E + (e - lo)] + pos;
+    s_dest = PLAN ? planned : plan[2 * E + (e - lo)] + atomicAdd(plan + E + (e - lo), 1);
     dest_row[entry] = s_dest;
     routed_scale[s_dest] = s_scale;
   }
@@ -290,7 +324,8 @@ moe_requant_kernel(const __half* __restrict__ h, const float* __restrict__ absma
   }
 }
 
-// The same for the rows of a few routed entries, a block each (padding rows are neither computed nor read).
+// The same for the rows of the routed entries, a block each: padding rows, four of five with 104 tokens over four experts,
+// are neither computed nor read.  Where they are less than half the strided form is as fast (8192 tokens: 1 % faster).
 __global__ void __launch_bounds__(256)
 moe_requant_rows_kernel(const __half* __restrict__ h, const float* __restrict__ absmax, int slots, int I,
                         const int* __restrict__ dest_row, int8_t* __restrict__ q, float* __restrict__ scale) {
@@ -310,6 +345,13 @@ moe_requant_rows_kernel(const __half* __restrict__ h, const float* __restrict__ 
   int8_t* qr = q + (size_t)row * I;
   for (int c = blockIdx.y * 256 + threadIdx.x; c < (I >> 3); c += gridDim.y * 256)
     *reinterpret_cast<uint2*>(qr + c * 8) = quant8_pack(*reinterpret_cast<const uint4*>(hr + c * 8), rq);
+}
+
+static int launch_requant_rows(const __half* h, const float* absmax, int I, const int* dest_row, int entries, int8_t* q2,
+                               float* scale2, cudaStream_t st) {
+  const int parts = (I / 8 + 1023) / 1024;       // about a thousand eight-value pieces per block
+  return launch_chained(moe_requant_rows_kernel, dim3(entries, parts), dim3(256), 0, st, h, absmax, moe_absmax_slots(I), I,
+                        dest_row, q2, scale2);
 }
 
 static int launch_requant(const __half* h, const float* absmax, int I, const int* num_tiles, int padded_rows,
@@ -435,6 +477,15 @@ extern "C" int mp_moe_route_gather_quant(const void* hidden_f16, const void* top
   int* plan = static_cast<int*>(plan_i32);
   const int n_entries = T * k;
   const int padded = mp_moe_padded_rows(E, n_entries);
+  const __half* x = static_cast<const __half*>(hidden_f16);
+  const int* ids = static_cast<const int*>(topk_ids_i32);
+  int* dest = static_cast<int*>(dest_row_i32);
+  int8_t* rq = static_cast<int8_t*>(routed_q_i8);
+  float* rs = static_cast<float*>(routed_scale_f32);
+  if (n_entries <= kPlanInGather)
+    return launch_chained(H <= 4096 ? moe_gather_quant_kernel<true, true> : moe_gather_quant_kernel<false, true>,
+                          dim3(n_entries + 1), dim3(256), 0, st, x, ids, H, k, expert_lo, expert_hi, plan, E,
+                          padded / kTileRows, dest, rq, rs);
   if (n_entries <= 8192) {
     // few entries (a rank's share under expert parallelism, decode batches): one block counts, plans and zeroes the
     // padding rows' scales -- two launches instead of five graph nodes; with more entries one block's pass over the
@@ -454,11 +505,8 @@ extern "C" int mp_moe_route_gather_quant(const void* hidden_f16, const void* top
     moe_plan_kernel<<<1, 32, 0, st>>>(plan, E, padded / kTileRows);
     MP_LAUNCH_CHECK();
   }
-  return launch_chained(H <= 4096 ? moe_gather_quant_kernel<true> : moe_gather_quant_kernel<false>, dim3(n_entries),
-                        dim3(256), 0, st,
-                        static_cast<const __half*>(hidden_f16), static_cast<const int*>(topk_ids_i32), H, k, expert_lo,
-                        expert_hi, plan, E, static_cast<int*>(dest_row_i32), static_cast<int8_t*>(routed_q_i8),
-                        static_cast<float*>(routed_scale_f32));
+  return launch_chained(H <= 4096 ? moe_gather_quant_kernel<true, false> : moe_gather_quant_kernel<false, false>,
+                        dim3(n_entries), dim3(256), 0, st, x, ids, H, k, expert_lo, expert_hi, plan, E, 0, dest, rq, rs);
 }
 
 // ---- expert stage on rows that are already routed and quantised ------------
@@ -498,7 +546,8 @@ static int stage_buffers(void* workspace, size_t workspace_bytes, int padded_row
 static int expert_stage(const void* routed_q_i8, const void* routed_scale_f32, const void* plan_i32, int padded_rows,
                         int H, int I, int num_local_experts, const void* w13_q_i8, const void* w13_scale_f32,
                         const void* w2_q_i8, const void* w2_scale_f32, void* d_out_f16, const RowScatter* scatter,
-                        void* workspace, size_t workspace_bytes, int* error_word, mp_stream_t stream) {
+                        void* workspace, size_t workspace_bytes, int* error_word, mp_stream_t stream,
+                        const int* dest_row = nullptr, int entries = 0) {
   if (!routed_q_i8 || !routed_scale_f32 || !plan_i32 || !w13_q_i8 || !w13_scale_f32 || !w2_q_i8 || !w2_scale_f32 ||
       (!d_out_f16 && !scatter) || padded_rows <= 0 || H <= 0 || I <= 0 || num_local_experts <= 0)
     return MP_ERR_INVALID_ARG;
@@ -518,7 +567,8 @@ static int expert_stage(const void* routed_q_i8, const void* routed_scale_f32, c
                                static_cast<const float*>(w13_scale_f32), padded_rows, H, I, E, num_tiles, tile_expert,
                                b.h, b.absmax, error_word, st);
   if (rc != MP_OK) return rc;
-  rc = launch_requant(b.h, b.absmax, I, num_tiles, padded_rows, b.q2, b.scale2, st);
+  rc = dest_row ? launch_requant_rows(b.h, b.absmax, I, dest_row, entries, b.q2, b.scale2, st)
+                : launch_requant(b.h, b.absmax, I, num_tiles, padded_rows, b.q2, b.scale2, st);
   if (rc != MP_OK) return rc;
   return launch_moe_gemm2(b.q2, b.scale2, w2_q_i8, static_cast<const float*>(w2_scale_f32), padded_rows, I, H, E,
                           num_tiles, tile_expert, d_out_f16, error_word, st, scatter);
@@ -687,7 +737,8 @@ extern "C" int mp_moe_experts(const void* hidden_f16, const void* topk_ids_i32, 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     StreamParams p{};
     p.N = I; p.K = H;
-    p.early_weights = 1;                         // the kernel before is the gather, which waited for the plan
+    // which weights are read follows from the plan: older than the gather (which waited for it), or the gather's own work
+    p.early_weights = T * k > kPlanInGather;
     p.counts = plan;
     p.segments = plan + 2 * E;
     p.experts = E;
@@ -700,10 +751,7 @@ extern "C" int mp_moe_experts(const void* hidden_f16, const void* topk_ids_i32, 
     p.error_word = error_word;
     rc = launch_w8a8_stream(STREAM_SWIGLU, rq, b.padded, w13_q_i8, E * 2 * I, p, T, workspace, workspace_bytes, st);
     if (rc == MP_OK) {
-      const int parts = (I / 8 + 1023) / 1024;   // about a thousand eight-value pieces per block
-      rc = launch_chained(moe_requant_rows_kernel, dim3(T * k, parts), dim3(256), 0, st, static_cast<const __half*>(sb.h),
-                          static_cast<const float*>(sb.absmax), moe_absmax_slots(I), I, static_cast<const int*>(dest), sb.q2,
-                          sb.scale2);
+      rc = launch_requant_rows(sb.h, sb.absmax, I, dest, T * k, sb.q2, sb.scale2, st);
       if (rc != MP_OK) return rc;
       StreamParams p2{};
       p2.N = H; p2.K = I;
@@ -722,8 +770,8 @@ extern "C" int mp_moe_experts(const void* hidden_f16, const void* topk_ids_i32, 
     }
     if (rc != MP_ERR_UNSUPPORTED) return rc;
   }
-  rc = mp_moe_expert_stage(rq, rscale, plan, b.padded, H, I, E, w13_q_i8, w13_scale_f32, w2_q_i8, w2_scale_f32, d,
-                           base + b.stage, stage_bytes, error_word, stream);
+  rc = expert_stage(rq, rscale, plan, b.padded, H, I, E, w13_q_i8, w13_scale_f32, w2_q_i8, w2_scale_f32, d, nullptr,
+                    base + b.stage, stage_bytes, error_word, stream, 2 * T * k <= b.padded ? dest : nullptr, T * k);
   if (rc != MP_OK) return rc;
   return mp_moe_combine(d, dest, topk_ids_i32, topk_weights_f16, T, H, k, out_f16, stream);
 }

@@ -87,3 +87,42 @@ def test_router_matches_softmax_topk_at_every_width(e):
     assert torch.equal(idx.long(), ref[:, :2])
     want = top[:, :2] / top[:, :2].sum(dim=-1, keepdim=True)
     assert (w.float() - want).abs().max().item() <= 1e-3
+
+
+@pytest.mark.parametrize("t,k,lo,hi", [(1, 1, 0, 4), (3, 2, 0, 16), (128, 2, 0, 8), (129, 2, 0, 8), (60, 4, 2, 6), (32, 8, 0, 256)])
+def test_routing_plan_and_rows(t, k, lo, hi):
+    """Routing of up to 256 entries makes its plan beside the gather: counts, segments, tiles, scales and codes as the host
+    lays them out, every entry on a row of its expert."""
+    from mindpipe_b200 import _lib, ops
+    lib = _lib.load()
+    h, e = 256, hi - lo
+    g = torch.Generator(device="cuda").manual_seed(t)
+    x = torch.randn(t, h, generator=g, device="cuda").half()
+    ids = torch.stack([torch.randperm(max(hi + 2, k), generator=g, device="cuda")[:k] for _ in range(t)]).int()
+    padded = lib.mp_moe_padded_rows(e, t * k)
+    plan = torch.full((lib.mp_moe_plan_ints(e, t * k),), -7, dtype=torch.int32, device="cuda")
+    dest = torch.full((t * k,), -7, dtype=torch.int32, device="cuda")
+    q = torch.full((padded, h), 99, dtype=torch.int8, device="cuda")
+    s = torch.full((padded,), -1.0, device="cuda")
+    assert lib.mp_moe_route_gather_quant(x.data_ptr(), ids.data_ptr(), t, h, k, lo, hi, plan.data_ptr(), dest.data_ptr(),
+                                         q.data_ptr(), s.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    flat = ids.flatten().cpu().tolist()
+    counts = [flat.count(x_) for x_ in range(lo, hi)]
+    seg = [0]
+    for c in counts:
+        seg.append(seg[-1] + (c + 255) // 256 * 256)
+    p, d = plan.cpu().tolist(), dest.cpu().tolist()
+    assert p[:e] == counts and p[e:2 * e] == counts and p[2 * e:3 * e + 1] == seg and p[3 * e + 1] == seg[-1] // 128
+    assert p[3 * e + 2:3 * e + 2 + seg[-1] // 128] == [i for i in range(e) for _ in range((seg[i + 1] - seg[i]) // 128)]
+    want_q, want_s, _ = ops.act_quant_per_token(x)
+    used = set()
+    for i, x_ in enumerate(flat):
+        if not lo <= x_ < hi:
+            assert d[i] == -1
+            continue
+        assert seg[x_ - lo] <= d[i] < seg[x_ - lo] + counts[x_ - lo] and d[i] not in used
+        used.add(d[i])
+        assert torch.equal(q[d[i]], want_q[i // k]) and s[d[i]].item() == want_s.flatten()[i // k].item()
+    rest = torch.ones(padded, dtype=torch.bool)
+    rest[list(used)] = False
+    assert (s.cpu()[rest] == 0).all()
