@@ -261,13 +261,8 @@ int mp_w4a16_linear_decode_static(const void* x_f16, const void* packed_i32, con
  * activations, bias and outputs are only touched after that kernel has
  * completed.  Enable it only when no kernel still in flight writes the weight
  * buffers (weights are loaded once and then static, as in serving).
- * The same switch covers the W8A8 GEMMs and the kernels of the MoE layer
- * (routing, expert-parallel exchange and barriers, re-quantisation, combine):
- * each of them may be scheduled early, sets up its shared / tensor memory, and
- * then waits on the device for the preceding kernel before it reads or writes
- * anything else -- the launch latencies of the chain overlap, results are
- * the same bits.  The setting is read when a launch is issued (for a CUDA
- * graph: at capture).
+ * Kernels that wait for their predecessor's results on the device (W8A8, MoE, W4A16 with many rows) are always launched
+ * this way; beyond the decode linears the switch covers the kernels that wait for other GPUs.
  */
 int mp_set_programmatic_launch(int enabled);
 

@@ -1,4 +1,4 @@
-// W4A16 linear for up to 64 rows on the tcgen05 tensor core with the weights as the TENSOR-MEMORY operand:
+// W4A16 linear for up to 128 rows (the dispatch sends more than 96 elsewhere where it can) on the tcgen05 tensor core with the weights as the TENSOR-MEMORY operand:
 // y = x @ dequant(W)^T, the packed weights streamed once.
 //
 // A thread owns ONE weight row: it reads 16 bytes (32 codes) of its row from the shared-memory ring, expands them and
@@ -29,17 +29,19 @@
 // order (results are identical from run to run).  A tile word is stored inverted and zero means "not there yet": the
 // reader polls the words themselves (bounded) and puts the zeros back, with no fence, counter or second round trip.
 //
-//   warps 0-11   expansion: three sets of four; set j takes units j, j + 3, ... and owns TMEM slot j
-//   warps 12-15  epilogue
-//   warp 16      TMA producer of weights and (scale, zero) pairs
-//   warp 17      TMEM allocation and the MMA issuer
-//   warp 18      TMA producer of activations
-// Expansion emits the columns of a packed word in the order (k0,k4,k1,k5,k2,k6,k3,k7).  The threads of a unit apply the
-// same permutation in place to the 16-byte chunks of the unit's activation tile (a chunk is one token's eight columns of
-// one word, so the swizzle does not matter): two chunks each at 16 tokens.  (Warps of their own for this were starved
-// by the expansion warps: 2100 clocks per stage with one.)
-// Up to 16 rows a block takes less than half an SM (shared memory, registers, 256 TMEM columns), so that in a chain of
-// linears the next one's blocks start, and with the caller's leave fetch weights, beside the ones that finish.
+//   warps 0-15   expansion: two sets of eight take stages in turn; a warp does 32 rows of half a stage
+//   warps 16-19  epilogue
+//   warp 20      TMA producer of weights and (scale, zero) pairs
+//   warp 21      TMEM allocation and the MMA issuer
+//   warp 22      TMA producer of activations
+// Expansion emits the columns of a packed word in the order (k0,k4,k1,k5,k2,k6,k3,k7).  Up to 16 rows the expansion warps
+// apply the same permutation in place to the 16-byte chunks of the stage's activation tile (a chunk is one token's eight
+// columns of one word, so the swizzle does not matter); with more rows they put the words back in order, see Cfg.  (Warps
+// of their own for the permutation were starved by the expansion warps: 2100 clocks per stage with one.)
+// One block fills an SM: its ring is what hides HBM's latency.  Smaller blocks, two of them to an SM so that the next linear
+// of a chain starts beside the end of this one, took 38 us where this takes 28 (28672x8192, 16 rows).
+// A launch of 12288x4096 at 16 rows, 12 us: 2.7 from the end of the kernel before to the first stage's data (all SMs ask at
+// once), 0.7 its expansion, 4.7 the stream, 2 the exchange of partial tiles, the rest launch and exit.
 // Every wait is bounded.
 #include "common.cuh"
 #include "tc.cuh"
