@@ -531,10 +531,13 @@ def run_ours(args, rank, world, local_rank):
     torch.cuda.synchronize()
     _lib.load().mp_set_programmatic_launch(1 if args.pdl else 0)
 
-    ws_bytes = max(ops.w4a16_decode_workspace_bytes(M_DECODE, n, k) for _, (n, k) in layer_shapes())
+    lib, error_word = _lib.load(), ops._error_word(torch.device(dev)).data_ptr()
     # one scratch buffer per linear: with --fuse 0 --concurrent 1 some of them run side by side
-    ws = {name: ops.new_workspace(ws_bytes, dev) for name, _ in layer_shapes()}
-    umma_names = [name for name, (n, k) in layer_shapes() if ops.w4a16_decode_kernel_choice(M_DECODE, n, k) == "umma"]
+    ws = {name: ops.new_workspace(max(64, lib.mp_w4a16_linear_workspace_bytes(M_DECODE, n, k, GROUP)), dev)
+          for name, (n, k) in layer_shapes()}
+    # the linear's own choice at 9 to 16 rows: the tcgen05 weight stream unless the shape is tiny or the choice is forced
+    umma_names = [name for name, (n, k) in layer_shapes()
+                  if args.decode_kernel != "mma_sync" and n >= 2048 and n * k // 2 >= 2 << 20]
     tma_names = [name for name, _ in layer_shapes() if name not in umma_names]
     kernel_names = " + ".join(
         f"{kern} ({', '.join(names)})" for kern, names in (("w4a16_decode_umma_kernel", umma_names),
@@ -544,7 +547,12 @@ def run_ours(args, rank, world, local_rank):
     side = [torch.cuda.Stream(device=dev) for _ in range(2)]
 
     def launch(name, mod):
-        ops.w4a16_linear_decode(x_dev[name], mod.weight_packed, mod._scale_zero, workspace=ws[name], out=y_dev[name])
+        # what the module's forward calls, with buffers of the bench's own (the step is captured)
+        status = lib.mp_w4a16_linear(x_dev[name].data_ptr(), mod.weight_packed.data_ptr(), mod._scale_zero.data_ptr(), None,
+                                     y_dev[name].data_ptr(), M_DECODE, mod.out_features, mod.in_features, GROUP,
+                                     ws[name].data_ptr(), ws[name].numel(), error_word,
+                                     torch.cuda.current_stream().cuda_stream)
+        _lib.check(status, "w4a16_linear")
 
     def step(layer):
         """The layer's dependency structure: q, k, v side by side; o; gate, up side by side; down."""
