@@ -1,0 +1,24 @@
+"""Per-token quantisation with few and many rows: the block shape follows the row count, the bits do not."""
+import pytest
+import torch
+
+from mindpipe_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("k", [2056, 4096, 4104, 8192, 8200, 11008, 16384, 16392])
+def test_same_bits_whatever_the_row_count(k):
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x = torch.randn(149, k, generator=g, device="cuda").half()
+    x[:, ::97] *= 20
+    x[3], x[5] = 0, x[5].abs()
+    q, s, fake = ops.act_quant_per_token(x, want_fake=True)
+    parts = [ops.act_quant_per_token(x[i:i + 50].contiguous(), want_fake=True) for i in range(0, 149, 50)]
+    for whole, j in ((q, 0), (s, 1), (fake, 2)):
+        assert torch.equal(whole, torch.cat([p[j] for p in parts]))
+    whole = ops.affine_quant_per_row(x)
+    parts = [ops.affine_quant_per_row(x[i:i + 50].contiguous()) for i in range(0, 149, 50)]
+    for j, t in enumerate(whole):
+        if t is not None:
+            assert torch.equal(t, torch.cat([p[j] for p in parts]))
