@@ -89,9 +89,10 @@ def test_router_matches_softmax_topk_at_every_width(e):
     assert (w.float() - want).abs().max().item() <= 1e-3
 
 
-@pytest.mark.parametrize("t,k,lo,hi", [(1, 1, 0, 4), (3, 2, 0, 16), (128, 2, 0, 8), (129, 2, 0, 8), (60, 4, 2, 6), (32, 8, 0, 256)])
+@pytest.mark.parametrize("t,k,lo,hi", [(1, 1, 0, 4), (3, 2, 0, 16), (128, 2, 0, 8), (129, 2, 0, 8), (60, 4, 2, 6), (32, 8, 0, 256), (149, 2, 0, 8),
+                                       (700, 3, 1, 6)])
 def test_routing_plan_and_rows(t, k, lo, hi):
-    """Routing of up to 256 entries makes its plan beside the gather: counts, segments, tiles, scales and codes as the host
+    """Routing of few entries makes its plan beside the gather, of many tokens goes token by token: counts, segments, tiles, scales and codes as the host
     lays them out, every entry on a row of its expert."""
     from mindpipe_b200 import _lib, ops
     lib = _lib.load()
