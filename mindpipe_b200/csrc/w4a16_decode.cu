@@ -821,9 +821,13 @@ extern "C" int mp_w4a16_linear_decode(const void* x_f16, const void* packed_i32,
 // with "stream" the tcgen05 kernel of w4a16_decode_umma.cu (needs a workspace) and "ring" the mma.sync kernel:
 enum LinearKernel { kRing, kStream, kGemm };
 
+// The only place that decides: the scratch that is asked for and the kernel that runs both follow from it.
 static LinearKernel linear_kernel(int M, int N, int K, int group) {
   const LinearKernel narrow = M <= 16 ? kRing : kGemm;
-  if (!decode_umma_shape_ok(M, N, K, group) || g_decode_kernel == MP_DECODE_KERNEL_MMA_SYNC) return narrow;
+  // K of half a 128-column chunk and N of half an 8-row group go to the GEMM: the stream kernel's own limits (64 and 4) are
+  // wider than what the decode entries accept
+  if (K % kChunk != 0 || N % 8 != 0 || !decode_umma_shape_ok(M, N, K, group)) return narrow;
+  if (g_decode_kernel == MP_DECODE_KERNEL_MMA_SYNC) return narrow;
   if (g_decode_kernel == MP_DECODE_KERNEL_UMMA) return M <= 64 ? kStream : kGemm;
   const size_t packed = (size_t)N * (size_t)K / 2;
   // Above 96 rows the pair kernel expands less often for its tokens (4096x11008 at 97 / 128 rows: 23.7 / 26.0 vs 21.7 / 22.3
@@ -860,7 +864,7 @@ int w4a16_linear(const void* x_f16, const void* packed_i32, const void* sz_f16x2
   if (!x_f16 || !packed_i32 || !sz_f16x2 || !y_f16 || M <= 0 || N <= 0 || K <= 0 || group <= 0) return MP_ERR_INVALID_ARG;
   if (K % group != 0) return MP_ERR_UNSUPPORTED;
   const LinearKernel kernel = linear_kernel(M, N, K, group);
-  if (kernel == kStream && N % 8 == 0 && K % kChunk == 0) {
+  if (kernel == kStream) {
     if (!aligned(x_f16, 16) || !aligned(packed_i32, 16) || !aligned(sz_f16x2, 4) || !aligned(y_f16, 2)) return MP_ERR_ALIGNMENT;
     const int rc = launch_decode_umma(x_f16, packed_i32, sz_f16x2, bias_f16, y_f16, M, N, K, group, workspace,
                                       workspace_bytes, static_cast<cudaStream_t>(stream),
@@ -870,7 +874,9 @@ int w4a16_linear(const void* x_f16, const void* packed_i32, const void* sz_f16x2
   if (M <= 16)
     return decode_linear(x_f16, packed_i32, sz_f16x2, bias_f16, y_f16, M, N, K, group, workspace, workspace_bytes, 0,
                          MP_DECODE_KERNEL_MMA_SYNC, early, stream);
-  const bool scratch = workspace && workspace_bytes > kPartialOffset;
+  // After the stream kernel has declined, the workspace is not one that was sized for the GEMM, whatever its size: none of it
+  // is used, so that the result does not depend on calls before.
+  const bool scratch = kernel == kGemm && workspace && workspace_bytes > kPartialOffset;
   return mp_w4a16_linear_prefill_ex(x_f16, packed_i32, sz_f16x2, bias_f16, y_f16, M, N, K, group,
                                     scratch ? static_cast<unsigned char*>(workspace) + kPartialOffset : nullptr,
                                     scratch ? workspace_bytes - kPartialOffset : 0, error_word, stream);
