@@ -41,6 +41,7 @@ int launch_decode_umma(const void* x, const void* packed, const void* sz, const 
 bool decode_umma_shape_ok(int M, int N, int K, int group);
 int decode_tma_cluster(int row_blocks, int stages);   // cluster size the ring kernel splits K over
 size_t decode_umma_workspace_bytes(int M, int K);
+size_t w4a16_gemm_partial_bytes(int M, int N, int K);   // w4a16_gemm.cu
 // Which kernel serves M <= 16 when a call does not say: one of the MP_DECODE_KERNEL_* values.  Shapes the
 // chosen one does not take fall through to the next.
 static int g_decode_kernel = MP_DECODE_KERNEL_AUTO;
@@ -851,7 +852,7 @@ extern "C" size_t mp_w4a16_linear_workspace_bytes(int M, int N, int K, int group
     case kStream: return decode_umma_workspace_bytes(M, K);
     case kRing: return 0;
     default: {
-      const size_t split = mp_w4a16_prefill_workspace_bytes(M, N, K);
+      const size_t split = w4a16_gemm_partial_bytes(M, N, K);
       return split ? kPartialOffset + split : 0;
     }
   }
@@ -876,7 +877,7 @@ int w4a16_linear(const void* x_f16, const void* packed_i32, const void* sz_f16x2
                          MP_DECODE_KERNEL_MMA_SYNC, early, stream);
   // After the stream kernel has declined, the workspace is not one that was sized for the GEMM, whatever its size: none of it
   // is used, so that the result does not depend on calls before.
-  const bool scratch = kernel == kGemm && workspace && workspace_bytes > kPartialOffset;
+  const bool scratch = kernel == kGemm && workspace && workspace_bytes > kPartialOffset && w4a16_gemm_partial_bytes(M, N, K) > 0;
   return mp_w4a16_linear_prefill_ex(x_f16, packed_i32, sz_f16x2, bias_f16, y_f16, M, N, K, group,
                                     scratch ? static_cast<unsigned char*>(workspace) + kPartialOffset : nullptr,
                                     scratch ? workspace_bytes - kPartialOffset : 0, error_word, stream);

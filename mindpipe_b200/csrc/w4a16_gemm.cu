@@ -720,16 +720,28 @@ static W4Shape w4_gemm_shape(int M, int N, int K, bool scratch, const int (&clus
 
 static size_t w4_partial_bytes(int pairs, int T) { return (size_t)pairs * 4 * T * w4::kRows * sizeof(float); }
 
+static W4Shape w4_gemm_shape_here(int M, int N, int K) {
+  const W4Device* d;
+  const int none[3] = {0, 0, 0};
+  return w4_gemm_shape(M, N, K, true, w4_device(&d) == MP_OK ? d->clusters : none);
+}
+
+// What the chosen cut writes: partial tiles for equal runs, nothing for whole tiles and clusters.
+size_t w4a16_gemm_partial_bytes(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0 || K % 64 != 0) return 0;
+  const W4Shape s = w4_gemm_shape_here(M, N, K);
+  return s.runs ? w4_partial_bytes(s.pairs, s.T) : 0;
+}
+
 }  // namespace mp
 
 using namespace mp;
 
-// Room for the partial tiles wherever they may be wanted: when the split is chosen, and for fewer tiles than pairs.
+// What the entry with scratch insists on: the same, and for fewer pairs than the device has also where the cut writes none of
+// it (a smaller buffer has always been refused there).
 extern "C" size_t mp_w4a16_prefill_workspace_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0 || K % 64 != 0) return 0;
-  const W4Device* d;
-  const int none[3] = {0, 0, 0};
-  const W4Shape s = w4_gemm_shape(M, N, K, true, w4_device(&d) == MP_OK ? d->clusters : none);
+  const W4Shape s = w4_gemm_shape_here(M, N, K);
   return s.runs || s.pairs < w4::kPairs ? w4_partial_bytes(s.pairs, s.T) : 0;
 }
 

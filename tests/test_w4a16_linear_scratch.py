@@ -76,3 +76,26 @@ def test_parameters_the_stream_kernel_declines_for_their_alignment(m):
     assert ((got[0].double() - ref).norm() / ref.norm()).item() <= 4e-4
     assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
     ops.check_device_errors()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,runs", [(128, 4096, 4096, False), (200, 1024, 1024, False), (512, 1024, 2048, False),
+                                        (97, 1024, 28672, True)])
+def test_only_equal_runs_ask_for_room(m, n, k, runs):
+    """Whole tiles and clusters of pairs write no partial tiles: no scratch, and the bits of a call that has some."""
+    mod = _module(n, k, 128)
+    mod._ensure_prepared()
+    x = torch.randn(m, k, device="cuda").half()
+    need = _lib.load().mp_w4a16_linear_workspace_bytes(m, n, k, 128)
+    assert (need > 0) == runs
+    y = torch.empty(m, n, dtype=torch.float16, device="cuda")
+    for nbytes in (need, need + (64 << 20)):
+        ws = torch.zeros(nbytes, dtype=torch.uint8, device="cuda") if nbytes else None
+        st = _lib.load().mp_w4a16_linear(x.data_ptr(), mod.weight_packed.data_ptr(), mod._scale_zero.data_ptr(), None,
+                                         y.data_ptr(), m, n, k, 128, None if ws is None else ws.data_ptr(), nbytes,
+                                         ops._error_word(x.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert st == 0
+        assert torch.equal(y, ops.w4a16_linear_prefill(x, mod.weight_packed, mod._scale_zero))
+    ref = x.double() @ mod.dequantize().double().T
+    assert ((y.double() - ref).norm() / ref.norm()).item() <= 4e-4
+    ops.check_device_errors()
