@@ -788,7 +788,9 @@ def run_ours(args, rank, world, local_rank):
         traffic = None
         tr = ROOT / "profiles" / "w4a16_decode_traffic.json"
         if tr.exists():
-            traffic = json.loads(tr.read_text()).get("dram_bytes_per_launch")
+            captured = json.loads(tr.read_text())
+            if captured.get("kernel") == kernel_names:         # a figure of these kernels on these launches, or none
+                traffic = captured.get("dram_bytes_per_launch")
         line = {
             "metric": "w4a16_decode_linear_algorithmic_hbm_gbs", "value": value, "unit": "GB/s",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms / args.steps,
@@ -855,9 +857,8 @@ def measure_other_configs(args, local_rank):
                                                           "linear_tops", "library_int8_gemm_tops")})
     if errors:
         out["errors"] = errors
-    out["note"] = ("decode: chains of launches under programmatic dependent launch, weights rotated; M=64 goes where "
-                   "ops.w4a16_linear sends it (tcgen05 weight-streaming kernel with a 64-token tile on the 70B-sized "
-                   "weights, split-K tensor-core GEMM otherwise); library_int8_gemm_tops is torch._int_mm on the same box, "
+    out["note"] = ("decode: chains of mp_w4a16_linear, the call behind the module's forward, under programmatic dependent "
+                   "launch, weights rotated; library_int8_gemm_tops is torch._int_mm on the same box, "
                    "a timing yardstick only (MEASURED_PEAKS.json has no int8 figure)")
     return out
 
@@ -938,25 +939,20 @@ def run_suite(args, local_rank, collect=None):
                 packed, scale, zero, _ = ops.w4a16_quantize(w, GROUP)
                 mods.append((packed, ops.w4a16_prepare(scale, zero, k)))
                 del w
-            _lib.load().mp_set_programmatic_launch(1 if args.suite_pdl else 0)
+            lib, error_word = _lib.load(), ops._error_word(dev).data_ptr()
+            lib.mp_set_programmatic_launch(1 if args.suite_pdl else 0)
             for m in [int(v) for v in args.decode_m.split(",")]:
                 x = synth.normal_activation(m, k, seed=0).to(dev)
                 y = torch.empty((m, n), dtype=torch.float16, device=dev)
-                ws_dec = ops.new_workspace(max(ops.w4a16_decode_workspace_bytes(m, n, k), 20 << 20), dev)
-                ws_pre = ops.new_workspace(_lib.load().mp_w4a16_prefill_workspace_bytes(m, n, k), dev) if m > 16 else None
-                # 17..64 rows: what ops.w4a16_linear does -- the tcgen05 weight-streaming kernel with a 32/64-token
-                # tile where the library's rule picks it (or when asked for), else the split-K tensor-core GEMM
-                wide_umma = 16 < m <= 64 and (args.decode_kernel == "umma" or (
-                    args.decode_kernel in ("default", "auto") and ops.w4a16_decode_kernel_choice(m, n, k) == "umma"))
-                opt_umma = ops.decode_options(kernel="umma")
+                nbytes = lib.mp_w4a16_linear_workspace_bytes(m, n, k, GROUP)
+                ws = ops.new_workspace(nbytes, dev) if nbytes else None
 
                 def call(pk, sz):
-                    if m <= 16:
-                        ops.w4a16_linear_decode(x, pk, sz, workspace=ws_dec, out=y)
-                    elif wide_umma:             # the tcgen05 weight-streaming kernel with a 32/64-token tile
-                        ops.w4a16_linear_decode(x, pk, sz, workspace=ws_dec, out=y, options=opt_umma)
-                    else:                       # above 16 rows ops.w4a16_linear takes the split-K tensor-core GEMM
-                        ops.w4a16_linear_prefill(x, pk, sz, workspace=ws_pre)
+                    # what the module's forward calls, with buffers of the bench's own (the chain is captured)
+                    status = lib.mp_w4a16_linear(x.data_ptr(), pk.data_ptr(), sz.data_ptr(), None, y.data_ptr(), m, n, k, GROUP,
+                                                 None if ws is None else ws.data_ptr(), nbytes, error_word,
+                                                 torch.cuda.current_stream().cuda_stream)
+                    _lib.check(status, "w4a16_linear")
                 g = torch.cuda.CUDAGraph()
                 for pk, sz in mods:
                     call(pk, sz)
@@ -968,7 +964,7 @@ def run_suite(args, local_rank, collect=None):
                 b = w4a16_bytes(n, k, m)
                 emit(suite="w4a16_decode", N=n, K=k, M=m, us=t * 1e6, gbs=b / t / 1e9,
                      frac_of_measured_hbm=b / t / 1e9 / peaks["hbm_gbs"],
-                     kernel=args.decode_kernel if m <= 16 else ("umma" if wide_umma else "gemm"),
+                     kernel="auto" if args.decode_kernel == "default" else args.decode_kernel,
                      **({"pdl": 1} if args.suite_pdl else {}))
             _lib.load().mp_set_programmatic_launch(0)
             del mods
@@ -999,7 +995,8 @@ def run_suite(args, local_rank, collect=None):
                      tflops=2 * m * n * k / t / 1e12)
             del mods
     if "midm" in want or "all" in want:
-        # the W8A8 linear (per-token quant + int8 GEMM) at decode / small-batch row counts
+        # the W8A8 operators one after the other (per-token quant, int8 GEMM) at decode / small-batch row counts: the
+        # stages of the runtime's op interface.  SmoothQuantLinear's forward is one call, mp_w8a8_linear.
         for (n, k) in [(4096, 4096), (14336, 4096), (4096, 14336)]:
             copies = max(2, int(300e6 // (n * k)) + 1)
             ws_ = []
@@ -1089,7 +1086,7 @@ def main():
     ap.add_argument("--suite", default="", help="comma list of extra per-kernel lines: decode,prefill,w8a8,moe,all")
     ap.add_argument("--suite-only", action="store_true", help="skip the headline workload")
     ap.add_argument("--decode-kernel", default="default", choices=["default", "auto", "umma", "mma_sync"],
-                    help="kernel behind the M <= 16 decode linears (default: the library's default)")
+                    help="process-wide kernel choice for the W4A16 linears (default: the library's, by shape)")
     ap.add_argument("--decode-m", default="1,16", help="token counts of the decode suite")
     ap.add_argument("--suite-pdl", type=int, default=0,
                     help="decode suite: launch the chain with programmatic dependent launch (adds \"pdl\": 1 to the line)")
