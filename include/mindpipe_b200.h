@@ -91,10 +91,12 @@ int mp_w4a16_linear_decode(const void* x_f16, const void* packed_i32, const void
                            const void* bias_f16, void* y_f16, int M, int N, int K, int group,
                            void* workspace, size_t workspace_bytes, mp_stream_t stream);
 /*
- * Same, with the K split chosen by the caller.  k_split == 0 is automatic: for
- * M <= 16 a thread-block-cluster kernel that reduces the K split through
- * distributed shared memory and touches no workspace; otherwise (M > 16, or
- * an explicit k_split >= 1) the workspace kernel.
+ * Same, with the K split chosen by the caller.  k_split == 0 is automatic: the
+ * kernel of mp_set_decode_kernel's choice.  For M <= 16 that is the ring kernel,
+ * which reduces its K split through distributed shared memory and touches no
+ * workspace, or the tcgen05 kernel, which keeps partial tiles there; for M > 16
+ * the tcgen05 kernel or the split-K workspace kernel.  An explicit k_split >= 1
+ * is always the split-K workspace kernel.
  */
 int mp_w4a16_linear_decode_ex(const void* x_f16, const void* packed_i32, const void* sz_f16x2,
                               const void* bias_f16, void* y_f16, int M, int N, int K, int group,
@@ -156,8 +158,8 @@ int mp_w4a16_linear_decode_host_ws(const void* x_host_f16, void* x_stage_f16, co
 /*
  * Several independent host-buffer linears on one stream in one call (the q/k/v or gate/up projections of a
  * decoder layer, which read the same activations and do not depend on one another): all H2D copies are enqueued
- * first, then the kernels back to back -- so that, with mp_set_programmatic_launch(1), each one fetches its weights
- * while its predecessor drains -- then the D2H copies.  Every field means what the argument of the same name
+ * first, then the kernels back to back -- each is set up beside its predecessor's tail and, with
+ * mp_set_programmatic_launch(1), already fetches its weights there -- then the D2H copies.  Every field means what the argument of the same name
  * means in mp_w4a16_linear_decode_host_ws; the entries must not share staging buffers or workspaces.  The call
  * stops at the first entry that fails and returns its status.
  */
@@ -195,7 +197,8 @@ int mp_host_buffer_device_alias(const void* host_ptr, size_t bytes, void** devic
 
 /*
  * The linear for any number of rows: the decode kernels, the tcgen05 weight-streaming kernel (up to 96 rows) or the
- * prefill GEMM below, whichever is fastest for the shape (with mp_set_decode_kernel set: as that says).  The forward of
+ * prefill GEMM below, whichever is fastest for the shape (its own rule, not that of the decode entries; with
+ * mp_set_decode_kernel set to one kernel: as that says).  The forward of
  * VllmPackedInt4Linear (exporters/vllm.py:85-86) in one call.  The workspace is one for all shapes, under the rules of
  * mp_w4a16_linear_decode: zero-filled when it is created, left ready for the next call, shared only by calls that cannot
  * overlap on the device; it may also be shared with the decode entries.  Without one the scratch-free kernels run.  Shapes
@@ -217,12 +220,12 @@ int mp_w4a16_linear_prefill(const void* x_f16, const void* packed_i32, const voi
                             const void* bias_f16, void* y_f16, int M, int N, int K, int group,
                             int* error_word, mp_stream_t stream);
 /*
- * Same, with scratch for split tiles: where whole tiles would leave CTA pairs
- * idle, every pair gets an equal run of the tiles' K steps; the fp32 partial
- * tiles of those cut in between go to `workspace` and a second kernel
- * adds them in K order (deterministic).  mp_w4a16_prefill_workspace_bytes
- * returns the size needed (0 = no split for this shape); a null workspace
- * means no split.
+ * Same, with scratch for split tiles.  The product is cut into whole tiles,
+ * into tiles shared by clusters of CTA pairs (sums exchanged in shared memory;
+ * both need no scratch) or, only with a workspace, into equal runs of K steps
+ * per pair, whose fp32 partial tiles go to `workspace` and are added in K order
+ * by a second kernel; all three are deterministic.  mp_w4a16_prefill_workspace_bytes
+ * returns the size a non-null workspace must have (0: none is used).
  */
 size_t mp_w4a16_prefill_workspace_bytes(int M, int N, int K);
 int mp_w4a16_linear_prefill_ex(const void* x_f16, const void* packed_i32, const void* sz_f16x2,
@@ -267,11 +270,13 @@ int mp_w4a16_linear_decode_static(const void* x_f16, const void* packed_i32, con
 int mp_set_programmatic_launch(int enabled);
 
 /*
- * The process-wide DEFAULT kernel behind the decode linears for M <= 16 (returns
+ * The process-wide DEFAULT kernel behind the decode linears (returns
  * the previous choice, or MP_ERR_INVALID_ARG); a call that must not depend on
  * what another host in the process has set passes its choice in the options of
  * mp_w4a16_linear_decode_opts instead.  Both compute F.linear(x, Wdq) of
- * awq/quantize/quantizer.py:109-130 with fp32 accumulation:
+ * awq/quantize/quantizer.py:109-130 with fp32 accumulation (with groups of a
+ * multiple of 128 the first up to 16 rows, the second up to 8, apply the scale to
+ * the group's sum in fp32, i.e. without the fp16 rounding of Wdq's elements):
  *   MP_DECODE_KERNEL_UMMA      tcgen05.mma with the dequantised weights as the
  *                              tensor-memory operand (a thread expands one
  *                              weight row and stores it with tcgen05.st)
@@ -280,7 +285,9 @@ int mp_set_programmatic_launch(int enabled);
  *   MP_DECODE_KERNEL_AUTO      (default) the tcgen05 kernel for 9..16 tokens on
  *                              weights of at least 40 MiB packed with at least
  *                              16384 output rows when a workspace was passed,
- *                              the mma.sync kernel otherwise
+ *                              the mma.sync kernel otherwise (17..64 rows: see
+ *                              mp_w4a16_decode_kernel_choice; mp_w4a16_linear
+ *                              chooses by a rule of its own)
  * The tcgen05 kernel divides the (row block, K stage) pairs evenly over a
  * persistent grid and needs the workspace of mp_w4a16_decode_workspace_bytes
  * (zero-filled when created, left ready for the next call, not shared by calls
@@ -296,8 +303,8 @@ int mp_set_decode_kernel(int kind);
  * (1 <= M <= 64), with or without a workspace; shapes the chosen kernel does not take still fall through.  For
  * 17..64 rows _UMMA means the tcgen05 kernel with a 32- or 64-token activation tile (by default up to 32 rows
  * on >= 24 MiB of packed weights with >= 8192 output rows, up to 64 rows on >= 40 MiB with >= 16384), and
- * _MMA_SYNC that mp_w4a16_linear_decode would run its split-K kernel -- a caller then does better with
- * mp_w4a16_linear_prefill, the tensor-core GEMM. */
+ * _MMA_SYNC that mp_w4a16_linear_decode would run its split-K kernel.  mp_w4a16_linear has a rule of its own, which
+ * sends 17..96 rows to the tcgen05 kernel and never to the split-K one, which is up to ten times slower there. */
 int mp_w4a16_decode_kernel_choice(int M, int N, int K, int have_workspace);
 
 /*

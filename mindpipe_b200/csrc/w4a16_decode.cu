@@ -1,5 +1,8 @@
-// W4A16 decode-shaped linear (M <= 64): y = x @ dequant(W)^T, streaming the
-// packed weights once at HBM rate.
+// W4A16 decode-shaped linear (M <= 64): y = x @ dequant(W)^T, the packed weights
+// streamed through registers; and, at the end, the dispatch among all W4A16 kernels.
+//
+// The register-streaming kernel runs for explicit K splits, behind the entry without
+// scratch, and where the decode entries' default sends 17..64 rows (see below).
 //
 // Work split: a block owns ROWS_PER_BLOCK output rows and one slice of K; its
 // warps are arranged WN (rows) x 4 (K).  A warp step covers 32 rows x 128
@@ -46,25 +49,28 @@ size_t w4a16_gemm_partial_bytes(int M, int N, int K);   // w4a16_gemm.cu
 // chosen one does not take fall through to the next.
 static int g_decode_kernel = MP_DECODE_KERNEL_AUTO;
 
-// AUTO: the tcgen05 kernel for 9 to 16 tokens (below that the mma.sync kernel's folded scales are cheaper
-// still) on weights of at least 40 MiB packed with at least 128 row blocks -- the shapes where the mma.sync
-// kernel cannot cut K without a second wave and stream-K's even split pays (28672x8192, M = 16: 43.9 vs
-// 52.2 us; 22016x4096: 23.4 vs 26.3 us, and 66.1 vs 69.4 us per 7B layer set when the fused gate/up
-// projection alone takes it).  With fewer row blocks the mma.sync kernel's one-wave cluster split is as
-// fast or faster (8192x28672: 45.1 vs 46.3 us; 8192x8192: 16.2 vs 21.9 us; 12288x4096 inside the layer
-// set: 71.1 us per set when it also goes to the tcgen05 kernel).
+// AUTO, for the decode entries only: the tcgen05 kernel for 9 to 16 tokens on weights of at least 40 MiB packed with at
+// least 128 row blocks.  This is the default that include/mindpipe_b200.h states, so it stays what it was; it is not where
+// the two kernels cross.  The linear does not use it (linear_kernel() below), and a caller of the decode entries who wants
+// the faster kernel outside the line names it in the call's options.  Chains of launches, us, mma.sync ring / tcgen05 kernel:
+//   inside, 16 tokens     28672x8192 49.5 / 30.0, 22016x4096 26.2 / 15.9
+//   outside, 16 tokens    8192x28672 42.6 / 30.0, 8192x8192 16.9 / 13.3, 12288x4096 17.8 / 11.5, 4096x11008 14.5 / 11.6,
+//                         4096x4096 7.2 / 6.5, 1024x8192 7.5 / 6.7
+//   outside, 8 tokens     28672x8192 34.3 / 28.6, 22016x4096 19.2 / 15.3, 8192x28672 30.3 / 28.5, 12288x4096 13.1 / 11.3,
+//                         8192x8192 12.0 / 12.7, 4096x11008 10.2 / 11.1, 4096x4096 6.8 / 6.1
 static int decode_kernel_for(int kind, int M, int N, int K, bool have_workspace) {
   if (kind != MP_DECODE_KERNEL_AUTO) return kind;
   if (have_workspace && M > 8 && N >= 16384 && (size_t)N * (size_t)K / 2 >= (size_t)40 << 20) return MP_DECODE_KERNEL_UMMA;
   return MP_DECODE_KERNEL_MMA_SYNC;
 }
 
-// 17..64 rows: the tcgen05 kernel with a 32- or 64-token activation tile streams the weights once, where the
-// register-streaming kernel re-reads its activations per chunk; taken when the call names it.
-// AUTO (measured against the split-K tensor-core GEMM, chains under programmatic dependent launch): up to 32
-// rows on at least 24 MiB of packed weights with at least 8192 output rows (28672x8192: 54 vs 98 us, 22016x4096:
-// 31 vs 53, 8192x28672: 58 vs 90, 12288x4096: 24 vs 26; 4096x11008 loses 35 vs 24), and 33..64 rows on the
-// 70B-sized weights of the M <= 16 rule (28672x8192: 83 vs 98, 22016x4096: 47 vs 53; 8192x8192 loses 53 vs 33).
+// The same for 17..64 rows, where the other side is the register-streaming kernel below, which re-reads its activations per
+// chunk: the tcgen05 kernel when the call names it, else the stated default -- up to 32 rows on at least 24 MiB of packed
+// weights with at least 8192 output rows, 33..64 rows on the 70B-sized weights of the line above.  Again not where they
+// cross: the tcgen05 kernel is the faster one everywhere (us, register-streaming / tcgen05).
+//   inside    28672x8192 148 / 35 at 32 rows, 409 / 43 at 64; 8192x28672 169 / 35 at 32; 12288x4096 46 / 13 at 32
+//   outside   8192x28672 399 / 42 at 64, 8192x8192 129 / 16 at 64, 12288x4096 113 / 14 at 64, 4096x11008 47 / 13 at 32 and
+//             104 / 16 at 64, 4096x4096 30 / 8 at 32 and 61 / 10 at 64, 1024x8192 17 / 9 at 32 and 34 / 12 at 64
 static bool umma_above_16_rows(int kind, int M, int N, int K) {
   if (kind == MP_DECODE_KERNEL_UMMA) return true;
   if (kind != MP_DECODE_KERNEL_AUTO) return false;
@@ -533,7 +539,7 @@ extern "C" size_t mp_w4a16_decode_workspace_bytes_ex(int M, int N, int K, int k_
   const DecodePlan pl = plan_decode(M, N, K, k_split);
   const size_t split_k = kPartialOffset + (size_t)pl.k_split * (size_t)M * (size_t)N * sizeof(float);
   if (k_split <= 0 && g_decode_kernel != MP_DECODE_KERNEL_MMA_SYNC && decode_umma_workspace_bytes(M, K) > split_k)
-    return decode_umma_workspace_bytes(M, K);   // 17..64 rows may take the tcgen05 kernel with a wider activation tile
+    return decode_umma_workspace_bytes(M, K);   // 17..64 rows: whichever of the two kernels the call names
   return split_k;
 }
 

@@ -1,5 +1,5 @@
-// W4A16 linear for up to 128 rows (the dispatch sends more than 96 elsewhere where it can) on the tcgen05 tensor core with the weights as the TENSOR-MEMORY operand:
-// y = x @ dequant(W)^T, the packed weights streamed once.
+// W4A16 linear for up to 128 rows (the linear's dispatch sends more than 96 to the GEMM, which takes no groups of 32) on the
+// tcgen05 tensor core with the weights as the TENSOR-MEMORY operand: y = x @ dequant(W)^T, the packed weights streamed once.
 //
 // A thread owns ONE weight row: it reads 16 bytes (32 codes) of its row from the shared-memory ring, expands them and
 // stores the packed registers straight into tensor memory (tcgen05.st, lane = row, column = pair of K).  One elected

@@ -17,8 +17,11 @@
 //   warp 20      TMA producer of the packed words (256 columns a stage)
 //   warp 21      MMA issuer (the even CTA's)
 //   warp 22      TMA producer of the activations (128 columns a step)
-// Work is cut into (tile, step) units, and with scratch every pair gets an equal run of them: a tile whose run ends in
-// between is left as fp32 partial tiles, which a second kernel adds in K order.  Without scratch pairs take whole tiles.
+// Work is cut in one of three ways, whichever an estimate of clocks says is shortest (see w4_gemm_shape): whole tiles to a
+// pair; a tile shared by a cluster of two or four pairs, each with its part of K, which exchange their sums through
+// distributed shared memory; or, with scratch, an equal run of all tiles' steps to every pair, the tiles cut in between left
+// as fp32 partial tiles that a second kernel adds in K order.  Whole tiles and clusters are the usual ones; equal runs win
+// where K is long beside few tiles that do not fill the pairs (97 rows of 1024 x 28672, 300 rows of 8192 x 28672).
 //
 // Measured (us, groups of 128; in brackets the form it replaces, expanded weights as the B operand in shared memory):
 // 12288 x 4096 at 129 / 333 / 512 / 2048 rows 22.0 / 35.8 / 42.1 / 155.8 [40.8 / 59.7 / 59.6 / 171.6], 4096 x 11008 at

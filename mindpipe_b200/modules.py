@@ -9,7 +9,14 @@ names, but hold integer weights and run the sm_100a kernels:
   group scales and, for the asymmetric format AWQ's ``pseudo_quantize_tensor``
   defines (algorithm/quantization/ptq/awq/source/awq/quantize/quantizer.py:
   63-105), a packed zero-point buffer.  Its results are those of the
-  reference's W4A16 forward, ``F.linear(x, pseudo_quantize_tensor(W))``.
+  reference's W4A16 forward, ``F.linear(x, pseudo_quantize_tensor(W))``, with
+  fp32 sums -- exactly so (to summation order) above 16 rows.  Up to 16 rows and
+  with groups of a multiple of 128 columns most shapes multiply the integers
+  ``u - z`` and apply the scale to a group's sum in fp32: the product of the
+  weights before their rounding to fp16, which differs from the reference's by
+  that rounding alone, about 3e-4 relative.  So a token's bits may differ between a batch of up to 16 and one of
+  more rows (and, on weights below 2 MiB packed or 2048 output rows, between 8
+  and 9), as they may with any change of the order of summation.
 """
 from __future__ import annotations
 

@@ -59,8 +59,8 @@ def w4a16_decode_workspace_bytes(m: int, n: int, k: int, k_split: int = 0) -> in
 
 
 def w4a16_decode_kernel_choice(m: int, n: int, k: int, have_workspace: bool = True) -> str:
-    """Name of the kernel the process default picks for a decode call of this shape (1 <= m <= 64); above 16 rows
-    ``"mma_sync"`` means the split-K kernel, which the tensor-core GEMM (``w4a16_linear_prefill``) beats."""
+    """Name of the kernel the process default picks for a call of :func:`w4a16_linear_decode` of this shape
+    (1 <= m <= 64); above 16 rows ``"mma_sync"`` means the split-K kernel.  :func:`w4a16_linear` has a rule of its own."""
     kind = _lib.load().mp_w4a16_decode_kernel_choice(m, n, k, 1 if have_workspace else 0)
     _lib.check(min(kind, 0), "w4a16_decode_kernel_choice", M=m, N=n, K=k)
     return {0: "mma_sync", 1: "umma"}[kind]
@@ -132,8 +132,8 @@ def decode_options(kernel: str | None = None, pdl: bool | None = None) -> int:
 
 def w4a16_linear_decode(x, weight_packed, scale_zero, bias=None, *, k_split: int = 0, workspace=None, out=None,
                         options: int = 0):
-    """``y[M,N] = x[M,K] @ dequant(W)^T (+bias)`` with the weight-streaming kernels (M <= 64; meant for
-    M <= 16 -- above that ``w4a16_linear`` prefers the split-K tensor-core GEMM).
+    """``y[M,N] = x[M,K] @ dequant(W)^T (+bias)`` with the weight-streaming kernels (M <= 64), for callers who choose
+    kernel, split or scratch themselves; :func:`w4a16_linear` picks the fastest kernel for the shape.
 
     ``workspace`` (uint8, zero-filled when created, not shared by calls that
     may overlap) defaults to a cached buffer per device and stream.  ``options``
@@ -271,7 +271,7 @@ def w4a16_linear_prefill(x, weight_packed, scale_zero, bias=None, *, workspace=N
 
 def w4a16_linear(x, weight_packed, scale_zero, bias=None):
     """W4A16 linear for any number of rows: the library picks among the decode kernels, the tcgen05 weight-streaming
-    kernel (up to 128 rows) and the tensor-core prefill kernel (``mp_w4a16_linear``).  Shapes the prefill kernel does
+    kernel (up to 96 rows) and the tensor-core prefill kernel (``mp_w4a16_linear``).  Shapes the prefill kernel does
     not take (K or the group size not a multiple of 64) are processed by the decode kernels in 64-row slabs.
     """
     x2 = _req(x, "x", torch.float16, 2)
@@ -322,10 +322,10 @@ _DECODE_KERNELS = {"mma_sync": 0, "umma": 1, "auto": 2}
 
 
 def set_decode_kernel(kind: str) -> str:
-    """Choose the kernel behind the decode linears for M <= 16; returns the previous choice.
+    """Choose the kernel behind the W4A16 linears of few rows; returns the previous choice.
 
     ``"umma"``: tcgen05.mma with the dequantised weights as the tensor-memory operand;
-    ``"mma_sync"``: the mma.sync ring kernel; ``"auto"`` (the default): by shape.  Shapes the
+    ``"mma_sync"``: the mma.sync kernels; ``"auto"`` (the default): by shape.  Shapes the
     chosen kernel does not take fall through to the other ones.  This is the process-wide default;
     a single call chooses with ``options=decode_options(kernel=...)``.
     """
