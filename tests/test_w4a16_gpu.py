@@ -395,10 +395,11 @@ def test_prefill_cfg2_m2048_row_sample(n, k):
 @pytest.mark.parametrize("m,n,k", [(17, 256, 2048), (65, 256, 2048), (128, 512, 4096), (200, 1024, 1024),
                                    (256, 4096, 4096), (512, 1024, 2048), (700, 512, 1024)])
 def test_prefill_split_k_small_batches(m, n, k):
-    """Few output tiles: K is cut into slices (fp32 partial tiles + an ordered sum).  Same result as the
-    unsplit kernel to fp32 summation order, run-to-run identical, and within tolerance of the oracle."""
+    """Few output tiles: narrow ones, or tiles shared by clusters of CTA pairs (equal runs of K steps with partial tiles:
+    test_w4a16_linear_scratch.py).  Same result without scratch to fp32 summation order, run-to-run identical, and
+    within tolerance of the oracle."""
     from mindpipe_b200 import _lib, ops
-    assert _lib.load().mp_w4a16_prefill_workspace_bytes(m, n, k) > 0          # these shapes do split
+    assert _lib.load().mp_w4a16_prefill_workspace_bytes(m, n, k) > 0          # fewer tiles than CTA pairs
     w = synth.normal_weight(n, k, seed=m, index=0).cuda()
     packed, scale, zero, _ = ops.w4a16_quantize(w, 128)
     sz = ops.w4a16_prepare(scale, zero, k)
@@ -410,7 +411,7 @@ def test_prefill_split_k_small_batches(m, n, k):
     wdq = ops.w4a16_dequant(packed, scale, zero, n, k).float()
     ref = x.float() @ wdq.T + bias.float()
     assert ((y.float() - ref).norm() / ref.norm()).item() <= TOL
-    # a null workspace turns the split off: one K slice per tile, same math
+    # without a workspace, same math
     y1 = torch.empty_like(y)
     st = _lib.load().mp_w4a16_linear_prefill(x.data_ptr(), packed.data_ptr(), sz.data_ptr(), bias.data_ptr(),
                                              y1.data_ptr(), m, n, k, 128, ops._error_word(x.device).data_ptr(),

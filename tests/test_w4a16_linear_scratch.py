@@ -99,3 +99,22 @@ def test_only_equal_runs_ask_for_room(m, n, k, runs):
     ref = x.double() @ mod.dequantize().double().T
     assert ((y.double() - ref).norm() / ref.norm()).item() <= 4e-4
     ops.check_device_errors()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,group", [(18, 260, 8256, 64), (101, 260, 12352, 64), (149, 1500, 20544, 64),
+                                         (311, 260, 12416, 128)])
+def test_equal_runs_at_ragged_edges(m, n, k, group):
+    """Tiles cut between pairs, their partial tiles added by the second kernel: edges of M, N and K inside a tile."""
+    mod = _module(n, k, group)
+    mod._ensure_prepared()
+    assert _lib.load().mp_w4a16_linear_workspace_bytes(m, n, k, group) > 0
+    wdq = mod.dequantize().double()
+    bias = torch.randn(n, device="cuda").half()
+    x = torch.randn(m, k, device="cuda").half()
+    for b in (None, bias):
+        y = ops.w4a16_linear(x, mod.weight_packed, mod._scale_zero, b)
+        ref = x.double() @ wdq.T + (0 if b is None else b.double())
+        assert ((y.double() - ref).norm() / ref.norm()).item() <= 4e-4
+        assert torch.equal(y, ops.w4a16_linear(x, mod.weight_packed, mod._scale_zero, b))
+    ops.check_device_errors()
