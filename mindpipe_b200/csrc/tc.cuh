@@ -23,6 +23,11 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   return t;
 }
 
+// This thread's warp within the block, as a value that the compiler knows to be the same in the whole warp.  A role chosen by
+// it keeps its descriptors and addresses in uniform registers; chosen by threadIdx.x >> 5 alone, every operand of a
+// tcgen05.mma or a TMA copy is moved there first (an MMA of 16 tokens issued every 47 clocks instead of 9).
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x) >> 5, 0); }
+
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(

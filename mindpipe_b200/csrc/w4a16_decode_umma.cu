@@ -1,21 +1,21 @@
 // W4A16 linear for up to 128 rows (the linear's dispatch sends more than 96 to the GEMM, which takes no groups of 32) on the
 // tcgen05 tensor core with the weights as the TENSOR-MEMORY operand: y = x @ dequant(W)^T, the packed weights streamed once.
 //
-// A thread owns ONE weight row: it reads 16 bytes (32 codes) of its row from the shared-memory ring, expands them and
-// stores the packed registers straight into tensor memory (tcgen05.st, lane = row, column = pair of K).  One elected
+// A thread owns ONE weight row: it reads its row of a stage from the shared-memory ring, expands it and stores the packed
+// registers straight into tensor memory (tcgen05.st, lane = row, column = pair of K).  One elected
 // thread then issues tcgen05.mma kind::f16 with A = those TMEM columns (128 rows x 16 K per instruction), B = the
 // activation tile in shared memory (token rows, K-major, 128-byte swizzle) and the fp32 accumulator [128 rows x tokens]
 // in TMEM.  No dequantised weight touches shared or global memory, and no dequant warp issues an MMA, shuffles a fragment
 // or touches an activation.
 //
 // What bounds it (clocks per 16 KB stage of weights and SM; HBM delivers one in about 700):
-//   expansion   exact f16((u - z) * s): 660 (thirteen instructions per eight weights, most of them half rate);
-//               FOLD, the exact integers u - z with the group's scale applied to its dot product: 460
-//   MMA         16 instructions of N / 2 clocks (operand A in tensor memory): 154 at 16 tokens, 517 at 64
-//   producer    one thread per stream, about 200 clocks per iteration plus 60 per TMA instruction: weights and
-//               activations have a thread each and no division in their loops (with both streams in one thread, seven
-//               TMA instructions and two divisions per stage, this thread was what held the kernel at 0.45 of HBM)
-// so every role has its own warps and its own barriers, and none waits for another that is not its input.
+//   expansion   alone, twelve warps: exact f16((u - z) * s) in order 750 (17 instructions per eight weights, nine of them half
+//               rate); FOLD, the exact integers u - z with the group's scale applied to its dot product, 460, of which the
+//               stores to tensor memory are 230.  Four warps, one on each scheduler, take 540, eight 480.
+//   MMA         16 instructions of N / 2 clocks (operand A in tensor memory): 154 at 16 tokens, 768 at 96
+//   producer    one thread per stream, weights and activations, with no division in their loops (with both streams in one
+//               thread this was what held the kernel at 0.45 of HBM)
+// every role has its own warps and its own barriers, and none waits for another that is not its input.
 //
 // FOLD (up to 16 rows, groups of a multiple of 128 columns): the accumulator of every 128-column unit is read back by
 // the epilogue warps, which add scale * dot to fp32 registers: more accurate than the fp16-rounded f16((u - z) * s) and
@@ -29,7 +29,8 @@
 // order (results are identical from run to run).  A tile word is stored inverted and zero means "not there yet": the
 // reader polls the words themselves (bounded) and puts the zeros back, with no fence, counter or second round trip.
 //
-//   warps 0-15   expansion: two sets of eight take stages in turn; a warp does 32 rows of half a stage
+//   warps 0-15   expansion: two sets of eight take stages in turn, a warp does 32 rows of half a stage (see Cfg::kParts); at
+//                the end they fetch the tiles of the row block that this block closes
 //   warps 16-19  epilogue
 //   warp 20      TMA producer of weights and (scale, zero) pairs
 //   warp 21      TMEM allocation and the MMA issuer
@@ -40,8 +41,12 @@
 // of their own for the permutation were starved by the expansion warps: 2100 clocks per stage with one.)
 // One block fills an SM: its ring is what hides HBM's latency.  Smaller blocks, two of them to an SM so that the next linear
 // of a chain starts beside the end of this one, took 38 us where this takes 28 (28672x8192, 16 rows).
-// A launch of 12288x4096 at 16 rows, 12 us: 2.7 from the end of the kernel before to the first stage's data (all SMs ask at
-// once), 0.7 its expansion, 4.7 the stream, 2 the exchange of partial tiles, the rest launch and exit.
+// What a launch costs beyond the stream: 1.3 us from the end of the kernel before to the first MMA, 1.3 from the last MMA to the
+// last block's end.  The first was 2.1 to 2.9 with the whole ring requested before the activations, which then queued behind
+// it, and the (scale, zero) pairs not brought to L2 with the weights; the second 2 to 2.6, and 5 at 77 rows, with the tiles
+// read, an element at a time, after the last MMA.  Measured without early weights (us; in brackets that form): 12288x4096 at 16
+// rows 9.4 [11.5], 10240x8192 at 8 12.0 [14.4], 28672x8192 at 8 25.6 [28.5], 12288x4096 at 77 13.6 [16.2].  Streaming the
+// same bytes with nothing done to them takes 5.0, 8.0, 19.0 and 5.0.
 // Every wait is bounded.
 #include "common.cuh"
 #include "tc.cuh"
@@ -53,16 +58,22 @@ using namespace tc;
 namespace du {
 constexpr int kRows = 128;
 constexpr int kStageK = 256;
-constexpr int kSets = 2;                              // expansion sets of eight warps, a stage each in turn
 constexpr int kSlots = 3;                             // stages between expansion and MMA: stage i is in slot i % 3
-constexpr int kEpiWarp0 = 8 * kSets;
-constexpr int kWeightWarp = kEpiWarp0 + 4, kMmaWarp = kWeightWarp + 1, kXWarp = kMmaWarp + 1;
-constexpr int kThreads = 32 * (kXWarp + 1);
 constexpr int kWBytes = kRows * (kStageK / 2);        // 16384
 constexpr int kMaxRing = 10, kMaxXRing = 8;
+// Weight stages requested before the activations, which queue behind them: with early weights the time up to the wait for
+// the kernel before is theirs (12288x4096 at 16 rows in a chain, us: 4 or 5 stages 9.2, 6 9.5, the whole ring 10.1).
+constexpr int kFirstEarly = 5, kFirst = 1;
+// Stages brought to L2 while the kernel before ends.  A prefetch and the load after it cost L2 more than the load alone, so
+// more of them slow a short stream, fewer a long one (us without early weights, 3 / 6 / 10 stages: 12288x4096 at 16 rows 9.5 /
+// 9.6 / 10.1, 28672x8192 at 8 27.1 / 26.7 / 26.5; 10.5 and 26.7 without the (scale, zero) pairs beside the weights).
+constexpr int kPrefetch = 4;
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kASlotCols = 128;                  // 256 columns of K, two per 32-bit register
+constexpr uint32_t kASlotCols = kStageK / 2;          // two columns of K per 32-bit register
 constexpr size_t kSmemMax = 224 * 1024;
+
+template <int N>
+struct Int { static constexpr int value = N; };
 
 // TOK: token rows of the MMA (its N); XROWS: token rows of the activation tile in shared memory (8 where no more exist:
 // the MMA then reads whatever follows for the other eight, whose results are not used)
@@ -71,7 +82,18 @@ struct Cfg {
   // the columns of an expanded word come out as (k0,k4) (k1,k5) ..: the activations are put into that order, in shared
   // memory, or (PERM false) the words back into theirs.  Permuting the activations of 64 tokens per block and stage cost the
   // expansion warps a third of their time, permuting them in a kernel of its own 2 us a call.
+  static constexpr int kTokens = XROWS;               // that can exist
   static constexpr bool PERM = TOK <= 16;
+  // Warps that share 32 rows of a stage.  Two, in two sets, have a stage expanded soonest; where a stage costs both the exact
+  // products and the permutation, one to a stage in three sets spends less on barriers (us without early weights, halves /
+  // whole stages: 28672x8192 at 8 rows 25.6 / 28.1, 10240x8192 12.0 / 13.8, 4096x4096 at 48 8.5 / 9.5; groups of 64:
+  // 8192x28672 at 9 rows 40.1 / 34.9).
+  static constexpr int kParts = PERM && !FOLD ? 1 : 2;
+  static constexpr int kSets = kParts == 1 ? 3 : 2;       // expansion sets, a stage each in turn
+  static constexpr int kPieces = 8 / kParts;              // 16-byte pieces of a row that a warp does
+  static constexpr int kEpiWarp0 = 4 * kParts * kSets;
+  static constexpr int kWeightWarp = kEpiWarp0 + 4, kMmaWarp = kWeightWarp + 1, kXWarp = kMmaWarp + 1;
+  static constexpr int kThreads = 32 * (kXWarp + 1);
   static constexpr int kXSub = XROWS * 128;           // [XROWS x 64 columns] fp16
   static constexpr int kXBytes = (PERM ? 4 : 2) * kXSub;        // a tile of the ring: a stage, or half of one
   // activation tiles in flight: enough to hide the latency of their loads behind the stages before (with one per slot the
@@ -113,6 +135,7 @@ struct DecodeUmmaParams {
   int groups_per_stage;    // rows of the (scale, zero) box
   int gshift;              // log2(group) for groups of up to 128 columns
   int ring;                // weight stages in the ring
+  int first;               // weight stages requested before the activations, at most `ring`
   int early_weights;       // 1: fetch weights before the previous kernel of the stream has finished
   uint32_t* tiles;         // workspace: [grid][TOK][128] inverted fp32 words, zero between calls
   int* error_word;
@@ -145,13 +168,13 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[8]) {
 
 // D[tmem] (+)= A[tmem] * B[smem]: the A operand is read from tensor memory (lane = row, one 32-bit
 // column = two consecutive K elements), 16 K per instruction.
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
-                                            uint32_t accumulate) {
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t desc_lo, uint32_t desc_hi,
+                                            uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .b64 b;\n\t.reg .pred p;\n\tmov.b64 b, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "r"(desc_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
@@ -216,7 +239,7 @@ __device__ __forceinline__ void expand8(uint32_t q, __half2 zl, __half2 zh, uint
 }
 
 template <int TOK, int XROWS, bool FOLD>
-__global__ void __launch_bounds__(du::kThreads, 1)
+__global__ void __launch_bounds__(du::Cfg<TOK, XROWS, FOLD>::kThreads, 1)
 w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                          const __grid_constant__ CUtensorMap tmap_sz, const DecodeUmmaParams p) {
   using C = du::Cfg<TOK, XROWS, FOLD>;
@@ -232,50 +255,58 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
   uint32_t* tmem_slot = s_scale + du::kScaleWords;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const uint32_t xring = smem_u32(base), wring = xring + kXRing * kXBytes;
-  const uint32_t full0 = smem_u32(bars);                      // a stage's weights (PERM: and activations) landed
+  const uint32_t full0 = smem_u32(bars);                      // a stage's weights landed
   const uint32_t empty0 = full0 + 8 * du::kMaxRing;           // its weights have been read
   const uint32_t xempty0 = empty0 + 8 * du::kMaxRing;         // activation tile has been read
-  const uint32_t xfull0 = xempty0 + 8 * du::kMaxXRing;        // not PERM: activation tile landed
+  const uint32_t xfull0 = xempty0 + 8 * du::kMaxXRing;        // activation tile landed
   const uint32_t ready0 = xfull0 + 8 * du::kMaxXRing;         // slot holds an expanded stage (FOLD: and its accumulators are free)
   const uint32_t done0 = ready0 + 8 * du::kSlots;             // its MMAs are complete
   const uint32_t dfull0 = done0 + 8 * du::kSlots;             // not FOLD: a segment's accumulator is complete
   const uint32_t dempty0 = dfull0 + 16;                       // ... and has been read
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int blk = static_cast<int>(blockIdx.x);
   const int ST = p.stages_per_row;
   const int t_lo = range_start(blk, p), t_hi = range_start(blk + 1, p) - 1;   // walked from t_hi down
   const int n_stages = t_hi - t_lo + 1;
 
+  // whether the block's last segment ends a row block that earlier blocks began, whose tiles it then adds (see the expansion)
+  const int rb_lo = t_lo / ST;
+  const bool closes = t_lo > rb_lo * ST && t_hi >= rb_lo * ST + ST - 1;
+  constexpr int kExpThreads = 32 * C::kEpiWarp0;
+  constexpr int kMine = (C::kTokens * (du::kRows / 4) + kExpThreads - 1) / kExpThreads;     // elements of an expansion thread
+  float others[kMine][4];
+
   // weight producer: the stage it is at (its first loads are issued before the block is set up)
   int w_row = 0, w_st = 0;
+  auto group_of = [&](int st) { return p.group <= du::kStageK ? st * p.groups_per_stage : (st * du::kStageK) / p.group; };
   auto load_weights = [&](int s) {
     const uint32_t full = full0 + 8 * s, dst = wring + s * stage_bytes;
     mbar_arrive_expect_tx(full, du::kWBytes + p.groups_per_stage * du::kRows * 4);
     tma_load_2d(dst, &tmap_w, full, w_st * (du::kStageK / 2), w_row);
-    const int group = p.group <= du::kStageK ? w_st * p.groups_per_stage : (w_st * du::kStageK) / p.group;
-    tma_load_2d(dst + du::kWBytes, &tmap_sz, full, w_row, group);
+    tma_load_2d(dst + du::kWBytes, &tmap_sz, full, w_row, group_of(w_st));
     if (--w_st < 0) { w_st = ST - 1; w_row -= du::kRows; }
   };
-  if (warp == du::kWeightWarp) {
+  if (warp == C::kWeightWarp) {
     if (elect_one()) {
       for (int s = 0; s < p.ring; ++s) {
-        mbar_init(full0 + 8 * s, PERM ? 2 : 1);               // the producers
-        mbar_init(empty0 + 8 * s, 8);
+        mbar_init(full0 + 8 * s, 1);
+        mbar_init(empty0 + 8 * s, 4 * C::kParts);
       }
       fence_mbar_init();
       w_row = (t_hi / ST) * du::kRows;
       w_st = t_hi % ST;
       if (!p.early_weights) {
-        for (int s = 0, row = w_row, st = w_st; s < p.ring && s < n_stages; ++s) {     // to L2 while the kernel before ends
+        for (int s = 0, row = w_row, st = w_st; s < du::kPrefetch && s < n_stages; ++s) {     // to L2 while the kernel before ends
+          tma_prefetch_2d(&tmap_sz, row, group_of(st));
           tma_prefetch_2d(&tmap_w, st * (du::kStageK / 2), row);
           if (--st < 0) { st = ST - 1; row -= du::kRows; }
         }
         chain_wait();
       }
-      for (int s = 0; s < p.ring && s < n_stages; ++s) load_weights(s);
+      for (int s = 0; s < p.first && s < n_stages; ++s) load_weights(s);
     }
-  } else if (warp == du::kXWarp) {
+  } else if (warp == C::kXWarp) {
     if (elect_one()) {
       prefetch_tensormap(&tmap_x);
       for (int s = 0; s < kXRing; ++s) {
@@ -283,7 +314,7 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
         mbar_init(xfull0 + 8 * s, 1);
       }
       for (int q = 0; q < du::kSlots; ++q) {
-        mbar_init(ready0 + 8 * q, FOLD ? 12 : 8);
+        mbar_init(ready0 + 8 * q, 4 * C::kParts + (FOLD ? 4 : 0));
         mbar_init(done0 + 8 * q, 1);
       }
       for (int d = 0; d < 2; ++d) {
@@ -293,7 +324,7 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
       *abort_flag = 0;
       fence_mbar_init();
     }
-  } else if (warp == du::kMmaWarp) {
+  } else if (warp == C::kMmaWarp) {
     tmem_alloc(smem_u32(tmem_slot), du::kTmemCols);
     tmem_relinquish();
   }
@@ -303,39 +334,39 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == du::kWeightWarp) {
+  if (warp == C::kWeightWarp) {
     // ------------------------------------------------------------ TMA producer: weights
     if (elect_one()) {
-      int s = 0;
-      uint32_t phase = 0;
-      for (int i = p.ring; i < n_stages; ++i) {
+      chain_wait();                // (early weights: the activations come before the rest of the ring)
+      int s = p.first;
+      uint32_t phase = 1;
+      if (s == p.ring) { s = 0; phase = 0; }
+      for (int i = p.first; i < n_stages; ++i) {
         if (!mbar_wait(empty0 + 8 * s, phase, abort_flag)) break;
         load_weights(s);
         if (++s == p.ring) { s = 0; phase ^= 1; }
       }
       chain_release();             // all of this block's loads are issued: the next kernel's blocks may start
     }
-  } else if (warp == du::kXWarp) {
+  } else if (warp == C::kXWarp) {
     // ------------------------------------------------------------ TMA producer: activations
     if (elect_one()) {
       chain_wait();
-      int st = t_hi % ST, s = 0, xs = 0;
+      int st = t_hi % ST, xs = 0;
       uint32_t phase = 1;
       bool ok = true;
       for (int i = 0; ok && i < n_stages; ++i) {
 #pragma unroll
         for (int h = 0; h < (PERM ? 1 : 2); ++h) {
           if (!mbar_wait(xempty0 + 8 * xs, phase, abort_flag)) { ok = false; break; }
-          const uint32_t bar = PERM ? full0 + 8 * s : xfull0 + 8 * xs;
-          mbar_arrive_expect_tx(bar, kXBytes);
-          tma_load_3d(xring + xs * kXBytes, &tmap_x, bar, 0, 0, st * (du::kStageK / 64) + h * 2);
+          mbar_arrive_expect_tx(xfull0 + 8 * xs, kXBytes);
+          tma_load_3d(xring + xs * kXBytes, &tmap_x, xfull0 + 8 * xs, 0, 0, st * (du::kStageK / 64) + h * 2);
           if (++xs == kXRing) { xs = 0; phase ^= 1; }
         }
         if (--st < 0) st = ST - 1;
-        if (++s == p.ring) s = 0;
       }
     }
-  } else if (warp == du::kMmaWarp) {
+  } else if (warp == C::kMmaWarp) {
     // ------------------------------------------------------------ MMA issuer: one wait, 16 MMAs, one commit per stage
     if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc(kIdescDFormatF32 | kIdescABFormatF16, du::kRows, TOK);
@@ -344,6 +375,7 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
       uint32_t phase = 0, xphase = 0, dphase = 1;
       bool ok = true;
       const uint64_t b_desc0 = umma_desc_k_sw128(xring);
+      const uint32_t desc_hi = static_cast<uint32_t>(b_desc0 >> 32), desc_lo0 = static_cast<uint32_t>(b_desc0);
       for (int i = 0; i < n_stages; ++i) {
         if (!FOLD && fresh && !mbar_wait(dempty0 + 8 * d, dphase, abort_flag)) break;
         if (!mbar_wait(ready0 + 8 * q, phase, abort_flag)) break;
@@ -352,13 +384,12 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           if (!PERM && !mbar_wait(xfull0 + 8 * xs, xphase, abort_flag)) { ok = false; break; }
-          const uint64_t b_desc = b_desc0 + ((xs * kXBytes + (PERM ? h * 2 * kXSub : 0)) >> 4);
+          const uint32_t d_tmem = tmem_base + (FOLD ? 2 * q + h : d) * TOK;
+          const uint32_t desc = desc_lo0 + ((xs * kXBytes + (PERM ? h * 2 * kXSub : 0)) >> 4);
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {     // 16 K per instruction: 8 TMEM columns of A, 32 bytes of B's rows
-            const uint32_t d_tmem = tmem_base + (FOLD ? 2 * q + h : d) * TOK;
-            umma_f16_ts(d_tmem, a_tmem + (h * 8 + kk) * 8, b_desc + ((kk >> 2) * kXSub >> 4) + 2 * (kk & 3), idesc,
+          for (int kk = 0; kk < 8; ++kk)       // 16 K per instruction: 8 TMEM columns of A, 32 bytes of B's rows
+            umma_f16_ts(d_tmem, a_tmem + (h * 8 + kk) * 8, desc + ((kk >> 2) * kXSub >> 4) + 2 * (kk & 3), desc_hi, idesc,
                         FOLD ? kk != 0 : !(fresh && h == 0 && kk == 0));
-          }
           if (!PERM || h == 1) {
             umma_commit(xempty0 + 8 * xs);
             if (++xs == kXRing) { xs = 0; xphase ^= 1; }
@@ -375,49 +406,53 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
         if (++q == du::kSlots) { q = 0; phase ^= 1; }
       }
     }
-  } else if (warp < du::kEpiWarp0) {
-    // ------------------------------------------------------------ expansion: a warp does 32 rows of half a stage
-    const int quarter = warp & 3, h = (warp >> 2) & 1, set = warp >> 3;
-    const int row = quarter * 32 + lane, sw = row & 7;
-    const uint32_t a_tmem0 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::kASlot0 + h * (du::kASlotCols / 2);
+  } else if (warp < C::kEpiWarp0) {
+    // ------------------------------------------------------------ expansion: a warp does 32 rows of a stage, or half of it
+    constexpr int kPieces = C::kPieces;
+    const int quarter = warp & 3, part = C::kParts == 1 ? 0 : (warp >> 2) & 1, set = warp / (4 * C::kParts);
+    const int row = quarter * 32 + lane;
+    const uint32_t a_tmem0 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::kASlot0 + part * kPieces * 16;
+    const uint32_t lane_w = row * 128 + ((row & 7) << 4);      // a swizzled row's 16-byte pieces are at lane_w ^ (piece << 4)
+    const uint32_t scale0 = smem_u32(s_scale + row);
+    const uint32_t sz_lane = du::kWBytes + row * 4;
     int s = set, xs = set, q = set;
-    uint32_t phase = 0, qphase = 1, parity = 0;
-    for (int i = set; i < n_stages; i += du::kSets) {
+    uint32_t phase = 0, xphase = 0, use = 0;
+    for (int i = set; i < n_stages; i += C::kSets) {
       if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, phase, abort_flag))) break;
-      const uint32_t stage = wring + s * stage_bytes + row * 128, sz = wring + s * stage_bytes + du::kWBytes + row * 4;
-      uint4 q4[4];
+      const uint32_t stage = wring + s * stage_bytes, src = (stage + lane_w) ^ (part * kPieces * 16), sz = stage + sz_lane;
+      uint4 q4[kPieces];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) q4[j] = du_lds_v4(stage + (((h * 4 + j) ^ sw) << 4));
-      uint32_t szw[FOLD ? 1 : 4];
-      if constexpr (FOLD) {
-        szw[0] = du_lds_u32(sz + (p.groups_per_stage > 1 ? h * (du::kRows * 4) : 0));
-      } else {
+      for (int j = 0; j < kPieces; ++j) q4[j] = du_lds_v4(src ^ (j << 4));
+      constexpr int kScales = FOLD ? kPieces / 4 : kPieces;    // one for 128 columns or one for 32
+      uint32_t szw[kScales];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          szw[j] = du_lds_u32(sz + (p.groups_per_stage > 1 ? ((h * 128 + j * 32) >> p.gshift) * (du::kRows * 4) : 0));
-      }
-      // (the slot's use before its last one is over: the activations of stage i were requested after the MMAs of stage
-      // i - kXRing >= i - 6, so the parity is not ambiguous)
-      if (!__all_sync(0xffffffffu, mbar_wait(done0 + 8 * q, qphase, abort_flag))) break;
+      for (int j = 0; j < kScales; ++j)
+        szw[j] = du_lds_u32(sz + (p.groups_per_stage > 1 ? ((part * 128 + j * (FOLD ? 128 : 32)) >> p.gshift) * (du::kRows * 4) : 0));
+      // (the slot's use before its last one is over: this warp has waited for the MMAs of a stage at most six before this
+      // one, and they complete in order, so the parity is not ambiguous)
+      if (!__all_sync(0xffffffffu, mbar_wait(done0 + 8 * q, use ^ 1, abort_flag))) break;
       mbar_arrive_warp(empty0 + 8 * s, lane);
       tcgen05_fence_after();
       const uint32_t a_tmem = a_tmem0 + q * du::kASlotCols;
       if constexpr (FOLD) {
-        du_sts_u32(smem_u32(s_scale + ((q * 2 + parity) * 2 + h) * du::kRows + row), szw[0]);
-        const __half2 z2 = __high2half2(*reinterpret_cast<const __half2*>(&szw[0]));
-        const __half2 zl = __hadd2(z2, __float2half2_rn(1024.0f)), zh = __hadd2(z2, __float2half2_rn(64.0f));
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint32_t r[16];
-          expand8(q4[j].x, zl, zh, r);
-          expand8(q4[j].y, zl, zh, r + 4);
-          expand8(q4[j].z, zl, zh, r + 8);
-          expand8(q4[j].w, zl, zh, r + 12);
-          tmem_st_32x32_x16(a_tmem + j * 16, r);
+        for (int h = 0; h < kScales; ++h) {
+          du_sts_u32(scale0 + ((q * 2 + use) * 2 + part + h) * (du::kRows * 4), szw[h]);
+          const __half2 z2 = __high2half2(*reinterpret_cast<const __half2*>(&szw[h]));
+          const __half2 zl = __hadd2(z2, __float2half2_rn(1024.0f)), zh = __hadd2(z2, __float2half2_rn(64.0f));
+#pragma unroll
+          for (int j = 4 * h; j < 4 * h + 4; ++j) {
+            uint32_t r[16];
+            expand8(q4[j].x, zl, zh, r);
+            expand8(q4[j].y, zl, zh, r + 4);
+            expand8(q4[j].z, zl, zh, r + 8);
+            expand8(q4[j].w, zl, zh, r + 12);
+            tmem_st_32x32_x16(a_tmem + j * 16, r);
+          }
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < kPieces; ++j) {
           const __half2 szh = *reinterpret_cast<const __half2*>(&szw[j]);
           const ScaleZero sp = make_scale_zero(__low2half(szh), __high2half(szh));
           uint32_t r[16];
@@ -434,27 +469,85 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
         }
       }
       if constexpr (PERM) {
-        // this half's activations: chunks of XROWS tokens x 128 columns
-        const uint32_t xt = xring + xs * kXBytes + h * (2 * kXSub) + row * 16;
+        // this warp's share of the stage's activations: chunks of XROWS tokens x 256 columns
+        if (!__all_sync(0xffffffffu, mbar_wait(xfull0 + 8 * xs, xphase, abort_flag))) break;
+        constexpr int kChunks = kXBytes / 2048 / C::kParts;
+        const uint32_t xt = xring + xs * kXBytes + part * (kXBytes / C::kParts) + row * 16;
+        uint4 v[kChunks];
 #pragma unroll
-        for (int c0 = 0; c0 < 2 * kXSub; c0 += 4096) {
-          constexpr int kAtOnce = 2 * kXSub < 4096 ? kXSub / 1024 : 2;
-          uint4 v[kAtOnce];
+        for (int j = 0; j < kChunks; ++j) v[j] = du_lds_v4(xt + j * 2048);
 #pragma unroll
-          for (int j = 0; j < kAtOnce; ++j) v[j] = du_lds_v4(xt + c0 + j * 2048);
-#pragma unroll
-          for (int j = 0; j < kAtOnce; ++j) du_sts_v4(xt + c0 + j * 2048, pair_permute_u4(v[j]));
-        }
-        fence_proxy_async_smem();                                // generic-proxy stores -> visible to the MMA's reads
+        for (int j = 0; j < kChunks; ++j) du_sts_v4(xt + j * 2048, pair_permute_u4(v[j]));
+        fence_proxy_async_smem();                                  // generic-proxy stores -> visible to the MMA's reads
       }
       tmem_st_wait();
       tcgen05_fence_before();
       mbar_arrive_warp(ready0 + 8 * q, lane);
-      s += du::kSets;
+      s += C::kSets;
       if (s >= p.ring) { s -= p.ring; phase ^= 1; }
-      if (PERM && (xs += du::kSets) >= kXRing) xs -= kXRing;
-      q += du::kSets;
-      if (q >= du::kSlots) { q -= du::kSlots; qphase ^= 1; parity ^= 1; }
+      if (PERM && (xs += C::kSets) >= kXRing) { xs -= kXRing; xphase ^= 1; }
+      q += C::kSets;
+      if (q >= du::kSlots) { q -= du::kSlots; use ^= 1; }
+    }
+    // The sums of the tiles that this block closes, fetched while the last MMAs and the epilogue run: four rows of a token to
+    // an element, ELEMENTS elements of TILES tiles requested together.
+    auto fetch = [&](auto elements, auto tiles) {
+      constexpr int ELEMENTS = decltype(elements)::value, TILES = decltype(tiles)::value;
+      const int first_block = block_of(rb_lo * ST, p);
+      uint32_t* tile0 = p.tiles + (size_t)first_block * TOK * du::kRows + tid * 4;
+      for (int b2 = first_block; b2 < blk && !*abort_flag; b2 += TILES, tile0 += (size_t)TILES * TOK * du::kRows) {
+        uint4 w[ELEMENTS][TILES];
+        uint64_t since = 0;
+        for (uint32_t it = 1;; ++it) {
+          bool there = true;
+#pragma unroll
+          for (int k = 0; k < ELEMENTS; ++k)
+#pragma unroll
+            for (int j = 0; j < TILES; ++j)
+              w[k][j] = b2 + j < blk && tid + k * kExpThreads < p.M * (du::kRows / 4)
+                            ? ld_relaxed_gpu_v4(tile0 + (size_t)j * TOK * du::kRows + k * kExpThreads * 4)
+                            : make_uint4(1u, 1u, 1u, 1u);
+#pragma unroll
+          for (int k = 0; k < ELEMENTS; ++k)
+#pragma unroll
+            for (int j = 0; j < TILES; ++j)
+              there = there && w[k][j].x != 0u && w[k][j].y != 0u && w[k][j].z != 0u && w[k][j].w != 0u;
+          if (there) break;
+          if ((it & 0x3F) == 0) {
+            const uint64_t now = globaltimer_ns();
+            if (since == 0) since = now;
+            if (now - since > kWaitLimitNs) *abort_flag = 1;
+            if (*abort_flag) break;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < ELEMENTS; ++k)
+#pragma unroll
+          for (int j = 0; j < TILES; ++j)
+            if (b2 + j < blk && tid + k * kExpThreads < p.M * (du::kRows / 4)) {
+              others[k][0] += __uint_as_float(~w[k][j].x);
+              others[k][1] += __uint_as_float(~w[k][j].y);
+              others[k][2] += __uint_as_float(~w[k][j].z);
+              others[k][3] += __uint_as_float(~w[k][j].w);
+              st_relaxed_gpu_v4_zero(tile0 + (size_t)j * TOK * du::kRows + k * kExpThreads * 4);       // ready for the next call
+            }
+      }
+    };
+    if (closes) {
+      chain_wait();       // (with more than 16 rows nothing that this warp waited for came after it) the tiles are this call's
+#pragma unroll
+      for (int k = 0; k < kMine; ++k)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) others[k][i] = 0.0f;
+      // as many requests as registers hold
+      const int mine = (p.M * (du::kRows / 4) + kExpThreads - 1) / kExpThreads;
+      if (kMine <= 3 || mine <= 3) {
+        fetch(du::Int<kMine < 3 ? kMine : 3>{}, du::Int<4>{});
+      } else if (mine <= 4) {
+        fetch(du::Int<kMine < 4 ? kMine : 4>{}, du::Int<2>{});
+      } else {
+        fetch(du::Int<kMine>{}, du::Int<1>{});
+      }
     }
   } else {
     // ------------------------------------------------------------ epilogue: lane = weight row, column = token
@@ -547,58 +640,23 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
 
   tcgen05_fence_before();
   __syncthreads();
-  {
-    // The closing step, all threads: when the block's last segment ends a row block that earlier blocks began, add their
-    // tiles to this block's sums.  Four rows of a token per thread; the words of up to four blocks are requested together.
-    const int rb = t_lo / ST, row_first = rb * ST;
-    if (t_lo > row_first && t_hi >= row_first + ST - 1 && !*abort_flag) {
-      const int first_block = block_of(row_first, p);
-      for (int e = tid; e < p.M * (du::kRows / 4); e += du::kThreads) {
-        const int m = e / (du::kRows / 4), r4 = (e % (du::kRows / 4)) * 4;
-        const uint4 own = du_lds_v4(wring + (m * du::kRows + r4) * 4);
-        float v[4] = {__uint_as_float(own.x), __uint_as_float(own.y), __uint_as_float(own.z), __uint_as_float(own.w)};
-        uint32_t* tile = p.tiles + ((size_t)first_block * TOK + m) * du::kRows + r4;
-        for (int b2 = first_block; b2 < blk && !*abort_flag; b2 += 4, tile += (size_t)4 * TOK * du::kRows) {
-          uint4 w[4];
-          uint64_t since = 0;
-          for (uint32_t it = 1;; ++it) {
-            bool there = true;
+  // The closing step: when the block's last segment ends a row block that earlier blocks began, their sums and this block's.
+  if (closes && warp < C::kEpiWarp0 && !*abort_flag) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              w[j] = b2 + j < blk ? ld_relaxed_gpu_v4(tile + (size_t)j * TOK * du::kRows) : make_uint4(1u, 1u, 1u, 1u);
-              there = there && w[j].x != 0u && w[j].y != 0u && w[j].z != 0u && w[j].w != 0u;
-            }
-            if (there) break;
-            if ((it & 0x3F) == 0) {
-              const uint64_t now = globaltimer_ns();
-              if (since == 0) since = now;
-              if (now - since > kWaitLimitNs) *abort_flag = 1;
-              if (*abort_flag) break;
-            }
-          }
+    for (int k = 0; k < kMine; ++k) {
+      const int e = tid + k * kExpThreads, m = e / (du::kRows / 4), r4 = (e % (du::kRows / 4)) * 4, n = rb_lo * du::kRows + r4;
+      if (m >= p.M || n >= p.N) continue;                      // N is a multiple of four
+      const uint4 own = du_lds_v4(wring + (m * du::kRows + r4) * 4);
+      float v[4] = {__uint_as_float(own.x) + others[k][0], __uint_as_float(own.y) + others[k][1],
+                    __uint_as_float(own.z) + others[k][2], __uint_as_float(own.w) + others[k][3]};
+      if (p.bias) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (b2 + j < blk) {
-              v[0] += __uint_as_float(~w[j].x);
-              v[1] += __uint_as_float(~w[j].y);
-              v[2] += __uint_as_float(~w[j].z);
-              v[3] += __uint_as_float(~w[j].w);
-              st_relaxed_gpu_v4_zero(tile + (size_t)j * TOK * du::kRows);          // ready for the next call
-            }
-        }
-        const int n = rb * du::kRows + r4;                     // N is a multiple of four
-        if (n < p.N && !*abort_flag) {
-          if (p.bias) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) v[i] += h2f(p.bias[n + i]);
-          }
-          __half* y = p.y + (size_t)m * p.N + n;
-          *reinterpret_cast<__half2*>(y) = __floats2half2_rn(v[0], v[1]);
-          *reinterpret_cast<__half2*>(y + 2) = __floats2half2_rn(v[2], v[3]);
-        }
+        for (int i = 0; i < 4; ++i) v[i] += h2f(p.bias[n + i]);
       }
+      __half* y = p.y + (size_t)m * p.N + n;
+      *reinterpret_cast<__half2*>(y) = __floats2half2_rn(v[0], v[1]);
+      *reinterpret_cast<__half2*>(y + 2) = __floats2half2_rn(v[2], v[3]);
     }
-    __syncthreads();
   }
   if (*abort_flag) {
     if (tid == 0 && p.error_word) atomicExch(p.error_word, 4);
@@ -606,7 +664,7 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
     while (globaltimer_ns() - t_start < 200000ull) __nanosleep(1000);  // let copies and MMAs in flight land
     __syncthreads();
   }
-  if (warp == du::kMmaWarp) {
+  if (warp == C::kMmaWarp) {
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, du::kTmemCols);
   }
@@ -638,7 +696,9 @@ static int launch_umma(const CUtensorMap& tw, const CUtensorMap& tx, const CUten
   const size_t fixed = 1024 + (size_t)C::kXRing * C::kXBytes + du::kTailBytes;
   p.ring = (int)((du::kSmemMax - fixed) / stage);
   if (p.ring > du::kMaxRing) p.ring = du::kMaxRing;
-  return launch_chained(kern, dim3(grid), dim3(du::kThreads), fixed + (size_t)p.ring * stage, st, tw, tx, tsz, p);
+  p.first = p.early_weights ? du::kFirstEarly : du::kFirst;
+  if (p.first > p.ring) p.first = p.ring;
+  return launch_chained(kern, dim3(grid), dim3(C::kThreads), fixed + (size_t)p.ring * stage, st, tw, tx, tsz, p);
 }
 
 // Returns MP_ERR_UNSUPPORTED for shapes this kernel does not take (M > 128, K % 64 != 0, N % 4 != 0, groups
