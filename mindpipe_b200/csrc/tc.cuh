@@ -172,6 +172,11 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int crd0
                ::"l"(reinterpret_cast<uint64_t>(map)), "r"(crd0), "r"(crd1) : "memory");
 }
 
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int crd0, int crd1, int crd2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(crd0), "r"(crd1), "r"(crd2) : "memory");
+}
+
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }

@@ -323,6 +323,14 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
       }
       *abort_flag = 0;
       fence_mbar_init();
+      // The first activations on their way to L2, where they are already unless the kernel before did not write them (a 7B
+      // layer at 16 rows 43.3 -> 42.1 us; with more than 16 rows nothing).
+      if (PERM) {
+        for (int i = 0, st = t_hi % ST; i < 2 && i < n_stages; ++i) {
+          tma_prefetch_3d(&tmap_x, 0, 0, st * (du::kStageK / 64));
+          if (--st < 0) st = ST - 1;
+        }
+      }
     }
   } else if (warp == C::kMmaWarp) {
     tmem_alloc(smem_u32(tmem_slot), du::kTmemCols);

@@ -45,3 +45,31 @@ def test_linear_of_extreme_values(m):
     y = ops.w4a16_linear(x, packed, sz)
     assert y[m - 1].isnan().all() and not torch.isfinite(y[0]).any() and not y[1:m - 1].any()
     ops.check_device_errors()
+
+
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 64, 77, 96])
+@pytest.mark.parametrize("n,k", [(1024, 8192), (512, 2048), (4104, 4096)])
+def test_chained_launches_with_early_weights_share_scratch(n, k, m):
+    """Blocks of few stages that close a row block, behind a launch whose partial tiles lie in the same scratch: none may
+    take the other's.  The same bits as one launch at a time."""
+    cases = [_case(n, k, m, group)[:3] for group in (128, 64)]
+    want = [ops.w4a16_linear(*c) for c in cases]
+    lib = _lib.load()
+    before = lib.mp_set_programmatic_launch(1)
+    stream = torch.cuda.Stream()
+    try:
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            ops.w4a16_linear(*cases[0])
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            got = [ops.w4a16_linear(*cases[i % 2]) for i in range(8)]
+        for _ in range(10):
+            graph.replay()
+        torch.cuda.synchronize()
+    finally:
+        lib.mp_set_programmatic_launch(before)
+    ops.check_device_errors()
+    for i, y in enumerate(got):
+        assert torch.equal(y, want[i % 2])
