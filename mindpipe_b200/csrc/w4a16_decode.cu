@@ -42,7 +42,6 @@ int read_and_clear_decode_error(int* value);
 int launch_decode_umma(const void* x, const void* packed, const void* sz, const void* bias, void* y, int M, int N, int K,
                        int group, void* workspace, size_t workspace_bytes, cudaStream_t st, bool pdl);
 bool decode_umma_shape_ok(int M, int N, int K, int group);
-int decode_tma_cluster(int row_blocks, int stages);   // cluster size the ring kernel splits K over
 size_t decode_umma_workspace_bytes(int M, int K);
 size_t w4a16_gemm_partial_bytes(int M, int N, int K);   // w4a16_gemm.cu
 // Which kernel serves M <= 16 when a call does not say: one of the MP_DECODE_KERNEL_* values.  Shapes the
@@ -840,16 +839,13 @@ static LinearKernel linear_kernel(int M, int N, int K, int group) {
   // Above 96 rows the pair kernel expands less often for its tokens (4096x11008 at 97 / 128 rows: 23.7 / 26.0 vs 21.7 / 22.3
   // us; the other 7B shapes are level at 97 and a few per cent better at 128); it takes no groups of 32.
   if (M > 16) return M > 96 && group % 64 == 0 ? kGemm : kStream;
-  // 9..16 rows double the ring kernel's MMAs and cost the stream kernel nothing; below 2 MiB or 16 row blocks the stream
-  // kernel's longer pipeline shows (2048x2048: 4.3 vs 4.5 us, 2048x8192: 6.4 vs 8.9, 12288x4096: 10.4 vs 15.7)
-  if (M > 8) return packed >= ((size_t)2 << 20) && N >= 2048 ? kStream : kRing;
-  // Up to 8 rows the ring kernel's folded form is as fast where its grid is one full wave (8192x8192: 11.0 vs 11.2 us).
-  // Elsewhere the stream kernel's even split wins: grids of more than one wave (6144x4096: 6.3 vs 9.4 us, 12288x4096:
-  // 10.0 vs 11.2), grids that leave SMs empty (2048x8192: 5.5 vs 6.3) and long runs per block (8192x28672: 26 vs 29).
-  const int row_blocks = (N + 127) / 128, stages = (K + 255) / 256;
-  const int blocks = row_blocks * decode_tma_cluster(row_blocks, stages);
-  if (packed < ((size_t)4 << 20)) return kRing;
-  return blocks > 2 * kSmCount || blocks <= kSmCount || packed >= ((size_t)64 << 20) ? kStream : kRing;
+  // Below, the stream kernel but for small weights, where its longer pipeline shows.  us, ring / stream, without early weights:
+  // 9..16 rows, which double the ring kernel's MMAs: 2048x2048 4.8 / 4.1, 1024x4096 5.0 / 5.2, 2048x4096 6.4 / 5.5,
+  // 1024x8192 7.2 / 6.0, 12288x4096 18.5 / 9.4.
+  if (M > 8) return packed >= ((size_t)4 << 20) || (packed >= ((size_t)2 << 20) && N >= 2048) ? kStream : kRing;
+  // Up to 8: 1024x4096 4.2 / 4.8, 2048x4096 5.1 / 5.2, 4096x2048 5.5 / 4.5, 3072x4096 5.5 / 5.3, 8192x8192 11.8 / 10.5,
+  // 28672x4096 19.5 / 15.1.
+  return packed >= ((size_t)5 << 20) || (packed >= ((size_t)4 << 20) && N >= 4096) ? kStream : kRing;
 }
 
 extern "C" size_t mp_w4a16_linear_workspace_bytes(int M, int N, int K, int group) {

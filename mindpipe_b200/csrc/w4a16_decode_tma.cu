@@ -524,7 +524,7 @@ static int launch_tma(const CUtensorMap& tw, const CUtensorMap& tx, const CUtens
   return MP_OK;
 }
 
-int decode_tma_cluster(int row_blocks, int stages) {
+static int decode_tma_cluster(int row_blocks, int stages) {
   // K is cut over a cluster of ck blocks: the smallest power of two (<= 8, the portable limit) that puts
   // about two blocks on every SM ...
   constexpr int kSlots = 2 * kSmCount;
