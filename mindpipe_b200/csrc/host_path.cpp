@@ -42,10 +42,16 @@ std::map<std::tuple<int, cudaStream_t, int>, at::Tensor> g_workspaces;
 
 // A copy of the tensor handle: it keeps the buffer alive until the launch is in the stream even if another thread
 // replaces it by a larger one meanwhile (the allocator hands freed memory on in stream order).
-at::Tensor workspace(size_t nbytes, int device, cudaStream_t stream, int kind) {
+// own_in_capture: a capture on a stream that has none yet gets a zeroed buffer of the call's own, from the graph's memory
+// (decode steps are often captured on a stream of their own, and small linears of up to 16 rows can do without scratch; they
+// are not to fail there for the sake of a faster kernel).
+at::Tensor workspace(size_t nbytes, int device, cudaStream_t stream, int kind, bool own_in_capture = false) {
   std::lock_guard<std::mutex> lock(g_workspace_mutex);
   at::Tensor& ws = g_workspaces[std::make_tuple(device, stream, kind)];
   if (!ws.defined() || static_cast<size_t>(ws.numel()) < nbytes) {
+    if (own_in_capture && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
+      return at::zeros({static_cast<int64_t>(nbytes)},
+                       at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
     TORCH_CHECK(c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None,
                 "scratch memory would be allocated during CUDA graph capture; "
                 "pass a preallocated workspace= (see new_workspace)");
@@ -142,9 +148,9 @@ struct Scratch {
   at::Tensor hold;
   void* ptr = nullptr;
   size_t bytes = 0;
-  Scratch(size_t wanted, int device, cudaStream_t st, int kind) {
+  Scratch(size_t wanted, int device, cudaStream_t st, int kind, bool own_in_capture = false) {
     if (!wanted) return;
-    hold = workspace(wanted, device, st, kind);
+    hold = workspace(wanted, device, st, kind, own_in_capture);
     ptr = hold.data_ptr();
     bytes = static_cast<size_t>(hold.numel());
   }
@@ -163,7 +169,7 @@ struct W4Plan : Plan {
     const int m = static_cast<int>(rows);
     const cudaStream_t st = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream();
     at::Tensor y = output_like(x, n, at::kHalf);
-    Scratch ws(mp_w4a16_linear_workspace_bytes(m, n, k, group), device, st, kDecode);
+    Scratch ws(mp_w4a16_linear_workspace_bytes(m, n, k, group), device, st, kDecode, m <= 16);
     const int rc = mp_w4a16_linear(x.data_ptr(), packed.data_ptr(), scale_zero.data_ptr(), data_or_null(bias), y.data_ptr(),
                                    m, n, k, group, ws.ptr, ws.bytes, error_word, st);
     return rc == MP_OK ? THPVariable_Wrap(std::move(y)) : none();
@@ -461,13 +467,13 @@ PyObject* w4_dequant(PyObject*, PyObject* args) {
 PyObject* py_workspace(PyObject*, PyObject* args) {
   HANDLE_TH_ERRORS
   unsigned long long nbytes;
-  int device;
+  int device, own_in_capture = 0;
   const char* name;
-  if (!PyArg_ParseTuple(args, "Kis", &nbytes, &device, &name)) return nullptr;
+  if (!PyArg_ParseTuple(args, "Kis|p", &nbytes, &device, &name, &own_in_capture)) return nullptr;
   for (int kind = 0; kind < kKinds; ++kind)
     if (std::string(name) == kKindNames[kind]) {
       const cudaStream_t st = c10::cuda::getCurrentCUDAStream().stream();
-      return THPVariable_Wrap(workspace(static_cast<size_t>(nbytes), device, st, kind));
+      return THPVariable_Wrap(workspace(static_cast<size_t>(nbytes), device, st, kind, own_in_capture != 0));
     }
   PyErr_Format(PyExc_ValueError, "unknown workspace kind %s", name);
   return nullptr;

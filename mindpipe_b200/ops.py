@@ -38,15 +38,17 @@ def _ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
-def _workspace(nbytes: int, device: torch.device, kind: str = "decode") -> torch.Tensor:
+def _workspace(nbytes: int, device: torch.device, kind: str = "decode", own_in_capture: bool = False) -> torch.Tensor:
     """Zero-initialised scratch, one per (device, stream, kind), grown on demand (``csrc/host_path.cpp`` keeps it).
 
     The decode kernels leave their part zeroed where it has to be, so it is
     cleared only when it is (re)allocated; the prefill and W8A8 split-K partial
-    sums overwrite theirs freely, hence the separate kinds.
+    sums overwrite theirs freely, hence the separate kinds.  With ``own_in_capture``
+    a graph capture on a stream that has none gets a zeroed buffer of its own from
+    the graph's memory instead of an error.
     """
     index = device.index if device.index is not None else torch.cuda.current_device()
-    return _lib.host().workspace(nbytes, index, kind)
+    return _lib.host().workspace(nbytes, index, kind, own_in_capture)
 
 
 def new_workspace(nbytes: int, device) -> torch.Tensor:
@@ -292,7 +294,7 @@ def w4a16_linear(x, weight_packed, scale_zero, bias=None):
     y = torch.empty((m, n), dtype=torch.float16, device=x2.device)
     lib = _lib.load()
     nbytes = lib.mp_w4a16_linear_workspace_bytes(m, n, k, group)
-    ws = _workspace(nbytes, x2.device) if nbytes else None
+    ws = _workspace(nbytes, x2.device, own_in_capture=m <= 16) if nbytes else None
     st = lib.mp_w4a16_linear(x2.data_ptr(), p.data_ptr(), sz.data_ptr(), _ptr(b), y.data_ptr(), m, n, k, group, _ptr(ws),
                              0 if ws is None else ws.numel(), _error_word(x2.device).data_ptr(), _stream())
     _lib.check(st, "w4a16_linear", M=m, N=n, K=k, group=group)

@@ -73,3 +73,20 @@ def test_chained_launches_with_early_weights_share_scratch(n, k, m):
     ops.check_device_errors()
     for i, y in enumerate(got):
         assert torch.equal(y, want[i % 2])
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 4096, 4096), (8, 8192, 8192), (16, 1024, 8192), (16, 12288, 4096)])
+def test_capture_on_a_stream_without_scratch(m, n, k):
+    """Up to 16 rows a capture needs no call on its stream before; the graph then brings zeroed scratch of its own."""
+    x, packed, sz, bias, _ = _case(n, k, m, 128)
+    want = ops.w4a16_linear(x, packed, sz, bias)
+    stream = torch.cuda.Stream()                           # (kept: another stream might get its handle and find scratch)
+    stream.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        got = [ops.w4a16_linear(x, packed, sz, bias) for _ in range(3)]
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    ops.check_device_errors()
+    assert all(torch.equal(y, want) for y in got)
