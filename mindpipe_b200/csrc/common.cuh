@@ -34,6 +34,42 @@ constexpr int kSmCount = 148;  // B200
 constexpr size_t kW4CounterBytes = 16384;                       // room for 4096 row blocks
 constexpr size_t kW4TileBytes = (size_t)kSmCount * 128 * 512;   // a tile of 128 tokens x 128 rows fp32 per block
 
+// Copies between page-locked host memory and the device in one launch, in pieces of 16 bytes (host_pipeline.cu): of a kernel's
+// own, or taken along by a product.
+constexpr int kMaxHostCopies = 16;
+struct HostCopies {
+  const uint4* src[kMaxHostCopies];
+  uint4* dst[kMaxHostCopies];
+  int end[kMaxHostCopies];     // running count of pieces
+  int count;
+};
+
+#ifdef __CUDACC__
+// Thread `i0` of `step` copies its pieces, four in flight.  Host memory is written again between calls, so loads from it
+// bypass the caches.
+__device__ __forceinline__ void copy_pieces(const HostCopies& list, int i0, int step, bool from_host) {
+  const int total = list.end[list.count - 1];
+  for (; i0 < total; i0 += 4 * step) {
+    uint4 v[4];
+    uint4* to[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int i = i0 + j * step;
+      to[j] = nullptr;
+      if (i >= total) continue;
+      int e = 0;
+      while (i >= list.end[e]) ++e;
+      const int at = i - (e ? list.end[e - 1] : 0);
+      v[j] = from_host ? __ldcv(list.src[e] + at) : __ldcg(list.src[e] + at);
+      to[j] = list.dst[e] + at;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (to[j]) *to[j] = v[j];
+  }
+}
+#endif
+
 // ---- programmatic dependent launch for chains of short kernels -------------
 // launch_chained() lets a kernel be scheduled while the previous kernel of the stream is still running; the kernel
 // itself waits for that kernel's results with chain_wait() before it reads or writes anything the stream ordered, so

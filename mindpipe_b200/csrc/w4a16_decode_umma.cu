@@ -35,6 +35,7 @@
 //   warp 20      TMA producer of weights and (scale, zero) pairs
 //   warp 21      TMEM allocation and the MMA issuer
 //   warp 22      TMA producer of activations
+//   warp 23      copies from host memory, where the call brings some
 // Expansion emits the columns of a packed word in the order (k0,k4,k1,k5,k2,k6,k3,k7).  Up to 16 rows the expansion warps
 // apply the same permutation in place to the 16-byte chunks of the stage's activation tile (a chunk is one token's eight
 // columns of one word, so the swizzle does not matter); with more rows they put the words back in order, see Cfg.  (Warps
@@ -93,7 +94,8 @@ struct Cfg {
   static constexpr int kPieces = 8 / kParts;              // 16-byte pieces of a row that a warp does
   static constexpr int kEpiWarp0 = 4 * kParts * kSets;
   static constexpr int kWeightWarp = kEpiWarp0 + 4, kMmaWarp = kWeightWarp + 1, kXWarp = kMmaWarp + 1;
-  static constexpr int kThreads = 32 * (kXWarp + 1);
+  static constexpr int kSideWarp = kXWarp + 1;
+  static constexpr int kThreads = 32 * (kSideWarp + 1);
   static constexpr int kXSub = XROWS * 128;           // [XROWS x 64 columns] fp16
   static constexpr int kXBytes = (PERM ? 4 : 2) * kXSub;        // a tile of the ring: a stage, or half of one
   // activation tiles in flight: enough to hide the latency of their loads behind the stages before (with one per slot the
@@ -137,6 +139,7 @@ struct DecodeUmmaParams {
   int ring;                // weight stages in the ring
   int first;               // weight stages requested before the activations, at most `ring`
   int early_weights;       // 1: fetch weights before the previous kernel of the stream has finished
+  HostCopies copies;       // from host memory, every block its share; count 0: none
   uint32_t* tiles;         // workspace: [grid][TOK][128] inverted fp32 words, zero between calls
   int* error_word;
 };
@@ -557,6 +560,12 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
         fetch(du::Int<kMine>{}, du::Int<1>{});
       }
     }
+  } else if (warp == C::kSideWarp) {
+    // ------------------------------------------------------------ copies: beside the product, which ends when they have ended
+    if (p.copies.count > 0) {
+      chain_wait();
+      copy_pieces(p.copies, blk * 32 + lane, static_cast<int>(gridDim.x) * 32, true);
+    }
   } else {
     // ------------------------------------------------------------ epilogue: lane = weight row, column = token
     constexpr int CH = FOLD ? XROWS : 16;                      // tokens held at a time
@@ -714,7 +723,8 @@ static int launch_umma(const CUtensorMap& tw, const CUtensorMap& tx, const CUten
 // caller then uses another kernel.  The workspace starts zeroed and is left ready for the next call;
 // calls that share it must not overlap on the GPU.
 int launch_decode_umma(const void* x, const void* packed, const void* sz, const void* bias, void* y, int M, int N, int K,
-                       int group, void* workspace, size_t workspace_bytes, cudaStream_t st, bool early_weights) {
+                       int group, void* workspace, size_t workspace_bytes, cudaStream_t st, bool early_weights,
+                       const HostCopies* copies) {
   if (!decode_umma_shape_ok(M, N, K, group)) return MP_ERR_UNSUPPORTED;
   const int tok = du::tokens_for(M);
   if (!workspace || workspace_bytes < du::workspace_bytes(M) || !aligned(workspace, 16)) return MP_ERR_UNSUPPORTED;
@@ -749,6 +759,7 @@ int launch_decode_umma(const void* x, const void* packed, const void* sz, const 
   p.groups_per_stage = gps;
   p.gshift = group == 32 ? 5 : group == 64 ? 6 : 7;
   p.early_weights = early_weights ? 1 : 0;
+  if (copies) p.copies = *copies;
   p.tiles = reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(workspace) + du::kTileOffset);
   int rc_err = MP_OK;
   p.error_word = decode_error_word_ptr(&rc_err);
