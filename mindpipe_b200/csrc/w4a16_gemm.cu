@@ -28,6 +28,9 @@
 // 129 / 2048 rows 23.5 / 142.4 [38.1 / 149.5].  With many rows the MMAs bound it (1050 clocks a step of 1024 at 256 tokens,
 // 5000 of 38000 a tile in the epilogue); below 160 rows the expansion warps (about 800 a step).
 //
+// With the warp's number a uniform value (uniform_warp, tc.cuh) the single-thread roles issue faster: the four linears of a
+// 7B layer at 100 / 200 / 333 rows 89.6 / 115.5 / 141.5 -> 87.2 / 112.9 / 139.8.
+//
 // Every mbarrier wait is bounded (tc.cuh); on a timeout the pair records an error word, lets its copies land, frees its
 // tensor memory and returns.
 #include <algorithm>
@@ -176,7 +179,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 8 * (2 * kMaxRing + 2 * kMaxSlots + 4));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank(), rank = cta & 1u, leader_cta = cta & ~1u;
   const bool leader = rank == 0;
   const int pair = static_cast<int>(blockIdx.x) >> 1, steps = p.steps, split = p.split;
