@@ -196,7 +196,7 @@ void mp_host_pipeline_destroy(void* pipeline);
 int mp_host_buffer_device_alias(const void* host_ptr, size_t bytes, void** device_ptr);
 
 /*
- * The linear for any number of rows: the decode kernels, the tcgen05 weight-streaming kernel (up to 96 rows) or the
+ * The linear for any number of rows: the decode kernels, the tcgen05 weight-streaming kernel (up to 128 rows) or the
  * prefill GEMM below, whichever is fastest for the shape (its own rule, not that of the decode entries; with
  * mp_set_decode_kernel set to one kernel: as that says).  The forward of
  * VllmPackedInt4Linear (exporters/vllm.py:85-86) in one call.  The workspace is one for all shapes, under the rules of

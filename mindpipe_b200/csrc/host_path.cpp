@@ -43,8 +43,8 @@ std::map<std::tuple<int, cudaStream_t, int>, at::Tensor> g_workspaces;
 // A copy of the tensor handle: it keeps the buffer alive until the launch is in the stream even if another thread
 // replaces it by a larger one meanwhile (the allocator hands freed memory on in stream order).
 // own_in_capture: a capture on a stream that has none yet gets a zeroed buffer of the call's own, from the graph's memory
-// (decode steps are often captured on a stream of their own, and small linears of up to 16 rows can do without scratch; they
-// are not to fail there for the sake of a faster kernel).
+// (decode steps are often captured on a stream of their own, and a linear that could do without scratch is not to fail there
+// for the sake of a faster kernel).
 at::Tensor workspace(size_t nbytes, int device, cudaStream_t stream, int kind, bool own_in_capture = false) {
   std::lock_guard<std::mutex> lock(g_workspace_mutex);
   at::Tensor& ws = g_workspaces[std::make_tuple(device, stream, kind)];
@@ -169,7 +169,7 @@ struct W4Plan : Plan {
     const int m = static_cast<int>(rows);
     const cudaStream_t st = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream();
     at::Tensor y = output_like(x, n, at::kHalf);
-    Scratch ws(mp_w4a16_linear_workspace_bytes(m, n, k, group), device, st, kDecode, m <= 16);
+    Scratch ws(mp_w4a16_linear_workspace_bytes(m, n, k, group), device, st, kDecode, true);
     const int rc = mp_w4a16_linear(x.data_ptr(), packed.data_ptr(), scale_zero.data_ptr(), data_or_null(bias), y.data_ptr(),
                                    m, n, k, group, ws.ptr, ws.bytes, error_word, st);
     return rc == MP_OK ? THPVariable_Wrap(std::move(y)) : none();

@@ -837,9 +837,16 @@ static LinearKernel linear_kernel(int M, int N, int K, int group) {
   if (g_decode_kernel == MP_DECODE_KERNEL_MMA_SYNC) return narrow;
   if (g_decode_kernel == MP_DECODE_KERNEL_UMMA) return M <= 64 ? kStream : kGemm;
   const size_t packed = (size_t)N * (size_t)K / 2;
-  // Above 96 rows the pair kernel expands less often for its tokens (4096x11008 at 97 / 128 rows: 23.7 / 26.0 vs 21.7 / 22.3
-  // us; the other 7B shapes are level at 97 and a few per cent better at 128); it takes no groups of 32.
-  if (M > 16) return M > 96 && group % 64 == 0 ? kGemm : kStream;
+  // Above 96 rows the pair kernel expands less often for its tokens and has no closing step, which the stream kernel makes up
+  // for by an even split, to 112 rows on all but small or narrow weights and to 128 on wide ones (us at 97 / 112 / 128 rows, stream vs
+  // pairs: 12288x4096 15.3 / 15.9 / 18.1 vs 19.4 / 19.4 / 19.8, 28672x8192 48.6 / 49.9 / 55.0 vs 55.8 / 56.7 / 58.0,
+  // 4096x11008 17.8 / 19.3 / 22.4 vs 20.7 / 20.8 / 21.2, 1024x8192 14.9 / 16.2 / 18.7 vs 13.3 / 13.4 / 13.3).  The pair
+  // kernel takes no groups of 32.
+  if (M > 96 && group % 64 == 0) {
+    const bool stream = M <= 112 ? packed >= ((size_t)6 << 20) && N >= 4096 : M <= 128 && N >= 8192;
+    return stream ? kStream : kGemm;
+  }
+  if (M > 16) return kStream;
   // Below, the stream kernel but for small weights, where its longer pipeline shows.  us, ring / stream, without early weights:
   // 9..16 rows, which double the ring kernel's MMAs: 2048x2048 4.8 / 4.1, 1024x4096 5.0 / 5.2, 2048x4096 6.4 / 5.5,
   // 1024x8192 7.2 / 6.0, 12288x4096 18.5 / 9.4.

@@ -273,7 +273,7 @@ def w4a16_linear_prefill(x, weight_packed, scale_zero, bias=None, *, workspace=N
 
 def w4a16_linear(x, weight_packed, scale_zero, bias=None):
     """W4A16 linear for any number of rows: the library picks among the decode kernels, the tcgen05 weight-streaming
-    kernel (up to 96 rows) and the tensor-core prefill kernel (``mp_w4a16_linear``).  Shapes the prefill kernel does
+    kernel (up to 128 rows) and the tensor-core prefill kernel (``mp_w4a16_linear``).  Shapes the prefill kernel does
     not take (K or the group size not a multiple of 64) are processed by the decode kernels in 64-row slabs.
     """
     x2 = _req(x, "x", torch.float16, 2)
@@ -294,7 +294,7 @@ def w4a16_linear(x, weight_packed, scale_zero, bias=None):
     y = torch.empty((m, n), dtype=torch.float16, device=x2.device)
     lib = _lib.load()
     nbytes = lib.mp_w4a16_linear_workspace_bytes(m, n, k, group)
-    ws = _workspace(nbytes, x2.device, own_in_capture=m <= 16) if nbytes else None
+    ws = _workspace(nbytes, x2.device, own_in_capture=True) if nbytes else None
     st = lib.mp_w4a16_linear(x2.data_ptr(), p.data_ptr(), sz.data_ptr(), _ptr(b), y.data_ptr(), m, n, k, group, _ptr(ws),
                              0 if ws is None else ws.numel(), _error_word(x2.device).data_ptr(), _stream())
     _lib.check(st, "w4a16_linear", M=m, N=n, K=k, group=group)

@@ -18,8 +18,8 @@ def _case(n, k, m, group):
     return x, packed, sz, bias, ops.w4a16_dequant(packed, scale, zero, n, k).float()
 
 
-@pytest.mark.parametrize("m", [1, 8, 9, 16, 17, 32, 33, 64, 65, 80, 96, 97, 128, 129])
-@pytest.mark.parametrize("n,k,group", [(264, 1280, 128), (4104, 512, 64), (40, 1408, 128), (2048, 2176, 128),
+@pytest.mark.parametrize("m", [1, 8, 9, 16, 17, 32, 33, 48, 49, 64, 65, 80, 81, 96, 97, 112, 113, 128, 129])
+@pytest.mark.parametrize("n,k,group", [(8200, 1664, 128), (264, 1280, 128), (4104, 512, 64), (40, 1408, 128), (2048, 2176, 128),
                                        (20480, 512, 256), (1032, 4096, 4096)])
 def test_linear_at_row_count_edges(m, n, k, group):
     x, packed, sz, bias, wdq = _case(n, k, m, group)
@@ -47,7 +47,7 @@ def test_linear_of_extreme_values(m):
     ops.check_device_errors()
 
 
-@pytest.mark.parametrize("m", [1, 16, 17, 33, 64, 77, 96])
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 48, 64, 77, 96, 112, 128])
 @pytest.mark.parametrize("n,k", [(1024, 8192), (512, 2048), (4104, 4096)])
 def test_chained_launches_with_early_weights_share_scratch(n, k, m):
     """Blocks of few stages that close a row block, behind a launch whose partial tiles lie in the same scratch: none may
@@ -75,9 +75,10 @@ def test_chained_launches_with_early_weights_share_scratch(n, k, m):
         assert torch.equal(y, want[i % 2])
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 4096, 4096), (8, 8192, 8192), (16, 1024, 8192), (16, 12288, 4096)])
+@pytest.mark.parametrize("m,n,k", [(1, 4096, 4096), (8, 8192, 8192), (16, 1024, 8192), (16, 12288, 4096),
+                                   (77, 4096, 4096), (100, 4096, 4096), (128, 8192, 2048)])
 def test_capture_on_a_stream_without_scratch(m, n, k):
-    """Up to 16 rows a capture needs no call on its stream before; the graph then brings zeroed scratch of its own."""
+    """A capture needs no call on its stream before; the graph then brings zeroed scratch of its own."""
     x, packed, sz, bias, _ = _case(n, k, m, 128)
     want = ops.w4a16_linear(x, packed, sz, bias)
     stream = torch.cuda.Stream()                           # (kept: another stream might get its handle and find scratch)
