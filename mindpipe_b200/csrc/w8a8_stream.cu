@@ -18,8 +18,8 @@
 //               scales, bias or SwiGLU, stores of 256 contiguous bytes
 //   warp 8      TMA producer: one copy of weights and one of activations per stage
 //   warp 9      TMEM allocation and the MMA issuer
-// A block takes less than half an SM, so the next product of a chain starts beside the end of this one; its
-// first weights are then already on the way (see early_weights).
+// Where its stream is short a block takes less than half an SM, so the next product of a chain starts beside the end of this
+// one; its first weights are then already on the way (see early_weights).  A long stream has a longer ring (kLongStream).
 #include "common.cuh"
 #include "tc.cuh"
 #include "moe_api.cuh"
@@ -38,21 +38,26 @@ constexpr int kWBytes = kRows * kStepK;
 constexpr int kChunk = 16;                       // tokens that pass through shared memory at a time
 constexpr int kPitch = kRows + 4;                // words between tokens there: 16-byte rows, lanes on different banks
 constexpr int kMaxRing = 8;
+// Blocks of at least kLongStream stages have kLongRing of them in flight, though they then take more than half an SM and the
+// next product of a chain starts behind their end: with four (32 tokens) an SM has too little under way, with more than six
+// the HBM rate falls again (the Mixtral-shaped experts at 32 tokens, us: 4 stages 284, 6 262, 7 263, 8 270; 28672x4096 at one
+// row, 5 / 6 / 8 stages 24.0 / 23.4 / 23.6; 12288x4096, where a block has 21, is level).
+constexpr int kLongRing = 6, kLongStream = 40;
 constexpr int kMaxExperts = 256;
 constexpr int kMaxGroups = 512;
 
-template <int TOK, int EPI>
+template <int TOK, int EPI, bool LONG>
 struct Cfg {
   static constexpr int kParts = EPI == STREAM_SWIGLU ? 2 : 1;       // gate rows and up rows
   static constexpr int kStageBytes = kWBytes + TOK * kStepK;
   static constexpr int kSmemMax = 112 * 1024;
   static constexpr int kFixed = 1024 + 2 * kChunk * kPitch * 4 + (2 * kMaxRing + 4) * 8 + 64;
   static constexpr int kFit = (kSmemMax - kFixed) / kStageBytes;
-  static constexpr int kRing = kFit < kMaxRing ? kFit : kMaxRing;
+  static constexpr int kRing = LONG ? kLongRing : kFit < kMaxRing ? kFit : kMaxRing;
   static constexpr int kSmem = kFixed + kRing * kStageBytes;
   static constexpr int kTmemUsed = 2 * kParts * TOK;                // two accumulator buffers
   static constexpr uint32_t kTmemCols = kTmemUsed <= 64 ? 64 : kTmemUsed <= 128 ? 128 : 256;
-  static_assert(kRing >= 3 && kTmemUsed <= 256, "shared or tensor memory");
+  static_assert(kRing >= 3 && kSmem <= 224 * 1024 && kTmemUsed <= 256, "shared or tensor memory");
 };
 }  // namespace ws
 
@@ -92,11 +97,11 @@ struct StreamAt {
   }
 };
 
-template <int TOK, int EPI>
+template <int TOK, int EPI, bool LONG>
 __global__ void __launch_bounds__(ws::kThreads, 2)
 w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                    const StreamParams p) {
-  using C = ws::Cfg<TOK, EPI>;
+  using C = ws::Cfg<TOK, EPI, LONG>;
   constexpr int kRing = C::kRing, kParts = C::kParts;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -410,10 +415,10 @@ w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   }
 }
 
-template <int TOK, int EPI>
+template <int TOK, int EPI, bool LONG>
 static int launch_stream(const CUtensorMap& tw, const CUtensorMap& tx, const StreamParams& p, int grid, cudaStream_t st) {
-  using C = ws::Cfg<TOK, EPI>;
-  auto kern = w8a8_stream_kernel<TOK, EPI>;
+  using C = ws::Cfg<TOK, EPI, LONG>;
+  auto kern = w8a8_stream_kernel<TOK, EPI, LONG>;
   static thread_local int configured_device = -1;
   int device = 0;
   MP_CUDA_TRY(cudaGetDevice(&device));
@@ -461,17 +466,23 @@ int launch_w8a8_stream(int epi, const void* x_i8, int x_rows, const void* w_i8, 
   p.tiles = reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(workspace) + kW4CounterBytes);
   const long long want = (most + p.min_share - 1) / p.min_share;
   const int grid = want < kSmCount ? (int)want : kSmCount;
-#define MP_STREAM(TOK)                                                               \
-  switch (epi) {                                                                     \
-    case STREAM_F16: return launch_stream<TOK, STREAM_F16>(tw, tx, p, grid, st);     \
-    case STREAM_AFFINE: return launch_stream<TOK, STREAM_AFFINE>(tw, tx, p, grid, st); \
-    default: return launch_stream<TOK, STREAM_SWIGLU>(tw, tx, p, grid, st); \
+  // (with every expert taken once)
+  const long long stages = (long long)(p.counts ? p.experts : 1) * p.row_blocks * p.steps * (epi == STREAM_SWIGLU ? 2 : 1);
+  const bool long_stream = stages >= (long long)ws::kLongStream * grid;
+#define MP_STREAM_EPI(TOK, EPI) \
+  return long_stream ? launch_stream<TOK, EPI, true>(tw, tx, p, grid, st) : launch_stream<TOK, EPI, false>(tw, tx, p, grid, st);
+#define MP_STREAM(TOK)                                     \
+  switch (epi) {                                           \
+    case STREAM_F16: MP_STREAM_EPI(TOK, STREAM_F16)        \
+    case STREAM_AFFINE: MP_STREAM_EPI(TOK, STREAM_AFFINE)  \
+    default: MP_STREAM_EPI(TOK, STREAM_SWIGLU)             \
   }
   switch (tok) {
     case 16: MP_STREAM(16)
     case 32: MP_STREAM(32)
     default: MP_STREAM(64)
   }
+#undef MP_STREAM_EPI
 #undef MP_STREAM
 }
 

@@ -127,3 +127,30 @@ def test_routing_plan_and_rows(t, k, lo, hi):
     rest = torch.ones(padded, dtype=torch.bool)
     rest[list(used)] = False
     assert (s.cpu()[rest] == 0).all()
+
+
+@pytest.mark.parametrize("kind", [SmoothQuantLinear.from_float, QuantLinear], ids=["symmetric", "affine"])
+@pytest.mark.parametrize("m,n,k", [(1, 24610, 4112), (8, 24610, 4112), (8, 6168, 16400)])
+def test_long_streams_give_the_tiled_gemm_s_bits(kind, m, n, k):
+    """Blocks of 40 stages and more, which take the longer ring."""
+    mod = kind(_linear(n, k, bias=True))
+    x = torch.randn(m, k, device="cuda").half()
+    want = mod._forward_checked(x)
+    for _ in range(3):
+        assert torch.equal(mod(x), want)
+    ops.check_device_errors()
+
+
+@pytest.mark.parametrize("t", [5, 17, 33, 64])
+def test_long_streams_of_experts_give_the_staged_layer_s_bits(t):
+    g = torch.Generator(device="cuda").manual_seed(t)
+    e, h, i = 8, 2064, 6400
+    mod = SmoothQuantPackedMoeExperts(torch.randn(e, 2 * i, h, generator=g, device="cuda").half() * 0.05,
+                                      torch.randn(e, h, i, generator=g, device="cuda").half() * 0.05)
+    x = torch.randn(t, h, generator=g, device="cuda").half()
+    ids = torch.rand(t, e, generator=g, device="cuda").topk(2, dim=1).indices.int()
+    w = torch.rand(t, 2, generator=g, device="cuda").half()
+    want = mod._forward_checked(x, ids, w)
+    for _ in range(3):
+        assert torch.equal(mod(x, ids, w), want)
+    ops.check_device_errors()
