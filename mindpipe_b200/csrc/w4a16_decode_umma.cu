@@ -61,7 +61,7 @@ constexpr int kRows = 128;
 constexpr int kStageK = 256;
 constexpr int kSlots = 3;                             // stages between expansion and MMA: stage i is in slot i % 3
 constexpr int kWBytes = kRows * (kStageK / 2);        // 16384
-constexpr int kMaxRing = 10, kMaxXRing = 8;
+constexpr int kMaxRing = 8, kMaxXRing = 8;          // (eight weight stages; ten 1 to 5 % slower: 40960x8192 at 8 rows 36.3 us, 34.7 with eight)
 // Weight stages requested before the activations, which queue behind them: with early weights the time up to the wait for
 // the kernel before is theirs (12288x4096 at 16 rows in a chain, us: 4 or 5 stages 9.2, 6 9.5, the whole ring 10.1).
 constexpr int kFirstEarly = 5, kFirst = 1;
