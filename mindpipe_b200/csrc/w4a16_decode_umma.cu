@@ -39,7 +39,8 @@
 // Expansion emits the columns of a packed word in the order (k0,k4,k1,k5,k2,k6,k3,k7).  Up to 16 rows the expansion warps
 // apply the same permutation in place to the 16-byte chunks of the stage's activation tile (a chunk is one token's eight
 // columns of one word, so the swizzle does not matter); with more rows they put the words back in order, see Cfg.  (Warps
-// of their own for the permutation were starved by the expansion warps: 2100 clocks per stage with one.)
+// of their own for the permutation were starved by the expansion warps: 2100 clocks per stage with one; in the epilogue warps it
+// took a 7B layer at 16 rows from 42 to 49 us.)
 // One block fills an SM: its ring is what hides HBM's latency.  Smaller blocks, two of them to an SM so that the next linear
 // of a chain starts beside the end of this one, took 38 us where this takes 28 (28672x8192, 16 rows).
 // What a launch costs beyond the stream: 1.3 us from the end of the kernel before to the first MMA, 1.3 from the last MMA to the
@@ -431,7 +432,12 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
     int s = set, xs = set, q = set;
     uint32_t phase = 0, xphase = 0, use = 0;
     for (int i = set; i < n_stages; i += C::kSets) {
-      if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, phase, abort_flag))) break;
+      // FOLD: one look at all three barriers and one vote, where nothing is to be waited for: a wait that is over and its vote
+      // cost 38 clocks a stage (the four linears of a 70B layer at 8 rows 95.1 -> 91.7 us; the exact form, whose arithmetic is
+      // longer, gains nothing)
+      const bool wait = !FOLD || !__all_sync(0xffffffffu, mbar_test(full0 + 8 * s, phase) & mbar_test(done0 + 8 * q, use ^ 1) &
+                                                              mbar_test(xfull0 + 8 * xs, xphase));
+      if (wait && !__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, phase, abort_flag))) break;
       const uint32_t stage = wring + s * stage_bytes, src = (stage + lane_w) ^ (part * kPieces * 16), sz = stage + sz_lane;
       uint4 q4[kPieces];
 #pragma unroll
@@ -443,7 +449,7 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
         szw[j] = du_lds_u32(sz + (p.groups_per_stage > 1 ? ((part * 128 + j * (FOLD ? 128 : 32)) >> p.gshift) * (du::kRows * 4) : 0));
       // (the slot's use before its last one is over: this warp has waited for the MMAs of a stage at most six before this
       // one, and they complete in order, so the parity is not ambiguous)
-      if (!__all_sync(0xffffffffu, mbar_wait(done0 + 8 * q, use ^ 1, abort_flag))) break;
+      if (wait && !__all_sync(0xffffffffu, mbar_wait(done0 + 8 * q, use ^ 1, abort_flag))) break;
       mbar_arrive_warp(empty0 + 8 * s, lane);
       tcgen05_fence_after();
       const uint32_t a_tmem = a_tmem0 + q * du::kASlotCols;
@@ -483,7 +489,7 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
       }
       if constexpr (PERM) {
         // this warp's share of the stage's activations: chunks of XROWS tokens x 256 columns
-        if (!__all_sync(0xffffffffu, mbar_wait(xfull0 + 8 * xs, xphase, abort_flag))) break;
+        if (wait && !__all_sync(0xffffffffu, mbar_wait(xfull0 + 8 * xs, xphase, abort_flag))) break;
         constexpr int kChunks = kXBytes / 2048 / C::kParts;
         const uint32_t xt = xring + xs * kXBytes + part * (kXBytes / C::kParts) + row * 16;
         uint4 v[kChunks];
