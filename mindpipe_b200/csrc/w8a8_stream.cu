@@ -117,7 +117,7 @@ w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * ws::kMaxRing;
   const uint32_t dfull0 = empty0 + 8 * ws::kMaxRing, dempty0 = dfull0 + 16;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int blk = static_cast<int>(blockIdx.x), grid = static_cast<int>(gridDim.x);
   const bool grouped = p.counts != nullptr;
   if (warp == ws::kLoadWarp && elect_one()) {
