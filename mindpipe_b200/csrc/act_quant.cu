@@ -27,7 +27,7 @@ __device__ __forceinline__ void emit_codes(const uint4& raw, const RowQuant& rq,
   }
 }
 
-// One warp per row (rows of up to 32 * 8 * NV columns): the row is read once with NV independent
+// One warp per row (many rows of up to 32 * 8 * NV columns): the row is read once with NV independent
 // 128-bit loads per lane, reduced with shuffles only, and quantised from registers -- no block-level
 // synchronisation at all.
 // CODES / FAKE select the outputs at compile time and the rare tiny-scale rows take a rolled loop that
@@ -53,9 +53,7 @@ act_quant_warp_kernel(const __half* __restrict__ x, int M, int K, int8_t* __rest
   __half2 m2 = __float2half2_rn(0.0f);
 #pragma unroll
   for (int v = 0; v < NV; ++v) m2 = absmax8(m2, held[v]);
-  float amax = absmax_to_float(m2);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  const float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(absmax_to_float(m2))));
   const float eps = h2f(f2h(1e-5f));                                   // clamp_(min=1e-5) on an fp16 tensor
   const float sf = h2f(f2h(__fdiv_rn(fmaxf(amax, eps), 127.0f)));      // div_(q_max), rounded to fp16
   RowQuant rq = make_row_quant(sf);
@@ -99,8 +97,7 @@ act_quant_kernel(const __half* __restrict__ x, int M, int K, int8_t* __restrict_
                  float* __restrict__ scale, __half* __restrict__ fake) {
   chain_wait();
   chain_release();
-  __shared__ float s_red[THREADS / 32];
-  __shared__ float s_scale;
+  __shared__ uint32_t s_red[THREADS / 32];
   const int row = blockIdx.x;
   const __half* xr = x + (size_t)row * K;
   const int chunks = K >> 3;
@@ -119,24 +116,15 @@ act_quant_kernel(const __half* __restrict__ x, int M, int K, int8_t* __restrict_
   } else {
     for (int c = threadIdx.x; c < chunks; c += THREADS) absmax_of(*reinterpret_cast<const uint4*>(xr + c * 8));
   }
-  float amax = absmax_to_float(m2);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = amax;
+  // (bit patterns of non-negative numbers order as the numbers do)
+  uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(absmax_to_float(m2)));
+  if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = top;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    float v = threadIdx.x < THREADS / 32 ? s_red[threadIdx.x] : 0.0f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (threadIdx.x == 0) {
-      const float eps = h2f(f2h(1e-5f));                      // clamp_(min=1e-5) on an fp16 tensor
-      const __half s = f2h(__fdiv_rn(fmaxf(v, eps), 127.0f)); // div_(q_max), rounded to fp16
-      s_scale = h2f(s);
-      if (scale) scale[row] = s_scale;
-    }
-  }
-  __syncthreads();
-  const RowQuant rq = make_row_quant(s_scale);
+  top = __reduce_max_sync(0xffffffffu, (threadIdx.x & 31) < THREADS / 32 ? s_red[threadIdx.x & 31] : 0u);
+  const float eps = h2f(f2h(1e-5f));                                                  // clamp_(min=1e-5) on an fp16 tensor
+  const float sf = h2f(f2h(__fdiv_rn(fmaxf(__uint_as_float(top), eps), 127.0f)));     // div_(q_max), rounded to fp16
+  if (threadIdx.x == 0 && scale) scale[row] = sf;
+  const RowQuant rq = make_row_quant(sf);
   auto emit = [&](int c, const uint4& raw) {
     emit_codes(raw, rq, q ? q + (size_t)row * K + c * 8 : nullptr,
                fake ? fake + (size_t)row * K + c * 8 : nullptr);
@@ -396,8 +384,11 @@ extern "C" int mp_add_rmsnorm_quant(const void* x_f16, void* residual_f16, const
 
 // A block of these kernels loads its row, reduces, then stores: an SM streams only while its blocks are in different phases.
 // With more rows than SMs narrow blocks with more pieces per thread keep more rows in flight (4096 rows, us: 14336 values 40.8
-// with 512 threads, 29.7 with 256; 8192 values 23.4 / 16.7 with 128; with zero points 35.9 / 32.0 and 26.3 / 17.9); with
-// fewer the wide block is done sooner (8 rows of 14336: 2.2 / 2.4).
+// with 512 threads, 29.7 with 256; 8192 values 23.4 / 16.7 with 128; with zero points 35.9 / 32.0 and 26.3 / 17.9; a warp per
+// row up to 4096 values).  With fewer there is one block to an SM and its chain of load, reduction, division and rounding is
+// the time, so a thread has one piece of the row, or two (the four products of a Llama-8B layer with their quantisations, 1 /
+// 4 / 16 / 64 / 148 rows, us: a warp per row of 4096 and 512 threads for 14336 took 58.8 / 60.4 / 65.0 / 69.1 / 86.5, this 56.3 /
+// 57.7 / 62.6 / 67.2 / 85.2; two and four pieces a thread above 4096 56.7 / 58.2 / 62.7 / 67.7 / 85.8).
 static bool many_rows(int M) { return M > kSmCount; }
 
 extern "C" int mp_act_quant_per_token(const void* x_f16, int M, int K, void* q_i8, void* scale_f32,
@@ -410,21 +401,23 @@ extern "C" int mp_act_quant_per_token(const void* x_f16, int M, int K, void* q_i
   int8_t* q = static_cast<int8_t*>(q_i8);
   float* sc = static_cast<float*>(scale_f32);
   __half* fk = static_cast<__half*>(fake_f16);
-  const bool many = many_rows(M);
+  if (!many_rows(M) && K <= 16384) {
+    if (K <= 1024) return launch_chained(act_quant_kernel<128, 1>, dim3(M), dim3(128), 0, st, x, M, K, q, sc, fk);
+    if (K <= 2048) return launch_chained(act_quant_kernel<256, 1>, dim3(M), dim3(256), 0, st, x, M, K, q, sc, fk);
+    if (K <= 4096) return launch_chained(act_quant_kernel<512, 1>, dim3(M), dim3(512), 0, st, x, M, K, q, sc, fk);
+    if (K <= 8192) return launch_chained(act_quant_kernel<1024, 1>, dim3(M), dim3(1024), 0, st, x, M, K, q, sc, fk);
+    return launch_chained(act_quant_kernel<1024, 2>, dim3(M), dim3(1024), 0, st, x, M, K, q, sc, fk);
+  }
   if (K <= 1024) {
     return launch_act_quant_warp<4>(x, M, K, q, sc, fk, st);
   } else if (K <= 2048) {
     return launch_act_quant_warp<8>(x, M, K, q, sc, fk, st);
   } else if (K <= 4096) {
     return launch_act_quant_warp<16>(x, M, K, q, sc, fk, st);
-  } else if (many && K <= 8192) {
-    return launch_chained(act_quant_kernel<128, 8>, dim3(M), dim3(128), 0, st, x, M, K, q, sc, fk);
-  } else if (many && K <= 16384) {
-    return launch_chained(act_quant_kernel<256, 8>, dim3(M), dim3(256), 0, st, x, M, K, q, sc, fk);
   } else if (K <= 8192) {
-    return launch_chained(act_quant_kernel<512, 2>, dim3(M), dim3(512), 0, st, x, M, K, q, sc, fk);
+    return launch_chained(act_quant_kernel<128, 8>, dim3(M), dim3(128), 0, st, x, M, K, q, sc, fk);
   } else if (K <= 16384) {
-    return launch_chained(act_quant_kernel<512, 4>, dim3(M), dim3(512), 0, st, x, M, K, q, sc, fk);
+    return launch_chained(act_quant_kernel<256, 8>, dim3(M), dim3(256), 0, st, x, M, K, q, sc, fk);
   } else {
     return launch_chained(act_quant_kernel<512, 0>, dim3(M), dim3(512), 0, st, x, M, K, q, sc, fk);
   }
