@@ -383,13 +383,16 @@ extern "C" int mp_add_rmsnorm_quant(const void* x_f16, void* residual_f16, const
 }
 
 // A block of these kernels loads its row, reduces, then stores: an SM streams only while its blocks are in different phases.
-// With more rows than SMs narrow blocks with more pieces per thread keep more rows in flight (4096 rows, us: 14336 values 40.8
-// with 512 threads, 29.7 with 256; 8192 values 23.4 / 16.7 with 128; with zero points 35.9 / 32.0 and 26.3 / 17.9; a warp per
-// row up to 4096 values).  With fewer there is one block to an SM and its chain of load, reduction, division and rounding is
-// the time, so a thread has one piece of the row, or two (the four products of a Llama-8B layer with their quantisations, 1 /
-// 4 / 16 / 64 / 148 rows, us: a warp per row of 4096 and 512 threads for 14336 took 58.8 / 60.4 / 65.0 / 69.1 / 86.5, this 56.3 /
-// 57.7 / 62.6 / 67.2 / 85.2; two and four pieces a thread above 4096 56.7 / 58.2 / 62.7 / 67.7 / 85.8).
-static bool many_rows(int M) { return M > kSmCount; }
+// With many rows narrow blocks with more pieces per thread keep more rows in flight (4096 rows, us: 14336 values 40.8 with 512
+// threads, 29.7 with 256; 8192 values 23.4 / 16.7 with 128; with zero points 35.9 / 32.0 and 26.3 / 17.9; a warp per row up to
+// 4096 values).  While all rows fit on the SMs side by side the chain of load, reduction, division and rounding is the time,
+// so a thread has one or two pieces of the row.  A Llama-8B layer's four products with their quantisations, 1 / 4 / 16 / 64 /
+// 148 rows, us: a warp per row of 4096 and 512 threads for 14336 58.8 / 60.4 / 65.0 / 69.1 / 86.5, this 56.3 / 57.7 / 62.6 /
+// 67.2 / 85.2 (two and four pieces a thread above 4096 56.7 / 58.2 / 62.7 / 67.7 / 85.8).
+// The line is four rows to an SM, which is what its threads hold of 512 to a row (200 / 333 / 500 / 1000 rows of that layer:
+// narrow blocks 89.8 / 114.9 / 124.5 / 189.2, wide ones 88.0 / 112.7 / 119.9 / 191.2; 333 and 2000 rows of a Llama-7B layer
+// with zero points 114.4 / 323.5 and 110.4 / 326.9; there one piece a thread is no better at 333 rows, 113.6).
+static bool many_rows(int M) { return M > 4 * kSmCount; }
 
 extern "C" int mp_act_quant_per_token(const void* x_f16, int M, int K, void* q_i8, void* scale_f32,
                                       void* fake_f16, mp_stream_t stream) {

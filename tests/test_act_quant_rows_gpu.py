@@ -24,16 +24,19 @@ def test_same_bits_whatever_the_row_count(k):
             assert torch.equal(t, torch.cat([p[j] for p in parts]))
 
 
-@pytest.mark.parametrize("k", [8, 128, 1016, 1024, 1032, 2048, 2056, 4088, 4096])
-def test_a_block_to_a_row_gives_the_bits_of_a_warp_to_a_row(k):
+@pytest.mark.parametrize("k", [8, 128, 1016, 1024, 1032, 2048, 2056, 4088, 4096, 4104, 8200, 11008])
+def test_wide_blocks_give_the_bits_of_narrow_ones(k):
     g = torch.Generator(device="cuda").manual_seed(k)
-    x = torch.randn(149, k, generator=g, device="cuda").half()
+    x = torch.randn(593, k, generator=g, device="cuda").half()
     x[:, -1] *= 20                                       # the last piece holds the largest value
     x[3], x[5], x[7] = 0, x[5].abs() * -1, 1e-5
+    whole, affine = ops.act_quant_per_token(x, want_fake=True), ops.affine_quant_per_row(x)
     x[9, 0], x[11, k - 1], x[13] = float("inf"), float("nan"), float("nan")
-    whole = ops.act_quant_per_token(x, want_fake=True)
-    for rows in (1, 148):
-        parts = [ops.act_quant_per_token(x[i:i + rows].contiguous(), want_fake=True) for i in range(0, 149, rows)]
-        q, s, fake = (torch.cat([p[j] for p in parts]) for j in range(3))
-        assert torch.equal(q, whole[0]) and torch.equal(s, whole[1])
-        assert torch.equal(fake.view(torch.int16), whole[2].view(torch.int16))
+    odd = ops.act_quant_per_token(x, want_fake=True)
+    for rows in (1, 592):
+        parts = [ops.affine_quant_per_row(p) for p in x[:9].split(rows)]
+        assert all(torch.equal(torch.cat([p[j] for p in parts]), t[:9]) for j, t in enumerate(affine) if t is not None)
+        for of, n in ((whole, 9), (odd, 593)):
+            q, s, fake = (torch.cat(t) for t in zip(*(ops.act_quant_per_token(p, want_fake=True) for p in x[:n].split(rows))))
+            assert torch.equal(q, of[0][:n]) and torch.equal(s, of[1][:n])
+            assert torch.equal(fake.view(torch.int16), of[2][:n].view(torch.int16))
