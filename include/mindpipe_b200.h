@@ -402,7 +402,8 @@ int mp_w8a8_gemm_ex(const void* qx_i8, const void* x_scale_f32, const void* w_i8
 /*
  * The whole W8A8 linear on fp16 rows: mp_act_quant_per_token, then the product -- SmoothQuantLinear.forward
  * (fake_quant.py:77-88) in one call, so that the product's weights are on their way while the rows are quantised.  Up to
- * 8 rows a weight-streaming kernel runs, else mp_w8a8_gemm_ex; the results are those of the two calls, bit for bit.
+ * 8 rows a weight-streaming kernel runs (with few values it quantises the rows as well), else mp_w8a8_gemm_ex; the results
+ * are those of the two calls, bit for bit.
  * qx_i8 [M,K] and x_scale_f32 [M] receive the codes and scales.  Workspace: as for mp_w4a16_linear (zero-filled when
  * created, one for all shapes, may be shared with it); the tiled GEMM runs unsplit without one.
  */

@@ -20,6 +20,11 @@
 //   warp 9      TMEM allocation and the MMA issuer
 // Where its stream is short a block takes less than half an SM, so the next product of a chain starts beside the end of this
 // one; its first weights are then already on the way (see early_weights).  A long stream has a longer ring (kLongStream).
+//
+// With few activation values (quantise_in_stream) the kernel quantises the rows itself (QUANT): a launch less between two
+// products of a chain, which was 1 to 2 us of its own chain of load, reduction and store.  The epilogue warps and four more
+// look through all rows for their maxima, then
+//   warps 10-13 quantise 128 columns of two rows each per stage, into the stage's activations as TMA would lay them out
 #include "common.cuh"
 #include "tc.cuh"
 #include "moe_api.cuh"
@@ -33,7 +38,8 @@ namespace ws {
 constexpr int kRows = 128;
 constexpr int kStepK = 128;
 constexpr int kEpiWarps = 8, kLoadWarp = 8, kMmaWarp = 9;
-constexpr int kThreads = 32 * 10;
+constexpr int kQuantWarp0 = 10, kQuantWarps = 4; // with rows quantised here: two rows to a warp
+constexpr int kMaxQuantRows = 2 * kQuantWarps;
 constexpr int kWBytes = kRows * kStepK;
 constexpr int kChunk = 16;                       // tokens that pass through shared memory at a time
 constexpr int kPitch = kRows + 4;                // words between tokens there: 16-byte rows, lanes on different banks
@@ -46,8 +52,10 @@ constexpr int kLongRing = 6, kLongStream = 40;
 constexpr int kMaxExperts = 256;
 constexpr int kMaxGroups = 512;
 
-template <int TOK, int EPI, bool LONG>
+template <int TOK, int EPI, bool LONG, bool QUANT>
 struct Cfg {
+  static_assert(!QUANT || (TOK >= kMaxQuantRows && EPI == STREAM_F16), "rows quantised here");
+  static constexpr int kThreads = 32 * (kMmaWarp + 1 + (QUANT ? kQuantWarps : 0));
   static constexpr int kParts = EPI == STREAM_SWIGLU ? 2 : 1;       // gate rows and up rows
   static constexpr int kStageBytes = kWBytes + TOK * kStepK;
   static constexpr int kSmemMax = 112 * 1024;
@@ -97,11 +105,11 @@ struct StreamAt {
   }
 };
 
-template <int TOK, int EPI, bool LONG>
-__global__ void __launch_bounds__(ws::kThreads, 2)
+template <int TOK, int EPI, bool LONG, bool QUANT>
+__global__ void __launch_bounds__(ws::Cfg<TOK, EPI, LONG, QUANT>::kThreads, 2)
 w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                    const StreamParams p) {
-  using C = ws::Cfg<TOK, EPI, LONG>;
+  using C = ws::Cfg<TOK, EPI, LONG, QUANT>;
   constexpr int kRing = C::kRing, kParts = C::kParts;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -113,6 +121,7 @@ w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   // launcher) and would be dropped
   __shared__ int s_group[EPI == STREAM_AFFINE ? 1 : ws::kMaxGroups];
   __shared__ int s_active;
+  __shared__ uint32_t s_top[QUANT ? ws::kMaxQuantRows : 1];     // the rows' largest magnitudes
   const uint32_t ring = smem_u32(base);
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * ws::kMaxRing;
   const uint32_t dfull0 = empty0 + 8 * ws::kMaxRing, dempty0 = dfull0 + 16;
@@ -124,7 +133,7 @@ w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     prefetch_tensormap(&tmap_w);
     prefetch_tensormap(&tmap_x);
     for (int s = 0; s < kRing; ++s) {
-      mbar_init(full0 + 8 * s, 1);
+      mbar_init(full0 + 8 * s, QUANT ? 1 + (p.M + 1) / 2 : 1);
       mbar_init(empty0 + 8 * s, 1);
     }
     for (int d = 0; d < 2; ++d) {
@@ -138,7 +147,8 @@ w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     tmem_alloc(smem_u32(tmem_slot), C::kTmemCols);
     tmem_relinquish();
   }
-  if (!p.early_weights) chain_wait();
+  if (QUANT && tid < ws::kMaxQuantRows) s_top[tid] = 0;
+  if (!QUANT && !p.early_weights) chain_wait();
   if (grouped && warp == 0) {
     // (the counts are complete: they are older than the previous kernel, or it was waited for)
     int n = 0;
@@ -182,7 +192,7 @@ w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       at.set(n_steps > 0 ? t_hi : 0, row_blocks, steps);
       auto load_w = [&](int s, const StreamAt& a, int part) {
         const int e = grouped ? s_group[a.group] & 0xFF : 0;
-        mbar_arrive_expect_tx(full0 + 8 * s, ws::kWBytes + p.x_box * ws::kStepK);
+        mbar_arrive_expect_tx(full0 + 8 * s, ws::kWBytes + (QUANT ? 0 : p.x_box * ws::kStepK));
         tma_load_2d(ring + s * C::kStageBytes, &tmap_w, full0 + 8 * s, a.kb * ws::kStepK,
                     e * p.rows_per_expert + part * p.up_row_offset + a.rb * ws::kRows);
       };
@@ -192,7 +202,12 @@ w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       };
       const int n_stages = n_steps * kParts;
       int ahead = 0;
-      if (p.early_weights) {                       // the ring's first weights, then what the previous kernel made
+      if constexpr (QUANT) {                       // the first weights as far as L2: a kernel before may write weights
+        StreamAt a = at;
+        for (int i = 0; i < kRing && i < n_stages; ++i, a.back(row_blocks, steps))
+          tma_prefetch_2d(&tmap_w, a.kb * ws::kStepK, a.rb * ws::kRows);
+        chain_wait();
+      } else if (p.early_weights) {                // the ring's first weights, then what the previous kernel made
         StreamAt a = at;
         for (; ahead < kRing && ahead < n_stages; ++ahead) {
           load_w(ahead, a, ahead % kParts);
@@ -207,7 +222,7 @@ w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
           if (!mbar_wait(empty0 + 8 * s, phase, abort_flag)) break;
           load_w(s, at, part);
         }
-        load_x(s, at);
+        if (!QUANT) load_x(s, at);
         if (++part == kParts) {
           part = 0;
           at.back(row_blocks, steps);
@@ -249,8 +264,92 @@ w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       }
     }
   } else {
+    float sa_here = 0.0f;                          // QUANT: the scale of row `warp`
+    if (QUANT || p.early_weights) chain_wait();    // before anything of the previous kernel is read or overwritten
+    if constexpr (QUANT) {
+      // a quantising warp has 128 columns of two rows per stage, eight values to a lane; the first stages' are on their way
+      // while the rows are looked through
+      const int r = 2 * (warp - ws::kQuantWarp0) + (lane >> 4), c = lane & 15;
+      const bool mine = warp >= ws::kEpiWarps && r < p.M;
+      auto load = [&](int kb) {
+        return mine && kb * ws::kStepK + 8 * c < p.K
+                   ? *reinterpret_cast<const uint4*>(p.x + (size_t)r * p.K + kb * ws::kStepK + 8 * c) : make_uint4(0, 0, 0, 0);
+      };
+      constexpr int kHeld = 4;                     // (3 is level, 6 is 2 us slower for four products)
+      uint4 held[kHeld];
+      StreamAt at, ahead;
+      at.set(n_steps > 0 ? t_hi : 0, row_blocks, steps);
+      ahead = at;
+      const int n = warp >= ws::kEpiWarps && 2 * (warp - ws::kQuantWarp0) < p.M ? n_steps : 0;
+#pragma unroll
+      for (int u = 0; u < kHeld; ++u) {
+        held[u] = u < n ? load(ahead.kb) : make_uint4(0, 0, 0, 0);
+        ahead.back(row_blocks, steps);
+      }
+      // the largest magnitude of every row: the epilogue and quantising warps in equal parts over the rows (all warps over
+      // all pieces, with a division and an atomic for each 32, took 0.8 us longer at four rows of 4096)
+      constexpr int kLookWarps = ws::kEpiWarps + ws::kQuantWarps, kBatch = 6;
+      const int me = warp < ws::kEpiWarps ? warp : warp - (ws::kQuantWarp0 - ws::kEpiWarps);
+      const int per_row = kLookWarps / p.M, of = me / per_row, chunks = p.K >> 3;
+      if (of < p.M) {
+        const uint4* xr = reinterpret_cast<const uint4*>(p.x + (size_t)of * p.K);
+        __half2 m2 = __float2half2_rn(0.0f);
+        for (int i0 = (me - of * per_row) * 32 + lane; i0 < chunks; i0 += kBatch * per_row * 32) {
+          uint4 look[kBatch];
+#pragma unroll
+          for (int j = 0; j < kBatch; ++j) {
+            const int i = i0 + j * per_row * 32;
+            look[j] = i < chunks ? xr[i] : make_uint4(0, 0, 0, 0);
+          }
+#pragma unroll
+          for (int j = 0; j < kBatch; ++j) m2 = absmax8(m2, look[j]);
+        }
+        // (bit patterns of non-negative numbers order as the numbers do)
+        __syncwarp();
+        const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(absmax_to_float(m2)));
+        if (lane == 0) atomicMax(&s_top[of], top);
+      }
+      asm volatile("bar.sync 2, %0;" ::"n"(32 * kLookWarps) : "memory");
+      // (as in act_quant.cu)
+      auto scale_of = [&](int r) {
+        const float eps = h2f(f2h(1e-5f));
+        return h2f(f2h(__fdiv_rn(fmaxf(__uint_as_float(s_top[r]), eps), 127.0f)));
+      };
+      if (warp < ws::kEpiWarps) {
+        sa_here = warp < p.M ? scale_of(warp) : 0.0f;
+      } else {
+        // ---------------------------------------------------------- quantising warps
+        const float sf = mine ? scale_of(r) : 1.0f;
+        const RowQuant rq = make_row_quant(sf);
+        int8_t* qr = p.qx + (size_t)r * p.K + 8 * c;
+        // row r of the stage's activations, 128 bytes, its 16-byte units swizzled as TMA would
+        const uint32_t slot = ws::kWBytes + r * ws::kStepK + (((c >> 1) ^ (r & 7)) << 4) + ((c & 1) << 3);
+        int s = 0;
+        uint32_t phase = 1;
+        bool ok = true;
+        for (int i0 = 0; ok && i0 < n; i0 += kHeld) {
+#pragma unroll
+          for (int u = 0; u < kHeld; ++u) {
+            if (i0 + u >= n) break;
+            const uint2 codes = quant8_pack(held[u], rq);
+            if (i0 + u + kHeld < n) held[u] = load(ahead.kb);
+            ahead.back(row_blocks, steps);
+            ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, phase, abort_flag));
+            if (!ok) break;
+            if (mine) *reinterpret_cast<uint2*>(base + s * C::kStageBytes + slot) = codes;
+            fence_proxy_async_smem();
+            mbar_arrive_warp(full0 + 8 * s, lane);
+            if (++s == kRing) { s = 0; phase ^= 1; }
+            if (at.rb == 0 && mine) {              // the caller's codes and scales, by the blocks of the first 128 rows
+              if (at.kb * ws::kStepK + 8 * c < p.K) *reinterpret_cast<uint2*>(qr + at.kb * ws::kStepK) = codes;
+              if (at.kb == 0 && c == 0) p.qx_scale[r] = sf;
+            }
+            at.back(row_blocks, steps);
+          }
+        }
+      }
+    }
     // ------------------------------------------------------------ epilogue
-    if (p.early_weights) chain_wait();             // before anything of the previous kernel is read or overwritten
     const int quarter = warp & 3, half = warp >> 2;
     const uint32_t lane_field = static_cast<uint32_t>(quarter * 32) << 16;
     const int row = quarter * 32 + lane;
@@ -258,7 +357,7 @@ w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     at.set(n_steps > 0 ? t_hi : 0, row_blocks, steps);
     int d = 0;
     uint32_t dphase = 0;
-    for (int t = t_hi; t >= t_lo;) {
+    for (int t = QUANT && warp >= ws::kEpiWarps ? t_lo - 1 : t_hi; t >= t_lo;) {
       const int seg_lo = max(t_lo, t - at.kb);                  // this segment: steps [seg_lo, t] of one row block
       const bool ends = at.kb == steps - 1, whole = ends && seg_lo == t - at.kb;
       // the first block of this row block (its tiles are added by the block that holds the end)
@@ -350,7 +449,7 @@ w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             if (gave_up) break;
           }
           const size_t out_row = (size_t)(x_row0 + m);
-          const float sa = __ldg(p.a_scale + out_row);
+          const float sa = QUANT ? sa_here : __ldg(p.a_scale + out_row);       // (QUANT: row j is warp j's)
           __half hv[4];
           if constexpr (EPI == STREAM_SWIGLU) {
             const int* g = reinterpret_cast<const int*>(&acc[0]);
@@ -415,10 +514,10 @@ w8a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   }
 }
 
-template <int TOK, int EPI, bool LONG>
+template <int TOK, int EPI, bool LONG, bool QUANT = false>
 static int launch_stream(const CUtensorMap& tw, const CUtensorMap& tx, const StreamParams& p, int grid, cudaStream_t st) {
-  using C = ws::Cfg<TOK, EPI, LONG>;
-  auto kern = w8a8_stream_kernel<TOK, EPI, LONG>;
+  using C = ws::Cfg<TOK, EPI, LONG, QUANT>;
+  auto kern = w8a8_stream_kernel<TOK, EPI, LONG, QUANT>;
   static thread_local int configured_device = -1;
   int device = 0;
   MP_CUDA_TRY(cudaGetDevice(&device));
@@ -426,7 +525,7 @@ static int launch_stream(const CUtensorMap& tw, const CUtensorMap& tx, const Str
     MP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem));
     configured_device = device;
   }
-  return launch_chained(kern, dim3(grid), dim3(ws::kThreads), C::kSmem, st, tw, tx, p);
+  return launch_chained(kern, dim3(grid), dim3(C::kThreads), C::kSmem, st, tw, tx, p);
 }
 
 static int stream_tokens(int rows) { return rows <= 16 ? 16 : rows <= 32 ? 32 : 64; }
@@ -469,6 +568,11 @@ int launch_w8a8_stream(int epi, const void* x_i8, int x_rows, const void* w_i8, 
   // (with every expert taken once)
   const long long stages = (long long)(p.counts ? p.experts : 1) * p.row_blocks * p.steps * (epi == STREAM_SWIGLU ? 2 : 1);
   const bool long_stream = stages >= (long long)ws::kLongStream * grid;
+  if (p.x) {
+    if (epi != STREAM_F16 || max_rows > ws::kMaxQuantRows || !aligned(p.x, 16)) return MP_ERR_UNSUPPORTED;
+    return long_stream ? launch_stream<16, STREAM_F16, true, true>(tw, tx, p, grid, st)
+                       : launch_stream<16, STREAM_F16, false, true>(tw, tx, p, grid, st);
+  }
 #define MP_STREAM_EPI(TOK, EPI) \
   return long_stream ? launch_stream<TOK, EPI, true>(tw, tx, p, grid, st) : launch_stream<TOK, EPI, false>(tw, tx, p, grid, st);
 #define MP_STREAM(TOK)                                     \
@@ -491,6 +595,22 @@ static size_t split_bytes(int M, int N, int K) { return mp_w8a8_gemm_workspace_b
 constexpr size_t kSplitOffset = kW4CounterBytes + kW4TileBytes;
 static bool stream_rows(int M, int K) { return M <= kStreamMaxRows && K % 16 == 0 && K < (1 << 17); }
 
+// Rows quantised inside the product: every block reads all of x for the rows' maxima, at about 45 bytes a clock, which has to
+// cost less than the kernel that it saves.  The four products of a Llama-8B layer, us, with the quantisation before / inside
+// all of them: 1 row 56.9 / 50.0, 4 rows 58.2 / 52.3, 6 rows 58.9 / 54.6, 8 rows 59.2 / 56.6 (56.1 without the 8 x 14336 one);
+// of a Llama-70B layer 1 row 157.1 / 146.1, 4 rows 159.8 / 151.8 (155.6 without 4 x 28672), 8 rows 162.9 / 161.5 (161.3).
+// x may not share memory with what other blocks write meanwhile.
+static bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
+  const char *p = static_cast<const char*>(a), *q = static_cast<const char*>(b);
+  return p < q + b_bytes && q < p + a_bytes;
+}
+static bool quantise_in_stream(const void* x, const void* qx, const void* scale, const void* y, int M, int N, int K) {
+  if (!x || M <= 0 || K <= 0 || !stream_rows(M, K) || (long long)M * K > (M <= 6 ? 131072 : 65536)) return false;
+  const size_t values = (size_t)M * K;
+  return !overlap(x, 2 * values, qx, values) && !overlap(x, 2 * values, scale, 4 * (size_t)M) &&
+         !overlap(x, 2 * values, y, 2 * (size_t)M * N);
+}
+
 static size_t linear_workspace_bytes(int epi, int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (stream_rows(M, K)) return w8a8_stream_workspace_bytes(epi, M);
@@ -508,18 +628,27 @@ extern "C" int mp_w8a8_linear(const void* x_f16, const void* w_i8, const void* w
                               int M, int N, int K, void* qx_i8, void* x_scale_f32, void* workspace, size_t workspace_bytes,
                               int* error_word, mp_stream_t stream) {
   if (!w_i8 || !w_scale_f32 || !y_f16 || !qx_i8 || !x_scale_f32 || N <= 0) return MP_ERR_INVALID_ARG;
+  StreamParams p{};
+  p.M = M; p.N = N; p.K = K;
+  p.b_scale = static_cast<const float*>(w_scale_f32);
+  p.bias = static_cast<const __half*>(bias_f16);
+  p.out = y_f16;
+  p.error_word = error_word;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (quantise_in_stream(x_f16, qx_i8, x_scale_f32, y_f16, M, N, K)) {
+    p.x = static_cast<const __half*>(x_f16);
+    p.qx = static_cast<int8_t*>(qx_i8);
+    p.qx_scale = static_cast<float*>(x_scale_f32);
+    const int rc = launch_w8a8_stream(STREAM_F16, qx_i8, M, w_i8, N, p, M, workspace, workspace_bytes, st);
+    if (rc != MP_ERR_UNSUPPORTED) return rc;
+    p.x = nullptr;
+  }
   int rc = mp_act_quant_per_token(x_f16, M, K, qx_i8, x_scale_f32, nullptr, stream);
   if (rc != MP_OK) return rc;
   if (stream_rows(M, K)) {
-    StreamParams p{};
-    p.M = M; p.N = N; p.K = K;
     p.early_weights = 1;                 // the kernel before is the quantisation, which waited for everything older
     p.a_scale = static_cast<const float*>(x_scale_f32);
-    p.b_scale = static_cast<const float*>(w_scale_f32);
-    p.bias = static_cast<const __half*>(bias_f16);
-    p.out = y_f16;
-    p.error_word = error_word;
-    rc = launch_w8a8_stream(STREAM_F16, qx_i8, M, w_i8, N, p, M, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+    rc = launch_w8a8_stream(STREAM_F16, qx_i8, M, w_i8, N, p, M, workspace, workspace_bytes, st);
     if (rc != MP_ERR_UNSUPPORTED) return rc;
   }
   const bool scratch = workspace && workspace_bytes > kSplitOffset;

@@ -32,6 +32,9 @@ struct StreamParams {
   int* error_word;
   int x_box;                   // activation rows a load brings: no more than there are (a copy that reaches beyond a small
                                // tensor is slow: 14 us instead of 8 for 24 rows of 4096 in a box of 128)
+  const __half* x;             // rows to quantise in the kernel, or null; then ...
+  int8_t* qx;                  // ... their codes and ...
+  float* qx_scale;             // ... scales are left here
 };
 
 // Rows of a linear, rows per expert.  From 9 rows on the tiled kernel is as fast or faster (16 rows, us: 4096x4096 10.6 vs

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from mindpipe_b200 import ops
+from mindpipe_b200 import _lib, ops
 from mindpipe_b200.modules import QuantLinear, SmoothQuantLinear, SmoothQuantPackedMoeExperts
 from oracle import pseudo_quant as O
 
@@ -34,6 +34,36 @@ def test_streamed_product_gives_the_tiled_gemm_s_bits(kind, m, n, k):
     for _ in range(3):
         assert torch.equal(mod(x), want)
     ops.check_device_errors()
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 7, 8])
+@pytest.mark.parametrize("n,k", [(40, 16), (8, 144), (384, 4112), (1026, 1024), (20480, 256), (256, 8192), (4096, 4096),
+                                 (264, 28672)])
+def test_rows_quantised_in_the_stream_give_the_quantiser_s_codes(m, n, k):
+    g = torch.Generator(device="cuda").manual_seed(m * n + k)
+    mod = SmoothQuantLinear.from_float(_linear(n, k, bias=m % 2 == 0))
+    x = torch.randn(m, k, generator=g, device="cuda").half()
+    x[:, ::97] *= 20
+    x[:, -1] *= 30                                             # the last piece of a row holds its largest value
+    if m > 2:
+        x[1], x[2] = 0, x[2] * 1e-4                            # a scale below 2^-14
+    q, s, _ = ops.act_quant_per_token(x)
+    w_scale = mod.weight_scale.flatten().float()
+    want = ops.w8a8_gemm(q, s, mod.weight, w_scale, mod.bias)
+    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    ws = torch.zeros(lib.mp_w8a8_linear_workspace_bytes(m, n, k), dtype=torch.uint8, device="cuda")
+    for _ in range(3):
+        q2, s2, y = torch.full_like(q, 85), torch.full_like(s, -1), torch.full_like(want, -1)
+        assert lib.mp_w8a8_linear(x.data_ptr(), mod.weight.data_ptr(), w_scale.data_ptr(),
+                                  mod.bias.data_ptr() if mod.bias is not None else None, y.data_ptr(), m, n, k,
+                                  q2.data_ptr(), s2.data_ptr(), ws.data_ptr(), ws.numel(), None, st) == 0
+        assert torch.equal(q2, q) and torch.equal(s2, s) and torch.equal(y, want)
+        assert torch.equal(mod(x), want)
+    if n == k:                                                 # results over the rows
+        assert lib.mp_w8a8_linear(x.data_ptr(), mod.weight.data_ptr(), w_scale.data_ptr(),
+                                  mod.bias.data_ptr() if mod.bias is not None else None, x.data_ptr(), m, n, k,
+                                  q2.data_ptr(), s2.data_ptr(), ws.data_ptr(), ws.numel(), None, st) == 0
+        assert torch.equal(x, want) and torch.equal(q2, q)
 
 
 @pytest.mark.filterwarnings("ignore::RuntimeWarning")
