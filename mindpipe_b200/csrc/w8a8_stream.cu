@@ -19,7 +19,7 @@
 //   warp 8      TMA producer: one copy of weights and one of activations per stage
 //   warp 9      TMEM allocation and the MMA issuer
 // Where its stream is short a block takes less than half an SM, so the next product of a chain starts beside the end of this
-// one; its first weights are then already on the way (see early_weights).  A long stream has a longer ring (kLongStream).
+// one; its first weights are then already on the way (see early_weights).  A long stream has a longer ring (long_stream).
 //
 // With few activation values (quantise_in_stream) the kernel quantises the rows itself (QUANT): a launch less between two
 // products of a chain, which was 1 to 2 us of its own chain of load, reduction and store.  The epilogue warps and four more
@@ -44,11 +44,16 @@ constexpr int kWBytes = kRows * kStepK;
 constexpr int kChunk = 16;                       // tokens that pass through shared memory at a time
 constexpr int kPitch = kRows + 4;                // words between tokens there: 16-byte rows, lanes on different banks
 constexpr int kMaxRing = 8;
-// Blocks of at least kLongStream stages have kLongRing of them in flight, though they then take more than half an SM and the
+// Blocks of at least long_stream() stages have kLongRing of them in flight, though they then take more than half an SM and the
 // next product of a chain starts behind their end: with four (32 tokens) an SM has too little under way, with more than six
 // the HBM rate falls again (the Mixtral-shaped experts at 32 tokens, us: 4 stages 284, 6 262, 7 263, 8 270; 28672x4096 at one
-// row, 5 / 6 / 8 stages 24.0 / 23.4 / 23.6; 12288x4096, where a block has 21, is level).
-constexpr int kLongRing = 6, kLongStream = 40;
+// row, 5 / 6 / 8 stages 24.0 / 23.4 / 23.6).  Rings of half an SM are four stages or less from 32 tokens on, so there, and
+// where the start of the next product has less to hide because it quantises its rows first, half the length is enough
+// (line at 40 / 20 stages: experts of 3072x3072 at 64 tokens 69.0 / 65.8, of 2048x2048 at 32 41.1 / 40.9, a layer with its
+// rows quantised inside 52.0 / 51.6; but experts of 2048x4096 at 16 tokens 54.7 / 55.0, an asymmetric layer at 8 rows 91.8 /
+// 92.8).
+constexpr int kLongRing = 6;
+constexpr int long_stream(int tokens, bool quantising) { return tokens > 16 || quantising ? 20 : 40; }
 constexpr int kMaxExperts = 256;
 constexpr int kMaxGroups = 512;
 
@@ -567,14 +572,14 @@ int launch_w8a8_stream(int epi, const void* x_i8, int x_rows, const void* w_i8, 
   const int grid = want < kSmCount ? (int)want : kSmCount;
   // (with every expert taken once)
   const long long stages = (long long)(p.counts ? p.experts : 1) * p.row_blocks * p.steps * (epi == STREAM_SWIGLU ? 2 : 1);
-  const bool long_stream = stages >= (long long)ws::kLongStream * grid;
+  const bool is_long = stages >= (long long)ws::long_stream(tok, p.x != nullptr) * grid;
   if (p.x) {
     if (epi != STREAM_F16 || max_rows > ws::kMaxQuantRows || !aligned(p.x, 16)) return MP_ERR_UNSUPPORTED;
-    return long_stream ? launch_stream<16, STREAM_F16, true, true>(tw, tx, p, grid, st)
+    return is_long ? launch_stream<16, STREAM_F16, true, true>(tw, tx, p, grid, st)
                        : launch_stream<16, STREAM_F16, false, true>(tw, tx, p, grid, st);
   }
 #define MP_STREAM_EPI(TOK, EPI) \
-  return long_stream ? launch_stream<TOK, EPI, true>(tw, tx, p, grid, st) : launch_stream<TOK, EPI, false>(tw, tx, p, grid, st);
+  return is_long ? launch_stream<TOK, EPI, true>(tw, tx, p, grid, st) : launch_stream<TOK, EPI, false>(tw, tx, p, grid, st);
 #define MP_STREAM(TOK)                                     \
   switch (epi) {                                           \
     case STREAM_F16: MP_STREAM_EPI(TOK, STREAM_F16)        \

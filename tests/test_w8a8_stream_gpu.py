@@ -38,7 +38,7 @@ def test_streamed_product_gives_the_tiled_gemm_s_bits(kind, m, n, k):
 
 @pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 7, 8])
 @pytest.mark.parametrize("n,k", [(40, 16), (8, 144), (384, 4112), (1026, 1024), (20480, 256), (256, 8192), (4096, 4096),
-                                 (264, 28672)])
+                                 (264, 28672), (24576, 2064)])
 def test_rows_quantised_in_the_stream_give_the_quantiser_s_codes(m, n, k):
     g = torch.Generator(device="cuda").manual_seed(m * n + k)
     mod = SmoothQuantLinear.from_float(_linear(n, k, bias=m % 2 == 0))
