@@ -13,12 +13,15 @@
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/zeros.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <atomic>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -31,14 +34,90 @@
 namespace {
 
 // ------------------------------------------------------------------------------------------------- scratch buffers
-// Zero-initialised scratch, one per (device, stream, kind), grown on demand.  The decode kernels leave their part
-// zeroed where it has to be, so it is cleared only when it is (re)allocated; the kinds whose kernels overwrite theirs
-// freely (split-K partial sums) have buffers of their own.  Launches of one stream run in order, so they may share.
+// Zero-initialised scratch, one per (device, stream, kind) and one per captured stream of a graph, grown on demand.  The
+// decode kernels leave their part zeroed where it has to be, so it is cleared only when it is (re)allocated; the kinds whose
+// kernels overwrite theirs freely (split-K partial sums) have buffers of their own.  Launches of one stream run in order, so
+// they may share.
 enum WorkspaceKind { kDecode = 0, kPrefill = 1, kW8A8 = 2, kKinds = 3 };
 const char* const kKindNames[kKinds] = {"decode", "prefill", "w8a8"};
 
 std::mutex g_workspace_mutex;
 std::map<std::tuple<int, cudaStream_t, int>, at::Tensor> g_workspaces;
+
+// Scratch of a graph capture.  A captured launch holds the address for as long as its graph lives, and graphs that were
+// captured on one stream may be replayed side by side; so a capture never takes the stream's buffer, which a later call that
+// wants more replaces, but one of its own per captured stream.  It belongs to the graph (a user object of it) and goes back
+// to the allocator at the first capture after the graph is gone.  It does not come from the graph's own pool, where memory of
+// other tensors of the capture is used again: its words have to stay zero from one replay to the next.
+struct CaptureScratch {
+  std::vector<at::Tensor> buffers;                   // the last is in use; launches captured before it grew hold the others
+  std::vector<std::shared_ptr<std::atomic<bool>>> released;
+  bool over() const {
+    for (const auto& r : released)
+      if (!r->load(std::memory_order_acquire)) return false;
+    return true;
+  }
+};
+using CaptureKey = std::tuple<int, cudaStream_t, int, unsigned long long>;
+// (never destroyed: a graph may be released after this library's static objects)
+std::map<CaptureKey, CaptureScratch>& captures() {
+  static auto* all = new std::map<CaptureKey, CaptureScratch>;
+  return *all;
+}
+
+// Runs on a thread of the CUDA library, where no CUDA call is allowed: the memory is given back later.
+void CUDART_CB graph_released(void* p) {
+  auto* released = static_cast<std::shared_ptr<std::atomic<bool>>*>(p);
+  (*released)->store(true, std::memory_order_release);
+  delete released;
+}
+
+// A stream of this library's own, on which captures' scratch is allocated and cleared while another stream captures.
+cudaStream_t clearing_stream(int device) {
+  static auto* streams = new std::map<int, cudaStream_t>;
+  cudaStream_t& st = (*streams)[device];
+  if (!st) C10_CUDA_CHECK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  return st;
+}
+
+at::Tensor zeroed_bytes(int64_t bytes, int device) {
+  return at::zeros({bytes}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
+}
+
+// The caller holds g_workspace_mutex.
+at::Tensor capture_workspace(size_t nbytes, int device, cudaStream_t stream, int kind, unsigned long long id,
+                             cudaGraph_t graph) {
+  auto& all = captures();
+  CaptureScratch& scratch = all[CaptureKey(device, stream, kind, id)];
+  if (!scratch.buffers.empty() && static_cast<size_t>(scratch.buffers.back().numel()) >= nbytes) return scratch.buffers.back();
+  for (auto it = all.begin(); it != all.end();)
+    it = &it->second != &scratch && it->second.over() ? all.erase(it) : std::next(it);
+  // at least twice the one before, so that those that are kept for earlier launches add up to less than the last
+  const size_t least = scratch.buffers.empty() ? size_t(1) << 20 : 2 * static_cast<size_t>(scratch.buffers.back().numel());
+  // the capture's mode may forbid allocation and synchronisation, also of streams that do not capture
+  c10::cuda::CUDAStreamCaptureModeGuard relaxed{cudaStreamCaptureModeRelaxed};
+  c10::cuda::CUDAGuard on(static_cast<c10::DeviceIndex>(device));
+  at::Tensor buffer;
+  const cudaStream_t clearing = clearing_stream(device);
+  {
+    c10::cuda::CUDAStreamGuard guard(c10::cuda::getStreamFromExternal(clearing, static_cast<c10::DeviceIndex>(device)));
+    buffer = at::empty({static_cast<int64_t>(nbytes > least ? nbytes : least)},
+                       at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
+    C10_CUDA_CHECK(cudaMemsetAsync(buffer.data_ptr(), 0, static_cast<size_t>(buffer.numel()), clearing));
+    C10_CUDA_CHECK(cudaStreamSynchronize(clearing));
+  }
+  auto released = std::make_shared<std::atomic<bool>>(false);
+  auto* handle = new std::shared_ptr<std::atomic<bool>>(released);
+  cudaUserObject_t object = nullptr;
+  if (cudaUserObjectCreate(&object, handle, graph_released, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+    delete handle;
+    TORCH_CHECK(false, "scratch memory of a CUDA graph capture: the graph takes no user object");
+  }
+  C10_CUDA_CHECK(cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove));
+  scratch.buffers.push_back(buffer);
+  scratch.released.push_back(std::move(released));
+  return buffer;
+}
 
 // A copy of the tensor handle: it keeps the buffer alive until the launch is in the stream even if another thread
 // replaces it by a larger one meanwhile (the allocator hands freed memory on in stream order).
@@ -46,18 +125,20 @@ std::map<std::tuple<int, cudaStream_t, int>, at::Tensor> g_workspaces;
 // (decode steps are often captured on a stream of their own, and a linear that could do without scratch is not to fail there
 // for the sake of a faster kernel).
 at::Tensor workspace(size_t nbytes, int device, cudaStream_t stream, int kind, bool own_in_capture = false) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(stream, &capturing, &id, &graph) != cudaSuccess) cudaGetLastError();    // the launch will tell
   std::lock_guard<std::mutex> lock(g_workspace_mutex);
   at::Tensor& ws = g_workspaces[std::make_tuple(device, stream, kind)];
   if (!ws.defined() || static_cast<size_t>(ws.numel()) < nbytes) {
-    if (own_in_capture && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
-      return at::zeros({static_cast<int64_t>(nbytes)},
-                       at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
-    TORCH_CHECK(c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None,
+    if (own_in_capture && capturing != cudaStreamCaptureStatusNone) return zeroed_bytes(static_cast<int64_t>(nbytes), device);
+    TORCH_CHECK(capturing == cudaStreamCaptureStatusNone,
                 "scratch memory would be allocated during CUDA graph capture; "
                 "pass a preallocated workspace= (see new_workspace)");
-    const int64_t bytes = static_cast<int64_t>(nbytes > (size_t(1) << 20) ? nbytes : (size_t(1) << 20));
-    ws = at::zeros({bytes}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
+    ws = zeroed_bytes(static_cast<int64_t>(nbytes > (size_t(1) << 20) ? nbytes : (size_t(1) << 20)), device);
   }
+  if (capturing == cudaStreamCaptureStatusActive) return capture_workspace(nbytes, device, stream, kind, id, graph);
   return ws;
 }
 
@@ -480,7 +561,7 @@ PyObject* py_workspace(PyObject*, PyObject* args) {
   END_HANDLE_TH_ERRORS
 }
 
-// every cached scratch buffer, as (device index, tensor)
+// every cached scratch buffer and every graph's, as (device index, tensor)
 PyObject* py_workspaces(PyObject*, PyObject*) {
   HANDLE_TH_ERRORS
   std::vector<std::pair<int, at::Tensor>> all;
@@ -488,6 +569,9 @@ PyObject* py_workspaces(PyObject*, PyObject*) {
     std::lock_guard<std::mutex> lock(g_workspace_mutex);
     for (auto& kv : g_workspaces)
       if (kv.second.defined()) all.emplace_back(std::get<0>(kv.first), kv.second);
+    for (auto& kv : captures())
+      if (!kv.second.over())
+        for (auto& t : kv.second.buffers) all.emplace_back(std::get<0>(kv.first), t);
   }
   PyObject* list = PyList_New(0);
   for (auto& it : all) {

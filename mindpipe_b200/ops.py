@@ -39,7 +39,8 @@ def _ptr(t: torch.Tensor | None) -> int | None:
 
 
 def _workspace(nbytes: int, device: torch.device, kind: str = "decode", own_in_capture: bool = False) -> torch.Tensor:
-    """Zero-initialised scratch, one per (device, stream, kind), grown on demand (``csrc/host_path.cpp`` keeps it).
+    """Zero-initialised scratch, one per (device, stream, kind) and, under capture, one per captured stream of the graph,
+    grown on demand (``csrc/host_path.cpp`` keeps it).
 
     The decode kernels leave their part zeroed where it has to be, so it is
     cleared only when it is (re)allocated; the prefill and W8A8 split-K partial
