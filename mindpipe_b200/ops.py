@@ -45,8 +45,7 @@ def _workspace(nbytes: int, device: torch.device, kind: str = "decode", own_in_c
     The decode kernels leave their part zeroed where it has to be, so it is
     cleared only when it is (re)allocated; the prefill and W8A8 split-K partial
     sums overwrite theirs freely, hence the separate kinds.  With ``own_in_capture``
-    a graph capture on a stream that has none gets a zeroed buffer of its own from
-    the graph's memory instead of an error.
+    a graph capture may begin on a stream that has none; else that is an error.
     """
     index = device.index if device.index is not None else torch.cuda.current_device()
     return _lib.host().workspace(nbytes, index, kind, own_in_capture)

@@ -139,3 +139,25 @@ def test_scratch_goes_back_with_its_graph():
     assert count[-1] <= count[1] and len(set(addresses)) <= 4       # the same memory again
     kept = [_capture(fn, stream) for _ in range(4)]
     assert len({held.data_ptr() for _, _, held in kept}) == 4       # never while the graph is there
+
+
+@pytest.mark.parametrize("m", [1, 8, 16, 77])
+@torch.no_grad()
+def test_a_capture_on_a_fresh_stream_records_the_products_alone(m):
+    """Its scratch is cleared once, not by a fill in front of every linear."""
+    from cuda.bindings import runtime
+    calls = [_call("w4", m, n, k) for n, k in ((4096, 4096), (4096, 2048), (5120, 4096))]
+    want = [f().clone() for f in calls]
+    stream = torch.cuda.Stream()                             # (kept: another stream might get its handle and find scratch)
+    stream.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=stream):
+        got = [f() for f in calls]
+    err, _, count = runtime.cudaGraphGetNodes(runtime.cudaGraph_t(graph.raw_cuda_graph()), 0)
+    assert int(err) == 0 and count == len(calls)
+    graph.instantiate()
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    ops.check_device_errors()
+    assert all(torch.equal(y, w) for y, w in zip(got, want))
