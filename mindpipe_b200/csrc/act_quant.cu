@@ -387,12 +387,22 @@ extern "C" int mp_add_rmsnorm_quant(const void* x_f16, void* residual_f16, const
 // threads, 29.7 with 256; 8192 values 23.4 / 16.7 with 128; with zero points 35.9 / 32.0 and 26.3 / 17.9; a warp per row up to
 // 4096 values).  While all rows fit on the SMs side by side the chain of load, reduction, division and rounding is the time,
 // so a thread has one or two pieces of the row.  A Llama-8B layer's four products with their quantisations, 1 / 4 / 16 / 64 /
-// 148 rows, us: a warp per row of 4096 and 512 threads for 14336 58.8 / 60.4 / 65.0 / 69.1 / 86.5, this 56.3 / 57.7 / 62.6 /
-// 67.2 / 85.2 (two and four pieces a thread above 4096 56.7 / 58.2 / 62.7 / 67.7 / 85.8).
-// The line is four rows to an SM, which is what its threads hold of 512 to a row (200 / 333 / 500 / 1000 rows of that layer:
-// narrow blocks 89.8 / 114.9 / 124.5 / 189.2, wide ones 88.0 / 112.7 / 119.9 / 191.2; 333 and 2000 rows of a Llama-7B layer
-// with zero points 114.4 / 323.5 and 110.4 / 326.9; there one piece a thread is no better at 333 rows, 113.6).
-static bool many_rows(int M) { return M > 4 * kSmCount; }
+// 148 rows, us: a warp per row of 4096 and 512 threads for 14336 58.8 / 60.4 / 65.0 / 69.1 / 86.5, wide blocks 56.3 / 57.7 /
+// 62.6 / 67.2 / 85.2 (two and four pieces a thread above 4096 56.7 / 58.2 / 62.7 / 67.7 / 85.8).
+// Where the line is, by a quantisation and its product (4096 / 14336 output columns), us, wide blocks / narrow ones:
+//   above 8192 values a block has 1024 threads with two pieces each, and two of them fill an SM: 296 rows (11008 values, 297
+//     rows 25.1 / 24.6 and 60.6 / 60.2, 500 rows 29.5 / 26.7 and 68.5 / 65.3; 14336 values, 200 rows 26.1 / 25.9 and 53.0 /
+//     54.2)
+//   up to 8192, one piece a thread (and with zero points, whose blocks have 512 threads, up to 16384), four rows to an SM: 592
+//     (8192 values, 333 rows 20.2 / 21.3 and 51.3 / 52.8, 500 rows 21.1 / 21.7 and 52.1 / 53.0, 740 rows 27.4 / 26.1 at 4096
+//     columns; with zero points 333 and 2000 rows of a Llama-7B layer 110.4 / 114.4 and 326.9 / 323.5)
+//   up to 4096 values narrow is a warp, eight rows to a block.  From 65 to 256 rows (200 with zero points, 160 above 3072
+//     values) the product gains more from the SMs this leaves to its blocks, which set up meanwhile (it seems: the times are
+//     what was measured), than from the shorter chain: 2048 values, 64 rows 7.3 / 7.3 and 10.4 / 10.3, 224 rows 9.2 / 8.7 and
+//     14.8 / 14.4, 333 rows 10.6 / 10.0 and 19.5 / 21.5; 4096 values, 148 rows 11.7 / 11.2 and 19.5 / 19.3, 333 rows
+//     13.3 / 14.0 and 27.0 / 29.9
+constexpr int kNarrowFrom = 65;
+static bool wide_blocks(int M, int narrow_to, int wide_to) { return M < kNarrowFrom || (M > narrow_to && M <= wide_to); }
 
 extern "C" int mp_act_quant_per_token(const void* x_f16, int M, int K, void* q_i8, void* scale_f32,
                                       void* fake_f16, mp_stream_t stream) {
@@ -404,7 +414,7 @@ extern "C" int mp_act_quant_per_token(const void* x_f16, int M, int K, void* q_i
   int8_t* q = static_cast<int8_t*>(q_i8);
   float* sc = static_cast<float*>(scale_f32);
   __half* fk = static_cast<__half*>(fake_f16);
-  if (!many_rows(M) && K <= 16384) {
+  if (K <= 16384 && wide_blocks(M, K > 4096 ? 0 : K > 3072 ? 160 : 256, K > 8192 ? 2 * kSmCount : 4 * kSmCount)) {
     if (K <= 1024) return launch_chained(act_quant_kernel<128, 1>, dim3(M), dim3(128), 0, st, x, M, K, q, sc, fk);
     if (K <= 2048) return launch_chained(act_quant_kernel<256, 1>, dim3(M), dim3(256), 0, st, x, M, K, q, sc, fk);
     if (K <= 4096) return launch_chained(act_quant_kernel<512, 1>, dim3(M), dim3(512), 0, st, x, M, K, q, sc, fk);
@@ -437,7 +447,7 @@ extern "C" int mp_affine_quant_per_row(const void* x_f16, int M, int K, void* q_
   float *sc = static_cast<float*>(scale_f32), *ze = static_cast<float*>(zero_f32);
   int* rs = static_cast<int*>(rowsum_i32);
   __half* fk = static_cast<__half*>(fake_f16);
-  if (many_rows(M) && K > 2048 && K <= 16384) {
+  if (K > 2048 && K <= 16384 && !wide_blocks(M, K > 4096 ? 0 : K > 3072 ? 160 : 200, 4 * kSmCount)) {
     if (K <= 4096) return launch_chained(affine_quant_kernel<128, 4>, dim3(M), dim3(128), 0, st, x, K, q, sc, ze, rs, fk);
     if (K <= 8192) return launch_chained(affine_quant_kernel<128, 8>, dim3(M), dim3(128), 0, st, x, K, q, sc, ze, rs, fk);
     return launch_chained(affine_quant_kernel<256, 8>, dim3(M), dim3(256), 0, st, x, K, q, sc, ze, rs, fk);

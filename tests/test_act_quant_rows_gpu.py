@@ -40,3 +40,20 @@ def test_wide_blocks_give_the_bits_of_narrow_ones(k):
             q, s, fake = (torch.cat(t) for t in zip(*(ops.act_quant_per_token(p, want_fake=True) for p in x[:n].split(rows))))
             assert torch.equal(q, of[0][:n]) and torch.equal(s, of[1][:n])
             assert torch.equal(fake.view(torch.int16), of[2][:n].view(torch.int16))
+
+
+@pytest.mark.parametrize("rows", [64, 65, 160, 161, 200, 201, 256, 257, 296, 297, 592])
+@pytest.mark.parametrize("k", [2048, 3072, 3080, 4096, 4104, 8192, 8200, 16384])
+def test_either_side_of_the_lines_between_wide_and_narrow_blocks(k, rows):
+    """The bits of the rows one at a time, at the row counts and widths where the block shape changes."""
+    g = torch.Generator(device="cuda").manual_seed(k + rows)
+    x = torch.randn(rows, k, generator=g, device="cuda").half()
+    x[:, -1] *= 20
+    few = torch.tensor([0, 1, rows // 2, rows - 1], device="cuda")
+    whole, parts = ops.act_quant_per_token(x, want_fake=True), [ops.act_quant_per_token(x[i:i + 1], want_fake=True) for i in few]
+    for j in range(3):
+        assert torch.equal(whole[j][few], torch.cat([p[j] for p in parts]))
+    whole, parts = ops.affine_quant_per_row(x), [ops.affine_quant_per_row(x[i:i + 1]) for i in few]
+    for j, t in enumerate(whole):
+        if t is not None:
+            assert torch.equal(t[few], torch.cat([p[j] for p in parts]))
