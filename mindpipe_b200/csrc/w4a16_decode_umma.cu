@@ -207,6 +207,9 @@ __device__ __forceinline__ uint4 ld_relaxed_gpu_v4(const uint32_t* p) {
   asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ void prefetch_l2(const uint32_t* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
 __device__ __forceinline__ void st_relaxed_gpu_v4_zero(uint32_t* p) {
   asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1,%1,%1,%1};" ::"l"(p), "r"(0u) : "memory");
 }
@@ -431,6 +434,17 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
     const uint32_t sz_lane = du::kWBytes + row * 4;
     int s = set, xs = set, q = set;
     uint32_t phase = 0, xphase = 0, use = 0;
+    // The tiles that this block will add on their way to L2, from which the weights of other linears push those of a graph that
+    // is not replayed all the time (three graphs of a 7B layer at 16 rows in turn 41.7 -> 41.0 us; at 77 rows, eagerly, where
+    // they are six times as many bytes and there already, 65.0 -> 67.2, so not beyond 16).
+    if (PERM && closes) {
+      const int first_block = block_of(rb_lo * ST, p);
+      for (int b2 = first_block; b2 < blk; ++b2)
+#pragma unroll
+        for (int k = 0; k < kMine; ++k)
+          if (tid + k * kExpThreads < p.M * (du::kRows / 4))
+            prefetch_l2(p.tiles + (size_t)b2 * TOK * du::kRows + (tid + k * kExpThreads) * 4);
+    }
     for (int i = set; i < n_stages; i += C::kSets) {
       // FOLD: one look at all three barriers and one vote, where nothing is to be waited for: a wait that is over and its vote
       // cost 38 clocks a stage (the four linears of a 70B layer at 8 rows 95.1 -> 91.7 us; the exact form, whose arithmetic is
