@@ -41,7 +41,7 @@ int read_and_clear_decode_error(int* value);
 // tcgen05 kernel for M <= 128 with the weights as the tensor-memory operand (w4a16_decode_umma.cu)
 int launch_decode_umma(const void* x, const void* packed, const void* sz, const void* bias, void* y, int M, int N, int K,
                        int group, void* workspace, size_t workspace_bytes, cudaStream_t st, bool pdl,
-                       const HostCopies* copies = nullptr);
+                       bool early_tiles = true, const HostCopies* copies = nullptr);
 bool decode_umma_shape_ok(int M, int N, int K, int group);
 size_t decode_umma_workspace_bytes(int M, int K);
 size_t w4a16_gemm_partial_bytes(int M, int N, int K);   // w4a16_gemm.cu
@@ -880,7 +880,7 @@ int w4a16_linear(const void* x_f16, const void* packed_i32, const void* sz_f16x2
     if (!aligned(x_f16, 16) || !aligned(packed_i32, 16) || !aligned(sz_f16x2, 4) || !aligned(y_f16, 2)) return MP_ERR_ALIGNMENT;
     const int rc = launch_decode_umma(x_f16, packed_i32, sz_f16x2, bias_f16, y_f16, M, N, K, group, workspace,
                                       workspace_bytes, static_cast<cudaStream_t>(stream),
-                                      early < 0 ? decode_programmatic_launch() : early > 0, copies);
+                                      early < 0 ? decode_programmatic_launch() : early > 0, early < 0, copies);
     if (carried) *carried = copies && rc == MP_OK;
     if (rc != MP_ERR_UNSUPPORTED) return rc;                     // (no workspace, odd alignment: the others)
   }

@@ -142,6 +142,7 @@ struct DecodeUmmaParams {
   int ring;                // weight stages in the ring
   int first;               // weight stages requested before the activations, at most `ring`
   int early_weights;       // 1: fetch weights before the previous kernel of the stream has finished
+  int early_tiles;         // 1: tiles to L2 before the first stage (up to 16 rows)
   HostCopies copies;       // from host memory, every block its share; count 0: none
   uint32_t* tiles;         // workspace: [grid][TOK][128] inverted fp32 words, zero between calls
   int* error_word;
@@ -435,9 +436,10 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
     int s = set, xs = set, q = set;
     uint32_t phase = 0, xphase = 0, use = 0;
     // The tiles that this block will add on their way to L2, from which the weights of other linears push those of a graph that
-    // is not replayed all the time (three graphs of a 7B layer at 16 rows in turn 41.7 -> 41.0 us; at 77 rows, eagerly, where
-    // they are six times as many bytes and there already, 65.0 -> 67.2, so not beyond 16).
-    if (PERM && closes) {
+    // is not replayed all the time (three graphs of a 7B layer at 16 rows in turn, us: without 41.7, here 41.0, by the side warp
+    // after the wait for the kernel before 41.1, from the loop below 43.0).  At 77 rows, where the tiles are six times as many
+    // bytes, it costs more than it gives (eager, 65.0 -> 67.2), so not beyond 16; and beside host copies too (65.7 -> 66.3).
+    if (PERM && closes && p.early_tiles) {
       const int first_block = block_of(rb_lo * ST, p);
       for (int b2 = first_block; b2 < blk; ++b2)
 #pragma unroll
@@ -746,7 +748,7 @@ static int launch_umma(const CUtensorMap& tw, const CUtensorMap& tx, const CUten
 // calls that share it must not overlap on the GPU.
 int launch_decode_umma(const void* x, const void* packed, const void* sz, const void* bias, void* y, int M, int N, int K,
                        int group, void* workspace, size_t workspace_bytes, cudaStream_t st, bool early_weights,
-                       const HostCopies* copies) {
+                       bool early_tiles, const HostCopies* copies) {
   if (!decode_umma_shape_ok(M, N, K, group)) return MP_ERR_UNSUPPORTED;
   const int tok = du::tokens_for(M);
   if (!workspace || workspace_bytes < du::workspace_bytes(M) || !aligned(workspace, 16)) return MP_ERR_UNSUPPORTED;
@@ -781,6 +783,7 @@ int launch_decode_umma(const void* x, const void* packed, const void* sz, const 
   p.groups_per_stage = gps;
   p.gshift = group == 32 ? 5 : group == 64 ? 6 : 7;
   p.early_weights = early_weights ? 1 : 0;
+  p.early_tiles = early_tiles ? 1 : 0;
   if (copies) p.copies = *copies;
   p.tiles = reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(workspace) + du::kTileOffset);
   int rc_err = MP_OK;
