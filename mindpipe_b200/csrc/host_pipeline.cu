@@ -4,10 +4,12 @@
 // What bounds it: PCIe (about 50 GB/s each way), the products, the first rows' way in and the last result's way out.  While
 // results leave, reads of host memory wait behind them (131 KB: 6 us alone, 59 beside a long copy out), so all rows come in
 // before the first result goes: a copy kernel brings the first linear's, and its product, on the weight stream, the others'
-// in a warp of its own.  Results leave by the copy engine, on a stream of their own, while the next product runs (the events
-// between products do not end the overlap of one's beginning with the end of the one before), so the linear with the smallest
-// result goes last: a copy kernel takes it.  Up to kDirectBytes each way one such kernel brings everything and one takes everything
-// back.
+// in a warp of its own.  So a linear that runs there goes first (outputs 1024, 1024 and 4096 of 4096 columns, given in that
+// order, at 16 rows 38.1 -> 33.5 us); where none does, a copy kernel on the side stream brings the others' rows beside the
+// first product (four linears of 256x11008 at 16 rows 66.3 us, by a launch behind that product 72.5).  Results leave by the copy
+// engine, on a stream of their own, while the next product runs (the events between products do not end the overlap of one's
+// beginning with the end of the one before), so the linear with the smallest result goes last: a copy kernel takes it.  Up to
+// kDirectBytes each way one such kernel brings everything and one takes everything back.
 // A 7B layer's four linears at 16 rows, 0.75 MB in and 1.36 MB out, 42 us of products: 68 us; 81 with the others' rows
 // on a stream of their own, where they kept the first one's from arriving (21 us); 76 with each product bringing the next
 // one's rows, against the results; 76 with the products taking the results along too, since a kernel that has stored to host
@@ -21,6 +23,8 @@
 
 namespace mp {
 
+// Whether mp_w4a16_linear takes copies along for such a call (with scratch and 16-byte aligned weights).  w4a16_decode.cu
+bool w4a16_linear_takes_copies(int M, int N, int K, int group);
 // mp_w4a16_linear with the kernels' weights requested before the kernel before has finished (early > 0), or as the
 // process-wide switch says (early < 0); `copies` go along where *carried says so afterwards.  w4a16_decode.cu
 int w4a16_linear(const void* x, const void* packed, const void* sz, const void* bias, void* y, int M, int N, int K, int group,
@@ -52,10 +56,15 @@ void add_copy(HostCopies& list, const void* src, void* dst, size_t bytes) {
 
 size_t row_bytes(const mp_host_linear& c) { return (size_t)c.M * c.K * 2; }
 size_t result_bytes(const mp_host_linear& c) { return (size_t)c.M * c.N * 2; }
+bool takes_copies(const mp_host_linear& c) {
+  return w4a16_linear_takes_copies(c.M, c.N, c.K, c.group) && c.workspace &&
+         c.workspace_bytes >= mp_w4a16_linear_workspace_bytes(c.M, c.N, c.K, c.group) && aligned(c.packed_i32, 16) &&
+         aligned(c.sz_f16x2, 16);
+}
 }  // namespace
 
-// The stream for results beside a caller's stream, shared by all pipelines that run there and given back with the last of
-// them (making one takes some 150 us; with two or four of them in turn a 7B layer took 73 to 87 us instead of 68 to 71).
+// The stream for results (and rows) beside a caller's stream, shared by all pipelines that run there and given back with the
+// last of them (making one takes some 150 us; with two or four of them in turn a 7B layer took 73 to 87 us instead of 68 to 71).
 struct SideStream {
   cudaStream_t out = nullptr;
   int users = 0;
@@ -73,11 +82,13 @@ struct HostPipeline {
   mp_host_linear linear[kMaxLinears];              // in the order they run
   HostCopies first{}, others{}, back{};            // rows of the first linear (or of all), of the others; the last result (or all)
   bool direct_out = false;
+  bool beside = false;                             // the others' rows come on the side stream, not with the first product
   cudaStream_t out = nullptr;
-  cudaEvent_t sent = nullptr, done[kMaxLinears] = {};
+  cudaEvent_t begun = nullptr, arrived = nullptr, sent = nullptr, done[kMaxLinears] = {};
   std::mutex enqueue;                              // a call's events are recorded and waited for before the next call's
   ~HostPipeline() {
-    if (sent) cudaEventDestroy(sent);
+    for (cudaEvent_t e : {begun, arrived, sent})
+      if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : done)
       if (e) cudaEventDestroy(e);
     if (has_side) {
@@ -94,7 +105,6 @@ struct HostPipeline {
 static int make_pipeline(HostPipeline& p, const mp_host_linear* linears, int count) {
   MP_CUDA_TRY(cudaGetDevice(&p.device));
   size_t x_bytes = 0, y_bytes = 0;
-  int smallest = 0;
   for (int i = 0; i < count; ++i) {
     const mp_host_linear& c = linears[i];
     if (!c.x_host_f16 || !c.x_stage_f16 || !c.y_stage_f16 || !c.y_host_f16 || c.M <= 0 || c.K <= 0 || c.N <= 0)
@@ -111,19 +121,37 @@ static int make_pipeline(HostPipeline& p, const mp_host_linear* linears, int cou
     if (!aligned(c.x_stage_f16, 16) || !aligned(c.y_stage_f16, 16)) return MP_ERR_ALIGNMENT;
     x_bytes += xb;
     y_bytes += yb;
-    if ((size_t)c.M * c.N < (size_t)linears[smallest].M * linears[smallest].N) smallest = i;
+  }
+  auto smallest_but = [&](int not_this) {
+    int best = -1;
+    for (int i = 0; i < count; ++i)
+      if (i != not_this && (best < 0 || result_bytes(linears[i]) < result_bytes(linears[best]))) best = i;
+    return best;
+  };
+  const bool rows_apart = count > 1 && x_bytes > kDirectBytes;
+  int first = -1, last = smallest_but(-1);
+  if (rows_apart) {
+    for (int i = 0; i < count && first < 0; ++i)
+      if (i != last && takes_copies(linears[i])) first = i;
+    if (first < 0 && takes_copies(linears[last])) {
+      first = last;
+      last = smallest_but(first);
+    }
+    p.beside = first < 0;
   }
   p.count = count;
-  for (int i = 0, at = 0; i < count; ++i)
-    if (i != smallest) p.linear[at++] = linears[i];
-  p.linear[count - 1] = linears[smallest];
+  int at = 0;
+  if (first >= 0) p.linear[at++] = linears[first];
+  for (int i = 0; i < count; ++i)
+    if (i != first && i != last) p.linear[at++] = linears[i];
+  p.linear[at] = linears[last];
   for (int i = 0; i < count; ++i) {
     const mp_host_linear& c = p.linear[i];
     add_copy(i == 0 || x_bytes <= kDirectBytes ? p.first : p.others, c.x_host_f16, c.x_stage_f16, row_bytes(c));
     if (i == count - 1 || y_bytes <= kDirectBytes) add_copy(p.back, c.y_stage_f16, c.y_host_f16, result_bytes(c));
   }
   p.direct_out = count == 1 || y_bytes <= kDirectBytes;
-  if (!p.direct_out) {
+  if (!p.direct_out || p.beside) {
     std::lock_guard<std::mutex> lock(g_sides_mutex);
     SideStream side;
     auto at = sides().find({p.device, p.stream});
@@ -136,6 +164,11 @@ static int make_pipeline(HostPipeline& p, const mp_host_linear* linears, int cou
     sides()[{p.device, p.stream}] = side;
     p.has_side = true;
     p.out = side.out;
+  }
+  if (p.beside) {
+    for (cudaEvent_t* e : {&p.begun, &p.arrived}) MP_CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  }
+  if (!p.direct_out) {
     MP_CUDA_TRY(cudaEventCreateWithFlags(&p.sent, cudaEventDisableTiming));
     for (int i = 0; i < count; ++i) MP_CUDA_TRY(cudaEventCreateWithFlags(&p.done[i], cudaEventDisableTiming));
   }
@@ -149,16 +182,25 @@ static int run_pipeline(HostPipeline& p) {
   if (capturing != cudaStreamCaptureStatusNone) return mp_w4a16_linear_decode_host_many(p.linear, p.count, st);
   std::lock_guard<std::mutex> lock(p.enqueue);
   int rc;
+  if (p.beside) {
+    MP_CUDA_TRY(cudaEventRecord(p.begun, st));               // the call before still reads its rows until here
+    MP_CUDA_TRY(cudaStreamWaitEvent(p.out, p.begun, 0));
+  }
   if ((rc = launch_copy(p.first, true, st)) != MP_OK) return rc;
   for (int i = 0; i < p.count; ++i) {
     const mp_host_linear& c = p.linear[i];
-    const HostCopies* others = i == 0 && p.others.count ? &p.others : nullptr;
+    const HostCopies* others = i == 0 && p.others.count && !p.beside ? &p.others : nullptr;
     bool carried = false;
     // the kernel before in the stream is this pipeline's own and writes no weights
     rc = w4a16_linear(c.x_stage_f16, c.packed_i32, c.sz_f16x2, c.bias_f16, c.y_stage_f16, c.M, c.N, c.K, c.group, c.workspace,
                       c.workspace ? c.workspace_bytes : 0, nullptr, 1, st, others, &carried);
     if (rc != MP_OK) return rc;
-    if (others && !carried && (rc = launch_copy(p.others, true, st)) != MP_OK) return rc;    // (small weights: a kernel without a place for them)
+    if (others && !carried && (rc = launch_copy(p.others, true, st)) != MP_OK) return rc;    // (the kernel was switched since)
+    if (i == 0 && p.beside) {
+      if ((rc = launch_copy(p.others, true, p.out)) != MP_OK) return rc;
+      MP_CUDA_TRY(cudaEventRecord(p.arrived, p.out));
+      MP_CUDA_TRY(cudaStreamWaitEvent(st, p.arrived, 0));
+    }
     if (!p.direct_out && i < p.count - 1) {
       MP_CUDA_TRY(cudaEventRecord(p.done[i], st));
       MP_CUDA_TRY(cudaStreamWaitEvent(p.out, p.done[i], 0));

@@ -869,6 +869,10 @@ extern "C" size_t mp_w4a16_linear_workspace_bytes(int M, int N, int K, int group
 }
 
 namespace mp {
+bool w4a16_linear_takes_copies(int M, int N, int K, int group) {
+  return M > 0 && M <= 16 && N > 0 && K > 0 && group > 0 && K % group == 0 && linear_kernel(M, N, K, group) == kStream;
+}
+
 int w4a16_linear(const void* x_f16, const void* packed_i32, const void* sz_f16x2, const void* bias_f16, void* y_f16, int M,
                  int N, int K, int group, void* workspace, size_t workspace_bytes, int* error_word, int early,
                  mp_stream_t stream, const HostCopies* copies, bool* carried) {

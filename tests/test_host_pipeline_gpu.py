@@ -11,7 +11,11 @@ pytestmark = pytest.mark.gpu
 SETS = {"carried": [(12288, 4096), (4096, 11008), (4096, 4096), (1024, 4096)],
         "first kernel takes none": [(512, 2048), (22016, 4096), (4096, 11008)],
         "one linear": [(22016, 4096)],
-        "everything in one copy each way": [(2048, 2048), (1024, 2048)]}
+        "everything in one copy each way": [(2048, 2048), (1024, 2048)],
+        "a later one goes first": [(1024, 2048), (22016, 4096), (512, 11008)],
+        "only the smallest result's kernel takes some": [(1536, 2048), (1536, 2048), (1024, 8192)],
+        "no kernel takes any": [(512, 4096)] * 6,
+        "no kernel takes any, results beside the products": [(2040, 3072)] * 9}
 
 
 @pytest.mark.parametrize("shapes", list(SETS.values()), ids=list(SETS))
