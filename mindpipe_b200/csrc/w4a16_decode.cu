@@ -877,6 +877,7 @@ int w4a16_linear(const void* x_f16, const void* packed_i32, const void* sz_f16x2
                  int N, int K, int group, void* workspace, size_t workspace_bytes, int* error_word, int early,
                  mp_stream_t stream, const HostCopies* copies, bool* carried) {
   if (carried) *carried = false;
+  if (M > 16) copies = nullptr;
   if (!x_f16 || !packed_i32 || !sz_f16x2 || !y_f16 || M <= 0 || N <= 0 || K <= 0 || group <= 0) return MP_ERR_INVALID_ARG;
   if (K % group != 0) return MP_ERR_UNSUPPORTED;
   const LinearKernel kernel = linear_kernel(M, N, K, group);

@@ -35,7 +35,7 @@
 //   warp 20      TMA producer of weights and (scale, zero) pairs
 //   warp 21      TMEM allocation and the MMA issuer
 //   warp 22      TMA producer of activations
-//   warp 23      copies from host memory, where the call brings some
+//   warp 23      copies from host memory, in a launch that brings some
 // Expansion emits the columns of a packed word in the order (k0,k4,k1,k5,k2,k6,k3,k7).  Up to 16 rows the expansion warps
 // apply the same permutation in place to the 16-byte chunks of the stage's activation tile (a chunk is one token's eight
 // columns of one word, so the swizzle does not matter); with more rows they put the words back in order, see Cfg.  (Warps
@@ -79,7 +79,8 @@ struct Int { static constexpr int value = N; };
 
 // TOK: token rows of the MMA (its N); XROWS: token rows of the activation tile in shared memory (8 where no more exist:
 // the MMA then reads whatever follows for the other eight, whose results are not used)
-template <int TOK, int XROWS, bool FOLD>
+// CARRY: a warp more, for copies from host memory (up to 16 rows)
+template <int TOK, int XROWS, bool FOLD, bool CARRY>
 struct Cfg {
   // the columns of an expanded word come out as (k0,k4) (k1,k5) ..: the activations are put into that order, in shared
   // memory, or (PERM false) the words back into theirs.  Permuting the activations of 64 tokens per block and stage cost the
@@ -96,7 +97,7 @@ struct Cfg {
   static constexpr int kEpiWarp0 = 4 * kParts * kSets;
   static constexpr int kWeightWarp = kEpiWarp0 + 4, kMmaWarp = kWeightWarp + 1, kXWarp = kMmaWarp + 1;
   static constexpr int kSideWarp = kXWarp + 1;
-  static constexpr int kThreads = 32 * (kSideWarp + 1);
+  static constexpr int kThreads = 32 * (kSideWarp + (CARRY ? 1 : 0));
   static constexpr int kXSub = XROWS * 128;           // [XROWS x 64 columns] fp16
   static constexpr int kXBytes = (PERM ? 4 : 2) * kXSub;        // a tile of the ring: a stage, or half of one
   // activation tiles in flight: enough to hide the latency of their loads behind the stages before (with one per slot the
@@ -143,9 +144,18 @@ struct DecodeUmmaParams {
   int first;               // weight stages requested before the activations, at most `ring`
   int early_weights;       // 1: fetch weights before the previous kernel of the stream has finished
   int early_tiles;         // 1: tiles to L2 before the first stage (up to 16 rows)
-  HostCopies copies;       // from host memory, every block its share; count 0: none
   uint32_t* tiles;         // workspace: [grid][TOK][128] inverted fp32 words, zero between calls
   int* error_word;
+};
+
+// The list of copies is in the arguments, and the warp that copies in the block, of the launches that bring copies alone: in
+// all of them they cost four captured linears of a 7B layer at 16 rows 0.15 us (41.15 -> 41.00), a 70B layer at 8 rows 0.5
+// (106.4 -> 105.8), and the exact form up to 16 rows a spilled register.
+template <bool CARRY>
+struct DecodeUmmaArgs : DecodeUmmaParams {};
+template <>
+struct DecodeUmmaArgs<true> : DecodeUmmaParams {
+  HostCopies copies;       // from host memory, every block its share
 };
 
 // The stage range of block b is [range_start(b), range_start(b + 1)): p.share stages each, one more for the first p.extra.
@@ -248,11 +258,11 @@ __device__ __forceinline__ void expand8(uint32_t q, __half2 zl, __half2 zh, uint
   v[3] = h2_as_u32(__hsub2(*reinterpret_cast<const __half2*>(&d), zh));
 }
 
-template <int TOK, int XROWS, bool FOLD>
-__global__ void __launch_bounds__(du::Cfg<TOK, XROWS, FOLD>::kThreads, 1)
+template <int TOK, int XROWS, bool FOLD, bool CARRY>
+__global__ void __launch_bounds__(du::Cfg<TOK, XROWS, FOLD, CARRY>::kThreads, 1)
 w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
-                         const __grid_constant__ CUtensorMap tmap_sz, const DecodeUmmaParams p) {
-  using C = du::Cfg<TOK, XROWS, FOLD>;
+                         const __grid_constant__ CUtensorMap tmap_sz, const DecodeUmmaArgs<CARRY> p) {
+  using C = du::Cfg<TOK, XROWS, FOLD, CARRY>;
   constexpr int kXSub = C::kXSub, kXBytes = C::kXBytes, kXRing = C::kXRing;
   constexpr bool PERM = C::PERM;
   extern __shared__ unsigned char smem_raw[];
@@ -586,7 +596,7 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
     }
   } else if (warp == C::kSideWarp) {
     // ------------------------------------------------------------ copies: beside the product, which ends when they have ended
-    if (p.copies.count > 0) {
+    if constexpr (CARRY) {
       chain_wait();
       copy_pieces(p.copies, blk * 32 + lane, static_cast<int>(gridDim.x) * 32, true);
     }
@@ -720,11 +730,14 @@ bool decode_umma_shape_ok(int M, int N, int K, int group) {
   return group == 32 || group == 64 || group == 128 || group == du::kStageK || group % du::kStageK == 0;
 }
 
-template <int TOK, int XROWS, bool FOLD>
-static int launch_umma(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tsz, DecodeUmmaParams p, int grid,
-                       cudaStream_t st) {
-  using C = du::Cfg<TOK, XROWS, FOLD>;
-  auto kern = w4a16_decode_umma_kernel<TOK, XROWS, FOLD>;
+template <int TOK, int XROWS, bool FOLD, bool CARRY = false>
+static int launch_umma(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& tsz, const DecodeUmmaParams& params,
+                       int grid, cudaStream_t st, const HostCopies* copies = nullptr) {
+  using C = du::Cfg<TOK, XROWS, FOLD, CARRY>;
+  auto kern = w4a16_decode_umma_kernel<TOK, XROWS, FOLD, CARRY>;
+  DecodeUmmaArgs<CARRY> p;
+  static_cast<DecodeUmmaParams&>(p) = params;
+  if constexpr (CARRY) p.copies = *copies;
   static thread_local int configured_device = -1;
   int device = 0;
   MP_CUDA_TRY(cudaGetDevice(&device));
@@ -784,12 +797,19 @@ int launch_decode_umma(const void* x, const void* packed, const void* sz, const 
   p.gshift = group == 32 ? 5 : group == 64 ? 6 : 7;
   p.early_weights = early_weights ? 1 : 0;
   p.early_tiles = early_tiles ? 1 : 0;
-  if (copies) p.copies = *copies;
   p.tiles = reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(workspace) + du::kTileOffset);
   int rc_err = MP_OK;
   p.error_word = decode_error_word_ptr(&rc_err);
   if (rc_err != MP_OK) return rc_err;
   const bool fold = group % 128 == 0;
+  if (copies) {
+    if (tok > 16) return MP_ERR_INVALID_ARG;
+    if (M <= 8)
+      return fold ? launch_umma<16, 8, true, true>(tw, tx, tsz, p, grid, st, copies)
+                  : launch_umma<16, 8, false, true>(tw, tx, tsz, p, grid, st, copies);
+    return fold ? launch_umma<16, 16, true, true>(tw, tx, tsz, p, grid, st, copies)
+                : launch_umma<16, 16, false, true>(tw, tx, tsz, p, grid, st, copies);
+  }
   if (M <= 8) return fold ? launch_umma<16, 8, true>(tw, tx, tsz, p, grid, st) : launch_umma<16, 8, false>(tw, tx, tsz, p, grid, st);
   if (tok == 16) return fold ? launch_umma<16, 16, true>(tw, tx, tsz, p, grid, st) : launch_umma<16, 16, false>(tw, tx, tsz, p, grid, st);
   switch (tok) {
