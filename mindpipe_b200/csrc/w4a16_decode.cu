@@ -847,12 +847,15 @@ static LinearKernel linear_kernel(int M, int N, int K, int group) {
     return stream ? kStream : kGemm;
   }
   if (M > 16) return kStream;
-  // Below, the stream kernel but for small weights, where its longer pipeline shows.  us, ring / stream, without early weights:
-  // 9..16 rows, which double the ring kernel's MMAs: 2048x2048 4.8 / 4.1, 1024x4096 5.0 / 5.2, 2048x4096 6.4 / 5.5,
-  // 1024x8192 7.2 / 6.0, 12288x4096 18.5 / 9.4.
+  // Below, the stream kernel but for small weights, where its longer pipeline shows.  us, ring / stream, without early weights,
+  // groups of 128 and (of 64): 9..16 rows, which double the ring kernel's MMAs, at 16 rows 1024x4096 5.0 / 5.5 (5.0 / 6.1),
+  // 2048x2048 4.9 / 4.4 (4.9 / 5.0), 2048x4096 6.5 / 5.8 (6.6 / 6.6), 1024x8192 7.5 / 6.3 (7.1 / 7.0), 4096x4096 7.3 / 5.9
+  // (7.4 / 6.7), 12288x4096 17.8 / 9.2 (18.0 / 10.3).  Groups of 32 are within 0.2 of those of 64 on either side.
   if (M > 8) return packed >= ((size_t)4 << 20) || (packed >= ((size_t)2 << 20) && N >= 2048) ? kStream : kRing;
-  // Up to 8: 1024x4096 4.2 / 4.8, 2048x4096 5.1 / 5.2, 4096x2048 5.5 / 4.5, 3072x4096 5.5 / 5.3, 8192x8192 11.8 / 10.5,
-  // 28672x4096 19.5 / 15.1.
+  // Up to 8, at 8 rows: 1024x4096 4.1 / 5.0 (4.4 / 5.4), 2048x4096 5.1 / 5.3 (5.7 / 5.8), 1024x8192 5.7 / 5.7 (6.3 / 6.2),
+  // 4096x2048 5.5 / 4.5 (5.5 / 5.1), 3072x4096 5.5 / 5.5 (6.1 / 6.1), 4096x4096 6.3 / 5.5 (6.7 / 6.2), 8192x8192 12.0 / 10.3
+  // (13.8 / 11.6), 12288x4096 13.2 / 8.8 (14.2 / 9.8).  The stream's exact form, for groups of 32 and 64, costs it as much as
+  // the ring kernel's costs that, so the line is the same for all groups.
   return packed >= ((size_t)5 << 20) || (packed >= ((size_t)4 << 20) && N >= 4096) ? kStream : kRing;
 }
 

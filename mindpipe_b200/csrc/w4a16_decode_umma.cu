@@ -66,9 +66,11 @@ constexpr int kMaxRing = 8, kMaxXRing = 8;          // (eight weight stages; ten
 // Weight stages requested before the activations, which queue behind them: with early weights the time up to the wait for
 // the kernel before is theirs (12288x4096 at 16 rows in a chain, us: 4 or 5 stages 9.2, 6 9.5, the whole ring 10.1).
 constexpr int kFirstEarly = 5, kFirst = 1;
-// Stages brought to L2 while the kernel before ends.  A prefetch and the load after it cost L2 more than the load alone, so
-// more of them slow a short stream, fewer a long one (us without early weights, 3 / 6 / 10 stages: 12288x4096 at 16 rows 9.5 /
-// 9.6 / 10.1, 28672x8192 at 8 27.1 / 26.7 / 26.5; 10.5 and 26.7 without the (scale, zero) pairs beside the weights).
+// Stages brought to L2 while the kernel before ends.  A prefetch and the load after it cost L2 more than the load alone (us
+// without early weights, 3 / 4 / 6 / 10 stages: 4096x4096 at 1 row 5.20 / 5.38 / 5.36 / 5.31, 12288x4096 at 16 9.22 / 9.13 /
+// 9.40 / 9.92 and at 77 13.20 / 13.03 / 13.06 / 13.43, 8192x28672 at 8 24.95 / 24.85 / 24.74 / 25.29, 28672x8192 at 8 24.46 /
+// 24.44 / 24.67 / 25.20; groups of 64: 12288x4096 at 16 10.14 / 10.10 / 10.34 / 10.93, 8192x28672 at 8 28.69 / 27.83 / 28.44 /
+// 29.37).
 constexpr int kPrefetch = 4;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kASlotCols = kStageK / 2;          // two columns of K per 32-bit register
@@ -102,7 +104,7 @@ struct Cfg {
   static constexpr int kXBytes = (PERM ? 4 : 2) * kXSub;        // a tile of the ring: a stage, or half of one
   // activation tiles in flight: enough to hide the latency of their loads behind the stages before (with one per slot the
   // expansion warps waited half their time); with PERM at most six, see the wait for a slot
-  static constexpr int kXRing = TOK == 16 ? 6 : TOK <= 64 ? 6 : 4;
+  static constexpr int kXRing = TOK <= 64 ? 6 : 4;
   // accumulators: FOLD two per slot (one for each 128 columns), else one per segment in turn
   static constexpr int kAccs = FOLD ? 2 * kSlots : TOK > 64 ? 1 : 2;
   static constexpr uint32_t kASlot0 = kAccs * TOK;
