@@ -23,3 +23,19 @@ def golden():
         return np.load(GOLDEN / name)
 
     return load
+
+
+@pytest.fixture
+def new_stream():
+    """Makes streams that have run nothing, and so have no scratch: torch hands out 32 in turn."""
+    import torch
+    from cuda.bindings import runtime
+
+    def make():
+        err, handle = runtime.cudaStreamCreateWithFlags(runtime.cudaStreamNonBlocking)
+        assert int(err) == 0
+        stream = torch.cuda.ExternalStream(int(handle))      # (never destroyed: its handle does not come back)
+        stream.wait_stream(torch.cuda.current_stream())
+        return stream
+
+    return make

@@ -8,19 +8,6 @@ from mindpipe_b200.modules import SmoothQuantLinear, SmoothQuantPackedMoeExperts
 pytestmark = pytest.mark.gpu
 
 
-_streams = []
-
-
-def _new_stream():
-    """A stream that has run nothing (torch hands out 32 in turn, and one that has been used has scratch)."""
-    from cuda.bindings import runtime
-    err, handle = runtime.cudaStreamCreateWithFlags(runtime.cudaStreamNonBlocking)
-    assert int(err) == 0
-    _streams.append(torch.cuda.ExternalStream(int(handle)))
-    _streams[-1].wait_stream(torch.cuda.current_stream())
-    return _streams[-1]
-
-
 def _linear(cls, n, k):
     lin = torch.nn.Linear(k, n, bias=False, device="meta", dtype=torch.float16)
     lin.weight = torch.nn.Parameter((torch.randn(n, k, device="cuda") * 0.02).half(), requires_grad=False)
@@ -61,10 +48,10 @@ CALLS = [("w4", 1, 4096, 4096), ("w4", 8, 8192, 8192), ("w4", 16, 4096, 2048), (
 
 @pytest.mark.parametrize("kind,m,n,k", CALLS)
 @torch.no_grad()
-def test_replay_after_the_stream_s_scratch_has_grown(kind, m, n, k):
+def test_replay_after_the_stream_s_scratch_has_grown(kind, m, n, k, new_stream):
     fn, larger = _call(kind, m, n, k), [_call("w4", 17, 4096, 4096), _call("w4", 128, 8192, 2048), _experts()]
     want = fn().clone()
-    stream = _new_stream()
+    stream = new_stream()
     with torch.cuda.stream(stream):
         fn()
         own = ops._workspace(1, torch.device("cuda"))
@@ -88,10 +75,10 @@ def test_replay_after_the_stream_s_scratch_has_grown(kind, m, n, k):
 
 @pytest.mark.parametrize("kind,m,n,k", CALLS)
 @torch.no_grad()
-def test_graphs_of_one_stream_side_by_side(kind, m, n, k):
+def test_graphs_of_one_stream_side_by_side(kind, m, n, k, new_stream):
     calls = [_call(kind, m, n, k) for _ in range(2)]
     want = [f().clone() for f in calls]
-    stream, streams = _new_stream(), [_new_stream(), _new_stream()]
+    stream, streams = new_stream(), [new_stream(), new_stream()]
     with torch.cuda.stream(stream):
         calls[0]()
     stream.synchronize()
@@ -108,11 +95,11 @@ def test_graphs_of_one_stream_side_by_side(kind, m, n, k):
 
 
 @torch.no_grad()
-def test_scratch_that_grows_within_a_capture():
+def test_scratch_that_grows_within_a_capture(new_stream):
     """Launches captured before it grew keep what they hold."""
     calls = [_call("w4", m, 4096, 4096) for m in (8, 32, 128, 16, 77)]
     want = [f().clone() for f in calls]
-    stream = _new_stream()
+    stream = new_stream()
     with torch.cuda.stream(stream):
         for f in calls:
             f()
@@ -128,9 +115,9 @@ def test_scratch_that_grows_within_a_capture():
 
 
 @torch.no_grad()
-def test_scratch_goes_back_with_its_graph():
+def test_scratch_goes_back_with_its_graph(new_stream):
     fn = _call("w4", 16, 4096, 4096)
-    stream = _new_stream()
+    stream = new_stream()
     with torch.cuda.stream(stream):
         want = fn().clone()
     stream.synchronize()
@@ -151,12 +138,12 @@ def test_scratch_goes_back_with_its_graph():
 
 @pytest.mark.parametrize("m", [1, 8, 16, 77])
 @torch.no_grad()
-def test_a_capture_on_a_fresh_stream_records_the_products_alone(m):
+def test_a_capture_on_a_fresh_stream_records_the_products_alone(m, new_stream):
     """Its scratch is cleared once, not by a fill in front of every linear."""
     from cuda.bindings import runtime
     calls = [_call("w4", m, n, k) for n, k in ((4096, 4096), (4096, 2048), (5120, 4096))]
     want = [f().clone() for f in calls]
-    stream = _new_stream()
+    stream = new_stream()
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(graph, stream=stream):
         got = [f() for f in calls]

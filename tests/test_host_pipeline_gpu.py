@@ -1,5 +1,5 @@
 """``forward_host_many``: rows that come beside the first product and results that leave beside the later ones, for sets in
-which the first linear's kernel takes copies along and for ones in which it does not; new rows at every call."""
+which a linear's kernel takes copies along, wherever it is given, and for ones in which none does; new rows at every call."""
 import pytest
 import torch
 
@@ -9,7 +9,7 @@ from mindpipe_b200.modules import VllmPackedInt4Linear, forward_host_many
 pytestmark = pytest.mark.gpu
 
 SETS = {"carried": [(12288, 4096), (4096, 11008), (4096, 4096), (1024, 4096)],
-        "first kernel takes none": [(512, 2048), (22016, 4096), (4096, 11008)],
+        "the smallest result given first": [(512, 2048), (22016, 4096), (4096, 11008)],
         "one linear": [(22016, 4096)],
         "everything in one copy each way": [(2048, 2048), (1024, 2048)],
         "a later one goes first": [(1024, 2048), (22016, 4096), (512, 11008)],

@@ -77,12 +77,11 @@ def test_chained_launches_with_early_weights_share_scratch(n, k, m):
 
 @pytest.mark.parametrize("m,n,k", [(1, 4096, 4096), (8, 8192, 8192), (16, 1024, 8192), (16, 12288, 4096),
                                    (77, 4096, 4096), (100, 4096, 4096), (128, 8192, 2048)])
-def test_capture_on_a_stream_without_scratch(m, n, k):
+def test_capture_on_a_stream_without_scratch(m, n, k, new_stream):
     """A capture needs no call on its stream before; the graph has zeroed scratch of its own."""
     x, packed, sz, bias, _ = _case(n, k, m, 128)
     want = ops.w4a16_linear(x, packed, sz, bias)
-    stream = torch.cuda.Stream()                           # (kept: another stream might get its handle and find scratch)
-    stream.wait_stream(torch.cuda.current_stream())
+    stream = new_stream()
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph, stream=stream):
         got = [ops.w4a16_linear(x, packed, sz, bias) for _ in range(3)]
