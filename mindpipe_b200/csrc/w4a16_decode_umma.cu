@@ -81,7 +81,7 @@ struct Int { static constexpr int value = N; };
 
 // TOK: token rows of the MMA (its N); XROWS: token rows of the activation tile in shared memory (8 where no more exist:
 // the MMA then reads whatever follows for the other eight, whose results are not used)
-// CARRY: a warp more, for copies from host memory (up to 16 rows)
+// CARRY: a warp more, for copies from host memory
 template <int TOK, int XROWS, bool FOLD, bool CARRY>
 struct Cfg {
   // the columns of an expanded word come out as (k0,k4) (k1,k5) ..: the activations are put into that order, in shared
@@ -152,12 +152,14 @@ struct DecodeUmmaParams {
 
 // The list of copies is in the arguments, and the warp that copies in the block, of the launches that bring copies alone: in
 // all of them they cost four captured linears of a 7B layer at 16 rows 0.15 us (41.15 -> 41.00), a 70B layer at 8 rows 0.5
-// (106.4 -> 105.8), and the exact form up to 16 rows a spilled register.
+// (106.4 -> 105.8), and the exact form up to 16 rows a spilled register.  Beyond 16 rows nothing is carried, but the forms keep
+// list and warp: the compiler's code without them is slower (us: 1024x8192 at 48 rows 10.5 -> 10.8, 12288x4096 at 64 12.3 ->
+// 12.6, 8192x8192 at 96 16.8 -> 17.2).
 template <bool CARRY>
 struct DecodeUmmaArgs : DecodeUmmaParams {};
 template <>
 struct DecodeUmmaArgs<true> : DecodeUmmaParams {
-  HostCopies copies;       // from host memory, every block its share
+  HostCopies copies;       // from host memory, every block its share; count 0: none
 };
 
 // The stage range of block b is [range_start(b), range_start(b + 1)): p.share stages each, one more for the first p.extra.
@@ -599,8 +601,10 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
   } else if (warp == C::kSideWarp) {
     // ------------------------------------------------------------ copies: beside the product, which ends when they have ended
     if constexpr (CARRY) {
-      chain_wait();
-      copy_pieces(p.copies, blk * 32 + lane, static_cast<int>(gridDim.x) * 32, true);
+      if (p.copies.count > 0) {
+        chain_wait();
+        copy_pieces(p.copies, blk * 32 + lane, static_cast<int>(gridDim.x) * 32, true);
+      }
     }
   } else {
     // ------------------------------------------------------------ epilogue: lane = weight row, column = token
@@ -739,7 +743,7 @@ static int launch_umma(const CUtensorMap& tw, const CUtensorMap& tx, const CUten
   auto kern = w4a16_decode_umma_kernel<TOK, XROWS, FOLD, CARRY>;
   DecodeUmmaArgs<CARRY> p;
   static_cast<DecodeUmmaParams&>(p) = params;
-  if constexpr (CARRY) p.copies = *copies;
+  if constexpr (CARRY) p.copies = copies ? *copies : HostCopies{};
   static thread_local int configured_device = -1;
   int device = 0;
   MP_CUDA_TRY(cudaGetDevice(&device));
@@ -815,13 +819,13 @@ int launch_decode_umma(const void* x, const void* packed, const void* sz, const 
   if (M <= 8) return fold ? launch_umma<16, 8, true>(tw, tx, tsz, p, grid, st) : launch_umma<16, 8, false>(tw, tx, tsz, p, grid, st);
   if (tok == 16) return fold ? launch_umma<16, 16, true>(tw, tx, tsz, p, grid, st) : launch_umma<16, 16, false>(tw, tx, tsz, p, grid, st);
   switch (tok) {
-    case 32: return launch_umma<32, 32, false>(tw, tx, tsz, p, grid, st);
-    case 48: return launch_umma<48, 48, false>(tw, tx, tsz, p, grid, st);
-    case 64: return launch_umma<64, 64, false>(tw, tx, tsz, p, grid, st);
-    case 80: return launch_umma<80, 80, false>(tw, tx, tsz, p, grid, st);
-    case 96: return launch_umma<96, 96, false>(tw, tx, tsz, p, grid, st);
-    case 112: return launch_umma<112, 112, false>(tw, tx, tsz, p, grid, st);
-    default: return launch_umma<128, 128, false>(tw, tx, tsz, p, grid, st);
+    case 32: return launch_umma<32, 32, false, true>(tw, tx, tsz, p, grid, st);
+    case 48: return launch_umma<48, 48, false, true>(tw, tx, tsz, p, grid, st);
+    case 64: return launch_umma<64, 64, false, true>(tw, tx, tsz, p, grid, st);
+    case 80: return launch_umma<80, 80, false, true>(tw, tx, tsz, p, grid, st);
+    case 96: return launch_umma<96, 96, false, true>(tw, tx, tsz, p, grid, st);
+    case 112: return launch_umma<112, 112, false, true>(tw, tx, tsz, p, grid, st);
+    default: return launch_umma<128, 128, false, true>(tw, tx, tsz, p, grid, st);
   }
 }
 
