@@ -451,8 +451,9 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
     uint32_t phase = 0, xphase = 0, use = 0;
     // The tiles that this block will add on their way to L2, from which the weights of other linears push those of a graph that
     // is not replayed all the time (three graphs of a 7B layer at 16 rows in turn, us: without 41.7, here 41.0, by the side warp
-    // after the wait for the kernel before 41.1, from the loop below 43.0).  At 77 rows, where the tiles are six times as many
-    // bytes, it costs more than it gives (eager, 65.0 -> 67.2), so not beyond 16; and beside host copies too (65.7 -> 66.3).
+    // after the wait for the kernel before 41.1, from the loop below 43.0; not beside host copies, 65.7 -> 66.3).  With more rows
+    // the idle side warp does it, a line at a time (that layer at 35 / 64 rows 51.3 / 58.8 -> 50.9 / 57.2; here, eagerly, 77
+    // rows took 65.0 -> 67.2), up to 64: at 77 rows the tiles are there already in an eager call, 55.7 -> 56.1.
     if (PERM && closes && p.early_tiles) {
       const int first_block = block_of(rb_lo * ST, p);
       for (int b2 = first_block; b2 < blk; ++b2)
@@ -600,6 +601,12 @@ w4a16_decode_umma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
     }
   } else if (warp == C::kSideWarp) {
     // ------------------------------------------------------------ copies: beside the product, which ends when they have ended
+    if (TOK > 16 && TOK <= 64 && closes) {       // tiles to L2, as the expansion warps do up to 16 rows
+      const int first_block = block_of(rb_lo * ST, p);
+      for (int b2 = first_block; b2 < blk; ++b2)
+        for (int e = lane; e < p.M * (du::kRows / 32); e += 32)
+          prefetch_l2(p.tiles + (size_t)b2 * TOK * du::kRows + e * 32);
+    }
     if constexpr (CARRY) {
       if (p.copies.count > 0) {
         chain_wait();
