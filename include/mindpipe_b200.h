@@ -178,7 +178,7 @@ typedef struct mp_host_linear {
 int mp_w4a16_linear_decode_host_many(const mp_host_linear* linears, int count, mp_stream_t stream);
 /*
  * The same set recorded once for a stream and run many times: rows and results cross PCIe beside the products, the results
- * on one more stream (joined to `stream` again at the end of each run).  All of x_host_f16 / y_host_f16 must be page-locked,
+ * on one more stream (joined to `stream` again at the end of each run, of one that fails too).  All of x_host_f16 / y_host_f16 must be page-locked,
  * at most 16 entries (MP_ERR_UNSUPPORTED otherwise: use the call above).  The entries' buffers and the host memory outlive
  * the pipeline.  Destroying it while a run is still
  * on the device is allowed.

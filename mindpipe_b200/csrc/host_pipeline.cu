@@ -168,19 +168,16 @@ static int make_pipeline(HostPipeline& p, const mp_host_linear* linears, int cou
   if (p.beside) {
     for (cudaEvent_t* e : {&p.begun, &p.arrived}) MP_CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   }
+  if (p.has_side) MP_CUDA_TRY(cudaEventCreateWithFlags(&p.sent, cudaEventDisableTiming));
   if (!p.direct_out) {
-    MP_CUDA_TRY(cudaEventCreateWithFlags(&p.sent, cudaEventDisableTiming));
     for (int i = 0; i < count; ++i) MP_CUDA_TRY(cudaEventCreateWithFlags(&p.done[i], cudaEventDisableTiming));
   }
   return MP_OK;
 }
 
-static int run_pipeline(HostPipeline& p) {
+// `apart`: work of this run is on the side stream and the caller's does not wait for it yet.
+static int enqueue_run(HostPipeline& p, bool& apart) {
   const cudaStream_t st = p.stream;
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  MP_CUDA_TRY(cudaStreamIsCapturing(st, &capturing));
-  if (capturing != cudaStreamCaptureStatusNone) return mp_w4a16_linear_decode_host_many(p.linear, p.count, st);
-  std::lock_guard<std::mutex> lock(p.enqueue);
   int rc;
   if (p.beside) {
     MP_CUDA_TRY(cudaEventRecord(p.begun, st));               // the call before still reads its rows until here
@@ -197,19 +194,35 @@ static int run_pipeline(HostPipeline& p) {
     if (rc != MP_OK) return rc;
     if (others && !carried && (rc = launch_copy(p.others, true, st)) != MP_OK) return rc;    // (the kernel was switched since)
     if (i == 0 && p.beside) {
+      apart = true;
       if ((rc = launch_copy(p.others, true, p.out)) != MP_OK) return rc;
       MP_CUDA_TRY(cudaEventRecord(p.arrived, p.out));
       MP_CUDA_TRY(cudaStreamWaitEvent(st, p.arrived, 0));
+      apart = false;
     }
     if (!p.direct_out && i < p.count - 1) {
       MP_CUDA_TRY(cudaEventRecord(p.done[i], st));
       MP_CUDA_TRY(cudaStreamWaitEvent(p.out, p.done[i], 0));
+      apart = true;
       MP_CUDA_TRY(cudaMemcpyAsync(c.y_host_f16, c.y_stage_f16, result_bytes(c), cudaMemcpyDeviceToHost, p.out));
     }
   }
-  if ((rc = launch_copy(p.back, false, st)) != MP_OK || p.direct_out) return rc;
-  MP_CUDA_TRY(cudaEventRecord(p.sent, p.out));
-  MP_CUDA_TRY(cudaStreamWaitEvent(st, p.sent, 0));
+  return launch_copy(p.back, false, st);
+}
+
+static int run_pipeline(HostPipeline& p) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  MP_CUDA_TRY(cudaStreamIsCapturing(p.stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) return mp_w4a16_linear_decode_host_many(p.linear, p.count, p.stream);
+  std::lock_guard<std::mutex> lock(p.enqueue);
+  bool apart = false;
+  const int rc = enqueue_run(p, apart);
+  if (!apart) return rc;
+  // also after an error: a caller who then waits for the stream may write its buffers again
+  const cudaError_t recorded = cudaEventRecord(p.sent, p.out);
+  const cudaError_t joined = recorded == cudaSuccess ? cudaStreamWaitEvent(p.stream, p.sent, 0) : recorded;
+  if (rc != MP_OK) return rc;
+  MP_CUDA_TRY(joined);
   return MP_OK;
 }
 

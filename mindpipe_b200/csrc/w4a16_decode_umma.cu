@@ -29,13 +29,16 @@
 // order (results are identical from run to run).  A tile word is stored inverted and zero means "not there yet": the
 // reader polls the words themselves (bounded) and puts the zeros back, with no fence, counter or second round trip.
 //
-//   warps 0-15   expansion: two sets of eight take stages in turn, a warp does 32 rows of half a stage (see Cfg::kParts); at
-//                the end they fetch the tiles of the row block that this block closes
-//   warps 16-19  epilogue
-//   warp 20      TMA producer of weights and (scale, zero) pairs
-//   warp 21      TMEM allocation and the MMA issuer
-//   warp 22      TMA producer of activations
-//   warp 23      copies from host memory, in a launch that brings some
+// Warps, by role and in this order (Cfg has the numbers):
+//   16 (or 12)   expansion: two sets of eight take stages in turn, a warp does 32 rows of half a stage; three sets of four and
+//                whole stages for the exact form up to 16 rows (see Cfg::kParts).  At the end they fetch the tiles of the row
+//                block that this block closes
+//   4            epilogue
+//   1            TMA producer of weights and (scale, zero) pairs
+//   1            TMEM allocation and the MMA issuer
+//   1            TMA producer of activations
+//   1            side warp: copies from host memory, in a launch that brings some; tiles to L2 from 17 to 64 rows.  Up to 16
+//                rows only a launch that brings copies has it
 // Expansion emits the columns of a packed word in the order (k0,k4,k1,k5,k2,k6,k3,k7).  Up to 16 rows the expansion warps
 // apply the same permutation in place to the 16-byte chunks of the stage's activation tile (a chunk is one token's eight
 // columns of one word, so the swizzle does not matter); with more rows they put the words back in order, see Cfg.  (Warps

@@ -15,8 +15,9 @@ names, but hold integer weights and run the sm_100a kernels:
   ``u - z`` and apply the scale to a group's sum in fp32: the product of the
   weights before their rounding to fp16, which differs from the reference's by
   that rounding alone, about 3e-4 relative.  So a token's bits may differ between a batch of up to 16 and one of
-  more rows (and, on weights below 4 MiB packed with fewer than 2048 output rows or
-  below 2 MiB, between 8 and 9), as they may with any change of the order of summation.
+  more rows, as they may with any change of the order of summation: on weights below 5 MiB packed (4 MiB from 4096
+  output rows on) also between 8 and 9 rows, and above 96, 112 or 128 rows, by shape, with the number of rows
+  (``linear_kernel`` in ``csrc/w4a16_decode.cu`` has the lines).
 """
 from __future__ import annotations
 

@@ -3,8 +3,8 @@ which a linear's kernel takes copies along, wherever it is given, and for ones i
 import pytest
 import torch
 
-from mindpipe_b200 import ops
-from mindpipe_b200.modules import VllmPackedInt4Linear, forward_host_many
+from mindpipe_b200 import _lib, ops
+from mindpipe_b200.modules import VllmPackedInt4Linear, _HostPipeline, forward_host_many
 
 pytestmark = pytest.mark.gpu
 
@@ -45,4 +45,41 @@ def test_results_are_those_of_the_single_forwards(shapes, rows):
             stream.synchronize()
             for y, v in zip(ys, w):
                 assert torch.equal(y, v)
+    ops.check_device_errors()
+
+
+def test_the_stream_waits_for_the_side_stream_after_an_error():
+    """The second product is refused (a group that does not divide K) when the first one's result is on its way: whoever
+    waits for the stream then may use the buffers again."""
+    rows, bad, shapes = 16, 1, [(262144, 256), (4096, 4096), (1024, 4096)]
+    g = torch.Generator(device="cuda").manual_seed(0)
+    stream = torch.cuda.Stream()
+    calls, keep = (_lib.HostLinear * len(shapes))(), []
+    for c, (n, k) in zip(calls, shapes):
+        lin = torch.nn.Linear(k, n, bias=False, device="meta", dtype=torch.float16)
+        lin.weight = torch.nn.Parameter((torch.randn(n, k, generator=g, device="cuda") * 0.02).half(), requires_grad=False)
+        mod = VllmPackedInt4Linear.from_float(lin, group_size=128)
+        mod.process_weights_after_loading()
+        x = torch.randn(rows, k, generator=g, device="cuda").half()
+        x_host, y_host = x.cpu().pin_memory(), torch.full((rows, n), float("nan"), dtype=torch.float16).pin_memory()
+        xs, ys = torch.empty_like(x), torch.empty((rows, n), dtype=torch.float16, device="cuda")
+        ws = ops.new_workspace(16 << 20, "cuda")
+        keep.append((mod, x, x_host, y_host, xs, ys, ws))
+        c.x_host_f16, c.x_stage_f16, c.y_stage_f16, c.y_host_f16 = (t.data_ptr() for t in (x_host, xs, ys, y_host))
+        c.packed_i32, c.sz_f16x2, c.bias_f16 = mod.weight_packed.data_ptr(), mod._scale_zero.data_ptr(), None
+        c.M, c.N, c.K, c.group = rows, n, k, 128
+        c.workspace, c.workspace_bytes = ws.data_ptr(), ws.numel()
+    calls[bad].group = 96
+    mod, x, _, y_host, *_ = keep[0]
+    want = mod(x).cpu()
+    pipeline = _HostPipeline(calls, len(shapes), stream.cuda_stream)
+    assert pipeline.status == 0
+    for _ in range(4):
+        y_host.fill_(float("nan"))
+        torch.cuda.synchronize()
+        assert pipeline.run() != 0
+        stream.synchronize()
+        last = float(y_host[-1, -1])                        # the copy's end, before a look at the rest gives it time
+        assert last == float(want[-1, -1]) and torch.equal(y_host, want)
+    torch.cuda.synchronize()
     ops.check_device_errors()
