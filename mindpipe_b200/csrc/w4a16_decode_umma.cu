@@ -771,6 +771,40 @@ static int launch_umma(const CUtensorMap& tw, const CUtensorMap& tx, const CUten
   return launch_chained(kern, dim3(grid), dim3(C::kThreads), fixed + (size_t)p.ring * stage, st, tw, tx, tsz, p);
 }
 
+// The tensor maps of weights and (scale, zero) pairs.  A map is made of an address and sizes and of nothing in memory, and a
+// program calls with the same weights again and again, so those made last are kept, per thread, in the place that the weights'
+// address gives.  Encoding all three in every call took what the stream kernel gains on a shape that the host bounds (one
+// 4096x4096 linear at one row, eager, us: the ring kernel, which keeps its maps, 6.05, this 6.25; kept 5.64 where that took
+// 5.84).  The activations' map is made in every call: their address is another one more often than not.
+static int weight_maps(const void* packed, const void* sz, int N, int K, int group, int gps, const CUtensorMap** tw,
+                       const CUtensorMap** tsz) {
+  struct Entry {
+    CUtensorMap tw, tsz;
+    const void *packed, *sz;
+    int N, K, group;
+  };
+  constexpr int kLog2Entries = 7;
+  static thread_local Entry entries[1 << kLog2Entries];
+  Entry& e = entries[(reinterpret_cast<uintptr_t>(packed) >> 4) * 0x9E3779B97F4A7C15ull >> (64 - kLog2Entries)];
+  if (e.packed != packed || e.sz != sz || e.N != N || e.K != K || e.group != group) {
+    e.packed = nullptr;
+    int rc = encode_tensor_map_2d(&e.tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, packed, (uint64_t)K / 2, (uint64_t)N,
+                                  (uint64_t)K / 2, 128, du::kRows, true);
+    if (rc != MP_OK) return rc;
+    rc = encode_tensor_map_2d(&e.tsz, CU_TENSOR_MAP_DATA_TYPE_UINT32, sz, (uint64_t)N, (uint64_t)(K / group),
+                              (uint64_t)N * 4, du::kRows, gps, false);
+    if (rc != MP_OK) return rc;
+    e.packed = packed;
+    e.sz = sz;
+    e.N = N;
+    e.K = K;
+    e.group = group;
+  }
+  *tw = &e.tw;
+  *tsz = &e.tsz;
+  return MP_OK;
+}
+
 // Returns MP_ERR_UNSUPPORTED for shapes this kernel does not take (M > 128, K % 64 != 0, N % 4 != 0, groups
 // other than 32, 64, 128, 256 or a multiple of 256) and when the workspace is missing or too small; the
 // caller then uses another kernel.  The workspace starts zeroed and is left ready for the next call;
@@ -783,18 +817,16 @@ int launch_decode_umma(const void* x, const void* packed, const void* sz, const 
   if (!workspace || workspace_bytes < du::workspace_bytes(M) || !aligned(workspace, 16)) return MP_ERR_UNSUPPORTED;
   if (!aligned(x, 16) || !aligned(packed, 16) || !aligned(sz, 16) || !aligned(y, 4)) return MP_ERR_UNSUPPORTED;
   const int row_blocks = (N + du::kRows - 1) / du::kRows;
-  CUtensorMap tw, tx, tsz;
-  int rc = encode_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, packed, (uint64_t)K / 2, (uint64_t)N,
-                                (uint64_t)K / 2, 128, du::kRows, true);
+  const int gps = group < du::kStageK ? du::kStageK / group : 1;
+  const CUtensorMap *tw_at = nullptr, *tsz_at = nullptr;
+  int rc = weight_maps(packed, sz, N, K, group, gps, &tw_at, &tsz_at);
   if (rc != MP_OK) return rc;
+  const CUtensorMap &tw = *tw_at, &tsz = *tsz_at;
   // [64 columns][token][chunk of 64 columns]: one copy brings the sub-tiles of a stage or half of one
+  CUtensorMap tx;
   const uint64_t x_dims[3] = {64, (uint64_t)M, (uint64_t)K / 64}, x_strides[2] = {(uint64_t)K * 2, 128};
   const uint32_t x_box[3] = {64, (uint32_t)(M <= 8 ? 8 : tok), tok <= 16 ? 4u : 2u};
   rc = encode_tensor_map_3d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, x_dims, x_strides, x_box);
-  if (rc != MP_OK) return rc;
-  const int gps = group < du::kStageK ? du::kStageK / group : 1;
-  rc = encode_tensor_map_2d(&tsz, CU_TENSOR_MAP_DATA_TYPE_UINT32, sz, (uint64_t)N, (uint64_t)(K / group),
-                            (uint64_t)N * 4, du::kRows, gps, false);
   if (rc != MP_OK) return rc;
   DecodeUmmaParams p{};
   p.bias = static_cast<const __half*>(bias);

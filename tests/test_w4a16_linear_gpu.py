@@ -90,3 +90,25 @@ def test_capture_on_a_stream_without_scratch(m, n, k, new_stream):
     torch.cuda.synchronize()
     ops.check_device_errors()
     assert all(torch.equal(y, want) for y in got)
+
+
+def test_weights_that_share_memory_and_more_of_them_than_maps_are_kept():
+    """Weights of other shapes and groups at the same addresses, and 160 of them in turn, again and again."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    codes = torch.randint(-2**31, 2**31 - 1, (4096 * 4096 // 8,), generator=g, dtype=torch.int32, device="cuda")
+    pairs = (torch.rand(4096 * 4096 // 64 * 2, generator=g, device="cuda") * 0.01).half()
+    forms = []
+    for n, k, group in ((4096, 4096, 128), (2048, 8192, 128), (8192, 2048, 64), (4096, 4096, 64), (4096, 2048, 128)):
+        packed = codes[:n * k // 8].view(n, k // 8)
+        sz = pairs[:k // group * n * 2].view(k // group, n, 2)
+        x = torch.randn(5, k, generator=g, device="cuda").half()
+        forms.append((x, packed, sz, ops.w4a16_linear(x, packed.clone(), sz.clone())))
+    many = []
+    for i in range(160):
+        packed, sz = codes[i * 4096:][:2048 * 2048 // 8].view(2048, 256), pairs[i * 64:][:16 * 2048 * 2].view(16, 2048, 2)
+        x = torch.randn(9, 2048, generator=g, device="cuda").half()
+        many.append((x, packed, sz, ops.w4a16_linear(x, packed.clone(), sz.clone())))
+    for _ in range(2):
+        for x, packed, sz, want in forms + many:
+            assert torch.equal(ops.w4a16_linear(x, packed, sz), want)
+    ops.check_device_errors()
