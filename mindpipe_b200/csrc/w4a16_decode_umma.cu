@@ -775,7 +775,7 @@ static int launch_umma(const CUtensorMap& tw, const CUtensorMap& tx, const CUten
 // program calls with the same weights again and again, so those made last are kept, per thread, in the place that the weights'
 // address gives.  Encoding all three in every call took what the stream kernel gains on a shape that the host bounds (one
 // 4096x4096 linear at one row, eager, us: the ring kernel, which keeps its maps, 6.05, this 6.25; kept 5.64 where that took
-// 5.84).  The activations' map is made in every call: their address is another one more often than not.
+// 5.84, and 6.14 where the ring kernel takes 6.14).  The activations' map is made in every call: their address is another one more often than not.
 static int weight_maps(const void* packed, const void* sz, int N, int K, int group, int gps, const CUtensorMap** tw,
                        const CUtensorMap** tsz) {
   struct Entry {
